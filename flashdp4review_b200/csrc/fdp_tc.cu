@@ -30,23 +30,30 @@ constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KiB
 constexpr int B_STAGE_BYTES = BN * BK * 2;  // 32 KiB
 constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
 constexpr int BAR_BYTES = 256;
-// EPI_STORE_SCALED keeps the clip factors of up to MAX_SMEM_FACTORS samples in shared memory
-constexpr int MAX_SMEM_FACTORS = 4096;
+constexpr int BOX_ROWS = 32, BOX_BYTES = BOX_ROWS * 128;   // an epilogue warp's output box: 32 rows of 128 bytes
+// EPI_STORE_SCALED keeps the clip factors of up to MAX_SMEM_FACTORS samples in shared memory (what the
+// ring and the output boxes leave of the 227 KB); larger batches read them from global memory
+constexpr int MAX_SMEM_FACTORS = 384;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + BAR_BYTES;
-constexpr int SMEM_BYTES_SCALED = SMEM_BYTES + MAX_SMEM_FACTORS * 4;
+constexpr int SMEM_BYTES_STORE = SMEM_BYTES + 8 * BOX_BYTES;
+constexpr int SMEM_BYTES_SCALED = SMEM_BYTES_STORE + MAX_SMEM_FACTORS * 4;
+static_assert(SMEM_BYTES_SCALED <= 227 * 1024, "shared memory of one CTA");
 constexpr int TMEM_COLS = 512;
 constexpr int MAX_SMS = 148;           // workers the split-K parking area is sized for
 
 // EPI_STORE_SCALED: the accumulator of each sample (K segment) is drained on its own and added, times
 // that sample's clip factor, to fp32 registers of eight epilogue warps; G needs no scaled copy.
-enum { EPI_STORE = 0, EPI_SUMSQ = 1, EPI_GRAM = 2, EPI_STORE_SCALED = 3 };
+// EPI_CHAIN / EPI_CHAIN_SUMSQ: the same with a constant factor for fp32 products in short chains; the first
+// stores the tile (+ bias), the second sums the squares of one sample's tile.
+enum { EPI_STORE = 0, EPI_SUMSQ = 1, EPI_GRAM = 2, EPI_STORE_SCALED = 3, EPI_CHAIN = 4, EPI_CHAIN_SUMSQ = 5 };
+__host__ __device__ constexpr bool epi_chained(int epi) { return epi >= EPI_STORE_SCALED; }
+__host__ __device__ constexpr bool epi_stores(int epi) { return epi == EPI_STORE || epi == EPI_STORE_SCALED || epi == EPI_CHAIN; }
 // eight epilogue warps (two per TMEM lane quarter, 128 columns each) for the store epilogues, four for the norms
-#ifndef FDP_EPI_STORE_WARPS
-#define FDP_EPI_STORE_WARPS 8
-#endif
-__host__ __device__ constexpr int epi_warps_for(int epi) { return epi == EPI_STORE_SCALED ? 8 : (epi == EPI_STORE ? FDP_EPI_STORE_WARPS : 4); }
+__host__ __device__ constexpr int epi_warps_for(int epi) { return (epi == EPI_STORE || epi_chained(epi)) ? 8 : 4; }
 constexpr int threads_for(int epi) { return 64 + 32 * epi_warps_for(epi); }
-constexpr int smem_for(int epi) { return epi == EPI_STORE_SCALED ? SMEM_BYTES_SCALED : SMEM_BYTES; }
+constexpr int smem_for(int epi) {
+  return epi == EPI_STORE_SCALED ? SMEM_BYTES_SCALED : epi_stores(epi) ? SMEM_BYTES_STORE : SMEM_BYTES;
+}
 
 struct TcArgs {
   int M, N;             // extents of the output space of one batch (masks)
@@ -62,9 +69,7 @@ struct TcArgs {
   int* status;          // status word of the call (workspace)
   int zero_status;      // this launch is the first of its call: its first thread clears the status word
   int dependent;        // host side: launch as a programmatic dependent of the kernel before it in the stream
-  int sub_stages;       // EPI_STORE_SCALED: K stages per accumulator hand-off (<= seg_stages; chains of fp32 tensor mode)
-  int norm_mode;        // EPI_STORE_SCALED: 1 = no store, sum of squares of the unit's accumulated tile -> partials;
-                        // 2 = plain product (factor = scale for every segment), stored as usual
+  int sub_stages;       // chained epilogues: K stages per accumulator hand-off (<= seg_stages; chains of fp32 tensor mode)
   int* sticky;          // this device's slot of the host-visible status array, or null
   uint32_t idesc;
   // split-K (store epilogues): work units [0, units_full) are whole tiles; each later tile is cut into
@@ -92,7 +97,7 @@ struct TcArgs {
   int gram_nb;          // 128-row blocks per sample
   uint32_t idesc_half;
   // store epilogue: optional bias[N] (same 16-bit type as the operands) added to every row
-  const void* bias; int bias_dt;
+  const void* bias; int bias_dt; int bias_vec;   // bias_vec: 16-byte aligned
   // fp32 inputs as three bf16 products.  Both operand matrices are then [rows, 2n]: the high bf16
   // halves of the n columns, then the low halves (x = hi + lo up to 2^-18 |x|).  With terms = 3 the K
   // loop visits every K range three times -- hi*hi, hi*lo, lo*hi -- into the same accumulator (lo*lo,
@@ -204,47 +209,88 @@ __device__ __forceinline__ void add_noise32(const NoiseKey& nk, size_t idx0, flo
   }
 }
 
-// Finish 32 adjacent output columns of row m starting at column n: bias, noise (NOISE), convert, store.
-template <bool NOISE>
-__device__ __forceinline__ void store_chunk32(const TcArgs& args, float v[32], int m, int n) {
-  if (m >= args.M || n >= args.N) return;
-  const size_t idx0 = static_cast<size_t>(m) * args.ld_out + n;
-  if (args.bias != nullptr) {
+// v[0..31] += bias[n .. n+31]; the same address in every lane.  16-byte loads: the columns are few, the
+// loads many (one set per 32 accumulator columns and warp), and as 32 scalar loads with a type switch
+// each they took half of the forward GEMM's time at K = 1024.
+__device__ __forceinline__ void add_bias32(const TcArgs& args, int n, float v[32]) {
+  if (args.bias_vec && n + 32 <= args.N) {
+    if (args.bias_dt == FDP_F32) {
+      const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(args.bias) + n);
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (n + j < args.N) v[j] += load_as(args.bias, args.bias_dt, n + j);
-  }
-  if (NOISE && args.nk.std != 0.f) add_noise32(args.nk, idx0, v);
-  const bool vec_ok = (args.ld_out * static_cast<long long>(dtype_size(args.out_dt))) % 16 == 0;
-  if (n + 32 <= args.N && vec_ok) {
-    if (args.out_dt == FDP_F32) {
-      float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(args.out) + idx0);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+      for (int j = 0; j < 8; ++j) {
+        const float4 b = __ldg(p + j);
+        v[4 * j] += b.x; v[4 * j + 1] += b.y; v[4 * j + 2] += b.z; v[4 * j + 3] += b.w;
+      }
     } else {
-      uint4* o = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(args.out) + idx0);
+      const uint4* p = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(args.bias) + n);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        uint32_t w[4];
+        const uint4 raw = __ldg(p + j);
+        float b[8];
+        if (args.bias_dt == FDP_BF16) unpack16<__nv_bfloat16>(raw, b); else unpack16<__half>(raw, b);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float lo = v[8 * j + 2 * e], hi = v[8 * j + 2 * e + 1];
-          if (args.out_dt == FDP_BF16) {
-            __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-            w[e] = *reinterpret_cast<uint32_t*>(&h);
-          } else {
-            __half2 h = __floats2half2_rn(lo, hi);
-            w[e] = *reinterpret_cast<uint32_t*>(&h);
-          }
-        }
-        o[j] = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int e = 0; e < 8; ++e) v[8 * j + e] += b[e];
       }
     }
   } else {
 #pragma unroll
     for (int j = 0; j < 32; ++j)
-      if (n + j < args.N) store_as(args.out, args.out_dt, idx0 + j, v[j]);
+      if (n + j < args.N) v[j] += load_as(args.bias, args.bias_dt, n + j);
   }
+}
+
+// ---- output boxes ------------------------------------------------------------------------------------
+// After tcgen05.ld a lane holds one row of the tile, so direct stores put the 32 lanes of an instruction
+// on 32 different rows: half-used sectors, 32 lines per request (16384 rows, 1024 -> 3072, bf16 forward with
+// bias: 171 us, tensor pipe 27 % busy; 86 us with the boxes and add_bias32).  Instead every epilogue warp writes boxes of 32 rows x 128 bytes into its own
+// 4 KB of shared memory, in the 128-byte swizzle of the tensor map (16-byte chunk j of row r at slot
+// j ^ (r & 7): no bank conflicts), and one lane hands each box to the copy engine, which also clips what
+// lies past the matrix.
+__device__ __forceinline__ void box_wait(int lane) {      // the previous box has been read out
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+  __syncwarp();
+}
+__device__ __forceinline__ void box_put(uint32_t box, int lane, int j, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+               ::"r"(box + lane * 128 + ((j ^ (lane & 7)) << 4)), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void box_send(uint32_t box, const CUtensorMap* map, int col, int row, int lane) {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  if (lane == 0) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(col), "r"(row), "r"(box) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  }
+}
+__device__ __forceinline__ void box_drain(int lane) {     // before the CTA leaves
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+// 32 fp32 values per lane = one box
+__device__ __forceinline__ void store_f32x32(uint32_t box, const CUtensorMap* map, const float v[32], int col, int row, int lane) {
+  box_wait(lane);
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    box_put(box, lane, j, __float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]), __float_as_uint(v[4 * j + 2]),
+            __float_as_uint(v[4 * j + 3]));
+  box_send(box, map, col, row, lane);
+}
+// chunk c4 (32 columns) of a warp's 128 columns, in the output type; 16-bit types fill a box with two chunks
+__device__ __forceinline__ void store_out32(const TcArgs& args, uint32_t box, const CUtensorMap* map, const float v[32], int c4,
+                                            int col0, int row, int lane) {
+  if (args.out_dt == FDP_F32) {
+    if (col0 + 32 * c4 < args.N) store_f32x32(box, map, v, col0 + 32 * c4, row, lane);
+    return;
+  }
+  if (col0 + 64 * (c4 >> 1) >= args.N) return;
+  if ((c4 & 1) == 0) box_wait(lane);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint4 w;
+    if (args.out_dt == FDP_BF16) w = pack16<__nv_bfloat16>(v + 8 * j); else w = pack16<__half>(v + 8 * j);
+    box_put(box, lane, 4 * (c4 & 1) + j, w.x, w.y, w.z, w.w);
+  }
+  if ((c4 & 1) == 1) box_send(box, map, col0 + 64 * (c4 >> 1), row, lane);
 }
 
 // accr[4g .. 4g+3] += z * f with g known only at run time: a switch keeps every index static, so
@@ -272,22 +318,24 @@ template <bool A_MN, bool B_MN, int EPI, int CTAS>
 __global__ void __launch_bounds__(threads_for(EPI), 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB2,
-               const __grid_constant__ TcArgs args) {
+               const __grid_constant__ CUtensorMap tmOut, const __grid_constant__ TcArgs args) {
   constexpr int NST = (CTAS == 2) ? 6 : STAGES;          // ring depth
   constexpr int B_BYTES = B_STAGE_BYTES / CTAS;          // this CTA's share of the B stage
   constexpr int STG = A_STAGE_BYTES + B_BYTES;
   constexpr int BN_CTA = BN / CTAS;                      // B columns (rows if K-major) loaded by this CTA
   constexpr int EPI_WARPS = epi_warps_for(EPI);
   static_assert(NST * STG <= STAGES * STAGE_BYTES, "ring size");
-  static_assert(CTAS == 1 || EPI == EPI_STORE || EPI == EPI_STORE_SCALED, "pairs: store epilogues only");
+  static_assert(CTAS == 1 || EPI == EPI_STORE || epi_chained(EPI), "pairs: store and chained epilogues only");
   const uint32_t cta_rank = (CTAS == 2) ? cluster_ctarank() : 0u;
   const bool is_leader = cta_rank == 0;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   uint8_t* gen_base = smem_raw + (base - raw_addr);
-  const uint32_t bar_base = base + NST * STG;
-  uint8_t* bar_gen = gen_base + NST * STG;
+  // ring | output boxes of the epilogue warps (store epilogues) | barriers | clip factors
+  constexpr int BOXES = epi_stores(EPI) ? EPI_WARPS * BOX_BYTES : 0;
+  const uint32_t bar_base = base + NST * STG + BOXES;
+  uint8_t* bar_gen = gen_base + NST * STG + BOXES;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (NST + s); };
   auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * NST + a); };
@@ -496,7 +544,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // one accumulator per segment: the whole unit, or one sample's share of it for EPI_STORE_SCALED
         while (ks < ks1 && ok) {
           const int seg_begin = ks;
-          const int seg_end = (EPI == EPI_STORE_SCALED) ? segment_end(ks, ks1) : ks1;
+          const int seg_end = epi_chained(EPI) ? segment_end(ks, ks1) : ks1;
           const int acc = it % NUM_ACC;
           const uint32_t acc_phase = (it / NUM_ACC) & 1u;
           if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, wctx, 2)) { ok = false; break; }
@@ -557,6 +605,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;
     const int ew = warp - 2;
+    const uint32_t box = base + NST * STG + ew * BOX_BYTES;
     int it = 0;
     bool ok = true;
     if (EPI == EPI_STORE_SCALED && args.norm_partials != nullptr) {
@@ -584,7 +633,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       decode_unit(u, tile, ks0, ks1, slot);
       decode(tile, b, m0, n0, half);
       const int m = m0 + row;
-      if (EPI == EPI_STORE_SCALED) {
+      if constexpr (epi_chained(EPI)) {
         // eight warps: two per lane quarter, each owning 128 of the tile's 256 columns in registers
         const int chalf = ew >> 2;
         float accr[128];
@@ -593,7 +642,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // A whole tile's Gaussian noise goes into the accumulators a few element groups per sample
         // segment, in the time these warps would otherwise wait for the next segment's MMAs; K-split
         // parts stay noise-free (the fix-up kernel adds the noise once per tile).
-        const bool pre_noise = slot < 0 && args.nk.std != 0.f && m < args.M;
+        const bool pre_noise = EPI == EPI_STORE_SCALED && slot < 0 && args.nk.std != 0.f && m < args.M;
         const uint64_t g0 = (static_cast<uint64_t>(m) * args.ld_out + n0 + chalf * 128) >> 2;
         const int nseg = (ks1 - 1) / args.sub_stages - ks0 / args.sub_stages + 1;
         int ng = 0, seg = 0;
@@ -604,7 +653,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           tc_fence_after();
           const int sample = ks / args.seg_stages;
           // the divisor goes into the factor, so the noise is added as it is drawn
-          const float cbs = args.norm_mode == 1 ? 1.0f : args.norm_mode == 2 ? args.scale
+          const float cbs = EPI != EPI_STORE_SCALED ? args.scale
                           : (args.norm_partials != nullptr ? sfac[sample] : __ldg(args.factors + sample)) * args.scale;
           const uint32_t tb = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN + chalf * 128;
 #pragma unroll
@@ -622,7 +671,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             else mbar_arrive_cluster(mapa_u32(tempty_bar(acc), 0));
           }
           ++seg;
-          if (pre_noise) {
+          if (EPI == EPI_STORE_SCALED && pre_noise) {
             const int target = (32 * seg) / nseg;
             for (; ng < target; ++ng) {
               float z[4];
@@ -632,7 +681,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
         }
         if (!ok) break;
-        if (args.norm_mode == 1) {
+        if constexpr (EPI == EPI_CHAIN_SUMSQ) {
           // the unit is one sample's product tile: its squares, without the rows and columns past the
           // matrix (with split operands a tile that overhangs reads the other half's columns, not zeros)
           float part = 0.f;
@@ -643,22 +692,20 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
           part = warp_sum(part);
           if (lane == 0) args.partials[(static_cast<size_t>(tile) * CTAS + cta_rank) * EPI_WARPS + ew] = part;
-          continue;
-        }
-        if (slot < 0) {
+        } else if (slot < 0) {
+          if (m0 + quarter * 32 < args.M) {
 #pragma unroll
-          for (int c4 = 0; c4 < 4; ++c4) {
-            float v[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = accr[c4 * 32 + j];
-            store_chunk32<false>(args, v, m, n0 + chalf * 128 + c4 * 32);
+            for (int c4 = 0; c4 < 4; ++c4) {
+              const int n = n0 + chalf * 128 + c4 * 32;
+              if (EPI == EPI_CHAIN && args.bias != nullptr && n < args.N) add_bias32(args, n, accr + c4 * 32);
+              store_out32(args, box, &tmOut, accr + c4 * 32, c4, n0 + chalf * 128, m0 + quarter * 32, lane);
+            }
           }
         } else {
           // park this part (already divided by the batch) for the fix-up kernel
-          float4* dst = reinterpret_cast<float4*>(args.split_ws + ((static_cast<size_t>(slot) * CTAS + cta_rank) * BM + row) * BN + chalf * 128);
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            dst[j] = make_float4(accr[4 * j], accr[4 * j + 1], accr[4 * j + 2], accr[4 * j + 3]);
+          for (int c4 = 0; c4 < 4; ++c4)
+            store_f32x32(box, &tmA2, accr + c4 * 32, chalf * 128 + c4 * 32, (slot * CTAS + cta_rank) * BM + quarter * 32, lane);
         }
         continue;
       }
@@ -668,32 +715,38 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       tc_fence_after();
       const uint32_t tbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + (EPI == EPI_GRAM ? 0 : acc * BN);
       float part = 0.f;
-      constexpr int C_SPAN = BN * 4 / EPI_WARPS;     // store epilogue: this warp's share of the tile's columns
-      const int c_begin = (ew >> 2) * C_SPAN;
-      if (EPI == EPI_STORE && slot >= 0) {
-        // K-split unit: park the raw accumulator for the fix-up kernel
-        float4* dst = reinterpret_cast<float4*>(args.split_ws + ((static_cast<size_t>(slot) * CTAS + cta_rank) * BM + row) * BN);
-#pragma unroll 1
-        for (int c = c_begin; c < c_begin + C_SPAN; c += 32) {
-          uint32_t r[32];
-          tc_ld32(tbase + c, r);
-          tc_wait_ld();
+      if (EPI == EPI_STORE) {
+        // this warp's 128 columns into registers, then the accumulator goes back to the MMA warp at once
+        const int col0 = (ew >> 2) * 128;
+        float v[128];
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            dst[c / 4 + j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
-                                         __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+        for (int c4 = 0; c4 < 4; ++c4) tc_ld32(tbase + col0 + c4 * 32, reinterpret_cast<uint32_t*>(v) + c4 * 32);
+        tc_wait_ld();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (CTAS == 1 || is_leader) mbar_arrive(tempty_bar(acc));
+          else mbar_arrive_cluster(mapa_u32(tempty_bar(acc), 0));
         }
-      } else if (EPI == EPI_STORE) {
-#pragma unroll 1
-        for (int c = c_begin; c < c_begin + C_SPAN; c += 32) {
-          uint32_t r[32];
-          tc_ld32(tbase + c, r);
-          tc_wait_ld();
-          float v[32];
+        ++it;
+        if (slot >= 0) {   // K-split unit: park the raw accumulator for the fix-up kernel
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * args.scale;
-          store_chunk32<true>(args, v, m, n0 + c);
+          for (int c4 = 0; c4 < 4; ++c4)
+            store_f32x32(box, &tmA2, v + c4 * 32, col0 + c4 * 32, (slot * CTAS + cta_rank) * BM + quarter * 32, lane);
+        } else if (m0 + quarter * 32 < args.M) {
+#pragma unroll
+          for (int c4 = 0; c4 < 4; ++c4) {
+            const int n = n0 + col0 + c4 * 32;
+            float* w = v + c4 * 32;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) w[j] *= args.scale;
+            if (args.bias != nullptr && n < args.N) add_bias32(args, n, w);
+            if (args.nk.std != 0.f && m < args.M && n < args.N)
+              add_noise32(args.nk, static_cast<size_t>(m) * args.ld_out + n, w);
+            store_out32(args, box, &tmOut, w, c4, n0 + col0, m0 + quarter * 32, lane);
+          }
         }
+        continue;
       } else if (EPI == EPI_SUMSQ) {
         // rows / columns outside the matrix were zero-filled by TMA, so they add nothing
 #pragma unroll 1
@@ -745,6 +798,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   }
 
   // ================= teardown =================
+  if (epi_stores(EPI) && warp >= 2) box_drain(lane);
   __syncwarp();
   tc_fence_before();
   __syncthreads();
@@ -875,6 +929,22 @@ bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, ui
   return r == CUDA_SUCCESS;
 }
 
+// Map of an output matrix [rows, cols] for the epilogue warps' boxes of 32 rows x 128 bytes.  The row pitch
+// has to be a multiple of 16 bytes and the base 16-byte aligned.
+bool make_out_map(CUtensorMap* m, void* base, uint64_t rows, uint64_t cols, int dt) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return false;
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {cols * dtype_size(dt)};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(128 / dtype_size(dt)), BOX_ROWS};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult r = fn(m, dt == FDP_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : dt == FDP_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                                                              : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+                        2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS;
+}
+
 uint32_t make_idesc(int dt, bool a_mn, bool b_mn, int ctas = 1, int n = BN) {
   uint32_t d = 0;
   d |= 1u << 4;                                   // accumulator format: F32
@@ -917,7 +987,7 @@ int launch_sms() {
 
 template <bool A_MN, bool B_MN, int EPI, int CTAS = 1>
 int launch(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& a2, const CUtensorMap& b2,
-           const TcArgs& args, cudaStream_t s) {
+           const CUtensorMap& out, const TcArgs& args, cudaStream_t s) {
   static std::mutex mu;
   static bool done[64];
   constexpr int SMEM = smem_for(EPI);
@@ -931,7 +1001,7 @@ int launch(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& a2, co
   const int grid = CTAS * (units < workers ? units : workers);
   const bool dependent = la.dependent != 0 && pdl_enabled();
   if (CTAS == 1 && !dependent) {
-    tc_gemm_kernel<A_MN, B_MN, EPI, CTAS><<<grid, threads_for(EPI), SMEM, s>>>(a, b, a2, b2, la);
+    tc_gemm_kernel<A_MN, B_MN, EPI, CTAS><<<grid, threads_for(EPI), SMEM, s>>>(a, b, a2, b2, out, la);
   } else {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -951,7 +1021,7 @@ int launch(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& a2, co
       ++na;
     }
     cfg.attrs = attr; cfg.numAttrs = na;
-    if (cudaLaunchKernelEx(&cfg, tc_gemm_kernel<A_MN, B_MN, EPI, CTAS>, a, b, a2, b2, la) != cudaSuccess) {
+    if (cudaLaunchKernelEx(&cfg, tc_gemm_kernel<A_MN, B_MN, EPI, CTAS>, a, b, a2, b2, out, la) != cudaSuccess) {
       cudaGetLastError();
       return FDP_ERR_LAUNCH;
     }
@@ -1145,9 +1215,9 @@ int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int
     args.plane_a = n_out; args.plane_b = n_in;
     args.idesc = make_idesc(dt, true, true, ctas);
     args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = chain_stages(args.seg_stages);
-    args.norm_mode = 1; args.scale = 1.0f; args.nk = NoiseKey{};
-    return ctas == 2 ? launch<true, true, EPI_STORE_SCALED, 2>(a, b, a, b, args, s)
-                     : launch<true, true, EPI_STORE_SCALED, 1>(a, b, a, b, args, s);
+    args.scale = 1.0f; args.nk = NoiseKey{};
+    return ctas == 2 ? launch<true, true, EPI_CHAIN_SUMSQ, 2>(a, b, a, b, a, args, s)
+                     : launch<true, true, EPI_CHAIN_SUMSQ, 1>(a, b, a, b, a, args, s);
   }
   if (pl.algo == FDP_NORM_DIRECT) {
     if (!make_map(&a, G, rows, wo, 64, BK, dt) || !make_map(&b, X, rows, wi, 64, BK, dt)) return FDP_ERR_LAUNCH;
@@ -1158,7 +1228,7 @@ int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int
     args.k_stages = terms * (T / BK);
     args.plane_a = n_out; args.plane_b = n_in;
     args.idesc = make_idesc(dt, true, true);
-    return launch<true, true, EPI_SUMSQ>(a, b, a, b, args, s);
+    return launch<true, true, EPI_SUMSQ>(a, b, a, b, a, args, s);
   }
   // A and B boxes are both 128 rows: a B stage is filled by two independent copies
   if (!make_map(&a, G, rows, wo, BK, BM, dt) || !make_map(&b, G, rows, wo, BK, BN / 2, dt) ||
@@ -1173,7 +1243,7 @@ int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int
   args.k_stages = terms * args.term_stages; args.k_stages2 = terms * args.term_stages2;
   args.plane_a = args.plane_b = n_out; args.plane_a2 = args.plane_b2 = n_in;
   args.idesc = make_idesc(dt, false, false);
-  return launch<false, false, EPI_GRAM>(a, b, a2, b2, args, s);
+  return launch<false, false, EPI_GRAM>(a, b, a2, b2, a, args, s);
 }
 
 int tc_prescale(const void* G, const float* factors, void* Gs, int B, int T, int n_out, int dt, cudaStream_t s) {
@@ -1196,7 +1266,7 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
   const uint64_t rows = static_cast<uint64_t>(B) * T;
   const bool scaled = fs != nullptr;  // Gs is then the unscaled G
   if (terms != 1 && !(terms == 3 && scaled)) return FDP_ERR_ARG;
-  CUtensorMap mg, mx;
+  CUtensorMap mg, mx, mo, mp;
   if (!make_map(&mg, Gs, rows, terms == 3 ? 2 * n_out : n_out, 64, BK, dt) ||
       !make_map(&mx, X, rows, terms == 3 ? 2 * n_in : n_in, 64, BK, dt)) return FDP_ERR_LAUNCH;
   TcArgs args{};
@@ -1238,9 +1308,12 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
     args.units_full = total - n_split_tiles;
     args.split_ws = split_ws;
   }
+  if (!make_out_map(&mo, dW, args.M, args.N, out_dt)) return FDP_ERR_LAUNCH;
+  // the parked parts: [slot * ctas + CTA of the pair][BM rows][BN columns] fp32
+  if (!make_out_map(&mp, split_ws, static_cast<uint64_t>(2) * MAX_SMS * BM, BN, FDP_F32)) return FDP_ERR_LAUNCH;
   int st;
-#define FDP_WGRAD_LAUNCH(EPI_, CT_) (oi ? launch<true, true, EPI_, CT_>(mg, mx, mg, mx, args, s) \
-                                        : launch<true, true, EPI_, CT_>(mx, mg, mx, mg, args, s))
+#define FDP_WGRAD_LAUNCH(EPI_, CT_) (oi ? launch<true, true, EPI_, CT_>(mg, mx, mp, mx, mo, args, s) \
+                                        : launch<true, true, EPI_, CT_>(mx, mg, mp, mg, mo, args, s))
   if (scaled) st = ctas == 2 ? FDP_WGRAD_LAUNCH(EPI_STORE_SCALED, 2) : FDP_WGRAD_LAUNCH(EPI_STORE_SCALED, 1);
   else st = ctas == 2 ? FDP_WGRAD_LAUNCH(EPI_STORE, 2) : FDP_WGRAD_LAUNCH(EPI_STORE, 1);
 #undef FDP_WGRAD_LAUNCH
@@ -1260,9 +1333,9 @@ bool tc_dgrad_ok(int rows, int n_in, int n_out, int dt) {
 
 int tc_dgrad(const void* G, const void* W, void* dX, int* dev_status, int rows, int n_in, int n_out,
              int dt, int out_dt, int w_layout, cudaStream_t s) {
-  CUtensorMap mg, mw;
+  CUtensorMap mg, mw, mo;
   const int ctas = ctas_per_tile();
-  if (!make_map(&mg, G, rows, n_out, BK, BM, dt)) return FDP_ERR_LAUNCH;
+  if (!make_map(&mg, G, rows, n_out, BK, BM, dt) || !make_out_map(&mo, dX, rows, n_in, out_dt)) return FDP_ERR_LAUNCH;
   TcArgs args{};
   args.batch = 1; args.batch_rows = 0; args.status = dev_status; args.zero_status = 1;
   args.M = rows; args.N = n_in; args.ld_out = n_in;
@@ -1276,23 +1349,23 @@ int tc_dgrad(const void* G, const void* W, void* dX, int* dev_status, int rows, 
   if (w_layout == FDP_OUT_IN) {  // W [n_out, n_in]: rows are K, N contiguous
     if (!make_map(&mw, W, n_out, n_in, 64, BK, dt)) return FDP_ERR_LAUNCH;
     args.idesc = make_idesc(dt, false, true, ctas);
-    return ctas == 2 ? launch<false, true, EPI_STORE, 2>(mg, mw, mg, mw, args, s)
-                     : launch<false, true, EPI_STORE, 1>(mg, mw, mg, mw, args, s);
+    return ctas == 2 ? launch<false, true, EPI_STORE, 2>(mg, mw, mg, mw, mo, args, s)
+                     : launch<false, true, EPI_STORE, 1>(mg, mw, mg, mw, mo, args, s);
   }
   // W [n_in, n_out]: K contiguous; a CTA of a pair loads half of the 256 B rows
   if (!make_map(&mw, W, n_in, n_out, BK, BN / ctas, dt)) return FDP_ERR_LAUNCH;
   args.idesc = make_idesc(dt, false, false, ctas);
-  return ctas == 2 ? launch<false, false, EPI_STORE, 2>(mg, mw, mg, mw, args, s)
-                   : launch<false, false, EPI_STORE, 1>(mg, mw, mg, mw, args, s);
+  return ctas == 2 ? launch<false, false, EPI_STORE, 2>(mg, mw, mg, mw, mo, args, s)
+                   : launch<false, false, EPI_STORE, 1>(mg, mw, mg, mw, mo, args, s);
 }
 
 // forward: A = X [rows, n_in] K-major; B = W, K-major for [n_out, n_in] (Linear), MN-major for
 // [n_in, n_out] (Conv1D); bias added in the epilogue
 int tc_fwd(const void* X, const void* W, const void* bias, void* Y, int* dev_status, int rows, int n_in,
            int n_out, int dt, int out_dt, int w_layout, cudaStream_t s) {
-  CUtensorMap mx, mw;
+  CUtensorMap mx, mw, mo;
   const int ctas = ctas_per_tile();
-  if (!make_map(&mx, X, rows, n_in, BK, BM, dt)) return FDP_ERR_LAUNCH;
+  if (!make_map(&mx, X, rows, n_in, BK, BM, dt) || !make_out_map(&mo, Y, rows, n_out, out_dt)) return FDP_ERR_LAUNCH;
   TcArgs args{};
   args.batch = 1; args.batch_rows = 0; args.status = dev_status; args.zero_status = 1;
   args.M = rows; args.N = n_out; args.ld_out = n_out;
@@ -1301,17 +1374,17 @@ int tc_fwd(const void* X, const void* W, const void* bias, void* Y, int* dev_sta
   args.k_stages = ceil_div(n_in, BK);
   args.n_fastest = 1;  // X is streamed once, W stays in L2
   args.out = Y; args.out_dt = out_dt; args.scale = 1.0f; args.nk = NoiseKey{};
-  args.bias = bias; args.bias_dt = dt;
+  args.bias = bias; args.bias_dt = dt; args.bias_vec = aligned16(bias);
   if (w_layout == FDP_OUT_IN) {  // W [n_out, n_in]: K contiguous
     if (!make_map(&mw, W, n_out, n_in, BK, BN / ctas, dt)) return FDP_ERR_LAUNCH;
     args.idesc = make_idesc(dt, false, false, ctas);
-    return ctas == 2 ? launch<false, false, EPI_STORE, 2>(mx, mw, mx, mw, args, s)
-                     : launch<false, false, EPI_STORE, 1>(mx, mw, mx, mw, args, s);
+    return ctas == 2 ? launch<false, false, EPI_STORE, 2>(mx, mw, mx, mw, mo, args, s)
+                     : launch<false, false, EPI_STORE, 1>(mx, mw, mx, mw, mo, args, s);
   }
   if (!make_map(&mw, W, n_in, n_out, 64, BK, dt)) return FDP_ERR_LAUNCH;  // W [n_in, n_out]: N contiguous
   args.idesc = make_idesc(dt, false, true, ctas);
-  return ctas == 2 ? launch<false, true, EPI_STORE, 2>(mx, mw, mx, mw, args, s)
-                   : launch<false, true, EPI_STORE, 1>(mx, mw, mx, mw, args, s);
+  return ctas == 2 ? launch<false, true, EPI_STORE, 2>(mx, mw, mx, mw, mo, args, s)
+                   : launch<false, true, EPI_STORE, 1>(mx, mw, mx, mw, mo, args, s);
 }
 
 // ---- fp32 products on the tensor cores: Y[rows, N] = A[rows, K] * W (+ bias) --------------------------
@@ -1326,9 +1399,9 @@ size_t tc_gemm3_ws_bytes(int rows, int K, int N) {
 }
 int tc_gemm3(const void* A3, const void* W3, const void* bias, void* Y, int* dev_status, int rows, int K, int N,
              int out_dt, bool w_kn, cudaStream_t s) {
-  CUtensorMap ma, mw;
+  CUtensorMap ma, mw, mo;
   const int ctas = ctas_per_tile();
-  if (!make_map(&ma, A3, rows, 2 * K, BK, BM, FDP_BF16)) return FDP_ERR_LAUNCH;
+  if (!make_map(&ma, A3, rows, 2 * K, BK, BM, FDP_BF16) || !make_out_map(&mo, Y, rows, N, out_dt)) return FDP_ERR_LAUNCH;
   TcArgs args{};
   args.batch = 1; args.batch_rows = 0; args.status = dev_status;
   args.dependent = 1;            // follows the split kernels of the same call
@@ -1341,19 +1414,18 @@ int tc_gemm3(const void* A3, const void* W3, const void* bias, void* Y, int* dev
   args.plane_a = K; args.plane_b = w_kn ? N : K;
   args.n_fastest = 1;
   args.out = Y; args.out_dt = out_dt; args.scale = 1.0f; args.nk = NoiseKey{};
-  args.bias = bias; args.bias_dt = FDP_F32;
+  args.bias = bias; args.bias_dt = FDP_F32; args.bias_vec = aligned16(bias);
   args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = chain_stages(args.seg_stages);
-  args.norm_mode = 2;
   if (w_kn) {   // rows of W3 are K, N contiguous
     if (!make_map(&mw, W3, K, 2 * N, 64, BK, FDP_BF16)) return FDP_ERR_LAUNCH;
     args.idesc = make_idesc(FDP_BF16, false, true, ctas);
-    return ctas == 2 ? launch<false, true, EPI_STORE_SCALED, 2>(ma, mw, ma, mw, args, s)
-                     : launch<false, true, EPI_STORE_SCALED, 1>(ma, mw, ma, mw, args, s);
+    return ctas == 2 ? launch<false, true, EPI_CHAIN, 2>(ma, mw, ma, mw, mo, args, s)
+                     : launch<false, true, EPI_CHAIN, 1>(ma, mw, ma, mw, mo, args, s);
   }
   if (!make_map(&mw, W3, N, 2 * K, BK, BN / ctas, FDP_BF16)) return FDP_ERR_LAUNCH;   // K contiguous
   args.idesc = make_idesc(FDP_BF16, false, false, ctas);
-  return ctas == 2 ? launch<false, false, EPI_STORE_SCALED, 2>(ma, mw, ma, mw, args, s)
-                   : launch<false, false, EPI_STORE_SCALED, 1>(ma, mw, ma, mw, args, s);
+  return ctas == 2 ? launch<false, false, EPI_CHAIN, 2>(ma, mw, ma, mw, mo, args, s)
+                   : launch<false, false, EPI_CHAIN, 1>(ma, mw, ma, mw, mo, args, s);
 }
 
 }  // namespace fdp
