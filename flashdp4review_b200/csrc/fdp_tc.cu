@@ -43,16 +43,19 @@ constexpr int MAX_SMS = 148;           // workers the split-K parking area is si
 
 // EPI_STORE_SCALED: the accumulator of each sample (K segment) is drained on its own and added, times
 // that sample's clip factor, to fp32 registers of eight epilogue warps; G needs no scaled copy.
-// EPI_CHAIN / EPI_CHAIN_SUMSQ: the same with a constant factor for fp32 products in short chains; the first
-// stores the tile (+ bias), the second sums the squares of one sample's tile.
-enum { EPI_STORE = 0, EPI_SUMSQ = 1, EPI_GRAM = 2, EPI_STORE_SCALED = 3, EPI_CHAIN = 4, EPI_CHAIN_SUMSQ = 5 };
+// EPI_SPLIT_*: fp32 inputs as bf16 halves, three products per K stage (see TcArgs::plane_a): the clipped sum,
+// a plain product (+ bias), and one sample's product tile squared and summed.
+enum { EPI_STORE = 0, EPI_SUMSQ = 1, EPI_GRAM = 2, EPI_STORE_SCALED = 3, EPI_SPLIT_SCALED = 4, EPI_SPLIT_STORE = 5,
+       EPI_SPLIT_SUMSQ = 6 };
 __host__ __device__ constexpr bool epi_chained(int epi) { return epi >= EPI_STORE_SCALED; }
-__host__ __device__ constexpr bool epi_stores(int epi) { return epi == EPI_STORE || epi == EPI_STORE_SCALED || epi == EPI_CHAIN; }
+__host__ __device__ constexpr bool epi_split(int epi) { return epi >= EPI_SPLIT_SCALED; }
+__host__ __device__ constexpr bool epi_scaled(int epi) { return epi == EPI_STORE_SCALED || epi == EPI_SPLIT_SCALED; }
+__host__ __device__ constexpr bool epi_stores(int epi) { return epi == EPI_STORE || epi_scaled(epi) || epi == EPI_SPLIT_STORE; }
 // eight epilogue warps (two per TMEM lane quarter, 128 columns each) for the store epilogues, four for the norms
 __host__ __device__ constexpr int epi_warps_for(int epi) { return (epi == EPI_STORE || epi_chained(epi)) ? 8 : 4; }
 constexpr int threads_for(int epi) { return 64 + 32 * epi_warps_for(epi); }
 constexpr int smem_for(int epi) {
-  return epi == EPI_STORE_SCALED ? SMEM_BYTES_SCALED : epi_stores(epi) ? SMEM_BYTES_STORE : SMEM_BYTES;
+  return epi_scaled(epi) ? SMEM_BYTES_SCALED : epi_stores(epi) ? SMEM_BYTES_STORE : SMEM_BYTES;
 }
 
 struct TcArgs {
@@ -98,14 +101,12 @@ struct TcArgs {
   uint32_t idesc_half;
   // store epilogue: optional bias[N] (same 16-bit type as the operands) added to every row
   const void* bias; int bias_dt; int bias_vec;   // bias_vec: 16-byte aligned
-  // fp32 inputs as three bf16 products.  Both operand matrices are then [rows, 2n]: the high bf16
-  // halves of the n columns, then the low halves (x = hi + lo up to 2^-18 |x|).  With terms = 3 the K
-  // loop visits every K range three times -- hi*hi, hi*lo, lo*hi -- into the same accumulator (lo*lo,
-  // 2^-18 of the product, is dropped).  term_stages: K stages of one term before the next term of the
-  // same range begins (a sample's rows for the per-sample kernels; pair 2 of EPI_GRAM: term_stages2).
-  // plane_*: columns of one half of the A / B matrix, i.e. the column offset of its low halves.
-  int terms, term_stages, term_stages2;
-  int plane_a, plane_b, plane_a2, plane_b2;
+  // fp32 inputs as three bf16 products (EPI_SPLIT_*).  Both operand matrices are then [rows, 2n]: the high
+  // bf16 halves of the n columns, then the low halves (x = hi + lo up to 2^-18 |x|); plane_a / plane_b is the
+  // column offset of the low halves.  A K stage holds all four tiles -- A hi, A lo, B hi, B lo -- and feeds
+  // three products, hi*lo, lo*hi and hi*hi, into the same accumulator (lo*lo, 2^-18 of the product, is
+  // dropped): four tile loads for three products instead of six.
+  int plane_a, plane_b;
   // store GEMMs: tiles are walked in groups of m_group tile rows (0 = plain order), so that the CTAs
   // running together cover a squarer patch of the output and re-read less of the operands
   int m_group;
@@ -319,9 +320,11 @@ __global__ void __launch_bounds__(threads_for(EPI), 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB2,
                const __grid_constant__ CUtensorMap tmOut, const __grid_constant__ TcArgs args) {
-  constexpr int NST = (CTAS == 2) ? 6 : STAGES;          // ring depth
-  constexpr int B_BYTES = B_STAGE_BYTES / CTAS;          // this CTA's share of the B stage
-  constexpr int STG = A_STAGE_BYTES + B_BYTES;
+  constexpr int PLANES = epi_split(EPI) ? 2 : 1;         // bf16 halves of fp32 operands
+  constexpr int NST = ((CTAS == 2) ? 6 : STAGES) / PLANES;   // ring depth
+  constexpr int A_BYTES = PLANES * A_STAGE_BYTES;
+  constexpr int B_BYTES = B_STAGE_BYTES / CTAS;          // this CTA's share of (one half of) the B stage
+  constexpr int STG = A_BYTES + PLANES * B_BYTES;
   constexpr int BN_CTA = BN / CTAS;                      // B columns (rows if K-major) loaded by this CTA
   constexpr int EPI_WARPS = epi_warps_for(EPI);
   static_assert(NST * STG <= STAGES * STAGE_BYTES, "ring size");
@@ -430,26 +433,20 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     ks1 = static_cast<int>(static_cast<long long>(kst_total) * (part + 1) / args.split);
     slot = v;
   };
-  // EPI_STORE_SCALED: end of the sample segment that contains stage ks, cut at the unit's end
-  // (sub_stages divides seg_stages: a hand-off never spans two samples.  With fp32 inputs it is a few
-  // stages only: the tensor cores add into the TMEM accumulator by truncation, about one unit in the
+  // chained epilogues: end of the hand-off that contains stage ks -- sub_stages further, cut at the
+  // sample's and at the unit's end.  (With fp32 inputs it is a few stages only: the tensor cores add into the TMEM accumulator by truncation, about one unit in the
   // last place per K = 16 step and all of one sign, so a long chain drifts; short chains summed in
   // registers with round-to-nearest do not.)
   auto segment_end = [&](int ks, int ks1) {
-    const int e = (ks / args.sub_stages + 1) * args.sub_stages;
+    const int s0 = ks / args.seg_stages * args.seg_stages;
+    const int sub = ((ks - s0) / args.sub_stages + 1) * args.sub_stages;
+    const int e = s0 + (sub < args.seg_stages ? sub : args.seg_stages);
     return e < ks1 ? e : ks1;
   };
-
-  // K stage `kl` of an operand pair's K order -> stage within the K range, and which term it belongs to
-  // (0: hi*hi, 1: hi*lo, 2: lo*hi); a no-op for 16-bit inputs (terms == 1)
-  auto term_of = [&](int& kl, bool second) {
-    if (args.terms <= 1) return 0;
-    const int ts = second ? args.term_stages2 : args.term_stages;
-    const int run = args.terms * ts;
-    const int blk = kl / run, w = kl - blk * run;
-    const int term = w / ts;
-    kl = blk * ts + (w - term * ts);
-    return term;
+  // running number of the hand-off that contains stage ks
+  auto segment_index = [&](int ks) {
+    const int sg = ks / args.seg_stages;
+    return sg * ((args.seg_stages + args.sub_stages - 1) / args.sub_stages) + (ks - sg * args.seg_stages) / args.sub_stages;
   };
 
   if (warp == 0) {
@@ -467,53 +464,42 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           const bool second = (EPI == EPI_GRAM) && ks >= args.k_stages;
           const CUtensorMap* ma = second ? &tmA2 : &tmA;
           const CUtensorMap* mb = second ? &tmB2 : &tmB;
-          int kl = second ? ks - args.k_stages : ks;
-          const int term = term_of(kl, second);
-          const int k0 = kl * BK;
-          // column offsets of the planes this term reads (A low halves in term 2, B low halves in term 1)
-          const int ca = term == 2 ? (second ? args.plane_a2 : args.plane_a) : 0;
-          const int cb = term == 1 ? (second ? args.plane_b2 : args.plane_b) : 0;
-          const uint32_t sa = base + stage * STG, sb = sa + A_STAGE_BYTES;
+          const int k0 = (second ? ks - args.k_stages : ks) * BK;
+          const uint32_t sa = base + stage * STG, sb = sa + A_BYTES;
           if (EPI == EPI_GRAM) {
             // A: the t-block; B: two independent 128-row s-blocks, one per half of the stage
             // (a unit that contains the diagonal block (i, i) has its t-block in the B stage already:
             // the MMA warp points the A descriptor there and no A copy is made)
             constexpr uint32_t HALF_B = B_STAGE_BYTES / 2;
-            const bool a_in_b = term == 0 && ((n0 == m0) || (gram_n1 == m0));
+            const bool a_in_b = (n0 == m0) || (gram_n1 == m0);
             mbar_expect_tx(full_bar(stage), (a_in_b ? 0 : A_STAGE_BYTES) + (gram_n1 >= 0 ? 2 : 1) * HALF_B);
-            if (!a_in_b) tma_load_2d(sa, ma, k0 + ca, row0 + m0, full_bar(stage));
-            tma_load_2d(sb, mb, k0 + cb, row0 + n0, full_bar(stage));
-            if (gram_n1 >= 0) tma_load_2d(sb + HALF_B, mb, k0 + cb, row0 + gram_n1, full_bar(stage));
-          } else if (CTAS == 1) {
-            mbar_expect_tx(full_bar(stage), STG);
-            if (A_MN) {
-#pragma unroll
-              for (int i = 0; i < BM / 64; ++i) tma_load_2d(sa + i * (BK * 128), ma, m0 + 64 * i + ca, row0 + k0, full_bar(stage));
-            } else {
-              tma_load_2d(sa, ma, k0 + ca, row0 + m0, full_bar(stage));
-            }
-            if (B_MN) {
-#pragma unroll
-              for (int j = 0; j < BN / 64; ++j) tma_load_2d(sb + j * (BK * 128), mb, n0 + 64 * j + cb, row0 + k0, full_bar(stage));
-            } else {
-              tma_load_2d(sb, mb, k0 + cb, row0 + n0, full_bar(stage));
-            }
+            if (!a_in_b) tma_load_2d(sa, ma, k0, row0 + m0, full_bar(stage));
+            tma_load_2d(sb, mb, k0, row0 + n0, full_bar(stage));
+            if (gram_n1 >= 0) tma_load_2d(sb + HALF_B, mb, k0, row0 + gram_n1, full_bar(stage));
           } else {
-            // both CTAs' copies complete on the leader's barrier, which expects the bytes of both
-            const uint32_t lbar = mapa_u32(full_bar(stage), 0);
-            if (is_leader) mbar_expect_tx(full_bar(stage), 2 * STG);
+            // both CTAs' copies of a pair complete on the leader's barrier, which expects the bytes of both
+            const uint32_t lbar = CTAS == 1 ? full_bar(stage) : mapa_u32(full_bar(stage), 0);
+            if (is_leader) mbar_expect_tx(full_bar(stage), CTAS * STG);
             const int nb0 = n0 + static_cast<int>(cta_rank) * BN_CTA;
-            if (A_MN) {
+            auto load = [&](uint32_t dst, const CUtensorMap* map, int c0, int c1) {
+              if (CTAS == 1) tma_load_2d(dst, map, c0, c1, lbar); else tma_load_2d_pair(dst, map, c0, c1, lbar);
+            };
 #pragma unroll
-              for (int i = 0; i < BM / 64; ++i) tma_load_2d_pair(sa + i * (BK * 128), ma, m0 + 64 * i + ca, row0 + k0, lbar);
-            } else {
-              tma_load_2d_pair(sa, ma, k0 + ca, row0 + m0, lbar);
-            }
-            if (B_MN) {
+            for (int pl = 0; pl < PLANES; ++pl) {
+              const int ca = pl * args.plane_a, cb = pl * args.plane_b;
+              const uint32_t da = sa + pl * A_STAGE_BYTES, db = sb + pl * B_BYTES;
+              if (A_MN) {
 #pragma unroll
-              for (int j = 0; j < BN_CTA / 64; ++j) tma_load_2d_pair(sb + j * (BK * 128), mb, nb0 + 64 * j + cb, row0 + k0, lbar);
-            } else {
-              tma_load_2d_pair(sb, mb, k0 + cb, row0 + nb0, lbar);
+                for (int i = 0; i < BM / 64; ++i) load(da + i * (BK * 128), ma, m0 + 64 * i + ca, row0 + k0);
+              } else {
+                load(da, ma, k0 + ca, row0 + m0);
+              }
+              if (B_MN) {
+#pragma unroll
+                for (int j = 0; j < BN_CTA / 64; ++j) load(db + j * (BK * 128), mb, nb0 + 64 * j + cb, row0 + k0);
+              } else {
+                load(db, mb, k0 + cb, row0 + nb0);
+              }
             }
           }
           if (++stage == NST) { stage = 0; phase ^= 1u; }
@@ -556,22 +542,20 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const uint32_t d = tmem_base + (EPI == EPI_GRAM ? (second ? BN : 0) : acc * BN);
             const bool first_stage = second ? (ks == args.k_stages) : (ks == seg_begin);
             uint32_t sa = base + stage * STG;
-            const uint32_t sb = sa + A_STAGE_BYTES;
+            const uint32_t sb = sa + A_BYTES;
             if (EPI == EPI_GRAM) {   // diagonal block in this unit: A is the matching half of the B stage
-              int kl = second ? ks - args.k_stages : ks;
-              if (term_of(kl, second) == 0) {
-                if (tn0 == tm0) sa = sb;
-                else if (gram_n1 == tm0) sa = sb + B_STAGE_BYTES / 2;
-              }
+              if (tn0 == tm0) sa = sb;
+              else if (gram_n1 == tm0) sa = sb + B_STAGE_BYTES / 2;
             }
 #pragma unroll
             for (int k16 = 0; k16 < BK / UMMA_K; ++k16) {
-              if (CTAS == 1)
-                tc_mma(d, operand_desc<A_MN>(sa, k16), operand_desc<B_MN>(sb, k16), idesc,
-                       (first_stage && k16 == 0) ? 0u : 1u);
-              else
-                tc_mma_pair(d, operand_desc<A_MN>(sa, k16), operand_desc<B_MN>(sb, k16), idesc,
-                            (first_stage && k16 == 0) ? 0u : 1u);
+#pragma unroll
+              for (int q = 0; q < (PLANES == 2 ? 3 : 1); ++q) {   // hi*lo, lo*hi, hi*hi
+                const uint64_t da = operand_desc<A_MN>(sa + (PLANES == 2 && q == 1 ? A_STAGE_BYTES : 0), k16);
+                const uint64_t db = operand_desc<B_MN>(sb + (PLANES == 2 && q == 0 ? B_BYTES : 0), k16);
+                const uint32_t acc_in = (first_stage && k16 == 0 && q == 0) ? 0u : 1u;
+                if (CTAS == 1) tc_mma(d, da, db, idesc, acc_in); else tc_mma_pair(d, da, db, idesc, acc_in);
+              }
             }
             // frees the stage (in both CTAs of a pair) once these MMAs have read it
             if (CTAS == 1) {
@@ -608,7 +592,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const uint32_t box = base + NST * STG + ew * BOX_BYTES;
     int it = 0;
     bool ok = true;
-    if (EPI == EPI_STORE_SCALED && args.norm_partials != nullptr) {
+    if (epi_scaled(EPI) && args.norm_partials != nullptr) {
       // clip factors of all samples from the norm pass's partial sums (fixed order: a lane adds every
       // 32nd partial, then the shuffle tree), while the producer and MMA warps start the main loop
       for (int b = ew; b < args.segs; b += EPI_WARPS) {
@@ -642,9 +626,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // A whole tile's Gaussian noise goes into the accumulators a few element groups per sample
         // segment, in the time these warps would otherwise wait for the next segment's MMAs; K-split
         // parts stay noise-free (the fix-up kernel adds the noise once per tile).
-        const bool pre_noise = EPI == EPI_STORE_SCALED && slot < 0 && args.nk.std != 0.f && m < args.M;
+        const bool pre_noise = epi_scaled(EPI) && slot < 0 && args.nk.std != 0.f && m < args.M;
         const uint64_t g0 = (static_cast<uint64_t>(m) * args.ld_out + n0 + chalf * 128) >> 2;
-        const int nseg = (ks1 - 1) / args.sub_stages - ks0 / args.sub_stages + 1;
+        const int nseg = segment_index(ks1 - 1) - segment_index(ks0) + 1;
         int ng = 0, seg = 0;
         for (int ks = ks0; ks < ks1 && ok; ks = segment_end(ks, ks1), ++it) {
           const int acc = it % NUM_ACC;
@@ -653,7 +637,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           tc_fence_after();
           const int sample = ks / args.seg_stages;
           // the divisor goes into the factor, so the noise is added as it is drawn
-          const float cbs = EPI != EPI_STORE_SCALED ? args.scale
+          const float cbs = !epi_scaled(EPI) ? args.scale
                           : (args.norm_partials != nullptr ? sfac[sample] : __ldg(args.factors + sample)) * args.scale;
           const uint32_t tb = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN + chalf * 128;
 #pragma unroll
@@ -671,7 +655,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             else mbar_arrive_cluster(mapa_u32(tempty_bar(acc), 0));
           }
           ++seg;
-          if (EPI == EPI_STORE_SCALED && pre_noise) {
+          if (epi_scaled(EPI) && pre_noise) {
             const int target = (32 * seg) / nseg;
             for (; ng < target; ++ng) {
               float z[4];
@@ -681,7 +665,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
         }
         if (!ok) break;
-        if constexpr (EPI == EPI_CHAIN_SUMSQ) {
+        if constexpr (EPI == EPI_SPLIT_SUMSQ) {
           // the unit is one sample's product tile: its squares, without the rows and columns past the
           // matrix (with split operands a tile that overhangs reads the other half's columns, not zeros)
           float part = 0.f;
@@ -697,7 +681,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
             for (int c4 = 0; c4 < 4; ++c4) {
               const int n = n0 + chalf * 128 + c4 * 32;
-              if (EPI == EPI_CHAIN && args.bias != nullptr && n < args.N) add_bias32(args, n, accr + c4 * 32);
+              if (EPI == EPI_SPLIT_STORE && args.bias != nullptr && n < args.N) add_bias32(args, n, accr + c4 * 32);
               store_out32(args, box, &tmOut, accr + c4 * 32, c4, n0 + chalf * 128, m0 + quarter * 32, lane);
             }
           }
@@ -1050,15 +1034,17 @@ int ctas_per_tile() { return forced_ctas() == 1 ? 1 : 2; }
 // unsplit (100.8 against 98.6 us per call: parking, the second round's hand-over and the fix-up
 // launch eat the 42 stages saved), while 16 tiles in four parts (52 against 82 us) and the tails of
 // the larger layers do pay.
-int plan_tail_split(int total_tiles, int k_stages, int workers) {
+int plan_tail_split(int total_tiles, int k_stages, int workers, int products) {
   const int rem = total_tiles <= workers ? total_tiles : total_tiles % workers;
-  if (rem == 0 || k_stages < 32) return 1;
+  // stages are counted by their work: with split fp32 operands one holds three products
+  const int min_stages = products == 3 ? 3 : 8;      // shortest part
+  if (rem == 0 || k_stages < 4 * min_stages) return 1;
   // FDP_TC_SPLIT=n forces the number of parts (measurements), within the same limits
   static const int forced = [] { const char* e = getenv("FDP_TC_SPLIT"); return e ? atoi(e) : 0; }();
-  if (forced >= 1) return (rem * forced > 2 * workers || k_stages / forced < 8) ? 1 : forced;
+  if (forced >= 1) return (rem * forced > 2 * workers || k_stages / forced < min_stages) ? 1 : forced;
   int best_s = 1; double best = 1.0;
   for (int sp = 2; sp <= 16; ++sp) {
-    if (rem * sp > 2 * workers || k_stages / sp < 8) break;
+    if (rem * sp > 2 * workers || k_stages / sp < min_stages) break;
     const double cost = static_cast<double>((rem * sp + workers - 1) / workers) / sp +
                         0.15 * (static_cast<double>(rem) * sp / workers) + 0.05;
     if (cost < best - 0.03) { best = cost; best_s = sp; }
@@ -1094,19 +1080,17 @@ int tc_wait_selftest(int* status, long long limit_cycles, cudaStream_t s) {
   return cudaPeekAtLastError() == cudaSuccess ? FDP_OK : (cudaGetLastError(), FDP_ERR_LAUNCH);
 }
 
-// K stages per accumulator hand-off for fp32 inputs (three bf16 products): the largest divisor of a
-// sample's stage count that is at most FDP_TC_CHAIN_STAGES (default 8: 32 steps of K = 16 per chain).
-// B=8, T=1024, 4096x4096, against float64: norms 1.1e-7 / 2.5e-7 / 4.4e-7 / 5e-6 and 2.15 / 1.48 /
-// 1.42 / 1.37 ms per call with 2 / 4 / 8 / all stages per chain (1e-5 at T=2048 with one chain).
+// K stages per accumulator hand-off for fp32 inputs (a stage = 12 MMA steps of K = 16, three products of
+// four): FDP_TC_CHAIN_STAGES, default 2.  B=8, T=1024, 4096x4096 against float64, 1 / 2 / 3 / 4 / 8 stages:
+// norms off by 2.0e-7 / 3.8e-7 / 5.2e-7 / 7.3e-7 / 1.4e-6 (the truncation of the accumulators grows with the
+// chain); B=8, T=1024, 1024->3072, all kernels of a forward and backward: 832 / 636 / 616 / 592 / 588 us.
 static int chain_stages(int seg_stages) {
   static const int cap = [] {
     const char* e = getenv("FDP_TC_CHAIN_STAGES");
-    const int v = e ? atoi(e) : 8;
+    const int v = e ? atoi(e) : 2;
     return v < 1 ? 1 : v;
   }();
-  int c = cap < seg_stages ? cap : seg_stages;
-  while (seg_stages % c != 0) --c;
-  return c;
+  return cap < seg_stages ? cap : seg_stages;
 }
 
 // The tensor-core path needs 16-bit inputs, row pitches that are multiples of 16 bytes, and
@@ -1194,13 +1178,11 @@ int tc_split3(const void* src, void* dst, size_t rows, int n, cudaStream_t s) {
 int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int B, int T, int n_in,
              int n_out, int dt, const TcPlan& pl, cudaStream_t s) {
   const uint64_t rows = static_cast<uint64_t>(B) * T;
-  const int terms = pl.split3 ? 3 : 1;
   const int wo = pl.split3 ? 2 * n_out : n_out, wi = pl.split3 ? 2 * n_in : n_in;   // matrix widths
   CUtensorMap a, b, a2, b2;
   TcArgs args{};
   args.batch = B; args.batch_rows = T; args.partials = partials; args.status = dev_status; args.T = T;
   args.zero_status = 1;      // the norm pass is the first launch of a weight-gradient call
-  args.terms = terms;
   if (pl.split3) {
     // fp32 inputs: the per-sample products G_b^T X_b themselves, on the tiles and CTA pairs of the
     // clipped-sum GEMM, handed to the epilogue every few K stages and summed there in registers; a
@@ -1210,23 +1192,20 @@ int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int
     args.M = n_out; args.N = n_in; args.ld_out = n_in;
     args.tiles_m = ceil_div(n_out, BM * ctas); args.tiles_n = ceil_div(n_in, BN);
     args.tiles_per_batch = args.tiles_m * args.tiles_n;
-    args.term_stages = T / BK;
-    args.k_stages = terms * (T / BK);
+    args.k_stages = T / BK;
     args.plane_a = n_out; args.plane_b = n_in;
     args.idesc = make_idesc(dt, true, true, ctas);
     args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = chain_stages(args.seg_stages);
     args.scale = 1.0f; args.nk = NoiseKey{};
-    return ctas == 2 ? launch<true, true, EPI_CHAIN_SUMSQ, 2>(a, b, a, b, a, args, s)
-                     : launch<true, true, EPI_CHAIN_SUMSQ, 1>(a, b, a, b, a, args, s);
+    return ctas == 2 ? launch<true, true, EPI_SPLIT_SUMSQ, 2>(a, b, a, b, a, args, s)
+                     : launch<true, true, EPI_SPLIT_SUMSQ, 1>(a, b, a, b, a, args, s);
   }
   if (pl.algo == FDP_NORM_DIRECT) {
     if (!make_map(&a, G, rows, wo, 64, BK, dt) || !make_map(&b, X, rows, wi, 64, BK, dt)) return FDP_ERR_LAUNCH;
     args.M = n_out; args.N = n_in;
     args.tiles_m = ceil_div(n_out, BM); args.tiles_n = ceil_div(n_in, BN);
     args.tiles_per_batch = args.tiles_m * args.tiles_n;
-    args.term_stages = T / BK;
-    args.k_stages = terms * (T / BK);
-    args.plane_a = n_out; args.plane_b = n_in;
+    args.k_stages = T / BK;
     args.idesc = make_idesc(dt, true, true);
     return launch<true, true, EPI_SUMSQ>(a, b, a, b, a, args, s);
   }
@@ -1239,9 +1218,7 @@ int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int
   args.tiles_m = args.gram_nb; args.tiles_n = args.gram_nb;
   args.tiles_per_batch = gram_tiles(T);
   args.idesc_half = make_idesc(dt, false, false, 1, BN / 2);
-  args.term_stages = ceil_div(n_out, BK); args.term_stages2 = ceil_div(n_in, BK);
-  args.k_stages = terms * args.term_stages; args.k_stages2 = terms * args.term_stages2;
-  args.plane_a = args.plane_b = n_out; args.plane_a2 = args.plane_b2 = n_in;
+  args.k_stages = ceil_div(n_out, BK); args.k_stages2 = ceil_div(n_in, BK);
   args.idesc = make_idesc(dt, false, false);
   return launch<false, false, EPI_GRAM>(a, b, a2, b2, a, args, s);
 }
@@ -1272,9 +1249,7 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
   TcArgs args{};
   args.batch = 1; args.batch_rows = 0; args.status = dev_status;
   args.dependent = 1;             // always follows a kernel of the same call (norm pass, clip factors or pre-scale)
-  args.terms = terms;
-  args.term_stages = T / BK;      // used when terms == 3: every sample's rows are visited three times
-  args.k_stages = terms * static_cast<int>((rows + BK - 1) / BK);
+  args.k_stages = static_cast<int>((rows + BK - 1) / BK);
   args.out = dW; args.out_dt = out_dt; args.scale = inv_div; args.nk = nk;
   // [out,in]: A = G (M = n_out), B = X (N = n_in); [in,out]: operands swap roles, no transpose pass
   const bool oi = (layout == FDP_OUT_IN);
@@ -1282,7 +1257,7 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
   const int ctas = ctas_per_tile();
   args.idesc = make_idesc(dt, true, true, ctas);
   if (scaled) {
-    args.segs = B; args.seg_stages = terms * (T / BK);
+    args.segs = B; args.seg_stages = T / BK;
     args.sub_stages = terms == 3 ? chain_stages(args.seg_stages) : args.seg_stages;
     args.factors = fs->factors;
     if (fs->factors == nullptr) {
@@ -1300,7 +1275,7 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
   // tail wave: split K so the SMs left idle by the tile count get work; the parts are parked in the
   // workspace and summed in fixed order by the fix-up kernel (deterministic, no waits)
   const int total = args.tiles_per_batch, workers = launch_sms() / ctas;
-  const int split = plan_tail_split(total, args.k_stages, workers);
+  const int split = plan_tail_split(total, args.k_stages, workers, terms);
   int n_split_tiles = 0;
   if (split > 1) {
     n_split_tiles = total <= workers ? total : total % workers;
@@ -1314,7 +1289,8 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
   int st;
 #define FDP_WGRAD_LAUNCH(EPI_, CT_) (oi ? launch<true, true, EPI_, CT_>(mg, mx, mp, mx, mo, args, s) \
                                         : launch<true, true, EPI_, CT_>(mx, mg, mp, mg, mo, args, s))
-  if (scaled) st = ctas == 2 ? FDP_WGRAD_LAUNCH(EPI_STORE_SCALED, 2) : FDP_WGRAD_LAUNCH(EPI_STORE_SCALED, 1);
+  if (terms == 3) st = ctas == 2 ? FDP_WGRAD_LAUNCH(EPI_SPLIT_SCALED, 2) : FDP_WGRAD_LAUNCH(EPI_SPLIT_SCALED, 1);
+  else if (scaled) st = ctas == 2 ? FDP_WGRAD_LAUNCH(EPI_STORE_SCALED, 2) : FDP_WGRAD_LAUNCH(EPI_STORE_SCALED, 1);
   else st = ctas == 2 ? FDP_WGRAD_LAUNCH(EPI_STORE, 2) : FDP_WGRAD_LAUNCH(EPI_STORE, 1);
 #undef FDP_WGRAD_LAUNCH
   if (st != FDP_OK || split <= 1) return st;
@@ -1408,9 +1384,7 @@ int tc_gemm3(const void* A3, const void* W3, const void* bias, void* Y, int* dev
   args.M = rows; args.N = N; args.ld_out = N;
   args.tiles_m = ceil_div(rows, BM * ctas); args.tiles_n = ceil_div(N, BN);
   args.tiles_per_batch = args.tiles_m * args.tiles_n;
-  args.terms = 3;
-  args.term_stages = K / BK;
-  args.k_stages = 3 * (K / BK);
+  args.k_stages = K / BK;
   args.plane_a = K; args.plane_b = w_kn ? N : K;
   args.n_fastest = 1;
   args.out = Y; args.out_dt = out_dt; args.scale = 1.0f; args.nk = NoiseKey{};
@@ -1419,13 +1393,13 @@ int tc_gemm3(const void* A3, const void* W3, const void* bias, void* Y, int* dev
   if (w_kn) {   // rows of W3 are K, N contiguous
     if (!make_map(&mw, W3, K, 2 * N, 64, BK, FDP_BF16)) return FDP_ERR_LAUNCH;
     args.idesc = make_idesc(FDP_BF16, false, true, ctas);
-    return ctas == 2 ? launch<false, true, EPI_CHAIN, 2>(ma, mw, ma, mw, mo, args, s)
-                     : launch<false, true, EPI_CHAIN, 1>(ma, mw, ma, mw, mo, args, s);
+    return ctas == 2 ? launch<false, true, EPI_SPLIT_STORE, 2>(ma, mw, ma, mw, mo, args, s)
+                     : launch<false, true, EPI_SPLIT_STORE, 1>(ma, mw, ma, mw, mo, args, s);
   }
   if (!make_map(&mw, W3, N, 2 * K, BK, BN / ctas, FDP_BF16)) return FDP_ERR_LAUNCH;   // K contiguous
   args.idesc = make_idesc(FDP_BF16, false, false, ctas);
-  return ctas == 2 ? launch<false, false, EPI_CHAIN, 2>(ma, mw, ma, mw, mo, args, s)
-                   : launch<false, false, EPI_CHAIN, 1>(ma, mw, ma, mw, mo, args, s);
+  return ctas == 2 ? launch<false, false, EPI_SPLIT_STORE, 2>(ma, mw, ma, mw, mo, args, s)
+                   : launch<false, false, EPI_SPLIT_STORE, 1>(ma, mw, ma, mw, mo, args, s);
 }
 
 }  // namespace fdp
