@@ -98,7 +98,8 @@ def dp_linear_weight_grad(input, grad_output, C, clamp_value, *, batch_divisor=N
     `fp32_tensor` (default: runtime.fp32_mode() == "tensor", which is the package default): fp32 inputs
     with 64-aligned shapes run on the tensor cores as three bf16 products with short accumulation
     chains -- about six times faster than the fp32-FMA kernels and within the same 1e-5 of float64;
-    False forces the FMA kernels.
+    other shapes (widths of at least 64, at least 128 rows) as six products, as close to float64 as the
+    FMA kernels.  False forces the FMA kernels.
     """
     lib = _lib.load()
     _require_cuda(input, grad_output)
@@ -123,7 +124,7 @@ def dp_linear_weight_grad(input, grad_output, C, clamp_value, *, batch_divisor=N
         from .. import runtime
         fp32_tensor = runtime.fp32_mode() == "tensor"
     if fp32_tensor and G.dtype == torch.float32:
-        algo |= _lib.FDP_FP32_TENSOR
+        algo |= _lib.FDP_FP32_TENSOR | _lib.FDP_FP32_WIDE
     nbytes = lib.fdp_linear_wgrad_workspace_bytes(B, T, n_in, n_out, _dt(G.dtype), algo)
     ws = _workspace(nbytes, G.device)
     p = _params(C, clamp_value, batch_divisor, noise)

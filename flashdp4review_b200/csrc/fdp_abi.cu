@@ -244,7 +244,7 @@ int fdp_linear_wgrad(const void* G, const void* X, void* dW, float* norms_out, f
   if (G == nullptr || X == nullptr || dW == nullptr) return FDP_ERR_ARG;
   if (B <= 0 || T <= 0 || n_in <= 0 || n_out <= 0) return FDP_ERR_ARG;
   if (layout != FDP_OUT_IN && layout != FDP_IN_OUT) return FDP_ERR_ARG;
-  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
+  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
     return FDP_ERR_ARG;
   if (!valid_dtype(in_dtype) || !valid_dtype(out_dtype)) return FDP_ERR_DTYPE;
   if (static_cast<long long>(B) * T >= (1ll << 31) / 2) return FDP_ERR_SHAPE;   // row indices are 32-bit
@@ -254,9 +254,9 @@ int fdp_linear_wgrad(const void* G, const void* X, void* dW, float* norms_out, f
   if (workspace == nullptr) return FDP_ERR_WORKSPACE;
   WgradWs w = wgrad_ws(workspace, B, T, n_in, n_out, in_dtype, norm_algo);
   if (workspace_bytes < w.bytes || !aligned16(workspace)) return FDP_ERR_WORKSPACE;
-  // the tensor-core path moves 16-byte vectors (TMA, vector stores); the generic kernels load and
-  // store single elements and take any naturally aligned pointer
-  if (w.tc.ok && (!aligned16(G) || !aligned16(X) || !aligned16(dW))) return FDP_ERR_ALIGN;
+  // the tensor-core path moves 16-byte vectors (TMA, vector stores); the generic kernels, and the split
+  // copies of fp32 operands with six products, take any naturally aligned pointer
+  if (w.tc.ok && !w.tc.any_align && (!aligned16(G) || !aligned16(X) || !aligned16(dW))) return FDP_ERR_ALIGN;
 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int div = p->batch_divisor > 0 ? p->batch_divisor : B;
@@ -273,11 +273,12 @@ int fdp_linear_wgrad(const void* G, const void* X, void* dW, float* norms_out, f
   const void* Gt = G;
   const void* Xt = X;
   int tdt = in_dtype;
-  if (w.tc.ok && w.tc.split3) {
+  const bool split = w.tc.ok && w.tc.planes > 1;
+  if (split) {
     char* sg = static_cast<char*>(w.tc_extra) + w.tc.split_bytes;
-    char* sx = sg + w.tc.split3_g_bytes;
-    if ((st = tc_split3(G, sg, static_cast<size_t>(B) * T, n_out, s)) != FDP_OK) return st;
-    if ((st = tc_split3(X, sx, static_cast<size_t>(B) * T, n_in, s)) != FDP_OK) return st;
+    char* sx = sg + w.tc.split_g_bytes;
+    if (!w.short_seq && (st = tc_split(G, sg, static_cast<size_t>(B) * T, n_out, w.tc.planes, nullptr, T, s)) != FDP_OK) return st;
+    if ((st = tc_split(X, sx, static_cast<size_t>(B) * T, n_in, w.tc.planes, nullptr, T, s)) != FDP_OK) return st;
     Gt = sg; Xt = sx; tdt = FDP_BF16;
   }
   if (w.short_seq) {
@@ -294,7 +295,9 @@ int fdp_linear_wgrad(const void* G, const void* X, void* dW, float* norms_out, f
   if (w.tc.ok) {
     float* split_ws = static_cast<float*>(w.tc_extra);
     char* gs = static_cast<char*>(w.tc_extra) + w.tc.split_bytes;
-    if (!w.tc.scaled_epilogue) {
+    if (split && w.short_seq) {     // c_b G in fp32, then its parts
+      if ((st = tc_split(G, gs, static_cast<size_t>(B) * T, n_out, w.tc.planes, w.factors, T, s)) != FDP_OK) return st;
+    } else if (!w.tc.scaled_epilogue) {
       if ((st = tc_prescale(G, w.factors, gs, B, T, n_out, in_dtype, s)) != FDP_OK) return st;
     }
     prof_mark(3, s);
@@ -307,7 +310,7 @@ int fdp_linear_wgrad(const void* G, const void* X, void* dW, float* norms_out, f
     }
     if ((st = tc_clipped_wgrad(w.tc.scaled_epilogue ? Gt : gs, Xt, w.tc.scaled_epilogue ? &fs : nullptr, split_ws,
                                dW, w.status, B, T, n_in, n_out, tdt, out_dtype, layout, inv_div, nk,
-                               s, w.tc.split3 ? 3 : 1)) != FDP_OK) return st;
+                               s, w.tc.planes)) != FDP_OK) return st;
   } else {
     prof_mark(3, s);
     simt_clipped_wgrad(G, X, w.factors, dW, B, T, n_in, n_out, in_dtype, out_dtype, layout, inv_div, nk, s);
@@ -379,9 +382,9 @@ static int gemm3_call(const void* A, const void* W, const void* bias, void* Y, i
   char* w3 = a3 + ((static_cast<size_t>(rows) * K * 4 + 255) & ~static_cast<size_t>(255));
   FDP_CUDA_OK(cudaMemsetAsync(status, 0, sizeof(int), s));
   int st;
-  if ((st = tc_split3(A, a3, static_cast<size_t>(rows), K, s)) != FDP_OK) return st;
+  if ((st = tc_split(A, a3, static_cast<size_t>(rows), K, 2, nullptr, 1, s)) != FDP_OK) return st;
   // W is [K, N] (w_kn) or [N, K]: either way its rows are split along their own columns
-  if ((st = tc_split3(W, w3, static_cast<size_t>(w_kn ? K : N), w_kn ? N : K, s)) != FDP_OK) return st;
+  if ((st = tc_split(W, w3, static_cast<size_t>(w_kn ? K : N), w_kn ? N : K, 2, nullptr, 1, s)) != FDP_OK) return st;
   return tc_gemm3(a3, w3, bias, Y, status, rows, K, N, out_dtype, w_kn, s);
 }
 

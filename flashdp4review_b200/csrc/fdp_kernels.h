@@ -122,15 +122,18 @@ struct TcPlan {
   int nparts;       // norm partials per sample
   bool scaled_epilogue;  // clip factors applied per sample in the GEMM epilogue, no pre-scale pass
   bool short_seq;        // T < SHORT_SEQ: norms by simt_norm_gram_small, clipped sum over the pre-scaled G
-  // fp32 inputs: G and X are first split into high and low bf16 halves ([rows, 2n] each, behind the
-  // parking area in the workspace), and every contraction runs as three bf16 products
-  bool split3;
-  size_t split3_g_bytes, split3_x_bytes;
+  bool any_align;        // takes operands and outputs of any alignment
+  // fp32 inputs (planes > 1): G and X are first split into 2 or 3 bf16 parts ([rows, planes * n] each, n
+  // rounded up to a multiple of 8, behind the parking area in the workspace), and every contraction runs as
+  // three or six bf16 products
+  int planes;
+  size_t split_g_bytes, split_x_bytes;
 };
 TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo);
-// fp32 [rows, n] -> bf16 [rows, 2n]: high halves, then low halves (x - hi rounded to bf16)
-int tc_split3(const void* src, void* dst, size_t rows, int n, cudaStream_t s);
-// With pl.split3, G and X are the split matrices and dt is FDP_BF16.
+// fp32 [rows, n] -> bf16 [rows, planes, n rounded up to 8]: high parts, then what is left of them, ...; row r is
+// multiplied by factors[r / T] first (factors may be null)
+int tc_split(const void* src, void* dst, size_t rows, int n, int planes, const float* factors, int T, cudaStream_t s);
+// With pl.planes > 1, G and X are the split matrices and dt is FDP_BF16.
 int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int B, int T, int n_in,
              int n_out, int dt, const TcPlan& pl, cudaStream_t s);
 // Gs[r,:] = factors[r / T] * G[r,:]
@@ -147,15 +150,15 @@ struct TcFactorSource {
 };
 bool tc_fused_factors_ok(int B);
 // dW = inv_div * sum_b c_b G_b^T X_b + noise over K = B*T.  fs == nullptr: Gs is the pre-scaled copy;
-// otherwise Gs is G itself and c_b is applied per sample in the epilogue.
+// otherwise Gs is G itself and c_b is applied per sample in the epilogue.  planes > 1: G and X are split.
 int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, float* split_ws,
                      void* dW, int* dev_status, int B, int T, int n_in, int n_out, int dt, int out_dt,
-                     int layout, float inv_div, NoiseKey nk, cudaStream_t s, int terms = 1);
+                     int layout, float inv_div, NoiseKey nk, cudaStream_t s, int planes = 1);
 // test aid: one warp waits `limit_cycles` on a barrier nobody arrives on and reports the timeout
 int tc_wait_selftest(int* status, long long limit_cycles, cudaStream_t s);
 bool tc_dgrad_ok(int rows, int n_in, int n_out, int dt);
 // fp32 product Y[rows, N] = A[rows, K] * W (+ bias) as three bf16 tensor-core products over operands split
-// by tc_split3 (A3 [rows, 2K]; W3 [K, 2N] if w_kn, else [N, 2K]); workspace for the two split copies
+// by tc_split (A3 [rows, 2K]; W3 [K, 2N] if w_kn, else [N, 2K]); workspace for the two split copies
 bool tc_gemm3_ok(int rows, int K, int N);
 size_t tc_gemm3_ws_bytes(int rows, int K, int N);
 int tc_gemm3(const void* A3, const void* W3, const void* bias, void* Y, int* dev_status, int rows, int K, int N,

@@ -45,11 +45,14 @@ constexpr int MAX_SMS = 148;           // workers the split-K parking area is si
 // that sample's clip factor, to fp32 registers of eight epilogue warps; G needs no scaled copy.
 // EPI_SPLIT_*: fp32 inputs as bf16 halves, three products per K stage (see TcArgs::plane_a): the clipped sum,
 // a plain product (+ bias), and one sample's product tile squared and summed.
+// EPI_SPLIT6_*: the same with bf16 thirds and six products.
 enum { EPI_STORE = 0, EPI_SUMSQ = 1, EPI_GRAM = 2, EPI_STORE_SCALED = 3, EPI_SPLIT_SCALED = 4, EPI_SPLIT_STORE = 5,
-       EPI_SPLIT_SUMSQ = 6 };
+       EPI_SPLIT_SUMSQ = 6, EPI_SPLIT6_SCALED = 7, EPI_SPLIT6_SUMSQ = 8 };
 __host__ __device__ constexpr bool epi_chained(int epi) { return epi >= EPI_STORE_SCALED; }
-__host__ __device__ constexpr bool epi_split(int epi) { return epi >= EPI_SPLIT_SCALED; }
-__host__ __device__ constexpr bool epi_scaled(int epi) { return epi == EPI_STORE_SCALED || epi == EPI_SPLIT_SCALED; }
+// bf16 parts of an operand
+__host__ __device__ constexpr int epi_planes(int epi) { return epi >= EPI_SPLIT6_SCALED ? 3 : epi >= EPI_SPLIT_SCALED ? 2 : 1; }
+__host__ __device__ constexpr bool epi_scaled(int epi) { return epi == EPI_STORE_SCALED || epi == EPI_SPLIT_SCALED || epi == EPI_SPLIT6_SCALED; }
+__host__ __device__ constexpr bool epi_sumsq(int epi) { return epi == EPI_SPLIT_SUMSQ || epi == EPI_SPLIT6_SUMSQ; }
 __host__ __device__ constexpr bool epi_stores(int epi) { return epi == EPI_STORE || epi_scaled(epi) || epi == EPI_SPLIT_STORE; }
 // eight epilogue warps (two per TMEM lane quarter, 128 columns each) for the store epilogues, four for the norms
 __host__ __device__ constexpr int epi_warps_for(int epi) { return (epi == EPI_STORE || epi_chained(epi)) ? 8 : 4; }
@@ -83,7 +86,7 @@ struct TcArgs {
   // sums then sit on the critical path of a few warps instead of spreading over the whole GPU.)
   int units_full, split;
   float* split_ws;
-  // EPI_STORE_SCALED: K is `segs` segments (samples) of `seg_stages` stages; every segment has its own
+  // EPI_STORE_SCALED: K is `segs` segments (samples; 0: the factors are in the operand, one segment) of `seg_stages` stages; every segment has its own
   // accumulator, scaled by that sample's clip factor when it is drained.  The factors come either from
   // `factors` (global, computed by an earlier kernel) or, when norm_partials != null, from the norm
   // pass's partial sums: the epilogue warps reduce them into shared memory while the first main loop
@@ -105,11 +108,14 @@ struct TcArgs {
   // bf16 halves of the n columns, then the low halves (x = hi + lo up to 2^-18 |x|); plane_a / plane_b is the
   // column offset of the low halves.  A K stage holds all four tiles -- A hi, A lo, B hi, B lo -- and feeds
   // three products, hi*lo, lo*hi and hi*hi, into the same accumulator (lo*lo, 2^-18 of the product, is
-  // dropped): four tile loads for three products instead of six.
+  // dropped): four tile loads for three products instead of six.  EPI_SPLIT6_*: [rows, 3n], x = hi + mid + lo
+  // up to 2^-27 |x|, and the six products down to 2^-18 (what is dropped is below 2^-26): fp32 accuracy.
   int plane_a, plane_b;
   // store GEMMs: tiles are walked in groups of m_group tile rows (0 = plain order), so that the CTAs
   // running together cover a squarer patch of the output and re-read less of the operands
   int m_group;
+  // the output cannot be written by the copy engine (row pitch or base not a multiple of 16 bytes)
+  int direct_out;
 };
 
 // ---- PTX wrappers (mbarrier helpers live in fdp_async.cuh) --------------------------------------------
@@ -117,6 +123,11 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar) : "memory");
 }
 // ---- CTA-pair (cta_group::2) helpers: the even CTA of a 2-CTA cluster issues one 256-row MMA for both;
 // loads are per CTA (no multicast), completion is signalled on the leader's mbarrier ------------------
@@ -142,6 +153,11 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(leader_bar) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t leader_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(leader_bar) : "memory");
 }
 __device__ __forceinline__ void tc_commit_pair(uint32_t cluster_bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar) : "memory");
@@ -294,6 +310,30 @@ __device__ __forceinline__ void store_out32(const TcArgs& args, uint32_t box, co
   if ((c4 & 1) == 1) box_send(box, map, col0 + 64 * (c4 >> 1), row, lane);
 }
 
+// 32 columns of an output that the copy engine cannot write: through the box all the same, then row by row, so
+// that an instruction writes 32 adjacent elements.  The noise is drawn per element here: a row pitch that is no
+// multiple of four puts an element group across rows.
+__device__ __forceinline__ void store_rows32(const TcArgs& args, uint32_t box, const float v[32], int n, int row, int lane,
+                                             bool noise) {
+  box_wait(lane);       // a parked part may still be on its way out of the box
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    box_put(box, lane, j, __float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]), __float_as_uint(v[4 * j + 2]),
+            __float_as_uint(v[4 * j + 3]));
+  __syncwarp();
+  const int rows = min(BOX_ROWS, args.M - row);
+  for (int r = 0; r < rows; ++r) {
+    float x;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x)
+                 : "r"(box + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4) : "memory");
+    if (n + lane < args.N) {
+      const size_t idx = static_cast<size_t>(row + r) * args.ld_out + n + lane;
+      if (noise) x += noise_at(args.nk, idx);
+      store_as(args.out, args.out_dt, idx, x);
+    }
+  }
+}
+
 // accr[4g .. 4g+3] += z * f with g known only at run time: a switch keeps every index static, so
 // the 128 accumulators stay in registers.
 __device__ __forceinline__ void add_group(float (&accr)[128], int g, const float z[4], float f) {
@@ -320,7 +360,7 @@ __global__ void __launch_bounds__(threads_for(EPI), 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB2,
                const __grid_constant__ CUtensorMap tmOut, const __grid_constant__ TcArgs args) {
-  constexpr int PLANES = epi_split(EPI) ? 2 : 1;         // bf16 halves of fp32 operands
+  constexpr int PLANES = epi_planes(EPI);                // bf16 parts of fp32 operands
   constexpr int NST = ((CTAS == 2) ? 6 : STAGES) / PLANES;   // ring depth
   constexpr int A_BYTES = PLANES * A_STAGE_BYTES;
   constexpr int B_BYTES = B_STAGE_BYTES / CTAS;          // this CTA's share of (one half of) the B stage
@@ -350,6 +390,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const WaitCtx wctx{abort_flag, args.status, args.sticky, WAIT_LIMIT_CYCLES};
 
   constexpr int NUM_ACC = (EPI == EPI_GRAM) ? 1 : 2;
+  // six products: accumulator hand-offs per K stage.  In the norm pass the truncation of the accumulators does not
+  // average out over the elements (it shrinks all of them), so its chains hold two large steps instead of four.
+  constexpr int SUBS = (EPI == EPI_SPLIT6_SUMSQ) ? 2 : 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int total_tiles = args.batch * args.tiles_per_batch;
   const int kst_total = args.k_stages + (EPI == EPI_GRAM ? args.k_stages2 : 0);
@@ -459,6 +502,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         decode_unit(u, tile, ks0, ks1, slot);
         decode(tile, b, m0, n0, half);
         const int row0 = b * args.batch_rows;
+        // K range along the rows: sample z, row t of it.  The maps are three-dimensional (column, row of the
+        // sample, sample), so the rows a sample's last stage is short of read as zeros, whatever its length.
+        int z = 0, t = 0;
+        if (A_MN && B_MN) { z = b + ks0 / args.seg_stages; t = ks0 % args.seg_stages * BK; }
         for (int ks = ks0; ks < ks1; ++ks) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, wctx, 1)) { ok = false; break; }
           const bool second = (EPI == EPI_GRAM) && ks >= args.k_stages;
@@ -484,22 +531,32 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             auto load = [&](uint32_t dst, const CUtensorMap* map, int c0, int c1) {
               if (CTAS == 1) tma_load_2d(dst, map, c0, c1, lbar); else tma_load_2d_pair(dst, map, c0, c1, lbar);
             };
+            auto load3 = [&](uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2) {
+              if (CTAS == 1) tma_load_3d(dst, map, c0, c1, c2, lbar); else tma_load_3d_pair(dst, map, c0, c1, c2, lbar);
+            };
 #pragma unroll
             for (int pl = 0; pl < PLANES; ++pl) {
               const int ca = pl * args.plane_a, cb = pl * args.plane_b;
               const uint32_t da = sa + pl * A_STAGE_BYTES, db = sb + pl * B_BYTES;
               if (A_MN) {
 #pragma unroll
-                for (int i = 0; i < BM / 64; ++i) load(da + i * (BK * 128), ma, m0 + 64 * i + ca, row0 + k0);
+                for (int i = 0; i < BM / 64; ++i) load3(da + i * (BK * 128), ma, m0 + 64 * i + ca, t, z);
               } else {
-                load(da, ma, k0 + ca, row0 + m0);
+                load(da, ma, k0 + ca, m0);
               }
               if (B_MN) {
 #pragma unroll
-                for (int j = 0; j < BN_CTA / 64; ++j) load(db + j * (BK * 128), mb, nb0 + 64 * j + cb, row0 + k0);
+                for (int j = 0; j < BN_CTA / 64; ++j) {
+                  if (A_MN) load3(db + j * (BK * 128), mb, nb0 + 64 * j + cb, t, z);
+                  else load(db + j * (BK * 128), mb, nb0 + 64 * j + cb, k0);
+                }
               } else {
-                load(db, mb, k0 + cb, row0 + nb0);
+                load(db, mb, k0 + cb, nb0);
               }
+            }
+            if (A_MN && B_MN) {
+              t += BK;
+              if (t >= args.seg_stages * BK) { t = 0; ++z; }
             }
           }
           if (++stage == NST) { stage = 0; phase ^= 1u; }
@@ -516,6 +573,28 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
   } else if (warp == 1) {
     // ================= MMA issuer (the leader CTA of a pair issues for both) =================
+    auto commit = [&](uint32_t bar) {   // signals `bar` (in both CTAs of a pair) when the MMAs issued so far are done
+      if (CTAS == 1) {
+        tc_commit(bar);
+      } else {
+        tc_commit_pair(bar);
+        tc_commit_pair(mapa_u32(bar, 1));
+      }
+    };
+    // The six products of K slices [k0, k1) of a stage, smallest first: the accumulator is added to by truncation,
+    // one unit in its last place per step, so the steps that come before it is large cost nothing.
+    auto issue_six = [&](uint32_t d, uint32_t sa, uint32_t idesc, int k0, int k1, bool fresh) {
+      constexpr int PA[6] = {0, 2, 1, 0, 1, 0}, PB[6] = {2, 0, 1, 1, 0, 0};   // hi*lo, lo*hi, mid*mid, hi*mid, mid*hi, hi*hi
+      const uint32_t sb = sa + A_BYTES;
+#pragma unroll
+      for (int q = 0; q < 6; ++q)
+        for (int k16 = k0; k16 < k1; ++k16) {
+          const uint64_t da = operand_desc<A_MN>(sa + PA[q] * A_STAGE_BYTES, k16);
+          const uint64_t db = operand_desc<B_MN>(sb + PB[q] * B_BYTES, k16);
+          const uint32_t acc_in = (fresh && k16 == k0 && q == 0) ? 0u : 1u;
+          if (CTAS == 1) tc_mma(d, da, db, idesc, acc_in); else tc_mma_pair(d, da, db, idesc, acc_in);
+        }
+    };
     if (lane == 0 && is_leader) {
       int stage = 0; uint32_t phase = 0;
       int it = 0;
@@ -528,6 +607,21 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const uint32_t idesc = half ? args.idesc_half : args.idesc;
         int ks = ks0;
         // one accumulator per segment: the whole unit, or one sample's share of it for EPI_STORE_SCALED
+        if constexpr (SUBS > 1) {
+          for (; ks < ks1 && ok; ++ks) {
+            if (!mbar_wait(full_bar(stage), phase, wctx, 3)) { ok = false; break; }
+            for (int sub = 0; sub < SUBS; ++sub, ++it) {
+              const int acc = it % NUM_ACC;
+              if (!mbar_wait(tempty_bar(acc), ((it / NUM_ACC) & 1u) ^ 1u, wctx, 2)) { ok = false; break; }
+              tc_fence_after();
+              issue_six(tmem_base + acc * BN, base + stage * STG, idesc, sub * (4 / SUBS), (sub + 1) * (4 / SUBS), true);
+              commit(tfull_bar(acc));
+            }
+            if (!ok) break;
+            commit(empty_bar(stage));
+            if (++stage == NST) { stage = 0; phase ^= 1u; }
+          }
+        }
         while (ks < ks1 && ok) {
           const int seg_begin = ks;
           const int seg_end = epi_chained(EPI) ? segment_end(ks, ks1) : ks1;
@@ -547,32 +641,26 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               if (tn0 == tm0) sa = sb;
               else if (gram_n1 == tm0) sa = sb + B_STAGE_BYTES / 2;
             }
+            if constexpr (PLANES == 3) {
+              issue_six(d, sa, idesc, 0, BK / UMMA_K, first_stage);
+            } else {
 #pragma unroll
-            for (int k16 = 0; k16 < BK / UMMA_K; ++k16) {
+              for (int k16 = 0; k16 < BK / UMMA_K; ++k16) {
 #pragma unroll
-              for (int q = 0; q < (PLANES == 2 ? 3 : 1); ++q) {   // hi*lo, lo*hi, hi*hi
-                const uint64_t da = operand_desc<A_MN>(sa + (PLANES == 2 && q == 1 ? A_STAGE_BYTES : 0), k16);
-                const uint64_t db = operand_desc<B_MN>(sb + (PLANES == 2 && q == 0 ? B_BYTES : 0), k16);
-                const uint32_t acc_in = (first_stage && k16 == 0 && q == 0) ? 0u : 1u;
-                if (CTAS == 1) tc_mma(d, da, db, idesc, acc_in); else tc_mma_pair(d, da, db, idesc, acc_in);
+                for (int q = 0; q < (PLANES == 2 ? 3 : 1); ++q) {   // hi*lo, lo*hi, hi*hi
+                  const uint64_t da = operand_desc<A_MN>(sa + (PLANES == 2 && q == 1 ? A_STAGE_BYTES : 0), k16);
+                  const uint64_t db = operand_desc<B_MN>(sb + (PLANES == 2 && q == 0 ? B_BYTES : 0), k16);
+                  const uint32_t acc_in = (first_stage && k16 == 0 && q == 0) ? 0u : 1u;
+                  if (CTAS == 1) tc_mma(d, da, db, idesc, acc_in); else tc_mma_pair(d, da, db, idesc, acc_in);
+                }
               }
             }
             // frees the stage (in both CTAs of a pair) once these MMAs have read it
-            if (CTAS == 1) {
-              tc_commit(empty_bar(stage));
-            } else {
-              tc_commit_pair(empty_bar(stage));
-              tc_commit_pair(mapa_u32(empty_bar(stage), 1));
-            }
+            commit(empty_bar(stage));
             if (++stage == NST) { stage = 0; phase ^= 1u; }
           }
           if (ok) {
-            if (CTAS == 1) {
-              tc_commit(tfull_bar(acc));
-            } else {
-              tc_commit_pair(tfull_bar(acc));
-              tc_commit_pair(mapa_u32(tfull_bar(acc), 1));
-            }
+            commit(tfull_bar(acc));
             ++it;
           }
         }
@@ -626,18 +714,18 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // A whole tile's Gaussian noise goes into the accumulators a few element groups per sample
         // segment, in the time these warps would otherwise wait for the next segment's MMAs; K-split
         // parts stay noise-free (the fix-up kernel adds the noise once per tile).
-        const bool pre_noise = epi_scaled(EPI) && slot < 0 && args.nk.std != 0.f && m < args.M;
+        const bool pre_noise = epi_scaled(EPI) && slot < 0 && args.nk.std != 0.f && m < args.M && !args.direct_out;
         const uint64_t g0 = (static_cast<uint64_t>(m) * args.ld_out + n0 + chalf * 128) >> 2;
         const int nseg = segment_index(ks1 - 1) - segment_index(ks0) + 1;
         int ng = 0, seg = 0;
-        for (int ks = ks0; ks < ks1 && ok; ks = segment_end(ks, ks1), ++it) {
+        for (int ks = ks0, sub = 0; ks < ks1 && ok; ++it) {
           const int acc = it % NUM_ACC;
           const uint32_t acc_phase = (it / NUM_ACC) & 1u;
           if (!mbar_wait_warp(tfull_bar(acc), acc_phase, wctx, 4)) { ok = false; break; }
           tc_fence_after();
           const int sample = ks / args.seg_stages;
           // the divisor goes into the factor, so the noise is added as it is drawn
-          const float cbs = !epi_scaled(EPI) ? args.scale
+          const float cbs = !epi_scaled(EPI) || args.segs == 0 ? args.scale
                           : (args.norm_partials != nullptr ? sfac[sample] : __ldg(args.factors + sample)) * args.scale;
           const uint32_t tb = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN + chalf * 128;
 #pragma unroll
@@ -654,6 +742,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (CTAS == 1 || is_leader) mbar_arrive(tempty_bar(acc));
             else mbar_arrive_cluster(mapa_u32(tempty_bar(acc), 0));
           }
+          if (++sub == SUBS) { sub = 0; ks = segment_end(ks, ks1); }
           ++seg;
           if (epi_scaled(EPI) && pre_noise) {
             const int target = (32 * seg) / nseg;
@@ -665,14 +754,17 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
         }
         if (!ok) break;
-        if constexpr (EPI == EPI_SPLIT_SUMSQ) {
+        if constexpr (epi_sumsq(EPI)) {
           // the unit is one sample's product tile: its squares, without the rows and columns past the
           // matrix (with split operands a tile that overhangs reads the other half's columns, not zeros)
           float part = 0.f;
           const int nb = n0 + chalf * 128;
           if (m < args.M) {
 #pragma unroll
-            for (int i = 0; i < 128; ++i) part = fmaf((nb + i < args.N) ? accr[i] : 0.f, accr[i], part);
+            for (int i = 0; i < 128; ++i) {
+              const float a = (nb + i < args.N) ? accr[i] : 0.f;
+              part = fmaf(a, a, part);
+            }
           }
           part = warp_sum(part);
           if (lane == 0) args.partials[(static_cast<size_t>(tile) * CTAS + cta_rank) * EPI_WARPS + ew] = part;
@@ -682,7 +774,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             for (int c4 = 0; c4 < 4; ++c4) {
               const int n = n0 + chalf * 128 + c4 * 32;
               if (EPI == EPI_SPLIT_STORE && args.bias != nullptr && n < args.N) add_bias32(args, n, accr + c4 * 32);
-              store_out32(args, box, &tmOut, accr + c4 * 32, c4, n0 + chalf * 128, m0 + quarter * 32, lane);
+              if (args.direct_out) store_rows32(args, box, accr + c4 * 32, n, m0 + quarter * 32, lane, epi_scaled(EPI) && args.nk.std != 0.f);
+              else store_out32(args, box, &tmOut, accr + c4 * 32, c4, n0 + chalf * 128, m0 + quarter * 32, lane);
             }
           }
         } else {
@@ -828,10 +921,15 @@ __global__ void __launch_bounds__(256) splitk_fixup_kernel(const float* __restri
   }
   float v[4] = {acc.x * scale, acc.y * scale, acc.z * scale, acc.w * scale};
   const size_t idx0 = static_cast<size_t>(m) * ld_out + n;
-  if (nk.std != 0.f) {   // idx0 is a multiple of 4: the row pitch and n are
-    float z[4];
-    noise_group(nk, idx0 >> 2, z);
-    v[0] += z[0]; v[1] += z[1]; v[2] += z[2]; v[3] += z[3];
+  if (nk.std != 0.f) {
+    if ((idx0 & 3) == 0) {
+      float z[4];
+      noise_group(nk, idx0 >> 2, z);
+      v[0] += z[0]; v[1] += z[1]; v[2] += z[2]; v[3] += z[3];
+    } else {     // a row pitch that is no multiple of four
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] += noise_at(nk, idx0 + j);
+    }
   }
   for (int j = 0; j < 4; ++j)
     if (n + j < N) store_as(out, out_dt, idx0 + j, v[j]);
@@ -854,25 +952,38 @@ __global__ void __launch_bounds__(256) prescale_kernel(const Tin* __restrict__ G
   }
 }
 
-// ---- fp32 -> (hi, lo) bf16 halves: dst[r, c] = bf16(x), dst[r, n + c] = bf16(x - hi) ---------------------
-__global__ void __launch_bounds__(256) split3_kernel(const float4* __restrict__ src, uint2* __restrict__ dst,
-                                                     size_t nvec, int vec_per_row) {
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < nvec;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const float4 v = __ldg(src + i);
-    const float f[4] = {v.x, v.y, v.z, v.w};
-    uint16_t hi[4], lo[4];
+// ---- fp32 -> PLANES bf16 parts: dst[r, 0, c] = bf16(f x), dst[r, 1, c] = bf16(f x - hi), ..., with the column
+// count rounded up to a multiple of 8 (zeros) and f a per-sample factor (1 when factors is null) --------------
+template <int PLANES, bool VEC>
+__global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ src, uint4* __restrict__ dst, unsigned nvec,
+                                                    int n, unsigned vec_per_row, const float* __restrict__ factors, int T) {
+  for (unsigned i = blockIdx.x * 256u + threadIdx.x; i < nvec; i += gridDim.x * 256u) {
+    const unsigned row = i / vec_per_row, cv = i - row * vec_per_row;
+    const int c0 = static_cast<int>(cv) * 8;
+    const float* p = src + static_cast<size_t>(row) * n + c0;
+    float f[8];
+    if (VEC) {     // n a multiple of 4, 16-byte aligned
+      unpack16<float>(__ldg(reinterpret_cast<const uint4*>(p)), f);
+      unpack16<float>(c0 + 4 < n ? __ldg(reinterpret_cast<const uint4*>(p) + 1) : make_uint4(0, 0, 0, 0), f + 4);
+    } else {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const __nv_bfloat16 h = __float2bfloat16_rn(f[e]);
-      const __nv_bfloat16 l = __float2bfloat16_rn(f[e] - __bfloat162float(h));
-      hi[e] = *reinterpret_cast<const uint16_t*>(&h);
-      lo[e] = *reinterpret_cast<const uint16_t*>(&l);
+      for (int e = 0; e < 8; ++e) f[e] = c0 + e < n ? __ldg(p + e) : 0.f;
     }
-    const size_t row = i / vec_per_row, cv = i - row * vec_per_row;
-    uint2* o = dst + row * (2 * static_cast<size_t>(vec_per_row)) + cv;
-    o[0] = make_uint2(hi[0] | (static_cast<uint32_t>(hi[1]) << 16), hi[2] | (static_cast<uint32_t>(hi[3]) << 16));
-    o[vec_per_row] = make_uint2(lo[0] | (static_cast<uint32_t>(lo[1]) << 16), lo[2] | (static_cast<uint32_t>(lo[3]) << 16));
+    if (factors != nullptr) {
+      const float c = __ldg(factors + row / T);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] *= c;
+    }
+    uint4* o = dst + static_cast<size_t>(row) * (PLANES * vec_per_row) + cv;
+#pragma unroll
+    for (int pl = 0; pl < PLANES; ++pl) {
+      const uint4 h = pack16<__nv_bfloat16>(f);
+      o[pl * vec_per_row] = h;
+      float hf[8];
+      unpack16<__nv_bfloat16>(h, hf);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] -= hf[e];
+    }
   }
 }
 
@@ -912,6 +1023,22 @@ bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, ui
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
+
+// [B * T, cols] as (column, row of the sample, sample), for K ranges that run over the rows: boxes of 64 x BK
+bool make_rows_map(CUtensorMap* m, const void* base, int B, uint64_t T, uint64_t cols, int dt) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return false;
+  const cuuint64_t dims[3] = {cols, T, static_cast<cuuint64_t>(B)};
+  const cuuint64_t strides[2] = {cols * 2, cols * 2 * T};
+  const cuuint32_t box[3] = {64, BK, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = fn(m, dt == FDP_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
+                        const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS;
+}
+int pitch8(int n) { return (n + 7) & ~7; }     // columns of one part in a split copy
 
 // Map of an output matrix [rows, cols] for the epilogue warps' boxes of 32 rows x 128 bytes.  The row pitch
 // has to be a multiple of 16 bytes and the base 16-byte aligned.
@@ -1036,8 +1163,8 @@ int ctas_per_tile() { return forced_ctas() == 1 ? 1 : 2; }
 // the larger layers do pay.
 int plan_tail_split(int total_tiles, int k_stages, int workers, int products) {
   const int rem = total_tiles <= workers ? total_tiles : total_tiles % workers;
-  // stages are counted by their work: with split fp32 operands one holds three products
-  const int min_stages = products == 3 ? 3 : 8;      // shortest part
+  // stages are counted by their work: with split fp32 operands one holds three or six products
+  const int min_stages = products == 6 ? 2 : products == 3 ? 3 : 8;      // shortest part
   if (rem == 0 || k_stages < 4 * min_stages) return 1;
   // FDP_TC_SPLIT=n forces the number of parts (measurements), within the same limits
   static const int forced = [] { const char* e = getenv("FDP_TC_SPLIT"); return e ? atoi(e) : 0; }();
@@ -1084,7 +1211,9 @@ int tc_wait_selftest(int* status, long long limit_cycles, cudaStream_t s) {
 // four): FDP_TC_CHAIN_STAGES, default 2.  B=8, T=1024, 4096x4096 against float64, 1 / 2 / 3 / 4 / 8 stages:
 // norms off by 2.0e-7 / 3.8e-7 / 5.2e-7 / 7.3e-7 / 1.4e-6 (the truncation of the accumulators grows with the
 // chain); B=8, T=1024, 1024->3072, all kernels of a forward and backward: 832 / 636 / 616 / 592 / 588 us.
-static int chain_stages(int seg_stages) {
+// Six products (24 steps a stage, of which only the four of hi*hi meet a large accumulator): one stage.
+static int chain_stages(int seg_stages, int planes) {
+  if (planes == 3) return 1;
   static const int cap = [] {
     const char* e = getenv("FDP_TC_CHAIN_STAGES");
     const int v = e ? atoi(e) : 2;
@@ -1093,28 +1222,57 @@ static int chain_stages(int seg_stages) {
   return cap < seg_stages ? cap : seg_stages;
 }
 
+// fp32 shapes of FDP_FP32_TENSOR's three products: whole 64-column and 64-row K stages, at least 128 of everything
+static bool three_products_ok(int T, int n_in, int n_out) {
+  return n_in % BK == 0 && n_out % BK == 0 && n_in >= 128 && n_out >= 128 && T % BK == 0 && T >= 2 * BK;
+}
+
+// ... and of FDP_FP32_WIDE's six
+static bool wide_ok(int B, int T, int n_in, int n_out, int norm_algo) {
+  if (n_in < 64 || n_out < 64) return false;
+  // (below 128 rows in all the FMA kernels' K loop is shorter than the extra launches: 64 samples of one row,
+  // 256 -> 256, 43 us a call against 52; 210 rows, 1024 -> 4096, 122 against 77)
+  return T >= SHORT_SEQ || (norm_algo != FDP_NORM_DIRECT && static_cast<long long>(B) * T >= 128);
+}
+
 // The tensor-core path needs 16-bit inputs, row pitches that are multiples of 16 bytes, and
 // matrices large enough that the 128x256 tile is not mostly padding.
 TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
   TcPlan p; p.ok = false; p.algo = FDP_NORM_DIRECT; p.ws_bytes = 0; p.nparts = 0; p.scaled_epilogue = false;
-  p.short_seq = false; p.split_bytes = 0;
-  p.split3 = false; p.split3_g_bytes = p.split3_x_bytes = 0;
-  const bool fp32_tensor = (norm_algo & FDP_FP32_TENSOR) != 0;
+  p.short_seq = false; p.any_align = false; p.split_bytes = 0;
+  p.planes = 1; p.split_g_bytes = p.split_x_bytes = 0;
+  const bool fp32_tensor = (norm_algo & FDP_FP32_TENSOR) != 0, fp32_wide = (norm_algo & FDP_FP32_WIDE) != 0;
   norm_algo &= FDP_NORM_MASK;
   if (dt == FDP_F32) {
-    // fp32 on the tensor cores as three bf16 products (hi*hi + hi*lo + lo*hi, fp32 accumulation), when
-    // the caller asks for it (FDP_FP32_TENSOR).  The tensor cores add into their fp32 accumulators by
-    // truncation, a one-sided error of about 2^-24 per K=16 step, so no accumulator runs for more than
-    // a few K stages: it is handed to the epilogue warps, which add it to registers with
-    // round-to-nearest (chain_stages).  Needs whole 64-column K stages per half, samples made of whole
-    // 64-row stages, and the per-sample epilogue (a pre-scaled copy would round c_b * G to bf16 again).
-    if (!fp32_tensor || n_in % BK != 0 || n_out % BK != 0 || n_in < 128 || n_out < 128 || T % BK != 0 || T < 2 * BK) return p;
-    p.split3 = true;
-    p.split3_g_bytes = align256(static_cast<size_t>(B) * T * n_out * 4);
-    p.split3_x_bytes = align256(static_cast<size_t>(B) * T * n_in * 4);
-  } else if (dt != FDP_BF16 && dt != FDP_F16) {
+    // fp32 on the tensor cores, when the caller asks for it.  FDP_FP32_TENSOR: three bf16 products (hi*hi +
+    // hi*lo + lo*hi).  FDP_FP32_WIDE: six products over three parts for the shapes the former does not take --
+    // any width (the split copies have padded rows), any T -- because those ran on FMA kernels and their
+    // results are to be no further from float64 than FMA ones.  The tensor cores add into their fp32
+    // accumulators by truncation, a one-sided error of about 2^-24 per K=16 step, so no accumulator runs for
+    // more than a few K stages: it is handed to the epilogue warps, which add it to registers with
+    // round-to-nearest (chain_stages).  The clip factors are applied there per sample (or, for short
+    // sequences, in fp32 before the split: a pre-scaled bf16 copy would round c_b * G).
+    if (fp32_tensor && three_products_ok(T, n_in, n_out)) p.planes = 2;
+    else if (fp32_wide && wide_ok(B, T, n_in, n_out, norm_algo)) p.planes = 3;
+    else return p;
+    p.any_align = p.planes == 3;
+    p.split_g_bytes = align256(static_cast<size_t>(B) * T * pitch8(n_out) * 2 * p.planes);
+    p.split_x_bytes = align256(static_cast<size_t>(B) * T * pitch8(n_in) * 2 * p.planes);
+    p.split_bytes = split_ws_bytes();
+    p.ws_bytes = p.split_bytes + p.split_g_bytes + p.split_x_bytes;
+    if (T < SHORT_SEQ) {
+      p.ok = true; p.algo = FDP_NORM_GRAM; p.short_seq = true; p.nparts = 1;
+      return p;
+    }
+    // always the product form, accumulated in short chains (tc_norms); the Gram form needs both T x T tiles
+    // complete in TMEM before its epilogue can multiply them, i.e. one chain of 3 * (in + out) / 16
+    // truncating additions.  The chained norm pass: tiles of the clipped-sum GEMM, eight epilogue warps per CTA
+    const int ctas = ctas_per_tile();
+    p.ok = true; p.algo = FDP_NORM_DIRECT; p.scaled_epilogue = true;
+    p.nparts = ceil_div(n_out, BM * ctas) * ceil_div(n_in, BN) * ctas * epi_warps_for(EPI_STORE_SCALED);
     return p;
   }
+  if (dt != FDP_BF16 && dt != FDP_F16) return p;
   if (n_in % 8 != 0 || n_out % 8 != 0 || n_in < 128 || n_out < 128) return p;
   if (T < SHORT_SEQ) {
     // short sequences: the norms come from the small Gram kernel (one partial per sample); the
@@ -1134,84 +1292,88 @@ TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
   constexpr long long PLAN_SMS = 148, UNIT_FIXED_STAGES = 4;
   const long long units_d = static_cast<long long>(B) * ceil_div(n_out, BM) * ceil_div(n_in, BN);
   const long long units_g = static_cast<long long>(B) * gram_tiles(T);
-  const int terms = p.split3 ? 3 : 1;
-  const double direct = static_cast<double>((units_d + PLAN_SMS - 1) / PLAN_SMS) * (terms * ceil_div(T, BK) + UNIT_FIXED_STAGES);
+  const double direct = static_cast<double>((units_d + PLAN_SMS - 1) / PLAN_SMS) * (ceil_div(T, BK) + UNIT_FIXED_STAGES);
   const double gram = static_cast<double>((units_g + PLAN_SMS - 1) / PLAN_SMS) *
-                      (terms * (ceil_div(n_in, BK) + ceil_div(n_out, BK)) + UNIT_FIXED_STAGES);
+                      (ceil_div(n_in, BK) + ceil_div(n_out, BK) + UNIT_FIXED_STAGES);
   int algo = norm_algo;
   if (algo == FDP_NORM_AUTO) algo = (direct_ok && direct <= gram) ? FDP_NORM_DIRECT : FDP_NORM_GRAM;
   if (algo == FDP_NORM_DIRECT && !direct_ok) algo = FDP_NORM_GRAM;
-  // split operands: always the product form, accumulated in short chains (tc_norms); the Gram form
-  // needs both T x T tiles complete in TMEM before its epilogue can multiply them, i.e. one chain of
-  // 3 * (in + out) / 16 truncating additions
-  if (p.split3) algo = FDP_NORM_DIRECT;
   p.ok = true;
   p.algo = algo;
   // clip factors applied in the GEMM epilogue (no scaled copy of G) when every 64-row K stage lies
   // inside one sample and a sample's main loop is long enough to hide the per-sample drain;
   // FDP_WGRAD_PRESCALE=1 forces the pre-scale pass (for A/B measurements)
   static const bool force_prescale = [] { const char* e = getenv("FDP_WGRAD_PRESCALE"); return e && e[0] == '1'; }();
-  p.scaled_epilogue = p.split3 || (!force_prescale && (T % BK == 0) && T >= 256);
+  p.scaled_epilogue = !force_prescale && (T % BK == 0) && T >= 256;
   // one partial per work unit and epilogue warp
   p.nparts = 4 * ((algo == FDP_NORM_DIRECT) ? ceil_div(n_out, BM) * ceil_div(n_in, BN) : gram_tiles(T));
-  if (p.split3) {   // the chained norm pass: tiles of the clipped-sum GEMM, eight epilogue warps per CTA
-    const int ctas = ctas_per_tile();
-    p.nparts = ceil_div(n_out, BM * ctas) * ceil_div(n_in, BN) * ctas * epi_warps_for(EPI_STORE_SCALED);
-  }
   // the parked accumulators of the split-K tail, then (pre-scale path only) the c_b-scaled copy of G
   p.split_bytes = split_ws_bytes();
-  p.ws_bytes = p.split_bytes + (p.scaled_epilogue ? 0 : align256(static_cast<size_t>(B) * T * n_out * 2)) +
-               p.split3_g_bytes + p.split3_x_bytes;
+  p.ws_bytes = p.split_bytes + (p.scaled_epilogue ? 0 : align256(static_cast<size_t>(B) * T * n_out * 2));
   return p;
 }
 
-int tc_split3(const void* src, void* dst, size_t rows, int n, cudaStream_t s) {
-  const size_t nvec = rows * n / 4;
-  size_t blocks = (nvec + 255) / 256;
-  const size_t cap = static_cast<size_t>(sm_count()) * 16;
-  split3_kernel<<<static_cast<unsigned>(blocks < cap ? blocks : cap), 256, 0, s>>>(
-      static_cast<const float4*>(src), static_cast<uint2*>(dst), nvec, n / 4);
-  note_launch();
+int tc_split(const void* src, void* dst, size_t rows, int n, int planes, const float* factors, int T, cudaStream_t s) {
+  const unsigned vpr = pitch8(n) / 8;
+  const bool vec = n % 4 == 0 && aligned16(src);
+  const size_t max_rows = (1u << 31) / vpr;       // 32-bit index arithmetic within a launch
+  for (size_t r = 0; r < rows; r += max_rows) {
+    const size_t nr = rows - r < max_rows ? rows - r : max_rows;
+    if (r != 0 && factors != nullptr) return FDP_ERR_SHAPE;     // (factors come with short sequences only)
+    const unsigned nvec = static_cast<unsigned>(nr) * vpr;
+    const unsigned blocks = (nvec + 255) / 256, cap = static_cast<unsigned>(sm_count()) * 16;
+    const unsigned grid = blocks < cap ? blocks : cap;
+    const float* in = static_cast<const float*>(src) + r * n;
+    uint4* out = static_cast<uint4*>(dst) + r * vpr * planes;
+#define FDP_SPLIT(P_, V_) split_kernel<P_, V_><<<grid, 256, 0, s>>>(in, out, nvec, n, vpr, factors, T)
+    if (planes == 2) { if (vec) FDP_SPLIT(2, true); else FDP_SPLIT(2, false); }
+    else { if (vec) FDP_SPLIT(3, true); else FDP_SPLIT(3, false); }
+#undef FDP_SPLIT
+    note_launch();
+  }
   return cudaPeekAtLastError() == cudaSuccess ? FDP_OK : (cudaGetLastError(), FDP_ERR_LAUNCH);
 }
 
 int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int B, int T, int n_in,
              int n_out, int dt, const TcPlan& pl, cudaStream_t s) {
   const uint64_t rows = static_cast<uint64_t>(B) * T;
-  const int wo = pl.split3 ? 2 * n_out : n_out, wi = pl.split3 ? 2 * n_in : n_in;   // matrix widths
   CUtensorMap a, b, a2, b2;
   TcArgs args{};
   args.batch = B; args.batch_rows = T; args.partials = partials; args.status = dev_status; args.T = T;
   args.zero_status = 1;      // the norm pass is the first launch of a weight-gradient call
-  if (pl.split3) {
+  if (pl.planes > 1) {
     // fp32 inputs: the per-sample products G_b^T X_b themselves, on the tiles and CTA pairs of the
     // clipped-sum GEMM, handed to the epilogue every few K stages and summed there in registers; a
     // unit is (sample, tile) and ends with the sum of its squares instead of a store
-    if (!make_map(&a, G, rows, wo, 64, BK, dt) || !make_map(&b, X, rows, wi, 64, BK, dt)) return FDP_ERR_LAUNCH;
+    const int po = pitch8(n_out), pi = pitch8(n_in);
+    if (!make_rows_map(&a, G, B, T, pl.planes * po, dt) || !make_rows_map(&b, X, B, T, pl.planes * pi, dt)) return FDP_ERR_LAUNCH;
     const int ctas = ctas_per_tile();
     args.M = n_out; args.N = n_in; args.ld_out = n_in;
     args.tiles_m = ceil_div(n_out, BM * ctas); args.tiles_n = ceil_div(n_in, BN);
     args.tiles_per_batch = args.tiles_m * args.tiles_n;
-    args.k_stages = T / BK;
-    args.plane_a = n_out; args.plane_b = n_in;
+    args.k_stages = ceil_div(T, BK);
+    args.plane_a = po; args.plane_b = pi;
     args.idesc = make_idesc(dt, true, true, ctas);
-    args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = chain_stages(args.seg_stages);
+    args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = chain_stages(args.seg_stages, pl.planes);
     args.scale = 1.0f; args.nk = NoiseKey{};
+    if (pl.planes == 3)
+      return ctas == 2 ? launch<true, true, EPI_SPLIT6_SUMSQ, 2>(a, b, a, b, a, args, s)
+                       : launch<true, true, EPI_SPLIT6_SUMSQ, 1>(a, b, a, b, a, args, s);
     return ctas == 2 ? launch<true, true, EPI_SPLIT_SUMSQ, 2>(a, b, a, b, a, args, s)
                      : launch<true, true, EPI_SPLIT_SUMSQ, 1>(a, b, a, b, a, args, s);
   }
   if (pl.algo == FDP_NORM_DIRECT) {
-    if (!make_map(&a, G, rows, wo, 64, BK, dt) || !make_map(&b, X, rows, wi, 64, BK, dt)) return FDP_ERR_LAUNCH;
+    if (!make_rows_map(&a, G, B, T, n_out, dt) || !make_rows_map(&b, X, B, T, n_in, dt)) return FDP_ERR_LAUNCH;
     args.M = n_out; args.N = n_in;
     args.tiles_m = ceil_div(n_out, BM); args.tiles_n = ceil_div(n_in, BN);
     args.tiles_per_batch = args.tiles_m * args.tiles_n;
-    args.k_stages = T / BK;
+    args.k_stages = T / BK; args.seg_stages = args.k_stages;
     args.idesc = make_idesc(dt, true, true);
     return launch<true, true, EPI_SUMSQ>(a, b, a, b, a, args, s);
   }
   // A and B boxes are both 128 rows: a B stage is filled by two independent copies
-  if (!make_map(&a, G, rows, wo, BK, BM, dt) || !make_map(&b, G, rows, wo, BK, BN / 2, dt) ||
-      !make_map(&a2, X, rows, wi, BK, BM, dt) || !make_map(&b2, X, rows, wi, BK, BN / 2, dt))
+  if (!make_map(&a, G, rows, n_out, BK, BM, dt) || !make_map(&b, G, rows, n_out, BK, BN / 2, dt) ||
+      !make_map(&a2, X, rows, n_in, BK, BM, dt) || !make_map(&b2, X, rows, n_in, BK, BN / 2, dt))
     return FDP_ERR_LAUNCH;
   args.M = T; args.N = T;
   args.gram_nb = ceil_div(T, BM);
@@ -1239,17 +1401,23 @@ bool tc_fused_factors_ok(int B) { return B <= MAX_SMEM_FACTORS; }
 
 int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, float* split_ws,
                      void* dW, int* dev_status, int B, int T, int n_in, int n_out, int dt, int out_dt,
-                     int layout, float inv_div, NoiseKey nk, cudaStream_t s, int terms) {
+                     int layout, float inv_div, NoiseKey nk, cudaStream_t s, int planes) {
   const uint64_t rows = static_cast<uint64_t>(B) * T;
   const bool scaled = fs != nullptr;  // Gs is then the unscaled G
-  if (terms != 1 && !(terms == 3 && scaled)) return FDP_ERR_ARG;
+  if (planes == 2 && !scaled) return FDP_ERR_ARG;
   CUtensorMap mg, mx, mo, mp;
-  if (!make_map(&mg, Gs, rows, terms == 3 ? 2 * n_out : n_out, 64, BK, dt) ||
-      !make_map(&mx, X, rows, terms == 3 ? 2 * n_in : n_in, 64, BK, dt)) return FDP_ERR_LAUNCH;
+  // samples are the segments of the K range; a pre-scaled G makes all rows one segment
+  const int segs = scaled ? B : 1;
+  const uint64_t seg_rows = scaled ? T : rows;
+  const int po = planes > 1 ? pitch8(n_out) : n_out, pi = planes > 1 ? pitch8(n_in) : n_in;
+  if (!make_rows_map(&mg, Gs, segs, seg_rows, static_cast<uint64_t>(planes) * po, dt) ||
+      !make_rows_map(&mx, X, segs, seg_rows, static_cast<uint64_t>(planes) * pi, dt)) return FDP_ERR_LAUNCH;
   TcArgs args{};
   args.batch = 1; args.batch_rows = 0; args.status = dev_status;
   args.dependent = 1;             // always follows a kernel of the same call (norm pass, clip factors or pre-scale)
-  args.k_stages = static_cast<int>((rows + BK - 1) / BK);
+  args.seg_stages = static_cast<int>((seg_rows + BK - 1) / BK);
+  args.k_stages = segs * args.seg_stages;
+  args.sub_stages = planes > 1 ? chain_stages(args.seg_stages, planes) : args.seg_stages;
   args.out = dW; args.out_dt = out_dt; args.scale = inv_div; args.nk = nk;
   // [out,in]: A = G (M = n_out), B = X (N = n_in); [in,out]: operands swap roles, no transpose pass
   const bool oi = (layout == FDP_OUT_IN);
@@ -1257,8 +1425,7 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
   const int ctas = ctas_per_tile();
   args.idesc = make_idesc(dt, true, true, ctas);
   if (scaled) {
-    args.segs = B; args.seg_stages = T / BK;
-    args.sub_stages = terms == 3 ? chain_stages(args.seg_stages) : args.seg_stages;
+    args.segs = B;
     args.factors = fs->factors;
     if (fs->factors == nullptr) {
       if (!tc_fused_factors_ok(B) || fs->norm_partials == nullptr) return FDP_ERR_ARG;
@@ -1267,7 +1434,8 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
       args.norms_out = fs->norms_out; args.factors_out = fs->factors_out;
     }
   }
-  args.plane_a = args.M; args.plane_b = args.N;
+  args.plane_a = oi ? po : pi; args.plane_b = oi ? pi : po;
+  args.direct_out = !aligned16(dW) || args.N * dtype_size(out_dt) % 16 != 0;
   args.tiles_m = ceil_div(args.M, BM * ctas); args.tiles_n = ceil_div(args.N, BN);
   args.tiles_per_batch = args.tiles_m * args.tiles_n;
   static const int m_group = [] { const char* e = getenv("FDP_TC_MGROUP"); return e ? atoi(e) : 8; }();
@@ -1275,7 +1443,7 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
   // tail wave: split K so the SMs left idle by the tile count get work; the parts are parked in the
   // workspace and summed in fixed order by the fix-up kernel (deterministic, no waits)
   const int total = args.tiles_per_batch, workers = launch_sms() / ctas;
-  const int split = plan_tail_split(total, args.k_stages, workers, terms);
+  const int split = plan_tail_split(total, args.k_stages, workers, planes == 3 ? 6 : planes == 2 ? 3 : 1);
   int n_split_tiles = 0;
   if (split > 1) {
     n_split_tiles = total <= workers ? total : total % workers;
@@ -1283,13 +1451,15 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
     args.units_full = total - n_split_tiles;
     args.split_ws = split_ws;
   }
-  if (!make_out_map(&mo, dW, args.M, args.N, out_dt)) return FDP_ERR_LAUNCH;
+  if (args.direct_out) mo = mg;   // not used
+  else if (!make_out_map(&mo, dW, args.M, args.N, out_dt)) return FDP_ERR_LAUNCH;
   // the parked parts: [slot * ctas + CTA of the pair][BM rows][BN columns] fp32
   if (!make_out_map(&mp, split_ws, static_cast<uint64_t>(2) * MAX_SMS * BM, BN, FDP_F32)) return FDP_ERR_LAUNCH;
   int st;
 #define FDP_WGRAD_LAUNCH(EPI_, CT_) (oi ? launch<true, true, EPI_, CT_>(mg, mx, mp, mx, mo, args, s) \
                                         : launch<true, true, EPI_, CT_>(mx, mg, mp, mg, mo, args, s))
-  if (terms == 3) st = ctas == 2 ? FDP_WGRAD_LAUNCH(EPI_SPLIT_SCALED, 2) : FDP_WGRAD_LAUNCH(EPI_SPLIT_SCALED, 1);
+  if (planes == 3) st = ctas == 2 ? FDP_WGRAD_LAUNCH(EPI_SPLIT6_SCALED, 2) : FDP_WGRAD_LAUNCH(EPI_SPLIT6_SCALED, 1);
+  else if (planes == 2) st = ctas == 2 ? FDP_WGRAD_LAUNCH(EPI_SPLIT_SCALED, 2) : FDP_WGRAD_LAUNCH(EPI_SPLIT_SCALED, 1);
   else if (scaled) st = ctas == 2 ? FDP_WGRAD_LAUNCH(EPI_STORE_SCALED, 2) : FDP_WGRAD_LAUNCH(EPI_STORE_SCALED, 1);
   else st = ctas == 2 ? FDP_WGRAD_LAUNCH(EPI_STORE, 2) : FDP_WGRAD_LAUNCH(EPI_STORE, 1);
 #undef FDP_WGRAD_LAUNCH
@@ -1298,7 +1468,7 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
   dim3 grid(BM * ctas * BN / (256 * 4), n_split_tiles);
   launch_dependent(splitk_fixup_kernel, grid, dim3(256), 0, s, args.split_ws, args.units_full, split, BM * ctas, args.M,
                    args.N, args.tiles_m, args.tiles_n, args.n_fastest, args.m_group, dW, out_dt, args.ld_out,
-                   scaled ? 1.0f : inv_div, nk);
+                   scaled || planes > 1 ? 1.0f : inv_div, nk);
   note_launch();
   return FDP_OK;
 }
@@ -1364,7 +1534,7 @@ int tc_fwd(const void* X, const void* W, const void* bias, void* Y, int* dev_sta
 }
 
 // ---- fp32 products on the tensor cores: Y[rows, N] = A[rows, K] * W (+ bias) --------------------------
-// A3 is [rows, 2K] and W3 [K, 2N] (w_kn) or [N, 2K] (else): bf16 high halves then low halves (tc_split3).
+// A3 is [rows, 2K] and W3 [K, 2N] (w_kn) or [N, 2K] (else): bf16 high halves then low halves (tc_split).
 // Three bf16 products per K range into accumulators that the epilogue warps take over every few K
 // stages and sum in registers (chain_stages), then the ordinary store epilogue.
 bool tc_gemm3_ok(int rows, int K, int N) {
@@ -1389,7 +1559,7 @@ int tc_gemm3(const void* A3, const void* W3, const void* bias, void* Y, int* dev
   args.n_fastest = 1;
   args.out = Y; args.out_dt = out_dt; args.scale = 1.0f; args.nk = NoiseKey{};
   args.bias = bias; args.bias_dt = FDP_F32; args.bias_vec = aligned16(bias);
-  args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = chain_stages(args.seg_stages);
+  args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = chain_stages(args.seg_stages, 2);
   if (w_kn) {   // rows of W3 are K, N contiguous
     if (!make_map(&mw, W3, K, 2 * N, 64, BK, FDP_BF16)) return FDP_ERR_LAUNCH;
     args.idesc = make_idesc(FDP_BF16, false, true, ctas);

@@ -31,8 +31,9 @@ extern "C" {
 
 /* 2: asynchronous status word, SM reservation, saturating LayerNorm mode, FDP_FP32_TENSOR.
  * 3: fdp_dp_params.step_device (appended; earlier fields keep their offsets); FDP_FP32_TENSOR also
- *    accepted in the dtype of fdp_linear_dgrad / fdp_linear_fwd. */
-#define FDP_ABI_VERSION 3
+ *    accepted in the dtype of fdp_linear_dgrad / fdp_linear_fwd.
+ * 4: FDP_FP32_WIDE. */
+#define FDP_ABI_VERSION 4
 
 typedef void* fdp_stream_t; /* a cudaStream_t */
 
@@ -74,7 +75,13 @@ enum fdp_norm_algo {
    * Without the flag fp32 inputs keep fp32 FMA arithmetic, the reference's own
    * (flashdp/core/utils.py:9-12: fp32 accumulates in fp32).  The Python layer sets the flag by default
    * (runtime.set_fp32_mode). */
-  FDP_FP32_TENSOR = 16
+  FDP_FP32_TENSOR = 16,
+  /* flag, OR-ed into the same arguments: fp32 inputs of other shapes (any widths of at least 64; T of at least 64,
+   * or T shorter than 64 with at least 128 rows in all) run on the tensor cores as six bf16 products (x = hi + mid + lo, dropping
+   * what lies below 2^-26 of a product).  Norms and gradients are as close to float64 as those of the FMA
+   * kernels.  Operands and output need no alignment.  The workspace grows by 1.5 times the size of the
+   * inputs. */
+  FDP_FP32_WIDE = 32
 };
 
 /* DP hyper-parameters of one call.  C / clamp_value are the arguments of

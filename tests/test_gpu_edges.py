@@ -43,3 +43,33 @@ def test_output_boxes(ops, rows, K, N, dtype, out_dtype, bias):
     if bias:
         want, absum = want + b.double(), absum + b.double().abs()
     _close_to_sum(Y, want, absum, K + 1, UNIT[out_dtype])
+
+
+# fp32 through six bf16 products: the ends of samples against 64-row K stages, sequences too short for the product
+# form of the norm (T < 64), the smallest widths and row counts, widths whose rows are not multiples of 16 bytes
+@pytest.mark.parametrize("B,T,n_in,n_out", [(1, 64, 64, 64), (2, 65, 72, 328), (3, 127, 257, 130), (5, 197, 520, 64),
+                                            (64, 1, 65, 129), (9, 63, 333, 100), (2, 1000, 300, 515), (400, 70, 66, 66)])
+@pytest.mark.parametrize("layout", ["out_in", "in_out"])
+def test_fp32_six_products(ops, B, T, n_in, n_out, layout):
+    X = _randn(B, T, n_in, seed=1, dtype=torch.float32)
+    G = _randn(B, T, n_out, seed=2, dtype=torch.float32, scale=1e-2)
+    G[0] *= 30.0
+    dW, norms, factors = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, layout=layout, return_norms=True, fp32_tensor=True)
+    per = torch.einsum("bto,bti->boi", G.double(), X.double())
+    want_n = per.flatten(1).norm(dim=1)
+    assert float(((norms.double() - want_n) / want_n).abs().max()) < 4 * 2.0 ** -23
+    f = (1.0 / (want_n + 1e-10)).clamp(max=1.0)
+    want = torch.einsum("boi,b->oi", per, f) / B
+    absum = torch.einsum("bto,bti,b->oi", G.double().abs(), X.double().abs(), f) / B
+    if layout == "in_out":
+        want, absum = want.t(), absum.t()
+    # 24 truncating steps within an accumulator, one rounded addition per 64 rows of a sample, the clip factor (4)
+    _close_to_sum(dW, want, absum, 28 + B * ((T + 63) // 64), 2.0 ** -23)
+    # the noise is the stream of the generic kernels, element for element, whatever the row pitch and alignment
+    noise = ops.NoiseSpec(0.01, 5, 2, 0, 9)
+    zero = torch.zeros_like(G)
+    flat = torch.zeros(n_in * n_out + 1, device=dev())
+    out = flat[1:].view(dW.shape)
+    ops.dp_linear_weight_grad(X, zero, 1.0, 1.0, layout=layout, noise=noise, fp32_tensor=True, out=out)
+    assert torch.equal(out, ops.dp_linear_weight_grad(X, zero, 1.0, 1.0, layout=layout, noise=noise, fp32_tensor=False))
+    assert float(flat[0]) == 0.0
