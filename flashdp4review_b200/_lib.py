@@ -88,6 +88,24 @@ def load():
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native call layer (csrc/fdp_host.cpp), bound to the library that load() has loaded."""
+    global _host
+    if _host is None:
+        lib = load()
+        try:
+            from . import _fdp_host
+        except ImportError as e:
+            raise ImportError("_fdp_host.so is missing or does not fit this torch: build it with "
+                              "`python -m flashdp4review_b200.build`") from e
+        _fdp_host.bind({n: ctypes.cast(getattr(lib, n), c_void_p).value for n in SIGNATURES})
+        _host = _fdp_host
+    return _host
+
+
 _EXC = {FDP_ERR_ARG: ValueError, FDP_ERR_DTYPE: KeyError, FDP_ERR_SHAPE: RuntimeError,
         FDP_ERR_ALIGN: RuntimeError, FDP_ERR_WORKSPACE: RuntimeError, FDP_ERR_ARCH: RuntimeError,
         FDP_ERR_LAUNCH: RuntimeError, FDP_ERR_TIMEOUT: RuntimeError}

@@ -13,8 +13,7 @@ from dataclasses import dataclass
 
 import torch
 
-from .. import _lib
-from .._lib import DPParams
+from .. import _lib, runtime
 
 _DT = {torch.float32: _lib.FDP_F32, torch.bfloat16: _lib.FDP_BF16, torch.float16: _lib.FDP_F16}
 NORM_ALGOS = {"auto": _lib.FDP_NORM_AUTO, "direct": _lib.FDP_NORM_DIRECT, "gram": _lib.FDP_NORM_GRAM}
@@ -49,10 +48,6 @@ def _aligned(t):
     return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
 
 
-def _workspace(nbytes, device):
-    return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
-
-
 @dataclass
 class NoiseSpec:
     """Where the Gaussian noise of one call comes from.
@@ -72,13 +67,16 @@ class NoiseSpec:
     step_device: object = None    # a one-element int32 CUDA tensor the kernels add to `step` when they run
 
 
+_NO_NOISE = NoiseSpec()
+
+
 def _params(C, clamp_value, batch_divisor, noise):
-    noise = noise or NoiseSpec()
-    return DPParams(float(C), float(clamp_value), float(noise.std), int(batch_divisor or 0),
-                    int(noise.seed) & (2 ** 64 - 1), int(noise.param_id) & 0xFFFFFFFF,
-                    int(noise.param_id2) & 0xFFFFFFFF, int(noise.step) & 0xFFFFFFFF,
-                    int(noise.rank), int(noise.world),
-                    noise.step_device.data_ptr() if noise.step_device is not None else None)
+    noise = noise or _NO_NOISE
+    return (float(C), float(clamp_value), float(noise.std), int(batch_divisor or 0),
+            int(noise.seed) & (2 ** 64 - 1), int(noise.param_id) & 0xFFFFFFFF,
+            int(noise.param_id2) & 0xFFFFFFFF, int(noise.step) & 0xFFFFFFFF,
+            int(noise.rank), int(noise.world),
+            noise.step_device.data_ptr() if noise.step_device is not None else None)
 
 
 # ------------------------------------------------------------------------------------------------
@@ -101,7 +99,7 @@ def dp_linear_weight_grad(input, grad_output, C, clamp_value, *, batch_divisor=N
     other shapes (widths of at least 64, at least 128 rows) as six products, as close to float64 as the
     FMA kernels.  False forces the FMA kernels.
     """
-    lib = _lib.load()
+    host = _lib.host()
     _require_cuda(input, grad_output)
     if input.dim() != 3 or grad_output.dim() != 3 or input.shape[:2] != grad_output.shape[:2]:
         raise RuntimeError(f"expected (B,T,in) and (B,T,out), got {tuple(input.shape)} and {tuple(grad_output.shape)}")
@@ -113,26 +111,17 @@ def dp_linear_weight_grad(input, grad_output, C, clamp_value, *, batch_divisor=N
     if out is not None:
         if tuple(out.shape) != shape or not out.is_contiguous() or out.device != G.device:
             raise RuntimeError(f"out must be a contiguous {shape} tensor on {G.device}")
-        dW, out_dtype = out, out.dtype
+        out_dtype = out.dtype
     else:
         out_dtype = out_dtype or G.dtype
-        dW = torch.empty(shape, dtype=out_dtype, device=G.device)
-    norms = torch.empty(B, dtype=torch.float32, device=G.device) if return_norms else None
-    factors = torch.empty(B, dtype=torch.float32, device=G.device) if return_norms else None
     algo = NORM_ALGOS[norm_algo]
     if fp32_tensor is None:
-        from .. import runtime
         fp32_tensor = runtime.fp32_mode() == "tensor"
     if fp32_tensor and G.dtype == torch.float32:
         algo |= _lib.FDP_FP32_TENSOR | _lib.FDP_FP32_WIDE
-    nbytes = lib.fdp_linear_wgrad_workspace_bytes(B, T, n_in, n_out, _dt(G.dtype), algo)
-    ws = _workspace(nbytes, G.device)
-    p = _params(C, clamp_value, batch_divisor, noise)
-    with torch.cuda.device(G.device):
-        st = lib.fdp_linear_wgrad(_ptr(G), _ptr(X), _ptr(dW), _ptr(norms), _ptr(factors), B, T, n_in,
-                                  n_out, _dt(G.dtype), _dt(out_dtype),
-                                  _lib.FDP_OUT_IN if layout == "out_in" else _lib.FDP_IN_OUT, algo,
-                                  p, _ptr(ws), ws.numel(), _stream(G.device))
+    st, dW, norms, factors = host.linear_wgrad(
+        G, X, out, _dt(G.dtype), _dt(out_dtype), _lib.FDP_OUT_IN if layout == "out_in" else _lib.FDP_IN_OUT, algo,
+        _params(C, clamp_value, batch_divisor, noise), return_norms)
     _lib.check(st, "fdp_linear_wgrad")
     return (dW, norms, factors) if return_norms else dW
 
@@ -179,7 +168,7 @@ def dp_bias_grad(grad_output, C, clamp_value, *, batch_divisor=None, noise=None,
                  return_norms=False):
     """(1/(divisor*T)) * sum_b c_b * sum_t G[b,t,:] + noise, with c_b from ||G_b||_F over T*out
     (flashdp/core/linear_clip.py:116-123)."""
-    lib = _lib.load()
+    host = _lib.host()
     _require_cuda(grad_output)
     if grad_output.dim() < 2:
         raise RuntimeError("grad_output must be at least (B, out)")
@@ -187,14 +176,8 @@ def dp_bias_grad(grad_output, C, clamp_value, *, batch_divisor=None, noise=None,
     B, n_out = G.shape[0], G.shape[-1]
     T = G.numel() // (B * n_out)
     out_dtype = out_dtype or G.dtype
-    db = torch.empty(n_out, dtype=out_dtype, device=G.device)
-    norms = torch.empty(B, dtype=torch.float32, device=G.device) if return_norms else None
-    factors = torch.empty(B, dtype=torch.float32, device=G.device) if return_norms else None
-    ws = _workspace(lib.fdp_bias_grad_workspace_bytes(B, T, n_out, _dt(G.dtype)), G.device)
-    p = _params(C, clamp_value, batch_divisor, noise)
-    with torch.cuda.device(G.device):
-        st = lib.fdp_bias_grad(_ptr(G), _ptr(db), _ptr(norms), _ptr(factors), B, T, n_out,
-                               _dt(G.dtype), _dt(out_dtype), p, _ptr(ws), ws.numel(), _stream(G.device))
+    st, db, norms, factors = host.bias_grad(G, B, T, _dt(G.dtype), _dt(out_dtype),
+                                            _params(C, clamp_value, batch_divisor, noise), return_norms)
     _lib.check(st, "fdp_bias_grad")
     return (db, norms, factors) if return_norms else db
 
@@ -214,7 +197,6 @@ def native_product_ok(dtype, rows, K, N):
     8-aligned features, at least 128 rows and output columns and 64 contracted ones; fp32 in mode "tensor"
     with K a multiple of 64 and at least 128 of everything (three bf16 products); "native" also for every
     other 16-bit shape (generic kernels)."""
-    from .. import runtime
     mode = runtime.input_grad_impl()
     if mode == "library":
         return False
@@ -231,7 +213,6 @@ def _gemm_dtype_code(dtype, fp32_tensor):
     code = _dt(dtype)
     if dtype == torch.float32:
         if fp32_tensor is None:
-            from .. import runtime
             fp32_tensor = runtime.fp32_mode() == "tensor"
         if fp32_tensor:
             code |= _lib.FDP_FP32_TENSOR
@@ -243,21 +224,13 @@ def linear_input_grad(grad_output, weight, w_layout="out_in", out_dtype=None, fp
     weight [in,out]) -- flashdp/layers/linear.py:62-67, transformers_conv1d.py:70-75.
     `out_dtype` (default: grad_output's) lets the kernel write the dtype autograd wants directly.
     `fp32_tensor` as in dp_linear_weight_grad: fp32 operands as three bf16 tensor-core products."""
-    lib = _lib.load()
+    host = _lib.host()
     _require_cuda(grad_output, weight)
     G = _aligned(grad_output.contiguous())
     W = _aligned(weight.to(G.dtype).contiguous())         # AMP: weight follows the grad dtype (linear.py:66)
     n_out = G.shape[-1]
-    n_in = W.shape[1] if w_layout == "out_in" else W.shape[0]
-    rows = G.numel() // n_out
-    out_dtype = out_dtype or G.dtype
-    dX = torch.empty(G.shape[:-1] + (n_in,), dtype=out_dtype, device=G.device)
-    code = _gemm_dtype_code(G.dtype, fp32_tensor)
-    ws = _workspace(lib.fdp_linear_dgrad_workspace_bytes(rows, n_in, n_out, code), G.device)
-    with torch.cuda.device(G.device):
-        st = lib.fdp_linear_dgrad(_ptr(G), _ptr(W), _ptr(dX), rows, n_in, n_out, code, _dt(out_dtype),
-                                  _lib.FDP_OUT_IN if w_layout == "out_in" else _lib.FDP_IN_OUT,
-                                  _ptr(ws), ws.numel(), _stream(G.device))
+    st, dX = host.linear_dgrad(G, W, G.numel() // n_out, _gemm_dtype_code(G.dtype, fp32_tensor),
+                               _dt(out_dtype or G.dtype), _lib.FDP_OUT_IN if w_layout == "out_in" else _lib.FDP_IN_OUT)
     _lib.check(st, "fdp_linear_dgrad")
     return dX
 
@@ -265,22 +238,14 @@ def linear_input_grad(grad_output, weight, w_layout="out_in", out_dtype=None, fp
 def linear_forward(input, weight, bias=None, w_layout="out_in", out_dtype=None, fp32_tensor=None):
     """input @ weight.t() + bias (nn.Linear, weight [out,in]) or input @ weight + bias (Conv1D, weight
     [in,out]) -- flashdp/layers/linear.py:41-46, transformers_conv1d.py:40-43."""
-    lib = _lib.load()
+    host = _lib.host()
     _require_cuda(input, weight, bias)
     X = _aligned(input.contiguous())
     W = _aligned(weight.to(X.dtype).contiguous())
     b = None if bias is None else _aligned(bias.to(X.dtype).contiguous())
     n_in = X.shape[-1]
-    n_out = W.shape[0] if w_layout == "out_in" else W.shape[1]
-    rows = X.numel() // n_in
-    out_dtype = out_dtype or X.dtype
-    Y = torch.empty(X.shape[:-1] + (n_out,), dtype=out_dtype, device=X.device)
-    code = _gemm_dtype_code(X.dtype, fp32_tensor)
-    ws = _workspace(lib.fdp_linear_dgrad_workspace_bytes(rows, n_out, n_in, code), X.device)
-    with torch.cuda.device(X.device):
-        st = lib.fdp_linear_fwd(_ptr(X), _ptr(W), _ptr(b), _ptr(Y), rows, n_in, n_out, code, _dt(out_dtype),
-                                _lib.FDP_OUT_IN if w_layout == "out_in" else _lib.FDP_IN_OUT,
-                                _ptr(ws), ws.numel(), _stream(X.device))
+    st, Y = host.linear_fwd(X, W, b, X.numel() // n_in, _gemm_dtype_code(X.dtype, fp32_tensor),
+                            _dt(out_dtype or X.dtype), _lib.FDP_OUT_IN if w_layout == "out_in" else _lib.FDP_IN_OUT)
     _lib.check(st, "fdp_linear_fwd")
     return Y
 
@@ -307,7 +272,7 @@ def mm_fused(tensor1, tensor2):
 def layernorm_fwd_fused(input, weight, bias, eps):
     """LayerNorm over the last dimension; returns (y, {'mean','rstd'}, args) like
     flashdp/core/layernorm_clip.py:201-239."""
-    lib = _lib.load()
+    host = _lib.host()
     _require_cuda(input, weight, bias)
     x = input.contiguous()
     d = x.shape[-1]
@@ -315,14 +280,9 @@ def layernorm_fwd_fused(input, weight, bias, eps):
     if d * x.element_size() >= 65536:
         # same limit and exception as the reference (flashdp/core/layernorm_clip.py:220-221)
         raise RuntimeError("This layer norm doesn't support feature dim >= 64KB.")
-    y = torch.empty_like(x)
-    mean = torch.empty(rows, dtype=torch.float32, device=x.device)
-    rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
     w = weight.contiguous()
     b = bias.to(w.dtype).contiguous()
-    with torch.cuda.device(x.device):
-        st = lib.fdp_layernorm_fwd(_ptr(x), _ptr(w), _ptr(b), _ptr(y), _ptr(mean), _ptr(rstd), rows, d,
-                                   float(eps), _dt(x.dtype), _dt(w.dtype), _stream(x.device))
+    st, y, mean, rstd = host.layernorm_fwd(x, w, b, float(eps), rows, _dt(x.dtype), _dt(w.dtype))
     _lib.check(st, "fdp_layernorm_fwd")
     return y, {"mean": mean, "rstd": rstd}, {"eps": eps}
 
@@ -336,7 +296,7 @@ def dp_layernorm_backward(grad_output, input, weight, mean, rstd, C, clamp_value
     with sum_t dy_b (flashdp/core/layernorm_clip.py:163-198; noise flashdp/layers/layernorm.py:139-155,
     drawn once per tensor).  The sample axis is dim 0; every other leading axis is summed.
     """
-    lib = _lib.load()
+    host = _lib.host()
     _require_cuda(grad_output, input, weight)
     dy = grad_output.contiguous()
     x = input.contiguous()
@@ -344,17 +304,9 @@ def dp_layernorm_backward(grad_output, input, weight, mean, rstd, C, clamp_value
     B = x.shape[0] if x.dim() > 1 else 1
     T = x.numel() // (B * d)
     w = weight.contiguous()
-    dx = torch.empty_like(x) if need_dx else None
-    dgamma = torch.empty(d, dtype=w.dtype, device=x.device)
-    dbeta = torch.empty(d, dtype=w.dtype, device=x.device) if need_dbeta else None
-    ng = torch.empty(B, dtype=torch.float32, device=x.device) if return_norms else None
-    nb = torch.empty(B, dtype=torch.float32, device=x.device) if return_norms and need_dbeta else None
-    ws = _workspace(lib.fdp_layernorm_bwd_workspace_bytes(B, T, d), x.device)
-    p = _params(C, clamp_value, batch_divisor, noise)
-    with torch.cuda.device(x.device):
-        st = lib.fdp_layernorm_bwd(_ptr(dy), _ptr(x), _ptr(w), _ptr(mean), _ptr(rstd), _ptr(dx),
-                                   _ptr(dgamma), _ptr(dbeta), _ptr(ng), _ptr(nb), B, T, d,
-                                   _dt(x.dtype), _dt(w.dtype), p, _ptr(ws), ws.numel(), _stream(x.device))
+    st, dx, dgamma, dbeta, ng, nb = host.layernorm_bwd(
+        dy, x, w, mean, rstd, B, T, _dt(x.dtype), _dt(w.dtype), _params(C, clamp_value, batch_divisor, noise),
+        need_dx, need_dbeta, return_norms)
     _lib.check(st, "fdp_layernorm_bwd")
     if return_norms:
         return dx, dgamma, dbeta, ng, nb

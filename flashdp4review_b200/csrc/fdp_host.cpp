@@ -1,0 +1,181 @@
+// Host side of the operator layer: allocates a call's outputs and workspace with torch's caching allocator and
+// enters the C ABI.  The checks on shapes, dtypes and devices, and all choices, stay in core/ops.py; what is
+// here is what every call pays for -- device guard, current stream, two to five allocations, argument
+// marshalling -- which through ctypes and torch's Python functions took 20 us an operator, more than the kernels
+// of a small layer.  Every function returns (status, outputs...).
+#include <torch/extension.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+
+#include "../../include/fdp_b200.h"
+
+namespace {
+
+namespace py = pybind11;
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+// Entry points of the library that _lib.py has loaded (it may be another build than the one beside this file).
+struct Abi {
+  decltype(&fdp_linear_wgrad_workspace_bytes) linear_wgrad_workspace_bytes;
+  decltype(&fdp_linear_wgrad) linear_wgrad;
+  decltype(&fdp_bias_grad_workspace_bytes) bias_grad_workspace_bytes;
+  decltype(&fdp_bias_grad) bias_grad;
+  decltype(&fdp_linear_dgrad_workspace_bytes) linear_dgrad_workspace_bytes;
+  decltype(&fdp_linear_dgrad) linear_dgrad;
+  decltype(&fdp_linear_fwd) linear_fwd;
+  decltype(&fdp_layernorm_fwd) layernorm_fwd;
+  decltype(&fdp_layernorm_bwd_workspace_bytes) layernorm_bwd_workspace_bytes;
+  decltype(&fdp_layernorm_bwd) layernorm_bwd;
+} abi;
+
+void bind(const std::map<std::string, uint64_t>& fns) {
+#define FDP_BIND(NAME) abi.NAME = reinterpret_cast<decltype(abi.NAME)>(fns.at("fdp_" #NAME))
+  FDP_BIND(linear_wgrad_workspace_bytes); FDP_BIND(linear_wgrad);
+  FDP_BIND(bias_grad_workspace_bytes); FDP_BIND(bias_grad);
+  FDP_BIND(linear_dgrad_workspace_bytes); FDP_BIND(linear_dgrad); FDP_BIND(linear_fwd);
+  FDP_BIND(layernorm_fwd); FDP_BIND(layernorm_bwd_workspace_bytes); FDP_BIND(layernorm_bwd);
+#undef FDP_BIND
+}
+
+at::ScalarType scalar_type(int dt) {
+  return dt == FDP_F32 ? at::kFloat : dt == FDP_BF16 ? at::kBFloat16 : at::kHalf;
+}
+Tensor new_tensor(const Tensor& like, at::IntArrayRef sizes, at::ScalarType t) {
+  return at::empty(sizes, like.options().dtype(t).memory_format(std::nullopt));
+}
+Tensor workspace(const Tensor& like, size_t bytes) {
+  return new_tensor(like, {static_cast<int64_t>(bytes < 256 ? 256 : bytes)}, at::kByte);
+}
+void* ptr(const Tensor& t) { return t.data_ptr(); }
+void* ptr(const OptTensor& t) { return t.has_value() ? t->data_ptr() : nullptr; }
+fdp_stream_t stream(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
+
+// (C, clamp_value, noise std, batch divisor, seed, param_id, param_id2, step, rank, world, step counter or None)
+fdp_dp_params params(const py::tuple& p) {
+  fdp_dp_params q{};
+  q.C = p[0].cast<float>(); q.clamp_value = p[1].cast<float>(); q.noise_std = p[2].cast<float>();
+  q.batch_divisor = p[3].cast<int32_t>(); q.seed = p[4].cast<uint64_t>();
+  q.param_id = p[5].cast<uint32_t>(); q.param_id2 = p[6].cast<uint32_t>(); q.step = p[7].cast<uint32_t>();
+  q.noise_rank = p[8].cast<int32_t>(); q.noise_world = p[9].cast<int32_t>();
+  q.step_device = p[10].is_none() ? nullptr : reinterpret_cast<decltype(q.step_device)>(p[10].cast<uint64_t>());
+  return q;
+}
+
+py::tuple linear_wgrad(const Tensor& G, const Tensor& X, const OptTensor& out, int in_dt, int out_dt, int layout, int algo,
+                       const py::tuple& p, bool want_norms) {
+  const fdp_dp_params q = params(p);
+  const c10::cuda::CUDAGuard guard(G.device());
+  const int B = static_cast<int>(X.size(0)), T = static_cast<int>(X.size(1));
+  const int n_in = static_cast<int>(X.size(2)), n_out = static_cast<int>(G.size(2));
+  Tensor dW = out.has_value() ? *out
+              : layout == FDP_OUT_IN ? new_tensor(G, {n_out, n_in}, scalar_type(out_dt)) : new_tensor(G, {n_in, n_out}, scalar_type(out_dt));
+  OptTensor norms, factors;
+  if (want_norms) { norms = new_tensor(G, {B}, at::kFloat); factors = new_tensor(G, {B}, at::kFloat); }
+  const size_t bytes = abi.linear_wgrad_workspace_bytes(B, T, n_in, n_out, in_dt, algo);
+  const Tensor ws = workspace(G, bytes);
+  int st;
+  {
+    py::gil_scoped_release nogil;
+    st = abi.linear_wgrad(ptr(G), ptr(X), ptr(dW), static_cast<float*>(ptr(norms)), static_cast<float*>(ptr(factors)), B, T, n_in,
+                          n_out, in_dt, out_dt, layout, algo, &q, ptr(ws), ws.numel(), stream(G));
+  }
+  return py::make_tuple(st, dW, norms, factors);
+}
+
+py::tuple bias_grad(const Tensor& G, int B, int T, int in_dt, int out_dt, const py::tuple& p, bool want_norms) {
+  const fdp_dp_params q = params(p);
+  const c10::cuda::CUDAGuard guard(G.device());
+  const int n_out = static_cast<int>(G.size(-1));
+  const Tensor db = new_tensor(G, {n_out}, scalar_type(out_dt));
+  OptTensor norms, factors;
+  if (want_norms) { norms = new_tensor(G, {B}, at::kFloat); factors = new_tensor(G, {B}, at::kFloat); }
+  const Tensor ws = workspace(G, abi.bias_grad_workspace_bytes(B, T, n_out, in_dt));
+  int st;
+  {
+    py::gil_scoped_release nogil;
+    st = abi.bias_grad(ptr(G), ptr(db), static_cast<float*>(ptr(norms)), static_cast<float*>(ptr(factors)), B, T, n_out, in_dt, out_dt,
+                       &q, ptr(ws), ws.numel(), stream(G));
+  }
+  return py::make_tuple(st, db, norms, factors);
+}
+
+// the leading sizes of `a` with `cols` columns
+Tensor with_columns(const Tensor& a, int64_t cols, int dt) {
+  c10::SmallVector<int64_t, 6> sizes(a.sizes().begin(), a.sizes().end());
+  sizes.back() = cols;
+  return new_tensor(a, sizes, scalar_type(dt));
+}
+
+py::tuple linear_dgrad(const Tensor& G, const Tensor& W, int rows, int code, int out_dt, int w_layout) {
+  const c10::cuda::CUDAGuard guard(G.device());
+  const int n_out = static_cast<int>(G.size(-1)), n_in = static_cast<int>(W.size(w_layout == FDP_OUT_IN ? 1 : 0));
+  const Tensor dX = with_columns(G, n_in, out_dt);
+  const Tensor ws = workspace(G, abi.linear_dgrad_workspace_bytes(rows, n_in, n_out, code));
+  int st;
+  {
+    py::gil_scoped_release nogil;
+    st = abi.linear_dgrad(ptr(G), ptr(W), ptr(dX), rows, n_in, n_out, code, out_dt, w_layout, ptr(ws), ws.numel(), stream(G));
+  }
+  return py::make_tuple(st, dX);
+}
+
+py::tuple linear_fwd(const Tensor& X, const Tensor& W, const OptTensor& bias, int rows, int code, int out_dt, int w_layout) {
+  const c10::cuda::CUDAGuard guard(X.device());
+  const int n_in = static_cast<int>(X.size(-1)), n_out = static_cast<int>(W.size(w_layout == FDP_OUT_IN ? 0 : 1));
+  const Tensor Y = with_columns(X, n_out, out_dt);
+  const Tensor ws = workspace(X, abi.linear_dgrad_workspace_bytes(rows, n_out, n_in, code));
+  int st;
+  {
+    py::gil_scoped_release nogil;
+    st = abi.linear_fwd(ptr(X), ptr(W), ptr(bias), ptr(Y), rows, n_in, n_out, code, out_dt, w_layout, ptr(ws), ws.numel(), stream(X));
+  }
+  return py::make_tuple(st, Y);
+}
+
+py::tuple layernorm_fwd(const Tensor& x, const Tensor& w, const Tensor& b, double eps, int rows, int dt, int pdt) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  const Tensor y = new_tensor(x, x.sizes(), x.scalar_type());
+  const Tensor mean = new_tensor(x, {rows}, at::kFloat), rstd = new_tensor(x, {rows}, at::kFloat);
+  int st;
+  {
+    py::gil_scoped_release nogil;
+    st = abi.layernorm_fwd(ptr(x), ptr(w), ptr(b), ptr(y), static_cast<float*>(ptr(mean)), static_cast<float*>(ptr(rstd)), rows,
+                           static_cast<int>(x.size(-1)), static_cast<float>(eps), dt, pdt, stream(x));
+  }
+  return py::make_tuple(st, y, mean, rstd);
+}
+
+py::tuple layernorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd, int B, int T,
+                        int dt, int pdt, const py::tuple& p, bool need_dx, bool need_dbeta, bool want_norms) {
+  const fdp_dp_params q = params(p);
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int d = static_cast<int>(x.size(-1));
+  OptTensor dx, dbeta, ng, nb;
+  if (need_dx) dx = new_tensor(x, x.sizes(), x.scalar_type());
+  const Tensor dgamma = new_tensor(x, {d}, w.scalar_type());
+  if (need_dbeta) dbeta = new_tensor(x, {d}, w.scalar_type());
+  if (want_norms) ng = new_tensor(x, {B}, at::kFloat);
+  if (want_norms && need_dbeta) nb = new_tensor(x, {B}, at::kFloat);
+  const Tensor ws = workspace(x, abi.layernorm_bwd_workspace_bytes(B, T, d));
+  int st;
+  {
+    py::gil_scoped_release nogil;
+    st = abi.layernorm_bwd(ptr(dy), ptr(x), ptr(w), static_cast<const float*>(ptr(mean)), static_cast<const float*>(ptr(rstd)), ptr(dx),
+                           ptr(dgamma), ptr(dbeta), static_cast<float*>(ptr(ng)), static_cast<float*>(ptr(nb)), B, T, d, dt, pdt, &q,
+                           ptr(ws), ws.numel(), stream(x));
+  }
+  return py::make_tuple(st, dx, dgamma, dbeta, ng, nb);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("bind", &bind);
+  m.def("linear_wgrad", &linear_wgrad);
+  m.def("bias_grad", &bias_grad);
+  m.def("linear_dgrad", &linear_dgrad);
+  m.def("linear_fwd", &linear_fwd);
+  m.def("layernorm_fwd", &layernorm_fwd);
+  m.def("layernorm_bwd", &layernorm_bwd);
+}
