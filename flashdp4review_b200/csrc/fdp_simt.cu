@@ -386,8 +386,50 @@ __global__ void __launch_bounds__(256) gram_small_norm_kernel(const Tin* __restr
   if (threadIdx.x == 0) sumsq[b] = v;
 }
 
+// sum of squares of n adjacent elements, by one warp
+template <typename Tin>
+__device__ __forceinline__ float slab_sumsq(const Tin* __restrict__ p, int n, bool vec, int lane) {
+  constexpr int VEC = 16 / sizeof(Tin);
+  float s = 0.f;
+  if (vec) {       // 16-byte aligned, n a multiple of VEC
+#pragma unroll 4
+    for (int i = lane * VEC; i < n; i += 32 * VEC) {
+      float f[VEC];
+      unpack16<Tin>(__ldg(reinterpret_cast<const uint4*>(p + i)), f);
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) s = fmaf(f[v], f[v], s);
+    }
+  } else {
+#pragma unroll 4
+    for (int i = lane; i < n; i += 32) { const float f = to_f32<Tin>(p[i]); s = fmaf(f, f, s); }
+  }
+  return warp_sum(s);
+}
+
+// sumsq[b] = ||g_b||^2 ||x_b||^2 = ||g_b^T x_b||_F^2 for samples of one row: one warp a sample
+template <typename Tin>
+__global__ void __launch_bounds__(256) row_norms_kernel(const Tin* __restrict__ G, const Tin* __restrict__ X,
+                                                        float* __restrict__ sumsq, int B, int n_in, int n_out, int vec_x, int vec_g) {
+  const int b = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (b >= B) return;
+  const float g = slab_sumsq<Tin>(G + static_cast<size_t>(b) * n_out, n_out, vec_g != 0, lane);
+  const float x = slab_sumsq<Tin>(X + static_cast<size_t>(b) * n_in, n_in, vec_x != 0, lane);
+  if (lane == 0) sumsq[b] = g * x;
+}
+
 void simt_norm_gram_small(const void* G, const void* X, float* sumsq, int B, int T, int n_in, int n_out,
                           int dt, cudaStream_t s) {
+  if (T == 1) {
+    // one row: no T x T block to form (1024 samples, 1024 and 1000 columns, fp32: 25 us in the kernel below)
+    const int vec = 16 / static_cast<int>(dtype_size(dt));
+    const int vx = n_in % vec == 0 && aligned16(X), vg = n_out % vec == 0 && aligned16(G);
+    const int grid = ceil_div(B, 8);
+    if (dt == FDP_F32) row_norms_kernel<float><<<grid, 256, 0, s>>>((const float*)G, (const float*)X, sumsq, B, n_in, n_out, vx, vg);
+    else if (dt == FDP_BF16) row_norms_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)G, (const __nv_bfloat16*)X, sumsq, B, n_in, n_out, vx, vg);
+    else row_norms_kernel<__half><<<grid, 256, 0, s>>>((const __half*)G, (const __half*)X, sumsq, B, n_in, n_out, vx, vg);
+    note_launch();
+    return;
+  }
   const int tb = ceil_div(T, 4);                 // T < 64: at most 16 x 16 thread groups
   int cs = 32;
   while (cs > 1 && tb * tb * cs > 256) cs >>= 1;
@@ -686,6 +728,129 @@ void gstats(const void* G, float* colsum_part, float* sq_part, int B, int T, int
   else
     gstats_kernel<__half, 8><<<grid, 256, 0, s>>>((const __half*)G, colsum_part, sq_part, T, n_out, pl.rows_per_chunk, vec_ok, pl.col_chunks, pl.row_chunks);
   note_launch();
+}
+
+// ---- short samples: many samples of few rows -------------------------------------------------------------
+// One partial column sum per sample is then as large as G itself, and adding B of them a long serial loop (1024
+// rows of 1000 fp32 columns, one row per sample: 17 us for the statistics and 94 us for the finalisation).  The
+// samples' norms are taken first -- a sample is T * n_out adjacent elements, one warp each -- and the column sums
+// carry the clip factors, so one partial covers many samples (the same call: 11 us).  G is read twice, the second
+// time mostly from L2.
+template <typename Tin>
+__global__ void __launch_bounds__(256) short_factors_kernel(const Tin* __restrict__ G, int B, int n, int vec, float C, float clamp,
+                                                            float* __restrict__ factors, float* __restrict__ norms_out,
+                                                            float* __restrict__ factors_out) {
+  pdl_trigger();
+  const int b = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (b >= B) return;
+  const float norm = sqrtf(slab_sumsq<Tin>(G + static_cast<size_t>(b) * n, n, vec != 0, lane));
+  if (lane == 0) {
+    const float f = clip_factor(norm, C, clamp);
+    factors[b] = f;
+    if (norms_out) norms_out[b] = norm;
+    if (factors_out) factors_out[b] = f;
+  }
+}
+
+// part[rc, o] = sum over the chunk's rows r of factors[r / T] * G[r, o]; block = row chunk * col_chunks + column chunk
+template <typename Tin, int VEC>
+__global__ void __launch_bounds__(256) short_colsum_kernel(const Tin* __restrict__ G, const float* __restrict__ factors,
+                                                           float* __restrict__ part, int rows, int T, int n_out, int vec_ok,
+                                                           int rows_per_chunk, int col_chunks) {
+  __shared__ float cs[8][32 * VEC];
+  pdl_trigger();
+  pdl_wait();
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int cc = blockIdx.x % col_chunks, rc = blockIdx.x / col_chunks;
+  const int c0 = (cc * 32 + x) * VEC;
+  const int r1 = min(rows, (rc + 1) * rows_per_chunk);
+  float acc[VEC];
+#pragma unroll
+  for (int v = 0; v < VEC; ++v) acc[v] = 0.f;
+  if (c0 < n_out) {
+#pragma unroll 4
+    for (int r = rc * rows_per_chunk + y; r < r1; r += 8) {
+      const float f = __ldg(factors + r / T);
+      const Tin* p = G + static_cast<size_t>(r) * n_out + c0;
+      if (vec_ok) {
+        float g[VEC];
+        unpack16<Tin>(__ldg(reinterpret_cast<const uint4*>(p)), g);
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) acc[v] = fmaf(f, g[v], acc[v]);
+      } else {
+#pragma unroll
+        for (int v = 0; v < VEC; ++v)
+          if (c0 + v < n_out) acc[v] = fmaf(f, to_f32<Tin>(p[v]), acc[v]);
+      }
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < VEC; ++v) cs[y][x * VEC + v] = acc[v];
+  __syncthreads();
+  for (int c = threadIdx.x; c < 32 * VEC; c += 256) {
+    const int col = cc * 32 * VEC + c;
+    if (col < n_out) {
+      float t = 0.f;
+#pragma unroll
+      for (int yy = 0; yy < 8; ++yy) t += cs[yy][c];
+      part[static_cast<size_t>(rc) * n_out + col] = t;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) short_finalize_kernel(const float* __restrict__ part, void* __restrict__ db, int n_out,
+                                                             int parts, int out_dt, float inv_div, NoiseKey nk) {
+  __shared__ float sm[8][32];
+  pdl_wait();
+  const int col = threadIdx.x & 31, sl = threadIdx.x >> 5;
+  const int o = blockIdx.x * 32 + col;
+  float acc = 0.f;
+  if (o < n_out) {
+#pragma unroll 4
+    for (int p = sl; p < parts; p += 8) acc += part[static_cast<size_t>(p) * n_out + o];
+  }
+  sm[sl][col] = acc;
+  __syncthreads();
+  if (sl == 0 && o < n_out) {
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t += sm[k][col];
+    float v = t * inv_div;
+    if (nk.std != 0.f) v += noise_at(nk, o);
+    store_as(db, out_dt, o, v);
+  }
+}
+
+// Few rows a sample and enough samples that the general kernels' finalisation, serial in the samples, is the
+// longer way (64 samples: 8 additions a slice, as here).
+bool bias_short_ok(int B, int T) { return T <= 16 && B > 64; }
+
+template <typename Tin>
+static void bias_short_t(const Tin* G, float* factors, float* part, void* db, float* norms_out, float* factors_out, int B, int T,
+                         int n_out, int out_dt, float C, float clamp, float inv_div, NoiseKey nk, cudaStream_t s) {
+  constexpr int VEC = 16 / sizeof(Tin);
+  const int slab = T * n_out, vec_ok = n_out % VEC == 0 && aligned16(G);
+  short_factors_kernel<Tin><<<ceil_div(B, 8), 256, 0, s>>>(G, B, slab, vec_ok, C, clamp, factors, norms_out, factors_out);
+  // two blocks an SM, at least 32 rows each, and no more parts than the workspace's B column sums
+  const int rows = B * T, col_chunks = ceil_div(n_out, 32 * VEC);
+  int chunks = ceil_div(2 * 148, col_chunks);
+  if (chunks > ceil_div(rows, 32)) chunks = ceil_div(rows, 32);
+  if (chunks > B) chunks = B;
+  const int per = ceil_div(rows, chunks);
+  chunks = ceil_div(rows, per);
+  launch_dependent(short_colsum_kernel<Tin, VEC>, dim3(static_cast<unsigned>(chunks * col_chunks)), dim3(256), 0, s, G, factors, part, rows, T, n_out,
+                   vec_ok, per, col_chunks);
+  launch_dependent(short_finalize_kernel, dim3(ceil_div(n_out, 32)), dim3(256), 0, s, part, db, n_out, chunks, out_dt, inv_div, nk);
+  note_launch(3);
+}
+
+void bias_short(const void* G, float* factors, float* part, void* db, float* norms_out, float* factors_out, int B, int T, int n_out,
+                int dt, int out_dt, float C, float clamp, float inv_div, NoiseKey nk, cudaStream_t s) {
+#define FDP_BIAS_SHORT(TY) bias_short_t<TY>((const TY*)G, factors, part, db, norms_out, factors_out, B, T, n_out, out_dt, C, clamp, inv_div, nk, s)
+  if (dt == FDP_F32) FDP_BIAS_SHORT(float);
+  else if (dt == FDP_BF16) FDP_BIAS_SHORT(__nv_bfloat16);
+  else FDP_BIAS_SHORT(__half);
+#undef FDP_BIAS_SHORT
 }
 
 // db[o] = inv_div * sum_b c_b * sum_rc colsum_part[b,rc,o] + noise.
