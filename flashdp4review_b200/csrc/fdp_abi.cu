@@ -277,8 +277,9 @@ int fdp_linear_wgrad(const void* G, const void* X, void* dW, float* norms_out, f
   if (split) {
     char* sg = static_cast<char*>(w.tc_extra) + w.tc.split_bytes;
     char* sx = sg + w.tc.split_g_bytes;
-    if (!w.short_seq && (st = tc_split(G, sg, static_cast<size_t>(B) * T, n_out, w.tc.planes, nullptr, T, s)) != FDP_OK) return st;
-    if ((st = tc_split(X, sx, static_cast<size_t>(B) * T, n_in, w.tc.planes, nullptr, T, s)) != FDP_OK) return st;
+    const SplitJob jobs[2] = {{G, sg, static_cast<size_t>(B) * T, n_out, nullptr, T}, {X, sx, static_cast<size_t>(B) * T, n_in, nullptr, T}};
+    // (short sequences: when the clip factors are there)
+    if (!w.short_seq && (st = tc_split(jobs, 2, w.tc.planes, w.status, s)) != FDP_OK) return st;
     Gt = sg; Xt = sx; tdt = FDP_BF16;
   }
   if (w.short_seq) {
@@ -296,7 +297,9 @@ int fdp_linear_wgrad(const void* G, const void* X, void* dW, float* norms_out, f
     float* split_ws = static_cast<float*>(w.tc_extra);
     char* gs = static_cast<char*>(w.tc_extra) + w.tc.split_bytes;
     if (split && w.short_seq) {     // c_b G in fp32, then its parts
-      if ((st = tc_split(G, gs, static_cast<size_t>(B) * T, n_out, w.tc.planes, w.factors, T, s)) != FDP_OK) return st;
+      const SplitJob jobs[2] = {{G, gs, static_cast<size_t>(B) * T, n_out, w.factors, T},
+                                {X, gs + w.tc.split_g_bytes, static_cast<size_t>(B) * T, n_in, nullptr, T}};
+      if ((st = tc_split(jobs, 2, w.tc.planes, nullptr, s)) != FDP_OK) return st;
     } else if (!w.tc.scaled_epilogue) {
       if ((st = tc_prescale(G, w.factors, gs, B, T, n_out, in_dtype, s)) != FDP_OK) return st;
     }
@@ -386,11 +389,11 @@ static int gemm3_call(const void* A, const void* W, const void* bias, void* Y, i
   int* status = static_cast<int*>(workspace);
   char* a3 = static_cast<char*>(workspace) + 256;
   char* w3 = a3 + ((static_cast<size_t>(rows) * K * 4 + 255) & ~static_cast<size_t>(255));
-  FDP_CUDA_OK(cudaMemsetAsync(status, 0, sizeof(int), s));
-  int st;
-  if ((st = tc_split(A, a3, static_cast<size_t>(rows), K, 2, nullptr, 1, s)) != FDP_OK) return st;
   // W is [K, N] (w_kn) or [N, K]: either way its rows are split along their own columns
-  if ((st = tc_split(W, w3, static_cast<size_t>(w_kn ? K : N), w_kn ? N : K, 2, nullptr, 1, s)) != FDP_OK) return st;
+  const SplitJob jobs[2] = {{A, a3, static_cast<size_t>(rows), K, nullptr, 1},
+                            {W, w3, static_cast<size_t>(w_kn ? K : N), w_kn ? N : K, nullptr, 1}};
+  const int st = tc_split(jobs, 2, 2, status, s);
+  if (st != FDP_OK) return st;
   return tc_gemm3(a3, w3, bias, Y, status, rows, K, N, out_dtype, w_kn, s);
 }
 

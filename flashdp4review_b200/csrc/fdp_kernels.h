@@ -135,8 +135,9 @@ struct TcPlan {
 };
 TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo);
 // fp32 [rows, n] -> bf16 [rows, planes, n rounded up to 8]: high parts, then what is left of them, ...; row r is
-// multiplied by factors[r / T] first (factors may be null)
-int tc_split(const void* src, void* dst, size_t rows, int n, int planes, const float* factors, int T, cudaStream_t s);
+// multiplied by factors[r / T] first (factors may be null).  One or two operands; clears *zero_status if not null
+struct SplitJob { const void* src; void* dst; size_t rows; int n; const float* factors; int T; };
+int tc_split(const SplitJob* jobs, int njobs, int planes, int* zero_status, cudaStream_t s);
 // With pl.planes > 1, G and X are the split matrices and dt is FDP_BF16.
 int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int B, int T, int n_in,
              int n_out, int dt, const TcPlan& pl, cudaStream_t s);

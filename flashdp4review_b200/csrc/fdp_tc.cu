@@ -953,32 +953,42 @@ __global__ void __launch_bounds__(256) prescale_kernel(const Tin* __restrict__ G
 }
 
 // ---- fp32 -> PLANES bf16 parts: dst[r, 0, c] = bf16(f x), dst[r, 1, c] = bf16(f x - hi), ..., with the column
-// count rounded up to a multiple of 8 (zeros) and f a per-sample factor (1 when factors is null) --------------
-template <int PLANES, bool VEC>
-__global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ src, uint4* __restrict__ dst, unsigned nvec,
-                                                    int n, unsigned vec_per_row, const float* __restrict__ factors, int T) {
-  for (unsigned i = blockIdx.x * 256u + threadIdx.x; i < nvec; i += gridDim.x * 256u) {
-    const unsigned row = i / vec_per_row, cv = i - row * vec_per_row;
+// count rounded up to a multiple of 8 (zeros) and f a per-sample factor (1 when factors is null).  Both operands
+// of a product in one launch: blocks below `first` work on job 0 ---------------------------------------------
+struct SplitRun {
+  const float* src; uint4* dst; const float* factors;
+  unsigned nvec, vec_per_row;
+  int n, T, vec;       // vec: n a multiple of 4, src 16-byte aligned
+};
+template <int PLANES>
+__global__ void __launch_bounds__(256) split_kernel(const SplitRun j0, const SplitRun j1, unsigned first, int* zero_status) {
+  pdl_trigger();       // the product that follows sets itself up meanwhile
+  if (zero_status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *zero_status = 0;
+  const bool second = blockIdx.x >= first;
+  const SplitRun& j = second ? j1 : j0;
+  const unsigned block = second ? blockIdx.x - first : blockIdx.x, blocks = second ? gridDim.x - first : first;
+  for (unsigned i = block * 256u + threadIdx.x; i < j.nvec; i += blocks * 256u) {
+    const unsigned row = i / j.vec_per_row, cv = i - row * j.vec_per_row;
     const int c0 = static_cast<int>(cv) * 8;
-    const float* p = src + static_cast<size_t>(row) * n + c0;
+    const float* p = j.src + static_cast<size_t>(row) * j.n + c0;
     float f[8];
-    if (VEC) {     // n a multiple of 4, 16-byte aligned
+    if (j.vec) {
       unpack16<float>(__ldg(reinterpret_cast<const uint4*>(p)), f);
-      unpack16<float>(c0 + 4 < n ? __ldg(reinterpret_cast<const uint4*>(p) + 1) : make_uint4(0, 0, 0, 0), f + 4);
+      unpack16<float>(c0 + 4 < j.n ? __ldg(reinterpret_cast<const uint4*>(p) + 1) : make_uint4(0, 0, 0, 0), f + 4);
     } else {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) f[e] = c0 + e < n ? __ldg(p + e) : 0.f;
+      for (int e = 0; e < 8; ++e) f[e] = c0 + e < j.n ? __ldg(p + e) : 0.f;
     }
-    if (factors != nullptr) {
-      const float c = __ldg(factors + row / T);
+    if (j.factors != nullptr) {
+      const float c = __ldg(j.factors + row / j.T);
 #pragma unroll
       for (int e = 0; e < 8; ++e) f[e] *= c;
     }
-    uint4* o = dst + static_cast<size_t>(row) * (PLANES * vec_per_row) + cv;
+    uint4* o = j.dst + static_cast<size_t>(row) * (PLANES * j.vec_per_row) + cv;
 #pragma unroll
     for (int pl = 0; pl < PLANES; ++pl) {
       const uint4 h = pack16<__nv_bfloat16>(f);
-      o[pl * vec_per_row] = h;
+      o[pl * j.vec_per_row] = h;
       float hf[8];
       unpack16<__nv_bfloat16>(h, hf);
 #pragma unroll
@@ -1313,22 +1323,37 @@ TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
   return p;
 }
 
-int tc_split(const void* src, void* dst, size_t rows, int n, int planes, const float* factors, int T, cudaStream_t s) {
-  const unsigned vpr = pitch8(n) / 8;
-  const bool vec = n % 4 == 0 && aligned16(src);
-  const size_t max_rows = (1u << 31) / vpr;       // 32-bit index arithmetic within a launch
-  for (size_t r = 0; r < rows; r += max_rows) {
-    const size_t nr = rows - r < max_rows ? rows - r : max_rows;
-    if (r != 0 && factors != nullptr) return FDP_ERR_SHAPE;     // (factors come with short sequences only)
-    const unsigned nvec = static_cast<unsigned>(nr) * vpr;
-    const unsigned blocks = (nvec + 255) / 256, cap = static_cast<unsigned>(sm_count()) * 16;
-    const unsigned grid = blocks < cap ? blocks : cap;
-    const float* in = static_cast<const float*>(src) + r * n;
-    uint4* out = static_cast<uint4*>(dst) + r * vpr * planes;
-#define FDP_SPLIT(P_, V_) split_kernel<P_, V_><<<grid, 256, 0, s>>>(in, out, nvec, n, vpr, factors, T)
-    if (planes == 2) { if (vec) FDP_SPLIT(2, true); else FDP_SPLIT(2, false); }
-    else { if (vec) FDP_SPLIT(3, true); else FDP_SPLIT(3, false); }
-#undef FDP_SPLIT
+int tc_split(const SplitJob* jobs, int njobs, int planes, int* zero_status, cudaStream_t s) {
+  SplitRun r[2] = {};
+  unsigned blocks[2] = {0, 0};
+  // 32-bit index arithmetic within a launch: an operand past that is cut along its rows
+  size_t done[2] = {0, 0};
+  for (;;) {
+    for (int k = 0; k < 2; ++k) {
+      blocks[k] = 0;
+      if (k >= njobs || done[k] >= jobs[k].rows) continue;
+      const SplitJob& j = jobs[k];
+      const unsigned vpr = pitch8(j.n) / 8;
+      const size_t most = (1u << 31) / vpr, left = j.rows - done[k], nr = left < most ? left : most;
+      if (nr < j.rows && j.factors != nullptr) return FDP_ERR_SHAPE;   // (factors come with short sequences only)
+      r[k].src = static_cast<const float*>(j.src) + done[k] * j.n;
+      r[k].dst = static_cast<uint4*>(j.dst) + done[k] * vpr * planes;
+      r[k].factors = j.factors; r[k].T = j.T; r[k].n = j.n; r[k].vec_per_row = vpr;
+      r[k].nvec = static_cast<unsigned>(nr * vpr);
+      r[k].vec = j.n % 4 == 0 && aligned16(r[k].src);
+      blocks[k] = (r[k].nvec + 255) / 256;
+      done[k] += nr;
+    }
+    if (blocks[0] + blocks[1] == 0) break;
+    // 16 blocks an SM in all, shared in proportion to the work
+    const unsigned cap = static_cast<unsigned>(sm_count()) * 16;
+    const unsigned long long all = static_cast<unsigned long long>(blocks[0]) + blocks[1];
+    if (all > cap) {
+      for (int k = 0; k < 2; ++k)
+        if (blocks[k] > 0) blocks[k] = static_cast<unsigned>(blocks[k] * static_cast<unsigned long long>(cap) / all) + 1;
+    }
+    if (planes == 2) split_kernel<2><<<blocks[0] + blocks[1], 256, 0, s>>>(r[0], r[1], blocks[0], zero_status);
+    else split_kernel<3><<<blocks[0] + blocks[1], 256, 0, s>>>(r[0], r[1], blocks[0], zero_status);
     note_launch();
   }
   return cudaPeekAtLastError() == cudaSuccess ? FDP_OK : (cudaGetLastError(), FDP_ERR_LAUNCH);
@@ -1356,6 +1381,7 @@ int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int
     args.idesc = make_idesc(dt, true, true, ctas);
     args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = chain_stages(args.seg_stages, pl.planes);
     args.scale = 1.0f; args.nk = NoiseKey{};
+    args.zero_status = 0; args.dependent = 1;      // follows the split kernel, which has cleared the status word
     if (pl.planes == 3)
       return ctas == 2 ? launch<true, true, EPI_SPLIT6_SUMSQ, 2>(a, b, a, b, a, args, s)
                        : launch<true, true, EPI_SPLIT6_SUMSQ, 1>(a, b, a, b, a, args, s);
