@@ -159,8 +159,11 @@ __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap
       "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(leader_bar) : "memory");
 }
-__device__ __forceinline__ void tc_commit_pair(uint32_t cluster_bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar) : "memory");
+// arrives on the barrier at this offset in both CTAs of the pair.  (One commit to both, not one each: a commit holds
+// the tensor pipe up by about 30 cycles; 32768 rows 4096 -> 4096 bf16: 732 -> 699 us.)
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
 }
 __device__ __forceinline__ void tc_mma_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -574,12 +577,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   } else if (warp == 1) {
     // ================= MMA issuer (the leader CTA of a pair issues for both) =================
     auto commit = [&](uint32_t bar) {   // signals `bar` (in both CTAs of a pair) when the MMAs issued so far are done
-      if (CTAS == 1) {
-        tc_commit(bar);
-      } else {
-        tc_commit_pair(bar);
-        tc_commit_pair(mapa_u32(bar, 1));
-      }
+      if (CTAS == 1) tc_commit(bar); else tc_commit_pair(bar);
     };
     // The six products of K slices [k0, k1) of a stage, smallest first: the accumulator is added to by truncation,
     // one unit in its last place per step, so the steps that come before it is large cost nothing.
@@ -606,6 +604,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // a single-block unit multiplies by the first 128 rows of the B stage only (N = 128)
         const uint32_t idesc = half ? args.idesc_half : args.idesc;
         int ks = ks0;
+        // stages left of the sample at ks, and how far into a hand-off a K split has put the unit's start
+        int sample_left = 0, sub_off = 0;
+        if (epi_chained(EPI)) {
+          sample_left = args.seg_stages - ks0 % args.seg_stages;
+          sub_off = (args.seg_stages - sample_left) % args.sub_stages;
+        }
         // one accumulator per segment: the whole unit, or one sample's share of it for EPI_STORE_SCALED
         if constexpr (SUBS > 1) {
           for (; ks < ks1 && ok; ++ks) {
@@ -624,7 +628,14 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         while (ks < ks1 && ok) {
           const int seg_begin = ks;
-          const int seg_end = epi_chained(EPI) ? segment_end(ks, ks1) : ks1;
+          int seg_end = ks1;
+          if (epi_chained(EPI)) {      // segment_end(ks, ks1) without its divisions
+            const int len = min(args.sub_stages - sub_off, sample_left);
+            sub_off = 0;
+            seg_end = min(ks + len, ks1);
+            sample_left -= len;
+            if (sample_left == 0) sample_left = args.seg_stages;
+          }
           const int acc = it % NUM_ACC;
           const uint32_t acc_phase = (it / NUM_ACC) & 1u;
           if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, wctx, 2)) { ok = false; break; }
@@ -667,7 +678,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       }
       if (!ok) {
         // let MMAs already issued finish before TMEM is released
-        if (CTAS == 1) tc_commit(drain_bar); else tc_commit_pair(drain_bar);
+        commit(drain_bar);
         const long long t0 = clock64();
         while (!mbar_try(drain_bar, 0) && clock64() - t0 < WAIT_LIMIT_CYCLES / 8) {}
       }
@@ -1165,12 +1176,10 @@ int ctas_per_tile() { return forced_ctas() == 1 ? 1 : 2; }
 // tiles than workers) are cut into s parts of equal K-stage count, so that the last round keeps more
 // SMs busy; cost in tile-times = ceil(rem*s/workers)/s plus the cost of parking and re-reading the
 // accumulators.  At most 2 * workers parked parts (workers <= MAX_SMS / CTAS).
-// That cost, in tile-times: 0.05 for the fix-up launch plus 0.15 per parked part and worker (the
-// parts are written and read again).  With 48 pair tiles of 128 K stages for 74 pairs (a GPT-2
-// layer, B=8, T=1024) three parts of 43 stages in two rounds measured no faster than the tiles
-// unsplit (100.8 against 98.6 us per call: parking, the second round's hand-over and the fix-up
-// launch eat the 42 stages saved), while 16 tiles in four parts (52 against 82 us) and the tails of
-// the larger layers do pay.
+// That cost, in K stages of bf16 (0.40 us each): 6 for the fix-up launch, 0.11 per part that it reads back
+// (256 KB), 4 for each further round.  Measured, GEMM + fix-up: 48 pair tiles of 256 stages for 74 pairs 110 us
+// unsplit, 117 in two parts, 91 in three; 16 tiles of 128 stages 54 / 37 / 30 / 26 us in one to four parts; 64 tiles
+// of 128 stages 62 us unsplit, 72 in two parts.
 int plan_tail_split(int total_tiles, int k_stages, int workers, int products) {
   const int rem = total_tiles <= workers ? total_tiles : total_tiles % workers;
   // stages are counted by their work: with split fp32 operands one holds three or six products
@@ -1182,8 +1191,9 @@ int plan_tail_split(int total_tiles, int k_stages, int workers, int products) {
   int best_s = 1; double best = 1.0;
   for (int sp = 2; sp <= 16; ++sp) {
     if (rem * sp > 2 * workers || k_stages / sp < min_stages) break;
-    const double cost = static_cast<double>((rem * sp + workers - 1) / workers) / sp +
-                        0.15 * (static_cast<double>(rem) * sp / workers) + 0.05;
+    const int rounds = (rem * sp + workers - 1) / workers;
+    const double cost = static_cast<double>(rounds) / sp +
+                        (6.0 + 0.11 * rem * sp + 4.0 * (rounds - 1)) / (static_cast<double>(k_stages) * products);
     if (cost < best - 0.03) { best = cost; best_s = sp; }
   }
   return best_s;

@@ -73,3 +73,30 @@ def test_fp32_six_products(ops, B, T, n_in, n_out, layout):
     ops.dp_linear_weight_grad(X, zero, 1.0, 1.0, layout=layout, noise=noise, fp32_tensor=True, out=out)
     assert torch.equal(out, ops.dp_linear_weight_grad(X, zero, 1.0, 1.0, layout=layout, noise=noise, fp32_tensor=False))
     assert float(flat[0]) == 0.0
+
+
+# many samples of few rows (at most 16 rows and more than 64 samples take kernels of their own): both sides of that line,
+# widths off the 16-byte vectors, one row a sample
+@pytest.mark.parametrize("B,T,n", [(64, 1, 256), (65, 1, 1000), (1025, 1, 257), (300, 3, 72), (66, 16, 130), (66, 17, 130), (4000, 2, 8)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_bias_gradient_of_short_samples(ops, B, T, n, dtype):
+    G = _randn(B, T, n, seed=3, dtype=dtype, scale=0.1)
+    db, norms, factors = ops.dp_bias_grad(G, 0.5, 1.0, out_dtype=torch.float32, return_norms=True)
+    want_n = G.double().flatten(1).norm(dim=1)
+    # sums of squares over T * n elements in chains of at most T * n / 32, then the root halves the error
+    assert float(((norms.double() - want_n) / want_n).abs().max()) < (T * n / 64 + 8) * 2.0 ** -23
+    f = (0.5 / (want_n + 1e-10)).clamp(max=1.0)
+    assert float(((factors.double() - f) / f).abs().max()) < (T * n / 64 + 10) * 2.0 ** -23
+    want = torch.einsum("bto,b->o", G.double(), f) / (B * T)
+    absum = torch.einsum("bto,b->o", G.double().abs(), f) / (B * T)
+    _close_to_sum(db, want, absum, B * T / 8 + T * n / 64 + 20, 2.0 ** -23)
+
+
+# the norm of samples of one row is the product of the rows' norms
+@pytest.mark.parametrize("B,n_in,n_out", [(1, 8, 8), (9, 1000, 1024), (300, 129, 65)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_norms_of_one_row_samples(ops, B, n_in, n_out, dtype):
+    X, G = _randn(B, 1, n_in, seed=4, dtype=dtype), _randn(B, 1, n_out, seed=5, dtype=dtype, scale=1e-2)
+    _, norms, _ = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, return_norms=True)
+    want = G.double().flatten(1).norm(dim=1) * X.double().flatten(1).norm(dim=1)
+    assert float(((norms.double() - want) / want).abs().max()) < ((n_in + n_out) / 64 + 12) * 2.0 ** -23
