@@ -235,6 +235,38 @@ def linear_input_grad(grad_output, weight, w_layout="out_in", out_dtype=None, fp
     return dX
 
 
+def dp_linear_backward(input, grad_output, weight, C, clamp_value, *, need_dx=True, need_dw=True, need_db=True,
+                       batch_divisor=None, noise=None, noise_bias=None, layout="out_in", dx_dtype=None, dw_dtype=None,
+                       db_dtype=None, norm_algo="auto", out=None):
+    """(dX, dW, db) of one layer in one library call: linear_input_grad, dp_linear_weight_grad and dp_bias_grad
+    with one normalisation of the operands, one workspace and, for fp32 on the tensor cores, one split of
+    grad_output.  input (B,T,in), grad_output (B,T,out); None in the place of what is not needed."""
+    host = _lib.host()
+    _require_cuda(input, grad_output, weight if need_dx else None)
+    if input.dim() != 3 or grad_output.dim() != 3 or input.shape[:2] != grad_output.shape[:2]:
+        raise RuntimeError(f"expected (B,T,in) and (B,T,out), got {tuple(input.shape)} and {tuple(grad_output.shape)}")
+    G = _aligned(grad_output.contiguous())
+    dt = G.dtype
+    X = _aligned(input.to(dt).contiguous())
+    W = _aligned(weight.to(dt).contiguous()) if need_dx else None
+    code = _dt(dt)
+    algo = NORM_ALGOS[norm_algo]
+    if dt == torch.float32 and runtime.fp32_mode() == "tensor":
+        algo |= _lib.FDP_FP32_TENSOR | _lib.FDP_FP32_WIDE
+    if out is not None:
+        shape = (G.shape[-1], X.shape[-1]) if layout == "out_in" else (X.shape[-1], G.shape[-1])
+        if tuple(out.shape) != shape or not out.is_contiguous() or out.device != G.device:
+            raise RuntimeError(f"out must be a contiguous {shape} tensor on {G.device}")
+        dw_dtype = out.dtype
+    p = _params(C, clamp_value, batch_divisor, noise)
+    st, dX, dW, db = host.linear_bwd(
+        G, X, W, out if need_dw else None, code, _dt(dx_dtype or dt), _dt(dw_dtype or dt), _dt(db_dtype or dt),
+        _lib.FDP_OUT_IN if layout == "out_in" else _lib.FDP_IN_OUT, algo, p,
+        _params(C, clamp_value, batch_divisor, noise_bias) if need_db else p, need_dx, need_dw, need_db)
+    _lib.check(st, "fdp_linear_bwd")
+    return dX, dW, db
+
+
 def linear_forward(input, weight, bias=None, w_layout="out_in", out_dtype=None, fp32_tensor=None):
     """input @ weight.t() + bias (nn.Linear, weight [out,in]) or input @ weight + bias (Conv1D, weight
     [in,out]) -- flashdp/layers/linear.py:41-46, transformers_conv1d.py:40-43."""

@@ -236,29 +236,12 @@ size_t fdp_linear_wgrad_workspace_bytes(int B, int T, int n_in, int n_out, int i
   return wgrad_ws(nullptr, B, T, n_in, n_out, in_dtype, norm_algo).bytes;
 }
 
-int fdp_linear_wgrad(const void* G, const void* X, void* dW, float* norms_out, float* factors_out,
-                     int B, int T, int n_in, int n_out, int in_dtype, int out_dtype, int layout,
-                     int norm_algo, const fdp_dp_params* p, void* workspace, size_t workspace_bytes,
-                     fdp_stream_t stream) {
-  NvtxRange nvtx_range("fdp_linear_wgrad");
-  if (G == nullptr || X == nullptr || dW == nullptr) return FDP_ERR_ARG;
-  if (B <= 0 || T <= 0 || n_in <= 0 || n_out <= 0) return FDP_ERR_ARG;
-  if (layout != FDP_OUT_IN && layout != FDP_IN_OUT) return FDP_ERR_ARG;
-  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
-    return FDP_ERR_ARG;
-  if (!valid_dtype(in_dtype) || !valid_dtype(out_dtype)) return FDP_ERR_DTYPE;
-  if (static_cast<long long>(B) * T >= (1ll << 31) / 2) return FDP_ERR_SHAPE;   // row indices are 32-bit
-  int st = check_params(p);
-  if (st != FDP_OK) return st;
-  if ((st = current_device_ok()) != FDP_OK) return st;
-  if (workspace == nullptr) return FDP_ERR_WORKSPACE;
-  WgradWs w = wgrad_ws(workspace, B, T, n_in, n_out, in_dtype, norm_algo);
-  if (workspace_bytes < w.bytes || !aligned16(workspace)) return FDP_ERR_WORKSPACE;
-  // the tensor-core path moves 16-byte vectors (TMA, vector stores); the generic kernels, and the split
-  // copies of fp32 operands with six products, take any naturally aligned pointer
-  if (w.tc.ok && !w.tc.any_align && (!aligned16(G) || !aligned16(X) || !aligned16(dW))) return FDP_ERR_ALIGN;
-
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
+// The launches of a weight gradient, behind the argument checks.  presplit: the bf16 parts of G and X are in the
+// workspace already and the status word is cleared.
+static int wgrad_run(const void* G, const void* X, void* dW, float* norms_out, float* factors_out, int B, int T, int n_in,
+                     int n_out, int in_dtype, int out_dtype, int layout, int norm_algo, const fdp_dp_params* p, WgradWs& w,
+                     bool presplit, cudaStream_t s) {
+  int st = FDP_OK;
   const int div = p->batch_divisor > 0 ? p->batch_divisor : B;
   const float inv_div = 1.0f / static_cast<float>(div);
   const NoiseKey nk = make_noise_key(p, p->param_id);
@@ -279,7 +262,7 @@ int fdp_linear_wgrad(const void* G, const void* X, void* dW, float* norms_out, f
     char* sx = sg + w.tc.split_g_bytes;
     const SplitJob jobs[2] = {{G, sg, static_cast<size_t>(B) * T, n_out, nullptr, T}, {X, sx, static_cast<size_t>(B) * T, n_in, nullptr, T}};
     // (short sequences: when the clip factors are there)
-    if (!w.short_seq && (st = tc_split(jobs, 2, w.tc.planes, w.status, s)) != FDP_OK) return st;
+    if (!w.short_seq && !presplit && (st = tc_split(jobs, 2, w.tc.planes, w.status, s)) != FDP_OK) return st;
     Gt = sg; Xt = sx; tdt = FDP_BF16;
   }
   if (w.short_seq) {
@@ -321,6 +304,32 @@ int fdp_linear_wgrad(const void* G, const void* X, void* dW, float* norms_out, f
   prof_mark(4, s);
   FDP_LAUNCH_OK();
   return FDP_OK;
+}
+
+int fdp_linear_wgrad(const void* G, const void* X, void* dW, float* norms_out, float* factors_out,
+                     int B, int T, int n_in, int n_out, int in_dtype, int out_dtype, int layout,
+                     int norm_algo, const fdp_dp_params* p, void* workspace, size_t workspace_bytes,
+                     fdp_stream_t stream) {
+  NvtxRange nvtx_range("fdp_linear_wgrad");
+  if (G == nullptr || X == nullptr || dW == nullptr) return FDP_ERR_ARG;
+  if (B <= 0 || T <= 0 || n_in <= 0 || n_out <= 0) return FDP_ERR_ARG;
+  if (layout != FDP_OUT_IN && layout != FDP_IN_OUT) return FDP_ERR_ARG;
+  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
+    return FDP_ERR_ARG;
+  if (!valid_dtype(in_dtype) || !valid_dtype(out_dtype)) return FDP_ERR_DTYPE;
+  if (static_cast<long long>(B) * T >= (1ll << 31) / 2) return FDP_ERR_SHAPE;   // row indices are 32-bit
+  int st = check_params(p);
+  if (st != FDP_OK) return st;
+  if ((st = current_device_ok()) != FDP_OK) return st;
+  if (workspace == nullptr) return FDP_ERR_WORKSPACE;
+  WgradWs w = wgrad_ws(workspace, B, T, n_in, n_out, in_dtype, norm_algo);
+  if (workspace_bytes < w.bytes || !aligned16(workspace)) return FDP_ERR_WORKSPACE;
+  // the tensor-core path moves 16-byte vectors (TMA, vector stores); the generic kernels, and the split
+  // copies of fp32 operands with six products, take any naturally aligned pointer
+  if (w.tc.ok && !w.tc.any_align && (!aligned16(G) || !aligned16(X) || !aligned16(dW))) return FDP_ERR_ALIGN;
+
+  return wgrad_run(G, X, dW, norms_out, factors_out, B, T, n_in, n_out, in_dtype, out_dtype, layout, norm_algo, p, w, false,
+                   static_cast<cudaStream_t>(stream));
 }
 
 // ---- bias gradient ----------------------------------------------------------------------------------
@@ -456,6 +465,117 @@ int fdp_linear_fwd(const void* X, const void* W, const void* bias, void* Y, int 
   }
   FDP_LAUNCH_OK();
   return FDP_OK;
+}
+
+// ---- the whole backward of a Linear / Conv1D layer ----------------------------------------------------------
+namespace {
+// Whether one set of split copies can serve both products: fp32 on the tensor cores with the parts made before the
+// norms, and an input gradient that takes them too.
+struct LinearBwdWs {
+  WgradWs w;
+  bool shared;
+  char* w_parts;      // split copy of W
+  GstatsPlan pl;
+  float* factors; float* sq_part; float* colsum_part;
+  size_t bytes;
+};
+LinearBwdWs linear_bwd_ws(void* base, int B, int T, int n_in, int n_out, int dtype, int norm_algo, int outputs) {
+  LinearBwdWs q{};
+  const int rows = B * T;
+  q.w = wgrad_ws(base, B, T, n_in, n_out, dtype, norm_algo);
+  q.shared = (outputs & FDP_BWD_DW) != 0 && (outputs & (FDP_BWD_DX | FDP_BWD_DB)) != 0 && q.w.tc.ok && q.w.tc.planes > 1 && !q.w.short_seq &&
+             ((outputs & FDP_BWD_DX) == 0 || tc_gemm3_ok(rows, n_out, n_in));
+  if (!q.shared) {
+    size_t most = q.w.bytes;
+    const size_t d = fdp_linear_dgrad_workspace_bytes(rows, n_in, n_out, dtype == FDP_F32 ? dtype | (norm_algo & FDP_FP32_TENSOR) : dtype);
+    const size_t g = fdp_bias_grad_workspace_bytes(B, T, n_out, dtype);
+    if (d > most) most = d;
+    if (g > most) most = g;
+    q.bytes = most;
+    return q;
+  }
+  Carver c(base);
+  c.off = q.w.bytes;
+  q.w_parts = c.take<char>((outputs & FDP_BWD_DX) ? tc_gemm3_w_bytes(n_out, n_in, q.w.tc.planes) : 0);
+  q.pl = gstats_plan(B, T, n_out, dtype);
+  q.factors = c.take<float>(B);
+  q.sq_part = c.take<float>(static_cast<size_t>(B) * q.pl.row_chunks * q.pl.col_chunks);
+  q.colsum_part = c.take<float>(static_cast<size_t>(B) * q.pl.row_chunks * n_out);
+  q.bytes = c.off;
+  return q;
+}
+}  // namespace
+
+size_t fdp_linear_bwd_workspace_bytes(int B, int T, int n_in, int n_out, int in_dtype, int norm_algo, int outputs) {
+  if (B <= 0 || T <= 0 || n_in <= 0 || n_out <= 0 || !valid_dtype(in_dtype)) return 0;
+  if (static_cast<long long>(B) * T >= (1ll << 31) / 2) return 0;
+  return linear_bwd_ws(nullptr, B, T, n_in, n_out, in_dtype, norm_algo, outputs).bytes;
+}
+
+int fdp_linear_bwd(const void* G, const void* X, const void* W, void* dX, void* dW, void* db, int B, int T, int n_in, int n_out,
+                   int in_dtype, int dx_dtype, int dw_dtype, int db_dtype, int layout, int norm_algo, const fdp_dp_params* p,
+                   const fdp_dp_params* p_bias, void* workspace, size_t workspace_bytes, fdp_stream_t stream) {
+  if (B <= 0 || T <= 0 || n_in <= 0 || n_out <= 0) return FDP_ERR_ARG;
+  if (static_cast<long long>(B) * T >= (1ll << 31) / 2) return FDP_ERR_SHAPE;   // row indices are 32-bit
+  if (!valid_dtype(in_dtype)) return FDP_ERR_DTYPE;
+  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
+    return FDP_ERR_ARG;
+  const int outputs = (dX ? FDP_BWD_DX : 0) | (dW ? FDP_BWD_DW : 0) | (db ? FDP_BWD_DB : 0);
+  if (outputs == 0) return FDP_ERR_ARG;
+  const int rows = B * T;
+  LinearBwdWs q = linear_bwd_ws(workspace, B, T, n_in, n_out, in_dtype, norm_algo, outputs);
+  if (workspace == nullptr || workspace_bytes < q.bytes || !aligned16(workspace)) return FDP_ERR_WORKSPACE;
+  // the shared form takes any operand the separate calls take: pointers that the input gradient's product cannot use,
+  // and everything else, go through them
+  if (q.shared && (dX == nullptr || (W != nullptr && aligned16(W) && aligned16(dX) && aligned16(G))) && aligned16(dW) && aligned16(X) && aligned16(G)) {
+    NvtxRange nvtx_range("fdp_linear_bwd");
+    if (G == nullptr || X == nullptr) return FDP_ERR_ARG;
+    if (layout != FDP_OUT_IN && layout != FDP_IN_OUT) return FDP_ERR_ARG;
+    if (!valid_dtype(dw_dtype) || (dX && !valid_dtype(dx_dtype)) || (db && !valid_dtype(db_dtype))) return FDP_ERR_DTYPE;
+    int st = check_params(p);
+    if (st == FDP_OK && db != nullptr) st = check_params(p_bias);
+    if (st != FDP_OK) return st;
+    if ((st = current_device_ok()) != FDP_OK) return st;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int planes = q.w.tc.planes;
+    char* sg = static_cast<char*>(q.w.tc_extra) + q.w.tc.split_bytes;
+    char* sx = sg + q.w.tc.split_g_bytes;
+    const SplitJob jg{G, sg, static_cast<size_t>(rows), n_out, nullptr, T}, jx{X, sx, static_cast<size_t>(rows), n_in, nullptr, T};
+    const bool w_kn = layout == FDP_OUT_IN;      // W's rows are the contraction of dX = G W
+    const SplitJob jw{W, q.w_parts, static_cast<size_t>(w_kn ? n_out : n_in), w_kn ? n_in : n_out, nullptr, 1};
+    const bool stats = db != nullptr && tc_split_stats_ok(G, n_out);
+    if (stats) {
+      if ((st = tc_split_stats(G, sg, q.colsum_part, q.sq_part, B, T, n_out, planes, q.pl, s)) != FDP_OK) return st;
+    } else {
+      if (db != nullptr) gstats(G, q.colsum_part, q.sq_part, B, T, n_out, in_dtype, q.pl, s);
+      if ((st = tc_split(&jg, 1, planes, nullptr, s)) != FDP_OK) return st;
+    }
+    const SplitJob jobs[2] = {jx, jw};
+    if ((st = tc_split(jobs, dX != nullptr ? 2 : 1, planes, q.w.status, s)) != FDP_OK) return st;
+    if ((st = wgrad_run(G, X, dW, nullptr, nullptr, B, T, n_in, n_out, in_dtype, dw_dtype, layout, norm_algo, p, q.w, true, s)) != FDP_OK)
+      return st;
+    if (dX != nullptr &&
+        (st = tc_gemm3(sg, q.w_parts, nullptr, dX, q.w.status, rows, n_out, n_in, dx_dtype, w_kn, s, planes)) != FDP_OK)
+      return st;
+    if (db != nullptr) {
+      const int div = p_bias->batch_divisor > 0 ? p_bias->batch_divisor : B;
+      bias_clip_finalize(q.colsum_part, q.sq_part, q.pl.row_chunks * q.pl.col_chunks, p_bias->C, p_bias->clamp_value, q.factors,
+                         nullptr, nullptr, db, B, n_out, q.pl.row_chunks, db_dtype,
+                         1.0f / (static_cast<float>(div) * static_cast<float>(T)), make_noise_key(p_bias, p_bias->param_id), s);
+    }
+    FDP_LAUNCH_OK();
+    return FDP_OK;
+  }
+  int st = FDP_OK;
+  if (dX != nullptr)
+    st = fdp_linear_dgrad(G, W, dX, rows, n_in, n_out, in_dtype == FDP_F32 ? in_dtype | (norm_algo & FDP_FP32_TENSOR) : in_dtype,
+                          dx_dtype, layout, workspace, workspace_bytes, stream);
+  if (st == FDP_OK && dW != nullptr)
+    st = fdp_linear_wgrad(G, X, dW, nullptr, nullptr, B, T, n_in, n_out, in_dtype, dw_dtype, layout, norm_algo, p, workspace,
+                          workspace_bytes, stream);
+  if (st == FDP_OK && db != nullptr)
+    st = fdp_bias_grad(G, db, nullptr, nullptr, B, T, n_out, in_dtype, db_dtype, p_bias, workspace, workspace_bytes, stream);
+  return st;
 }
 
 // ---- LayerNorm ------------------------------------------------------------------------------------------

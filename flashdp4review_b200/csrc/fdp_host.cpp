@@ -23,6 +23,8 @@ struct Abi {
   decltype(&fdp_bias_grad) bias_grad;
   decltype(&fdp_linear_dgrad_workspace_bytes) linear_dgrad_workspace_bytes;
   decltype(&fdp_linear_dgrad) linear_dgrad;
+  decltype(&fdp_linear_bwd_workspace_bytes) linear_bwd_workspace_bytes;
+  decltype(&fdp_linear_bwd) linear_bwd;
   decltype(&fdp_linear_fwd) linear_fwd;
   decltype(&fdp_layernorm_fwd) layernorm_fwd;
   decltype(&fdp_layernorm_bwd_workspace_bytes) layernorm_bwd_workspace_bytes;
@@ -33,6 +35,7 @@ void bind(const std::map<std::string, uint64_t>& fns) {
 #define FDP_BIND(NAME) abi.NAME = reinterpret_cast<decltype(abi.NAME)>(fns.at("fdp_" #NAME))
   FDP_BIND(linear_wgrad_workspace_bytes); FDP_BIND(linear_wgrad);
   FDP_BIND(bias_grad_workspace_bytes); FDP_BIND(bias_grad);
+  FDP_BIND(linear_bwd_workspace_bytes); FDP_BIND(linear_bwd);
   FDP_BIND(linear_dgrad_workspace_bytes); FDP_BIND(linear_dgrad); FDP_BIND(linear_fwd);
   FDP_BIND(layernorm_fwd); FDP_BIND(layernorm_bwd_workspace_bytes); FDP_BIND(layernorm_bwd);
 #undef FDP_BIND
@@ -120,6 +123,29 @@ py::tuple linear_dgrad(const Tensor& G, const Tensor& W, int rows, int code, int
   return py::make_tuple(st, dX);
 }
 
+// G, X as (B, T, .); W only where dX is wanted
+py::tuple linear_bwd(const Tensor& G, const Tensor& X, const OptTensor& W, const OptTensor& out, int in_dt, int dx_dt, int dw_dt, int db_dt,
+                     int layout, int algo, const py::tuple& p, const py::tuple& p_bias, bool need_dx, bool need_dw, bool need_db) {
+  const fdp_dp_params q = params(p), qb = params(p_bias);
+  const c10::cuda::CUDAGuard guard(G.device());
+  const int B = static_cast<int>(X.size(0)), T = static_cast<int>(X.size(1));
+  const int n_in = static_cast<int>(X.size(2)), n_out = static_cast<int>(G.size(2));
+  OptTensor dX, dW, db;
+  if (need_dx) dX = with_columns(G, n_in, dx_dt);
+  if (need_dw) dW = out.has_value() ? *out
+                    : layout == FDP_OUT_IN ? new_tensor(G, {n_out, n_in}, scalar_type(dw_dt)) : new_tensor(G, {n_in, n_out}, scalar_type(dw_dt));
+  if (need_db) db = new_tensor(G, {n_out}, scalar_type(db_dt));
+  const int outputs = (need_dx ? FDP_BWD_DX : 0) | (need_dw ? FDP_BWD_DW : 0) | (need_db ? FDP_BWD_DB : 0);
+  const Tensor ws = workspace(G, abi.linear_bwd_workspace_bytes(B, T, n_in, n_out, in_dt, algo, outputs));
+  int st;
+  {
+    py::gil_scoped_release nogil;
+    st = abi.linear_bwd(ptr(G), ptr(X), ptr(W), ptr(dX), ptr(dW), ptr(db), B, T, n_in, n_out, in_dt, dx_dt, dw_dt, db_dt, layout, algo,
+                        &q, &qb, ptr(ws), ws.numel(), stream(G));
+  }
+  return py::make_tuple(st, dX, dW, db);
+}
+
 py::tuple linear_fwd(const Tensor& X, const Tensor& W, const OptTensor& bias, int rows, int code, int out_dt, int w_layout) {
   const c10::cuda::CUDAGuard guard(X.device());
   const int n_in = static_cast<int>(X.size(-1)), n_out = static_cast<int>(W.size(w_layout == FDP_OUT_IN ? 0 : 1));
@@ -175,6 +201,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("linear_wgrad", &linear_wgrad);
   m.def("bias_grad", &bias_grad);
   m.def("linear_dgrad", &linear_dgrad);
+  m.def("linear_bwd", &linear_bwd);
   m.def("linear_fwd", &linear_fwd);
   m.def("layernorm_fwd", &layernorm_fwd);
   m.def("layernorm_bwd", &layernorm_bwd);

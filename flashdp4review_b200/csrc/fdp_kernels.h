@@ -91,6 +91,11 @@ void bias_clip_finalize(const float* colsum_part, const float* sq_part, int npar
                         float* factors_ws, float* norms_out, float* factors_out, void* db, int B, int n_out,
                         int row_chunks, int out_dt, float inv_div, NoiseKey nk, cudaStream_t s);
 
+// tc_split of G [B * T, n_out] and gstats in one pass (fp32, plan of gstats_plan)
+bool tc_split_stats_ok(const void* G, int n_out);
+int tc_split_stats(const void* G, void* dst, float* colsum_part, float* sq_part, int B, int T, int n_out, int planes,
+                   const GstatsPlan& pl, cudaStream_t s);
+
 // ---- LayerNorm -----------------------------------------------------------------------------------
 struct LnPlan { int tpr, cpt, cw, rows_per_block, chunks; bool vec; };
 LnPlan ln_plan(int B, int T, int d, int dt);
@@ -166,8 +171,9 @@ bool tc_dgrad_ok(int rows, int n_in, int n_out, int dt);
 // by tc_split (A3 [rows, 2K]; W3 [K, 2N] if w_kn, else [N, 2K]); workspace for the two split copies
 bool tc_gemm3_ok(int rows, int K, int N);
 size_t tc_gemm3_ws_bytes(int rows, int K, int N);
+size_t tc_gemm3_w_bytes(int K, int N, int planes);     // the split copy of W alone
 int tc_gemm3(const void* A3, const void* W3, const void* bias, void* Y, int* dev_status, int rows, int K, int N,
-             int out_dt, bool w_kn, cudaStream_t s);
+             int out_dt, bool w_kn, cudaStream_t s, int planes = 2);
 int tc_fwd(const void* X, const void* W, const void* bias, void* Y, int* dev_status, int rows, int n_in,
            int n_out, int dt, int out_dt, int w_layout, cudaStream_t s);
 int tc_dgrad(const void* G, const void* W, void* dX, int* dev_status, int rows, int n_in, int n_out,

@@ -1008,6 +1008,63 @@ __global__ void __launch_bounds__(256) split_kernel(const SplitRun j0, const Spl
   }
 }
 
+// ---- the same for G, with the bias gradient's statistics taken from the pass (grid and partials of gstats_kernel) ---
+// In a whole backward G is split once for both products, and the column sums and sums of squares cost no read of
+// their own: 8192 x 3072 fp32, G 33 + 33 + 23 us (two splits and the statistics) as separate passes, one pass here.
+template <int PLANES>
+__global__ void __launch_bounds__(256, 4) split_stats_kernel(const float* __restrict__ G, uint2* __restrict__ dst,
+                                                             float* __restrict__ colsum_part, float* __restrict__ sq_part,
+                                                             int T, int n_out, int pitch, int rows_per_chunk,
+                                                             int col_chunks, int row_chunks) {
+  __shared__ float cs[8][32 * 4];
+  __shared__ float red[32];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int cc = blockIdx.x % col_chunks, rc = (blockIdx.x / col_chunks) % row_chunks;
+  const int b = blockIdx.x / (col_chunks * row_chunks);
+  const int c0 = (cc * 32 + x) * 4;
+  const int r0 = rc * rows_per_chunk, r1 = min(T, r0 + rows_per_chunk);
+  float acc[4] = {0.f, 0.f, 0.f, 0.f}, sq = 0.f;
+  if (c0 < n_out) {
+    const bool pad = c0 + 4 == n_out && pitch > n_out;
+    auto take = [&](int r, const float4& v) {
+      float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { acc[e] += f[e]; sq = fmaf(f[e], f[e], sq); }
+      uint2* o = dst + ((static_cast<size_t>(b) * T + r) * PLANES * pitch + c0) / 4;
+#pragma unroll
+      for (int pl = 0; pl < PLANES; ++pl) {
+        const __nv_bfloat162 h0 = __floats2bfloat162_rn(f[0], f[1]), h1 = __floats2bfloat162_rn(f[2], f[3]);
+        o[pl * pitch / 4] = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+        if (pad) o[pl * pitch / 4 + 1] = make_uint2(0u, 0u);
+        f[0] -= __low2float(h0); f[1] -= __high2float(h0); f[2] -= __low2float(h1); f[3] -= __high2float(h1);
+      }
+    };
+    constexpr int U = 4;
+    int r = r0 + y;
+    for (; r + 8 * (U - 1) < r1; r += 8 * U) {
+      float4 v[U];
+#pragma unroll
+      for (int k = 0; k < U; ++k) v[k] = __ldg(reinterpret_cast<const float4*>(G + (static_cast<size_t>(b) * T + r + 8 * k) * n_out + c0));
+#pragma unroll
+      for (int k = 0; k < U; ++k) take(r + 8 * k, v[k]);
+    }
+    for (; r < r1; r += 8) take(r, __ldg(reinterpret_cast<const float4*>(G + (static_cast<size_t>(b) * T + r) * n_out + c0)));
+  }
+#pragma unroll
+  for (int v = 0; v < 4; ++v) cs[y][x * 4 + v] = acc[v];
+  sq = block_sum(sq, red);  // contains the __syncthreads that publishes cs
+  if (threadIdx.x == 0) sq_part[blockIdx.x] = sq;
+  for (int c = threadIdx.x; c < 128; c += 256) {
+    const int col = cc * 128 + c;
+    if (col < n_out) {
+      float t = 0.f;
+#pragma unroll
+      for (int yy = 0; yy < 8; ++yy) t += cs[yy][c];
+      colsum_part[(static_cast<size_t>(b) * row_chunks + rc) * n_out + col] = t;
+    }
+  }
+}
+
 // ---- host side ------------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1369,6 +1426,17 @@ int tc_split(const SplitJob* jobs, int njobs, int planes, int* zero_status, cuda
   return cudaPeekAtLastError() == cudaSuccess ? FDP_OK : (cudaGetLastError(), FDP_ERR_LAUNCH);
 }
 
+bool tc_split_stats_ok(const void* G, int n_out) { return n_out % 4 == 0 && aligned16(G); }
+int tc_split_stats(const void* G, void* dst, float* colsum_part, float* sq_part, int B, int T, int n_out, int planes,
+                   const GstatsPlan& pl, cudaStream_t s) {
+  const unsigned grid = static_cast<unsigned>(static_cast<size_t>(B) * pl.row_chunks * pl.col_chunks);
+  auto kernel = planes == 2 ? split_stats_kernel<2> : split_stats_kernel<3>;
+  kernel<<<grid, 256, 0, s>>>(static_cast<const float*>(G), static_cast<uint2*>(dst), colsum_part, sq_part, T, n_out, pitch8(n_out),
+                              pl.rows_per_chunk, pl.col_chunks, pl.row_chunks);
+  note_launch();
+  return cudaPeekAtLastError() == cudaSuccess ? FDP_OK : (cudaGetLastError(), FDP_ERR_LAUNCH);
+}
+
 int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int B, int T, int n_in,
              int n_out, int dt, const TcPlan& pl, cudaStream_t s) {
   const uint64_t rows = static_cast<uint64_t>(B) * T;
@@ -1570,20 +1638,22 @@ int tc_fwd(const void* X, const void* W, const void* bias, void* Y, int* dev_sta
 }
 
 // ---- fp32 products on the tensor cores: Y[rows, N] = A[rows, K] * W (+ bias) --------------------------
-// A3 is [rows, 2K] and W3 [K, 2N] (w_kn) or [N, 2K] (else): bf16 high halves then low halves (tc_split).
+// A3 is [rows, 2K] and W3 [K, 2N] (w_kn) or [N, 2K] (else): bf16 high halves then low halves (tc_split), or three
+// parts each (planes), of which the first two are the halves.
 // Three bf16 products per K range into accumulators that the epilogue warps take over every few K
 // stages and sum in registers (chain_stages), then the ordinary store epilogue.
 bool tc_gemm3_ok(int rows, int K, int N) {
   return rows >= 128 && K >= 128 && N >= 128 && K % BK == 0 && N % 8 == 0;
 }
+size_t tc_gemm3_w_bytes(int K, int N, int planes) { return align256(static_cast<size_t>(K) * N * 2 * planes); }
 size_t tc_gemm3_ws_bytes(int rows, int K, int N) {
   return align256(static_cast<size_t>(rows) * K * 4) + align256(static_cast<size_t>(K) * N * 4);
 }
 int tc_gemm3(const void* A3, const void* W3, const void* bias, void* Y, int* dev_status, int rows, int K, int N,
-             int out_dt, bool w_kn, cudaStream_t s) {
+             int out_dt, bool w_kn, cudaStream_t s, int planes) {
   CUtensorMap ma, mw, mo;
   const int ctas = ctas_per_tile();
-  if (!make_map(&ma, A3, rows, 2 * K, BK, BM, FDP_BF16) || !make_out_map(&mo, Y, rows, N, out_dt)) return FDP_ERR_LAUNCH;
+  if (!make_map(&ma, A3, rows, static_cast<uint64_t>(planes) * K, BK, BM, FDP_BF16) || !make_out_map(&mo, Y, rows, N, out_dt)) return FDP_ERR_LAUNCH;
   TcArgs args{};
   args.batch = 1; args.batch_rows = 0; args.status = dev_status;
   args.dependent = 1;            // follows the split kernels of the same call
@@ -1597,12 +1667,12 @@ int tc_gemm3(const void* A3, const void* W3, const void* bias, void* Y, int* dev
   args.bias = bias; args.bias_dt = FDP_F32; args.bias_vec = aligned16(bias);
   args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = chain_stages(args.seg_stages, 2);
   if (w_kn) {   // rows of W3 are K, N contiguous
-    if (!make_map(&mw, W3, K, 2 * N, 64, BK, FDP_BF16)) return FDP_ERR_LAUNCH;
+    if (!make_map(&mw, W3, K, static_cast<uint64_t>(planes) * N, 64, BK, FDP_BF16)) return FDP_ERR_LAUNCH;
     args.idesc = make_idesc(FDP_BF16, false, true, ctas);
     return ctas == 2 ? launch<false, true, EPI_SPLIT_STORE, 2>(ma, mw, ma, mw, mo, args, s)
                      : launch<false, true, EPI_SPLIT_STORE, 1>(ma, mw, ma, mw, mo, args, s);
   }
-  if (!make_map(&mw, W3, N, 2 * K, BK, BN / ctas, FDP_BF16)) return FDP_ERR_LAUNCH;   // K contiguous
+  if (!make_map(&mw, W3, N, static_cast<uint64_t>(planes) * K, BK, BN / ctas, FDP_BF16)) return FDP_ERR_LAUNCH;   // K contiguous
   args.idesc = make_idesc(FDP_BF16, false, false, ctas);
   return ctas == 2 ? launch<false, false, EPI_SPLIT_STORE, 2>(ma, mw, ma, mw, mo, args, s)
                    : launch<false, false, EPI_SPLIT_STORE, 1>(ma, mw, ma, mw, mo, args, s);

@@ -44,33 +44,33 @@ class _DPLinearFunc(Function):
         B = x3.shape[0]
         step = layer._next_step()
         grad_input = grad_weight = grad_bias = None
+        need_dx, need_dw = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
+        need_db = bias is not None and ctx.needs_input_grad[2]
 
-        if ctx.needs_input_grad[0]:
-            if ops.native_product_ok(
-                    g3.dtype, g3.numel() // g3.shape[-1], w_for_dx.shape[0], w_for_dx.shape[1]):
-                grad_input = ops.linear_input_grad(g3, w_for_dx, "out_in", out_dtype=ctx.input_dtype)
-            else:
-                grad_input = g3 @ w_for_dx.to(g3.dtype)
-            grad_input = grad_input.reshape(input.shape)
+        native_dx = need_dx and ops.native_product_ok(
+            g3.dtype, g3.numel() // g3.shape[-1], w_for_dx.shape[0], w_for_dx.shape[1])
+        if need_dx and not native_dx:
+            grad_input = g3 @ w_for_dx.to(g3.dtype)
 
-        if ctx.needs_input_grad[1]:
+        if native_dx or need_dw or need_db:
             div, noise = dp_scalars(B, layer.noise_multiplier, layer._dp_param_ids[0], step)
-            target = direct_grad_target(weight)      # a gradient-bucket slice, or None
-            grad_weight = ops.dp_linear_weight_grad(
-                x3, g3, layer.C, layer.clamp_value, batch_divisor=div, noise=noise,
-                layout="out_in", out_dtype=weight.dtype, norm_algo=layer.norm_algo, out=target)
-            if grad_weight.shape != weight.shape:
+            _, noise_bias = dp_scalars(B, layer.noise_multiplier, layer._dp_param_ids[1], step)
+            target = direct_grad_target(weight) if need_dw else None      # a gradient-bucket slice, or None
+            dx, grad_weight, grad_bias = ops.dp_linear_backward(
+                x3, g3, w_for_dx, layer.C, layer.clamp_value, need_dx=native_dx, need_dw=need_dw, need_db=need_db,
+                batch_divisor=div, noise=noise, noise_bias=noise_bias, layout="out_in", dx_dtype=ctx.input_dtype,
+                dw_dtype=weight.dtype, db_dtype=bias.dtype if need_db else None, norm_algo=layer.norm_algo, out=target)
+            if native_dx:
+                grad_input = dx
+            if need_dw and grad_weight.shape != weight.shape:
                 raise RuntimeError(f"grad_weight shape {grad_weight.shape} is not equal to weight shape {weight.shape}")
             if target is not None:
                 direct_grad_done(weight)
                 grad_weight = None                    # already where the optimizer and the all-reduce read it
-
-        if bias is not None and ctx.needs_input_grad[2]:
-            div, noise = dp_scalars(B, layer.noise_multiplier, layer._dp_param_ids[1], step)
-            grad_bias = ops.dp_bias_grad(g3, layer.C, layer.clamp_value, batch_divisor=div,
-                                         noise=noise, out_dtype=bias.dtype)
-            if grad_bias.shape != bias.shape:
+            if need_db and grad_bias.shape != bias.shape:
                 raise RuntimeError(f"grad_bias shape {grad_bias.shape} is not equal to bias shape {bias.shape}")
+        if need_dx:
+            grad_input = grad_input.reshape(input.shape)
 
         return grad_input, grad_weight, grad_bias, None
 

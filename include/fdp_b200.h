@@ -32,7 +32,7 @@ extern "C" {
 /* 2: asynchronous status word, SM reservation, saturating LayerNorm mode, FDP_FP32_TENSOR.
  * 3: fdp_dp_params.step_device (appended; earlier fields keep their offsets); FDP_FP32_TENSOR also
  *    accepted in the dtype of fdp_linear_dgrad / fdp_linear_fwd.
- * 4: FDP_FP32_WIDE. */
+ * 4: FDP_FP32_WIDE, fdp_linear_bwd. */
 #define FDP_ABI_VERSION 4
 
 typedef void* fdp_stream_t; /* a cudaStream_t */
@@ -218,6 +218,18 @@ size_t fdp_linear_dgrad_workspace_bytes(int rows, int n_in, int n_out, int dtype
 int fdp_linear_dgrad(const void* G, const void* W, void* dX, int rows, int n_in, int n_out,
                      int dtype, int out_dtype, int w_layout, void* workspace, size_t workspace_bytes,
                      fdp_stream_t stream);
+
+/* ---- the whole backward of a Linear / Conv1D layer ----------------------------------------------
+ * What fdp_linear_dgrad, fdp_linear_wgrad and fdp_bias_grad compute, in one call with one workspace; each of dX, dW, db
+ * may be null (W too when dX is).  `layout` is that of W and of dW.  p belongs to the weight, p_bias to the bias.
+ * fp32 inputs with FDP_FP32_TENSOR / FDP_FP32_WIDE in norm_algo: G is split into its bf16 parts once for both
+ * products, in the pass that also takes the bias gradient's statistics. */
+enum fdp_bwd_outputs { FDP_BWD_DX = 1, FDP_BWD_DW = 2, FDP_BWD_DB = 4 };
+size_t fdp_linear_bwd_workspace_bytes(int B, int T, int n_in, int n_out, int in_dtype, int norm_algo, int outputs);
+int fdp_linear_bwd(const void* G, const void* X, const void* W, void* dX, void* dW, void* db, int B, int T,
+                   int n_in, int n_out, int in_dtype, int dx_dtype, int dw_dtype, int db_dtype, int layout,
+                   int norm_algo, const fdp_dp_params* p, const fdp_dp_params* p_bias, void* workspace,
+                   size_t workspace_bytes, fdp_stream_t stream);
 
 /* ---- forward -----------------------------------------------------------------------------------
  * `input @ weight.t() + bias` of flashdp/layers/linear.py:41-46 (w_layout FDP_OUT_IN, W [n_out,n_in]) and

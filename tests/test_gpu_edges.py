@@ -100,3 +100,25 @@ def test_norms_of_one_row_samples(ops, B, n_in, n_out, dtype):
     _, norms, _ = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, return_norms=True)
     want = G.double().flatten(1).norm(dim=1) * X.double().flatten(1).norm(dim=1)
     assert float(((norms.double() - want) / want).abs().max()) < ((n_in + n_out) / 64 + 12) * 2.0 ** -23
+
+
+# one call for the whole backward: bit for bit what the three calls give, whether or not the split copies are shared
+# (fp32: three products, six products with and without 16-byte rows, short sequences; 16 bit: plain)
+@pytest.mark.parametrize("dtype,B,T,n_in,n_out", [
+    (torch.float32, 4, 128, 256, 384), (torch.float32, 3, 197, 264, 320), (torch.float32, 2, 100, 136, 196), (torch.float32, 5, 70, 130, 128),
+    (torch.float32, 40, 7, 128, 128), (torch.float32, 2, 130, 128, 129), (torch.bfloat16, 3, 256, 264, 136), (torch.float16, 4, 77, 128, 192)])
+@pytest.mark.parametrize("layout", ["out_in", "in_out"])
+@pytest.mark.parametrize("need", [(True, True, True), (True, True, False), (False, True, True), (True, False, True)])
+def test_whole_backward_equals_its_parts(ops, dtype, B, T, n_in, n_out, layout, need):
+    X, G = _randn(B, T, n_in, seed=6, dtype=dtype), _randn(B, T, n_out, seed=7, dtype=dtype, scale=1e-2)
+    W = _randn(*((n_out, n_in) if layout == "out_in" else (n_in, n_out)), seed=8, dtype=dtype, scale=0.05)
+    nw, nb = ops.NoiseSpec(0.01, 5, 2, 0, 9), ops.NoiseSpec(0.01, 5, 3, 0, 9)
+    dX, dW, db = ops.dp_linear_backward(X, G, W, 0.7, 1.0, need_dx=need[0], need_dw=need[1], need_db=need[2], noise=nw,
+                                        noise_bias=nb, layout=layout, dw_dtype=torch.float32, db_dtype=torch.float32)
+    assert (dX is not None, dW is not None, db is not None) == need
+    if need[0]:
+        assert torch.equal(dX, ops.linear_input_grad(G, W, layout))
+    if need[1]:
+        assert torch.equal(dW, ops.dp_linear_weight_grad(X, G, 0.7, 1.0, noise=nw, layout=layout, out_dtype=torch.float32))
+    if need[2]:
+        assert torch.equal(db, ops.dp_bias_grad(G, 0.7, 1.0, noise=nb, out_dtype=torch.float32))
