@@ -122,3 +122,23 @@ def test_whole_backward_equals_its_parts(ops, dtype, B, T, n_in, n_out, layout, 
         assert torch.equal(dW, ops.dp_linear_weight_grad(X, G, 0.7, 1.0, noise=nw, layout=layout, out_dtype=torch.float32))
     if need[2]:
         assert torch.equal(db, ops.dp_bias_grad(G, 0.7, 1.0, noise=nb, out_dtype=torch.float32))
+
+
+# LayerNorm backward with rows whose ring stages are 64 KB (wide fp32): a chunk shorter than the ring, a ragged last
+# stage, widths that do and do not fill the threads' columns
+@pytest.mark.parametrize("B,T,d", [(2, 3, 1024), (3, 37, 1000), (2, 70, 4096), (2, 33, 8192), (1, 130, 5000)])
+def test_layernorm_backward_of_wide_fp32_rows(ops, B, T, d):
+    x, dy = _randn(B, T, d, seed=9, dtype=torch.float32), _randn(B, T, d, seed=10, dtype=torch.float32, scale=0.1)
+    w, b = 1.0 + _randn(d, seed=11, dtype=torch.float32, scale=0.1), torch.zeros(d, device=dev())
+    _, buf, _ = ops.layernorm_fwd_fused(x, w, b, 1e-5)
+    dx, dg, db = ops.dp_layernorm_backward(dy, x, w, buf["mean"], buf["rstd"], 1e6, 1.0, batch_divisor=1)
+    xd, dyd, wd = x.double(), dy.double(), w.double()
+    rs = 1.0 / torch.sqrt(xd.var(-1, unbiased=False, keepdim=True) + 1e-5)
+    xh = (xd - xd.mean(-1, keepdim=True)) * rs
+    wdy = dyd * wd
+    want = rs * (wdy - xh * (wdy * xh).mean(-1, keepdim=True) - wdy.mean(-1, keepdim=True))
+    absum = rs * (wdy.abs() + xh.abs() * (wdy * xh).abs().mean(-1, keepdim=True) + wdy.abs().mean(-1, keepdim=True))
+    # a row's sums run in chains of at most d / 32 additions; mean and rstd carry as many
+    _close_to_sum(dx, want, absum, d / 16 + 16, 2.0 ** -23)
+    _close_to_sum(dg, (dyd * xh).sum((0, 1)), (dyd * xh).abs().sum((0, 1)) + rs.mean() * dyd.abs().sum((0, 1)), B * T + d / 32 + 16, 2.0 ** -23)
+    _close_to_sum(db, dyd.sum((0, 1)), dyd.abs().sum((0, 1)), B * T + 8, 2.0 ** -23)
