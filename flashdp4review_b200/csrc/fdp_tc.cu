@@ -1360,8 +1360,6 @@ TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
     p.ws_bytes = p.split_bytes + align256(static_cast<size_t>(B) * T * n_out * 2);
     return p;
   }
-  // direct: a K stage must not run into the next sample's rows
-  const bool direct_ok = (T % BK == 0);
   // Cost of the two norm algorithms in K stages on the critical path: both kernels deal equal work
   // units (128x256 tiles) round-robin to one CTA per SM, so a pass takes
   // ceil(units / SMs) * (stages per unit + a fixed cost per unit of about four stages).  The SM
@@ -1373,15 +1371,16 @@ TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
   const double gram = static_cast<double>((units_g + PLAN_SMS - 1) / PLAN_SMS) *
                       (ceil_div(n_in, BK) + ceil_div(n_out, BK) + UNIT_FIXED_STAGES);
   int algo = norm_algo;
-  if (algo == FDP_NORM_AUTO) algo = (direct_ok && direct <= gram) ? FDP_NORM_DIRECT : FDP_NORM_GRAM;
-  if (algo == FDP_NORM_DIRECT && !direct_ok) algo = FDP_NORM_GRAM;
+  if (algo == FDP_NORM_AUTO) algo = direct <= gram ? FDP_NORM_DIRECT : FDP_NORM_GRAM;
   p.ok = true;
   p.algo = algo;
-  // clip factors applied in the GEMM epilogue (no scaled copy of G) when every 64-row K stage lies
-  // inside one sample and a sample's main loop is long enough to hide the per-sample drain;
-  // FDP_WGRAD_PRESCALE=1 forces the pre-scale pass (for A/B measurements)
+  // clip factors applied in the GEMM epilogue (no scaled copy of G) when a sample's main loop is long
+  // enough to hide the per-sample drain and its last K stage is not mostly padding: the padded rows cost
+  // pad * n_in * n_out multiply-adds a sample, the pre-scale pass reads and writes T * n_out elements, about
+  // 400 multiply-adds' time each.  FDP_WGRAD_PRESCALE=1 forces the pre-scale pass (for A/B measurements)
   static const bool force_prescale = [] { const char* e = getenv("FDP_WGRAD_PRESCALE"); return e && e[0] == '1'; }();
-  p.scaled_epilogue = !force_prescale && (T % BK == 0) && T >= 256;
+  const long long pad = static_cast<long long>(ceil_div(T, BK)) * BK - T;
+  p.scaled_epilogue = !force_prescale && T >= 256 && pad * n_in <= 400ll * T;
   // one partial per work unit and epilogue warp
   p.nparts = 4 * ((algo == FDP_NORM_DIRECT) ? ceil_div(n_out, BM) * ceil_div(n_in, BN) : gram_tiles(T));
   // the parked accumulators of the split-K tail, then (pre-scale path only) the c_b-scaled copy of G
@@ -1471,7 +1470,7 @@ int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int
     args.M = n_out; args.N = n_in;
     args.tiles_m = ceil_div(n_out, BM); args.tiles_n = ceil_div(n_in, BN);
     args.tiles_per_batch = args.tiles_m * args.tiles_n;
-    args.k_stages = T / BK; args.seg_stages = args.k_stages;
+    args.k_stages = ceil_div(T, BK); args.seg_stages = args.k_stages;
     args.idesc = make_idesc(dt, true, true);
     return launch<true, true, EPI_SUMSQ>(a, b, a, b, a, args, s);
   }

@@ -142,3 +142,22 @@ def test_layernorm_backward_of_wide_fp32_rows(ops, B, T, d):
     _close_to_sum(dx, want, absum, d / 16 + 16, 2.0 ** -23)
     _close_to_sum(dg, (dyd * xh).sum((0, 1)), (dyd * xh).abs().sum((0, 1)) + rs.mean() * dyd.abs().sum((0, 1)), B * T + d / 32 + 16, 2.0 ** -23)
     _close_to_sum(db, dyd.sum((0, 1)), dyd.abs().sum((0, 1)), B * T + 8, 2.0 ** -23)
+
+
+# 16-bit weight gradients whose samples end inside a K stage: factors in the epilogue or in a copy of G, norms by product
+# tiles or by Gram blocks
+@pytest.mark.parametrize("B,T,n_in,n_out", [(3, 257, 136, 264), (2, 300, 520, 128), (12, 500, 256, 256), (2, 319, 2048, 128), (5, 65, 128, 128)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("algo", ["auto", "direct", "gram"])
+def test_ragged_samples_16bit(ops, B, T, n_in, n_out, dtype, algo):
+    X, G = _randn(B, T, n_in, seed=12, dtype=dtype), _randn(B, T, n_out, seed=13, dtype=dtype, scale=1e-2)
+    G[0] *= 30.0
+    dW, norms, _ = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, norm_algo=algo, out_dtype=torch.float32, return_norms=True)
+    per = torch.einsum("bto,bti->boi", G.double(), X.double())
+    want_n = per.flatten(1).norm(dim=1)
+    assert float(((norms.double() - want_n) / want_n).abs().max()) < 1e-4
+    f = (1.0 / (want_n + 1e-10)).clamp(max=1.0)
+    absum = torch.einsum("bto,bti,b->oi", G.double().abs(), X.double().abs(), f) / B
+    # fp32 sums; the pre-scaled copy rounds c_b G to the input type, half a unit each
+    err = (dW.double() - torch.einsum("boi,b->oi", per, f) / B).abs()
+    assert bool((err <= (UNIT[dtype] / 2 + (B * T / 16 + 32) * 2.0 ** -23) * absum).all())
