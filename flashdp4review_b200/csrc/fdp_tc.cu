@@ -3,11 +3,12 @@
 // accumulators in TMEM -> tcgen05.ld epilogue.  Instances (A major, B major, epilogue, CTAs per tile):
 //   wgrad   MN, MN, STORE_SCALED, 2   dW = scale * sum_b c_b G_b^T X_b + noise; every sample's K segment has
 //                                     its own TMEM accumulator, added times c_b into registers
-//           MN, MN, STORE, 2          same from a pre-scaled copy of G (T not a multiple of 64, or short T)
+//           MN, MN, STORE, 2          same from a pre-scaled copy of G (T < 256, or mostly padded K stages)
 //   direct  MN, MN, SUMSQ, 1          per-sample ||G_b^T X_b||_F^2: tile squared in the epilogue, never stored
 //   gram    K,  K,  GRAM, 1           sum_{t,s} (G_b G_b^T)_{ts} (X_b X_b^T)_{ts}, two accumulators in TMEM
 //   dgrad   K,  MN or K, STORE, 2     dX = G W
 //   forward K,  K or MN, STORE, 2     Y = X W^T + bias
+//   fp32    the same products over bf16 parts of the operands: SPLIT_* three products, SPLIT6_* six
 // Roles in a CTA: warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner, warps 2-5 (2-9 for the
 // store epilogues) = epilogue, each on the TMEM lane quarter warp % 4.  With two CTAs per tile the
 // even CTA of a 2-CTA cluster issues tcgen05.mma.cta_group::2 for both.  Every mbarrier wait is

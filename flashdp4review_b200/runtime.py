@@ -198,8 +198,9 @@ def set_fp32_mode(name: str):
     features and sequence length (at least 128 each) run on the tensor cores as three bf16 products
     (x = hi + lo; hi*hi + hi*lo + lo*hi) whose fp32 accumulators are drained into registers every few K
     stages -- within 1e-5 of float64 like the fp32-FMA kernels (measured 4e-6 on the gradient, 4e-7 on the
-    norms at 4096x4096) and about six times faster; other shapes use the FMA kernels.  "exact": always
-    the fp32-FMA kernels, the reference's own arithmetic."""
+    norms at 4096x4096) and about six times faster; other shapes (widths of at least 64) as six products over
+    three parts, no further from float64 than the FMA kernels.  "exact": always the fp32-FMA kernels, the
+    reference's own arithmetic."""
     if name not in ("exact", "tensor"):
         raise ValueError("fp32_mode must be 'exact' or 'tensor'")
     _run.fp32_mode = name
