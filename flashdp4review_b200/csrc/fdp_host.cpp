@@ -50,6 +50,18 @@ Tensor new_tensor(const Tensor& like, at::IntArrayRef sizes, at::ScalarType t) {
 Tensor workspace(const Tensor& like, size_t bytes) {
   return new_tensor(like, {static_cast<int64_t>(bytes < 256 ? 256 : bytes)}, at::kByte);
 }
+// The workspace of a call with `algo`.  Split copies of fp32 operands are 1.5 times the inputs: where they do not
+// fit the card the shapes of FDP_FP32_WIDE stay on the FMA kernels, which need next to nothing.
+template <typename Query>
+Tensor algo_workspace(const Tensor& like, int& algo, Query query) {
+  try {
+    return workspace(like, query(algo));
+  } catch (const c10::OutOfMemoryError&) {
+    if ((algo & FDP_FP32_WIDE) == 0) throw;
+    algo &= ~FDP_FP32_WIDE;
+    return workspace(like, query(algo));
+  }
+}
 void* ptr(const Tensor& t) { return t.data_ptr(); }
 void* ptr(const OptTensor& t) { return t.has_value() ? t->data_ptr() : nullptr; }
 fdp_stream_t stream(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
@@ -75,8 +87,7 @@ py::tuple linear_wgrad(const Tensor& G, const Tensor& X, const OptTensor& out, i
               : layout == FDP_OUT_IN ? new_tensor(G, {n_out, n_in}, scalar_type(out_dt)) : new_tensor(G, {n_in, n_out}, scalar_type(out_dt));
   OptTensor norms, factors;
   if (want_norms) { norms = new_tensor(G, {B}, at::kFloat); factors = new_tensor(G, {B}, at::kFloat); }
-  const size_t bytes = abi.linear_wgrad_workspace_bytes(B, T, n_in, n_out, in_dt, algo);
-  const Tensor ws = workspace(G, bytes);
+  const Tensor ws = algo_workspace(G, algo, [&](int a) { return abi.linear_wgrad_workspace_bytes(B, T, n_in, n_out, in_dt, a); });
   int st;
   {
     py::gil_scoped_release nogil;
@@ -136,7 +147,7 @@ py::tuple linear_bwd(const Tensor& G, const Tensor& X, const OptTensor& W, const
                     : layout == FDP_OUT_IN ? new_tensor(G, {n_out, n_in}, scalar_type(dw_dt)) : new_tensor(G, {n_in, n_out}, scalar_type(dw_dt));
   if (need_db) db = new_tensor(G, {n_out}, scalar_type(db_dt));
   const int outputs = (need_dx ? FDP_BWD_DX : 0) | (need_dw ? FDP_BWD_DW : 0) | (need_db ? FDP_BWD_DB : 0);
-  const Tensor ws = workspace(G, abi.linear_bwd_workspace_bytes(B, T, n_in, n_out, in_dt, algo, outputs));
+  const Tensor ws = algo_workspace(G, algo, [&](int a) { return abi.linear_bwd_workspace_bytes(B, T, n_in, n_out, in_dt, a, outputs); });
   int st;
   {
     py::gil_scoped_release nogil;

@@ -161,3 +161,20 @@ def test_ragged_samples_16bit(ops, B, T, n_in, n_out, dtype, algo):
     # fp32 sums; the pre-scaled copy rounds c_b G to the input type, half a unit each
     err = (dW.double() - torch.einsum("boi,b->oi", per, f) / B).abs()
     assert bool((err <= (UNIT[dtype] / 2 + (B * T / 16 + 32) * 2.0 ** -23) * absum).all())
+
+
+def test_six_products_fall_back_where_their_workspace_does_not_fit(ops):
+    """fp32 shapes that ran in little memory before still do: without room for the split copies and the parking area
+    (38.8 MB) the FMA kernels take the call."""
+    X, G = _randn(4, 100, 256, seed=14, dtype=torch.float32), _randn(4, 100, 192, seed=15, dtype=torch.float32)
+    want = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, fp32_tensor=False)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (24 << 20)) / total)
+        got = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, fp32_tensor=True)
+        _, dW, _ = ops.dp_linear_backward(X, G, None, 1.0, 1.0, need_dx=False)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.equal(got, want) and torch.equal(dW, want)
