@@ -209,3 +209,55 @@ def test_forward_and_input_gradient_gemm_selection():
     finally:
         runtime.set_input_grad_impl(before)
         runtime.set_fp32_mode(before32)
+
+
+@pytest.fixture
+def no_launch(monkeypatch):
+    """The operator layer on CPU tensors, with a call layer that fails the test when it is entered."""
+    from flashdp4review_b200 import _lib
+    from flashdp4review_b200.core import ops
+
+    class Launched(Exception):
+        pass
+
+    class Host:
+        def __getattr__(self, name):
+            def call(*args):
+                raise Launched(name)
+            return call
+    monkeypatch.setattr(_lib, "host", Host)
+    monkeypatch.setattr(ops, "_require_cuda", lambda *tensors: None)
+    return ops, Launched
+
+
+@pytest.mark.parametrize("layout", ["out_in", "in_out"])
+def test_operands_that_do_not_fit_are_refused_before_a_launch(no_launch, layout):
+    """The kernels take the weight as a bare pointer: another shape than (out, in) or (in, out) would be misread, a
+    smaller one read past its end."""
+    ops, Launched = no_launch
+    X, G = torch.zeros(2, 3, 16), torch.zeros(2, 3, 8)
+    right = (8, 16) if layout == "out_in" else (16, 8)
+    shapes = [right[::-1], (right[0], right[1] + 1), (right[0] + 1, right[1]), (right[0] - 1, right[1]), (4, 4), right + (1,), (128,)]
+    for shape in shapes:
+        with pytest.raises(RuntimeError, match="weight"):
+            ops.dp_linear_backward(X, G, torch.zeros(shape), 1.0, 1.0, layout=layout)
+        if len(shape) != 2 or shape[0 if layout == "out_in" else 1] != 8:
+            with pytest.raises(RuntimeError, match="weight"):
+                ops.linear_input_grad(G, torch.zeros(shape), layout)
+        if len(shape) != 2 or shape[1 if layout == "out_in" else 0] != 16:
+            with pytest.raises(RuntimeError, match="weight"):
+                ops.linear_forward(X, torch.zeros(shape), None, layout)
+    W = torch.zeros(right)
+    with pytest.raises(RuntimeError, match="weight"):
+        ops.dp_linear_backward(X, G, W.to("meta"), 1.0, 1.0, layout=layout)
+    with pytest.raises(RuntimeError, match="input is on"):
+        ops.dp_linear_backward(X.to("meta"), G, W, 1.0, 1.0, layout=layout)
+    with pytest.raises(RuntimeError, match="bias"):
+        ops.linear_forward(X, W, torch.zeros(7), layout)
+    # what fits goes through, and a weight that is not needed is not looked at
+    for call in (lambda: ops.dp_linear_backward(X, G, W, 1.0, 1.0, layout=layout),
+                 lambda: ops.dp_linear_backward(X, G, None, 1.0, 1.0, layout=layout, need_dx=False),
+                 lambda: ops.linear_input_grad(G, W, layout), lambda: ops.linear_forward(X, W, torch.zeros(8), layout),
+                 lambda: ops.linear_forward(X, W, None, layout)):
+        with pytest.raises(Launched):
+            call()
