@@ -250,7 +250,8 @@ def dp_linear_backward(input, grad_output, weight, C, clamp_value, *, need_dx=Tr
                        db_dtype=None, norm_algo="auto", out=None):
     """(dX, dW, db) of one layer in one library call: linear_input_grad, dp_linear_weight_grad and dp_bias_grad
     with one normalisation of the operands, one workspace and, for fp32 on the tensor cores, one split of
-    grad_output.  input (B,T,in), grad_output (B,T,out); None in the place of what is not needed."""
+    grad_output.  input (B,T,in), grad_output (B,T,out); None in the place of what is not needed.  Only the weight
+    gradient reads the input's values: without it the input is neither cast nor copied."""
     host = _lib.host()
     _require_cuda(input, grad_output, weight if need_dx else None)
     if input.dim() != 3 or grad_output.dim() != 3 or input.shape[:2] != grad_output.shape[:2]:
@@ -259,22 +260,25 @@ def dp_linear_backward(input, grad_output, weight, C, clamp_value, *, need_dx=Tr
         raise RuntimeError(f"input is on {input.device}, grad_output on {grad_output.device}")
     if need_dx:
         _check_weight(weight, input.shape[-1], grad_output.shape[-1], layout, grad_output.device)
-    G = _aligned(grad_output.contiguous())
+    n_in = input.shape[-1]
+    G = grad_output.contiguous()
+    if need_dx or need_dw:
+        G = _aligned(G)
     dt = G.dtype
-    X = _aligned(input.to(dt).contiguous())
+    X = _aligned(input.to(dt).contiguous()) if need_dw else None
     W = _aligned(weight.to(dt).contiguous()) if need_dx else None
     code = _dt(dt)
     algo = NORM_ALGOS[norm_algo]
     if dt == torch.float32 and runtime.fp32_mode() == "tensor":
         algo |= _lib.FDP_FP32_TENSOR | _lib.FDP_FP32_WIDE
     if out is not None:
-        shape = (G.shape[-1], X.shape[-1]) if layout == "out_in" else (X.shape[-1], G.shape[-1])
+        shape = (G.shape[-1], n_in) if layout == "out_in" else (n_in, G.shape[-1])
         if tuple(out.shape) != shape or not out.is_contiguous() or out.device != G.device:
             raise RuntimeError(f"out must be a contiguous {shape} tensor on {G.device}")
         dw_dtype = out.dtype
     p = _params(C, clamp_value, batch_divisor, noise)
     st, dX, dW, db = host.linear_bwd(
-        G, X, W, out if need_dw else None, code, _dt(dx_dtype or dt), _dt(dw_dtype or dt), _dt(db_dtype or dt),
+        G, X, W, out if need_dw else None, n_in, code, _dt(dx_dtype or dt), _dt(dw_dtype or dt), _dt(db_dtype or dt),
         _lib.FDP_OUT_IN if layout == "out_in" else _lib.FDP_IN_OUT, algo, p,
         _params(C, clamp_value, batch_divisor, noise_bias) if need_db else p, need_dx, need_dw, need_db)
     _lib.check(st, "fdp_linear_bwd")

@@ -482,13 +482,16 @@ struct LinearBwdWs {
 LinearBwdWs linear_bwd_ws(void* base, int B, int T, int n_in, int n_out, int dtype, int norm_algo, int outputs) {
   LinearBwdWs q{};
   const int rows = B * T;
-  q.w = wgrad_ws(base, B, T, n_in, n_out, dtype, norm_algo);
-  q.shared = (outputs & FDP_BWD_DW) != 0 && (outputs & (FDP_BWD_DX | FDP_BWD_DB)) != 0 && q.w.tc.ok && q.w.tc.planes > 1 && !q.w.short_seq &&
-             ((outputs & FDP_BWD_DX) == 0 || tc_gemm3_ok(rows, n_out, n_in));
+  const bool dx = (outputs & FDP_BWD_DX) != 0, dw = (outputs & FDP_BWD_DW) != 0, db = (outputs & FDP_BWD_DB) != 0;
+  if (dw) {
+    q.w = wgrad_ws(base, B, T, n_in, n_out, dtype, norm_algo);
+    q.shared = (dx || db) && q.w.tc.ok && q.w.tc.planes > 1 && !q.w.short_seq && (!dx || tc_gemm3_ok(rows, n_out, n_in));
+  }
   if (!q.shared) {
+    // one output after another in the same memory: what the hungriest of those that are wanted takes
     size_t most = q.w.bytes;
-    const size_t d = fdp_linear_dgrad_workspace_bytes(rows, n_in, n_out, dtype == FDP_F32 ? dtype | (norm_algo & FDP_FP32_TENSOR) : dtype);
-    const size_t g = fdp_bias_grad_workspace_bytes(B, T, n_out, dtype);
+    const size_t d = dx ? fdp_linear_dgrad_workspace_bytes(rows, n_in, n_out, dtype == FDP_F32 ? dtype | (norm_algo & FDP_FP32_TENSOR) : dtype) : 0;
+    const size_t g = db ? fdp_bias_grad_workspace_bytes(B, T, n_out, dtype) : 0;
     if (d > most) most = d;
     if (g > most) most = g;
     q.bytes = most;
@@ -496,7 +499,7 @@ LinearBwdWs linear_bwd_ws(void* base, int B, int T, int n_in, int n_out, int dty
   }
   Carver c(base);
   c.off = q.w.bytes;
-  q.w_parts = c.take<char>((outputs & FDP_BWD_DX) ? tc_gemm3_w_bytes(n_out, n_in, q.w.tc.planes) : 0);
+  q.w_parts = c.take<char>(dx ? tc_gemm3_w_bytes(n_out, n_in, q.w.tc.planes) : 0);
   q.pl = gstats_plan(B, T, n_out, dtype);
   q.factors = c.take<float>(B);
   q.sq_part = c.take<float>(static_cast<size_t>(B) * q.pl.row_chunks * q.pl.col_chunks);

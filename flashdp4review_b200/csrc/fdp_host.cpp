@@ -134,13 +134,12 @@ py::tuple linear_dgrad(const Tensor& G, const Tensor& W, int rows, int code, int
   return py::make_tuple(st, dX);
 }
 
-// G, X as (B, T, .); W only where dX is wanted
-py::tuple linear_bwd(const Tensor& G, const Tensor& X, const OptTensor& W, const OptTensor& out, int in_dt, int dx_dt, int dw_dt, int db_dt,
+// G, X as (B, T, .); X only where dW is wanted, W only where dX is
+py::tuple linear_bwd(const Tensor& G, const OptTensor& X, const OptTensor& W, const OptTensor& out, int n_in, int in_dt, int dx_dt, int dw_dt, int db_dt,
                      int layout, int algo, const py::tuple& p, const py::tuple& p_bias, bool need_dx, bool need_dw, bool need_db) {
   const fdp_dp_params q = params(p), qb = params(p_bias);
   const c10::cuda::CUDAGuard guard(G.device());
-  const int B = static_cast<int>(X.size(0)), T = static_cast<int>(X.size(1));
-  const int n_in = static_cast<int>(X.size(2)), n_out = static_cast<int>(G.size(2));
+  const int B = static_cast<int>(G.size(0)), T = static_cast<int>(G.size(1)), n_out = static_cast<int>(G.size(2));
   OptTensor dX, dW, db;
   if (need_dx) dX = with_columns(G, n_in, dx_dt);
   if (need_dw) dW = out.has_value() ? *out

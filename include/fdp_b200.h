@@ -221,7 +221,8 @@ int fdp_linear_dgrad(const void* G, const void* W, void* dX, int rows, int n_in,
 
 /* ---- the whole backward of a Linear / Conv1D layer ----------------------------------------------
  * What fdp_linear_dgrad, fdp_linear_wgrad and fdp_bias_grad compute, in one call with one workspace; each of dX, dW, db
- * may be null (W too when dX is).  `layout` is that of W and of dW.  p belongs to the weight, p_bias to the bias.
+ * may be null (W too when dX is, X when dW is).  The workspace is that of the outputs named in `outputs`: a call without
+ * dW needs none of the weight gradient's.  `layout` is that of W and of dW.  p belongs to the weight, p_bias to the bias.
  * fp32 inputs with FDP_FP32_TENSOR / FDP_FP32_WIDE in norm_algo: G is split into its bf16 parts once for both
  * products, in the pass that also takes the bias gradient's statistics. */
 enum fdp_bwd_outputs { FDP_BWD_DX = 1, FDP_BWD_DW = 2, FDP_BWD_DB = 4 };

@@ -223,7 +223,7 @@ def no_launch(monkeypatch):
     class Host:
         def __getattr__(self, name):
             def call(*args):
-                raise Launched(name)
+                raise Launched(name, args)
             return call
     monkeypatch.setattr(_lib, "host", Host)
     monkeypatch.setattr(ops, "_require_cuda", lambda *tensors: None)
@@ -261,3 +261,33 @@ def test_operands_that_do_not_fit_are_refused_before_a_launch(no_launch, layout)
                  lambda: ops.linear_forward(X, W, None, layout)):
         with pytest.raises(Launched):
             call()
+
+
+def test_partial_backward_takes_only_what_it_needs(no_launch):
+    """Without the weight gradient (a frozen weight, a bias alone) the workspace of a whole backward is that of the
+    remaining outputs, and the layer input stays out of the call: no cast, no copy."""
+    from flashdp4review_b200 import _lib
+    lib = _lib.load()
+    q, d, b = lib.fdp_linear_bwd_workspace_bytes, lib.fdp_linear_dgrad_workspace_bytes, lib.fdp_bias_grad_workspace_bytes
+    w = lib.fdp_linear_wgrad_workspace_bytes
+    DX, DW, DB = 1, 2, 4
+    wide = _lib.FDP_FP32_TENSOR | _lib.FDP_FP32_WIDE
+    for (B, T, n_in, n_out) in ((4, 128, 768, 768), (3, 197, 264, 320), (2, 100, 136, 196), (64, 1, 1024, 1000), (3, 50, 72, 40)):
+        for dt in (_lib.FDP_F32, _lib.FDP_BF16):
+            algo = wide if dt == _lib.FDP_F32 else 0
+            dx = d(B * T, n_in, n_out, dt | (algo & _lib.FDP_FP32_TENSOR))
+            db = b(B, T, n_out, dt)
+            assert q(B, T, n_in, n_out, dt, algo, DX) == dx
+            assert q(B, T, n_in, n_out, dt, algo, DB) == db
+            assert q(B, T, n_in, n_out, dt, algo, DX | DB) == max(dx, db)
+            assert q(B, T, n_in, n_out, dt, algo, DW) == w(B, T, n_in, n_out, dt, algo)
+    ops, Launched = no_launch
+    X, G, W = torch.zeros(2, 3, 16, dtype=torch.float64), torch.zeros(2, 3, 8), torch.zeros(8, 16)
+    for need in ((True, False, True), (True, False, False), (False, False, True)):
+        with pytest.raises(Launched) as e:
+            ops.dp_linear_backward(X, G, W, 1.0, 1.0, need_dx=need[0], need_dw=need[1], need_db=need[2])
+        passed_X = e.value.args[1][1]
+        assert passed_X is None
+    with pytest.raises(Launched) as e:
+        ops.dp_linear_backward(X, G, W, 1.0, 1.0)
+    assert e.value.args[1][1].dtype == torch.float32
