@@ -485,7 +485,9 @@ LinearBwdWs linear_bwd_ws(void* base, int B, int T, int n_in, int n_out, int dty
   const bool dx = (outputs & FDP_BWD_DX) != 0, dw = (outputs & FDP_BWD_DW) != 0, db = (outputs & FDP_BWD_DB) != 0;
   if (dw) {
     q.w = wgrad_ws(base, B, T, n_in, n_out, dtype, norm_algo);
-    q.shared = (dx || db) && q.w.tc.ok && q.w.tc.planes > 1 && !q.w.short_seq && (!dx || tc_gemm3_ok(rows, n_out, n_in));
+    // (the input gradient takes part as three products, which is FDP_FP32_TENSOR's to allow)
+    q.shared = (dx || db) && q.w.tc.ok && q.w.tc.planes > 1 && !q.w.short_seq &&
+               (!dx || ((norm_algo & FDP_FP32_TENSOR) != 0 && tc_gemm3_ok(rows, n_out, n_in)));
   }
   if (!q.shared) {
     // one output after another in the same memory: what the hungriest of those that are wanted takes

@@ -224,7 +224,8 @@ int fdp_linear_dgrad(const void* G, const void* W, void* dX, int rows, int n_in,
  * may be null (W too when dX is, X when dW is).  The workspace is that of the outputs named in `outputs`: a call without
  * dW needs none of the weight gradient's.  `layout` is that of W and of dW.  p belongs to the weight, p_bias to the bias.
  * fp32 inputs with FDP_FP32_TENSOR / FDP_FP32_WIDE in norm_algo: G is split into its bf16 parts once for both
- * products, in the pass that also takes the bias gradient's statistics. */
+ * products, in the pass that also takes the bias gradient's statistics.  dX runs on the tensor cores with
+ * FDP_FP32_TENSOR only, as in fdp_linear_dgrad. */
 enum fdp_bwd_outputs { FDP_BWD_DX = 1, FDP_BWD_DW = 2, FDP_BWD_DB = 4 };
 size_t fdp_linear_bwd_workspace_bytes(int B, int T, int n_in, int n_out, int in_dtype, int norm_algo, int outputs);
 int fdp_linear_bwd(const void* G, const void* X, const void* W, void* dX, void* dW, void* db, int B, int T,

@@ -178,3 +178,23 @@ def test_six_products_fall_back_where_their_workspace_does_not_fit(ops):
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert torch.equal(got, want) and torch.equal(dW, want)
+
+
+# FDP_FP32_WIDE without FDP_FP32_TENSOR through the C ABI: the input gradient is that of the FMA kernels, bit for bit,
+# whatever the pointers' alignment lets the weight gradient do
+@pytest.mark.parametrize("B,T,n_in,n_out", [(2, 130, 128, 256), (4, 128, 256, 384), (40, 7, 128, 128)])
+@pytest.mark.parametrize("layout", ["out_in", "in_out"])
+def test_wide_flag_alone_leaves_the_input_gradient_exact(ops, B, T, n_in, n_out, layout):
+    from flashdp4review_b200 import _lib
+    lib = _lib.load()
+    X, G = _randn(B, T, n_in, seed=16, dtype=torch.float32), _randn(B, T, n_out, seed=17, dtype=torch.float32, scale=1e-2)
+    W = _randn(*((n_out, n_in) if layout == "out_in" else (n_in, n_out)), seed=18, dtype=torch.float32, scale=0.05)
+    dX, dW = torch.empty_like(X), torch.empty_like(W)
+    p = _lib.DPParams(1.0, 1.0, 0.0, 0, 0, 0, 0, 0, 0, 1, None)
+    algo, lay = _lib.FDP_FP32_WIDE, _lib.FDP_OUT_IN if layout == "out_in" else _lib.FDP_IN_OUT
+    ws = torch.empty(lib.fdp_linear_bwd_workspace_bytes(B, T, n_in, n_out, _lib.FDP_F32, algo, 3), dtype=torch.uint8, device=dev())
+    st = lib.fdp_linear_bwd(G.data_ptr(), X.data_ptr(), W.data_ptr(), dX.data_ptr(), dW.data_ptr(), None, B, T, n_in, n_out,
+                            *[_lib.FDP_F32] * 4, lay, algo, p, p, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+    assert st == _lib.FDP_OK
+    assert torch.equal(dX, ops.linear_input_grad(G, W, layout, fp32_tensor=False))
+    assert _lib.load().fdp_device_status(None, torch.cuda.current_stream().cuda_stream) == _lib.FDP_OK

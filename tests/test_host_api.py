@@ -291,3 +291,16 @@ def test_partial_backward_takes_only_what_it_needs(no_launch):
     with pytest.raises(Launched) as e:
         ops.dp_linear_backward(X, G, W, 1.0, 1.0)
     assert e.value.args[1][1].dtype == torch.float32
+
+
+def test_input_gradient_of_a_whole_backward_needs_its_own_flag():
+    """FDP_FP32_WIDE alone asks for six products in the weight gradient; the input gradient's three products are
+    FDP_FP32_TENSOR's.  Without it nothing is shared, so the workspace holds no parts of W."""
+    from flashdp4review_b200 import _lib
+    q = _lib.load().fdp_linear_bwd_workspace_bytes
+    w = _lib.load().fdp_linear_wgrad_workspace_bytes
+    wide, both = _lib.FDP_FP32_WIDE, _lib.FDP_FP32_WIDE | _lib.FDP_FP32_TENSOR
+    for (B, T, n_in, n_out) in ((2, 130, 128, 256), (4, 128, 256, 384), (3, 197, 264, 320)):
+        plain = w(B, T, n_in, n_out, _lib.FDP_F32, wide)
+        assert q(B, T, n_in, n_out, _lib.FDP_F32, wide, 3) == plain
+        assert q(B, T, n_in, n_out, _lib.FDP_F32, both, 3) > w(B, T, n_in, n_out, _lib.FDP_F32, both)
