@@ -50,8 +50,9 @@ Tensor new_tensor(const Tensor& like, at::IntArrayRef sizes, at::ScalarType t) {
 Tensor workspace(const Tensor& like, size_t bytes) {
   return new_tensor(like, {static_cast<int64_t>(bytes < 256 ? 256 : bytes)}, at::kByte);
 }
-// The workspace of a call with `algo`.  Split copies of fp32 operands are 1.5 times the inputs: where they do not
-// fit the card the shapes of FDP_FP32_WIDE stay on the FMA kernels, which need next to nothing.
+// The workspace of a weight gradient with `algo`.  The split copies of fp32 operands (1.5 times the inputs with
+// FDP_FP32_WIDE) and the 38.8 MB parking area may not fit the card: the shapes of FDP_FP32_WIDE then stay on the FMA
+// kernels, which need next to nothing.
 template <typename Query>
 Tensor algo_workspace(const Tensor& like, int& algo, Query query) {
   try {
@@ -141,17 +142,42 @@ py::tuple linear_bwd(const Tensor& G, const OptTensor& X, const OptTensor& W, co
   const c10::cuda::CUDAGuard guard(G.device());
   const int B = static_cast<int>(G.size(0)), T = static_cast<int>(G.size(1)), n_out = static_cast<int>(G.size(2));
   OptTensor dX, dW, db;
-  if (need_dx) dX = with_columns(G, n_in, dx_dt);
-  if (need_dw) dW = out.has_value() ? *out
-                    : layout == FDP_OUT_IN ? new_tensor(G, {n_out, n_in}, scalar_type(dw_dt)) : new_tensor(G, {n_in, n_out}, scalar_type(dw_dt));
-  if (need_db) db = new_tensor(G, {n_out}, scalar_type(db_dt));
-  const int outputs = (need_dx ? FDP_BWD_DX : 0) | (need_dw ? FDP_BWD_DW : 0) | (need_db ? FDP_BWD_DB : 0);
-  const Tensor ws = algo_workspace(G, algo, [&](int a) { return abi.linear_bwd_workspace_bytes(B, T, n_in, n_out, in_dt, a, outputs); });
-  int st;
-  {
+  const auto allocate = [&](int outputs) {
+    if (outputs & FDP_BWD_DX) dX = with_columns(G, n_in, dx_dt);
+    if (outputs & FDP_BWD_DW) dW = out.has_value() ? *out
+                                   : layout == FDP_OUT_IN ? new_tensor(G, {n_out, n_in}, scalar_type(dw_dt)) : new_tensor(G, {n_in, n_out}, scalar_type(dw_dt));
+    if (outputs & FDP_BWD_DB) db = new_tensor(G, {n_out}, scalar_type(db_dt));
+  };
+  // one call for the outputs that are named, in the workspace `ws`
+  const auto call = [&](int outputs, int a, const Tensor& ws) {
     py::gil_scoped_release nogil;
-    st = abi.linear_bwd(ptr(G), ptr(X), ptr(W), ptr(dX), ptr(dW), ptr(db), B, T, n_in, n_out, in_dt, dx_dt, dw_dt, db_dt, layout, algo,
-                        &q, &qb, ptr(ws), ws.numel(), stream(G));
+    return abi.linear_bwd(ptr(G), ptr(X), ptr(W), (outputs & FDP_BWD_DX) ? ptr(dX) : nullptr, (outputs & FDP_BWD_DW) ? ptr(dW) : nullptr,
+                          (outputs & FDP_BWD_DB) ? ptr(db) : nullptr, B, T, n_in, n_out, in_dt, dx_dt, dw_dt, db_dt, layout, a,
+                          &q, &qb, ptr(ws), ws.numel(), stream(G));
+  };
+  const auto bytes = [&](int outputs, int a) { return abi.linear_bwd_workspace_bytes(B, T, n_in, n_out, in_dt, a, outputs); };
+  const int outputs = (need_dx ? FDP_BWD_DX : 0) | (need_dw ? FDP_BWD_DW : 0) | (need_db ? FDP_BWD_DB : 0);
+  int st = FDP_OK;
+  OptTensor ws;
+  try {
+    allocate(outputs);
+    ws = workspace(G, bytes(outputs, algo));
+  } catch (const c10::OutOfMemoryError&) {
+    // below
+  }
+  if (ws.has_value()) {
+    st = call(outputs, algo, *ws);
+  } else {
+    // One output at a time: the same results from less memory.  The workspaces follow one another, and no parts of W
+    // and no statistics lie beside the parts of G and X.
+    dX.reset(); dW.reset(); db.reset();
+    for (const int one : {FDP_BWD_DX, FDP_BWD_DW, FDP_BWD_DB}) {
+      if ((outputs & one) == 0 || st != FDP_OK) continue;
+      allocate(one);
+      int a = algo;
+      const Tensor own = algo_workspace(G, a, [&](int b) { return bytes(one, b); });
+      st = call(one, a, own);
+    }
   }
   return py::make_tuple(st, dX, dW, db);
 }

@@ -198,3 +198,29 @@ def test_wide_flag_alone_leaves_the_input_gradient_exact(ops, B, T, n_in, n_out,
     assert st == _lib.FDP_OK
     assert torch.equal(dX, ops.linear_input_grad(G, W, layout, fp32_tensor=False))
     assert _lib.load().fdp_device_status(None, torch.cuda.current_stream().cuda_stream) == _lib.FDP_OK
+
+
+@pytest.mark.parametrize("T", [128, 130])
+def test_whole_backward_one_output_at_a_time_where_its_workspace_does_not_fit(ops, T):
+    """Where the workspace of the whole call does not fit, that of one output after the other may: the same bits, with
+    three products (T = 128) and with six (T = 130)."""
+    from flashdp4review_b200 import _lib
+    B, n = 4, 4096
+    X, G = _randn(B, T, n, seed=19, dtype=torch.float32), _randn(B, T, n, seed=20, dtype=torch.float32, scale=1e-2)
+    W = _randn(n, n, seed=21, dtype=torch.float32, scale=0.05)
+    want = [t.cpu() for t in ops.dp_linear_backward(X, G, W, 1.0, 1.0)]
+    q = lambda outputs: _lib.load().fdp_linear_bwd_workspace_bytes(B, T, n, n, _lib.FDP_F32, _lib.FDP_FP32_TENSOR | _lib.FDP_FP32_WIDE, outputs)
+    # what the results (dX in a segment of 20 MB, db in one of 2 MB, dW) and the largest single workspace take, 6 MB for
+    # the allocator's rounding; dW and the whole call's workspace alone take more
+    room = (22 << 20) + 4 * n * n + max(q(1), q(2), q(4)) + (6 << 20)
+    assert 4 * n * n + q(7) > room + (2 << 20)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + room) / total)
+        got = ops.dp_linear_backward(X, G, W, 1.0, 1.0)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for a, b in zip(got, want):
+        assert torch.equal(a.cpu(), b)
