@@ -82,6 +82,13 @@ __device__ __forceinline__ float load_as(const void* in, int dt, size_t i) {
   return __half2float(reinterpret_cast<const __half*>(in)[i]);
 }
 
+// The norm of a sum of squares.  A Gram form may round to just below zero.  A sum that is not a number comes from a sample
+// with an infinity or a NaN (inf - inf in the split of an fp32 operand, inf * 0 in a product): it counts as infinite, like
+// a sum that overflows, so that the sample's clip factor is 0 and not the clamp value.
+__device__ __forceinline__ float norm_of_sumsq(float sq) {
+  return isnan(sq) ? __int_as_float(0x7f800000) : sqrtf(fmaxf(sq, 0.f));
+}
+
 // ---- clip factor: min(clamp_value, C / (norm + 1e-10))  (flashdp/core/clip_fn.py:6-8) -----
 __device__ __forceinline__ float clip_factor(float norm, float C, float clamp_value) {
   return fminf(clamp_value, C / (norm + 1e-10f));

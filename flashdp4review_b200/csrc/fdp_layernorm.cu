@@ -822,7 +822,7 @@ __global__ void __launch_bounds__(256) ln_clip_finalize_kernel(
     for (int i = lane; i < nparts; i += 32) sq += sumsq[static_cast<size_t>(tensor * B + b) * nparts + i];
     sq = warp_sum(sq);
     if (lane == 0) {
-      const float n = sqrtf(fmaxf(sq, 0.f));
+      const float n = norm_of_sumsq(sq);
       s_fac[b] = clip_factor(n, C, clamp);
       float* no = tensor == 0 ? norms0 : norms1;
       if (blockIdx.x == 0 && no != nullptr) no[b] = n;

@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(256) clip_factors_kernel(const float* __restri
   for (int i = threadIdx.x; i < nparts; i += blockDim.x) s += partials[static_cast<size_t>(b) * nparts + i];
   s = block_sum(s, red);
   if (threadIdx.x == 0) {
-    const float n = sqrtf(fmaxf(s, 0.f));
+    const float n = norm_of_sumsq(s);
     const float f = clip_factor(n, C, clamp);
     if (norms) norms[b] = n;
     factors[b] = f;
@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(256) short_factors_kernel(const Tin* __restric
   pdl_trigger();
   const int b = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (b >= B) return;
-  const float norm = sqrtf(slab_sumsq<Tin>(G + static_cast<size_t>(b) * n, n, vec != 0, lane));
+  const float norm = norm_of_sumsq(slab_sumsq<Tin>(G + static_cast<size_t>(b) * n, n, vec != 0, lane));
   if (lane == 0) {
     const float f = clip_factor(norm, C, clamp);
     factors[b] = f;
@@ -904,7 +904,7 @@ __global__ void __launch_bounds__(256) bias_finalize_fused_kernel(
     for (int i = col; i < nparts; i += 32) sq += sq_part[static_cast<size_t>(b) * nparts + i];
     sq = warp_sum(sq);
     if (col == 0) {
-      const float n = sqrtf(fmaxf(sq, 0.f));
+      const float n = norm_of_sumsq(sq);
       const float f = clip_factor(n, C, clamp);
       s_fac[b] = f;
       if (blockIdx.x == 0) {

@@ -701,7 +701,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         for (int i = lane; i < args.norm_nparts; i += 32) sq += pp[i];
         sq = warp_sum(sq);
         if (lane == 0) {
-          const float n = sqrtf(fmaxf(sq, 0.f));
+          const float n = norm_of_sumsq(sq);
           const float f = clip_factor(n, args.C, args.clamp);
           sfac[b] = f;
           if (blockIdx.x == 0) {

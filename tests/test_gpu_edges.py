@@ -224,3 +224,56 @@ def test_whole_backward_one_output_at_a_time_where_its_workspace_does_not_fit(op
         torch.cuda.set_per_process_memory_fraction(1.0)
     for a, b in zip(got, want):
         assert torch.equal(a.cpu(), b)
+
+
+# a sample with an infinity or a NaN: its norm is infinite, its clip factor 0, and only the rows (columns) that hold the
+# element are lost; every norm algorithm and every kernel that derives factors
+@pytest.mark.parametrize("dtype,B,T,n_in,n_out,algo,fp32_tensor", [
+    (torch.float32, 3, 197, 128, 136, "auto", True), (torch.float32, 3, 128, 128, 192, "auto", True),
+    (torch.float32, 40, 7, 128, 136, "auto", True), (torch.float32, 130, 1, 128, 136, "auto", True),
+    (torch.float32, 3, 197, 40, 40, "direct", False), (torch.float32, 3, 197, 40, 40, "gram", False), (torch.float32, 3, 50, 40, 40, "auto", False),
+    (torch.bfloat16, 3, 256, 128, 128, "direct", None), (torch.bfloat16, 3, 256, 128, 128, "gram", None),
+    (torch.float16, 3, 300, 136, 128, "auto", None), (torch.bfloat16, 400, 64, 128, 128, "auto", None)])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("where", ["input", "grad_output"])
+def test_non_finite_samples_are_clipped_away(ops, dtype, B, T, n_in, n_out, algo, fp32_tensor, value, where):
+    X, G = _randn(B, T, n_in, seed=22, dtype=dtype), _randn(B, T, n_out, seed=23, dtype=dtype, scale=1e-2)
+    X[1] *= 4.0
+    rest = [b for b in range(B) if b != 1]
+    row, col = (T - 1) // 2, 5
+    (X if where == "input" else G)[1, row, col] = value
+    dW, norms, factors = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, norm_algo=algo, return_norms=True, out_dtype=torch.float32,
+                                                   fp32_tensor=fp32_tensor)
+    assert float(norms[1]) == float("inf") and float(factors[1]) == 0.0
+    assert bool(norms[rest].isfinite().all()) and bool((factors[rest] > 0).all())
+    # the other elements are the sums of the other samples, at the same divisor
+    want = ops.dp_linear_weight_grad(X[rest].contiguous(), G[rest].contiguous(), 1.0, 1.0, batch_divisor=B, norm_algo=algo,
+                                     out_dtype=torch.float32, fp32_tensor=fp32_tensor)
+    lost = ~dW.isfinite()
+    mask = torch.zeros_like(lost)
+    (mask[:, col] if where == "input" else mask[col]).fill_(True)
+    assert bool((lost <= mask).all())
+    err = (dW - want)[~mask].abs().max() / want.abs().max()
+    assert float(err) < 1e-2 if dtype != torch.float32 else float(err) < 1e-5
+    if where == "grad_output":
+        db, norms, factors = ops.dp_bias_grad(G, 1.0, 1.0, out_dtype=torch.float32, return_norms=True)
+        assert float(norms[1]) == float("inf") and float(factors[1]) == 0.0
+        keep = [o for o in range(n_out) if o != col]
+        assert bool(db[keep].isfinite().all())
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_non_finite_samples_of_a_layernorm_are_clipped_away(ops, value):
+    B, T, d = 3, 17, 96
+    x, dy = _randn(B, T, d, seed=24, dtype=torch.float32), _randn(B, T, d, seed=25, dtype=torch.float32)
+    w, b = torch.ones(d, device=dev()), torch.zeros(d, device=dev())
+    _, buf, _ = ops.layernorm_fwd_fused(x, w, b, 1e-5)
+    dy[1, 3, 5] = value
+    _, dg, db, ng, nb = ops.dp_layernorm_backward(dy, x, w, buf["mean"], buf["rstd"], 1.0, 1.0, return_norms=True)
+    assert float(ng[1]) == float("inf") and float(nb[1]) == float("inf")
+    keep = [c for c in range(d) if c != 5]
+    rest = [0, 2]
+    _, wg, wb = ops.dp_layernorm_backward(dy[rest].contiguous(), x[rest].contiguous(), w, buf["mean"].view(B, T)[rest].reshape(-1).contiguous(),
+                                          buf["rstd"].view(B, T)[rest].reshape(-1).contiguous(), 1.0, 1.0, batch_divisor=B)
+    for got, want in ((dg, wg), (db, wb)):
+        assert float((got - want)[keep].abs().max() / want.abs().max()) < 1e-5
