@@ -386,22 +386,49 @@ __global__ void __launch_bounds__(256) gram_small_norm_kernel(const Tin* __restr
   if (threadIdx.x == 0) sumsq[b] = v;
 }
 
-// sum of squares of n adjacent elements, by one warp
+// Sum of squares of n adjacent elements, by one warp.  Eight loads at a time, each a chain of its own from zero, and a
+// tree over the eight: the one running sum of a lane is added to once per 32 * 8 loads.  As one chain over all of a
+// lane's elements the norms of long samples were further from float64 than those of the general kernels, root mean
+// square of the relative error, 16 rows of 11008 columns: fp32 1.4e-7 against 3.1e-8, bf16 1.7e-6 against 3.2e-8.
+// The warp is alone with its sample, so the next eight loads are under way while eight are added up.
 template <typename Tin>
 __device__ __forceinline__ float slab_sumsq(const Tin* __restrict__ p, int n, bool vec, int lane) {
-  constexpr int VEC = 16 / sizeof(Tin);
+  constexpr int VEC = 16 / sizeof(Tin), U = 8;
+  const unsigned end = static_cast<unsigned>(n);
   float s = 0.f;
   if (vec) {       // 16-byte aligned, n a multiple of VEC
-#pragma unroll 4
-    for (int i = lane * VEC; i < n; i += 32 * VEC) {
-      float f[VEC];
-      unpack16<Tin>(__ldg(reinterpret_cast<const uint4*>(p + i)), f);
+    const auto load = [&](unsigned i, uint4* raw) {
 #pragma unroll
-      for (int v = 0; v < VEC; ++v) s = fmaf(f[v], f[v], s);
+      for (int u = 0; u < U; ++u, i += 32 * VEC) raw[u] = i < end ? __ldg(reinterpret_cast<const uint4*>(p + i)) : make_uint4(0, 0, 0, 0);
+    };
+    uint4 raw[U], next[U];
+    unsigned i = lane * VEC;
+    load(i, raw);
+    while (i < end) {
+      i += 32 * VEC * U;
+      load(i, next);
+      float q[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float f[VEC];
+        unpack16<Tin>(raw[u], f);
+        q[u] = 0.f;
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) q[u] = fmaf(f[v], f[v], q[u]);
+        raw[u] = next[u];
+      }
+      s += ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
     }
   } else {
-#pragma unroll 4
-    for (int i = lane; i < n; i += 32) { const float f = to_f32<Tin>(p[i]); s = fmaf(f, f, s); }
+    for (unsigned i = lane; i < end; i += 32 * U) {
+      float q[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float f = u * 32 < end - i ? to_f32<Tin>(p[i + u * 32]) : 0.f;
+        q[u] = f * f;
+      }
+      s += ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
+    }
   }
   return warp_sum(s);
 }

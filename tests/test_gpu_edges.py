@@ -277,3 +277,17 @@ def test_non_finite_samples_of_a_layernorm_are_clipped_away(ops, value):
                                           buf["rstd"].view(B, T)[rest].reshape(-1).contiguous(), 1.0, 1.0, batch_divisor=B)
     for got, want in ((dg, wg), (db, wb)):
         assert float((got - want)[keep].abs().max() / want.abs().max()) < 1e-5
+
+
+# norms of short samples with long rows: as close to float64 as those of the general kernels (64 samples and fewer)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,T,n", [(300, 1, 8192), (300, 4, 4096), (300, 8, 4096), (300, 2, 4097)])
+def test_norms_of_short_samples_are_as_accurate(ops, dtype, B, T, n):
+    G = _randn(B, T, n, seed=26, dtype=dtype, scale=0.1)
+    want = G[:64].double().flatten(1).norm(dim=1)
+    rms = []
+    for part in (G[:64], G):
+        _, norms, _ = ops.dp_bias_grad(part, 1.0, 1.0, return_norms=True)
+        rms.append(float(((norms[:64].double() - want) / want).square().mean().sqrt()))
+    # half as much again, and half a unit in the last place for the root
+    assert rms[1] < 1.5 * rms[0] + 2.0 ** -25, rms
