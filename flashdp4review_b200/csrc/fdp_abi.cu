@@ -366,7 +366,7 @@ int fdp_bias_grad(const void* G, void* db, float* norms_out, float* factors_out,
   const int div = p->batch_divisor > 0 ? p->batch_divisor : B;
   // mean over the B*T rows (flashdp/core/linear_clip.py:122)
   const float inv_div = 1.0f / (static_cast<float>(div) * static_cast<float>(T));
-  if (bias_short_ok(B, T)) {
+  if (bias_short_ok(B, T, n_out, in_dtype)) {
     bias_short(G, factors, colsum_part, db, norms_out, factors_out, B, T, n_out, in_dtype, out_dtype, p->C, p->clamp_value,
                inv_div, make_noise_key(p, p->param_id), s);
     FDP_LAUNCH_OK();

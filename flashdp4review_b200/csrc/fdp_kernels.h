@@ -81,7 +81,7 @@ GstatsPlan gstats_plan(int B, int T, int n_out, int dt);
 void gstats(const void* G, float* colsum_part, float* sq_part, int B, int T, int n_out, int dt,
             const GstatsPlan& pl, cudaStream_t s);
 // many samples of few rows: factors[B], then part[<= B, n_out] column sums that carry them, then db
-bool bias_short_ok(int B, int T);
+bool bias_short_ok(int B, int T, int n_out, int dt);
 void bias_short(const void* G, float* factors, float* part, void* db, float* norms_out, float* factors_out, int B, int T, int n_out,
                 int dt, int out_dt, float C, float clamp, float inv_div, NoiseKey nk, cudaStream_t s);
 void bias_finalize(const float* colsum_part, const float* factors, void* db, int B, int n_out,

@@ -848,9 +848,21 @@ __global__ void __launch_bounds__(256) short_finalize_kernel(const float* __rest
   }
 }
 
-// Few rows a sample and enough samples that the general kernels' finalisation, serial in the samples, is the
-// longer way (64 samples: 8 additions a slice, as here).
-bool bias_short_ok(int B, int T) { return T <= 16 && B > 64; }
+// The general kernels add up one column sum a sample and row chunk, serially in the samples: about 0.1 us a sample and
+// 0.017 us for every 1000 columns of it.  The kernels above walk a sample with one warp, 0.5 us for every 1000 words of 4
+// bytes (0.8 when G comes from HBM).  So the line between them is in words a sample, and grows with the samples and a
+// little with the width.  Measured, general / short, us a call with G in L2 and (in brackets) from HBM:
+//   fp32, 65 samples:   1 x 11008 21.8 / 8.0    4 x 4096 13.2 / 9.9 (13.3 / 13.0)    16 x 11008 24.8 / 58.9 (31.7 / 113)
+//   fp32, 256 samples:  8 x 4096 41.8 / 20.0 (46.3 / 31.7)                          16 x 11008 117 / 169
+//   fp32, 1024 samples: 1 x 1000 112 / 6.7      16 x 1000 118 / 39.6 (126 / 45.7)    16 x 11008 466 / 419
+//   bf16, 256 samples:  16 x 4096 37.9 / 24.4 (42.1 / 35.5)                         16 x 11008 73 / 89
+// Samples of more rows have fewer partial sums than elements by far and stay with the general kernels (32 rows, 65
+// samples: 256 columns 8.7 / 8.4, 1000 columns 10.9 / 19.4); 64 samples and fewer leave their finalisation too short to
+// gain from (8 additions a slice, as here).
+bool bias_short_ok(int B, int T, int n_out, int dt) {
+  const long long words = static_cast<long long>(T) * n_out * static_cast<long long>(dtype_size(dt)) / 4;
+  return T <= 16 && B > 64 && words < 1024 + static_cast<long long>(B) * (144 + n_out / 56);
+}
 
 template <typename Tin>
 static void bias_short_t(const Tin* G, float* factors, float* part, void* db, float* norms_out, float* factors_out, int B, int T,

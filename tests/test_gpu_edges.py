@@ -291,3 +291,23 @@ def test_norms_of_short_samples_are_as_accurate(ops, dtype, B, T, n):
         rms.append(float(((norms[:64].double() - want) / want).square().mean().sqrt()))
     # half as much again, and half a unit in the last place for the root
     assert rms[1] < 1.5 * rms[0] + 2.0 ** -25, rms
+
+
+# ... and long rows against few samples take the general kernels: both sides of the line, by the launches of a call
+# (three of the short kernels, two of the general ones) and against float64
+@pytest.mark.parametrize("dtype,B,T,n,short", [
+    (torch.float32, 65, 16, 11008, False), (torch.float32, 65, 16, 4096, False), (torch.bfloat16, 65, 16, 4096, False),
+    (torch.float32, 65, 1, 11008, True), (torch.float32, 65, 11, 1000, True), (torch.float32, 65, 12, 1000, False),
+    (torch.bfloat16, 65, 16, 1000, True), (torch.float32, 200, 16, 1000, True), (torch.float16, 128, 16, 11008, False)])
+def test_bias_gradient_of_short_samples_with_long_rows(ops, dtype, B, T, n, short):
+    from flashdp4review_b200 import _lib
+    G = _randn(B, T, n, seed=27, dtype=dtype, scale=0.1)
+    before = _lib.load().fdp_launch_count()
+    db, norms, _ = ops.dp_bias_grad(G, 0.5, 1.0, out_dtype=torch.float32, return_norms=True)
+    assert _lib.load().fdp_launch_count() - before == (3 if short else 2)
+    want_n = G.double().flatten(1).norm(dim=1)
+    assert float(((norms.double() - want_n) / want_n).abs().max()) < (T * n / 256 + 8) * 2.0 ** -23
+    f = (0.5 / (want_n + 1e-10)).clamp(max=1.0)
+    want = torch.einsum("bto,b->o", G.double(), f) / (B * T)
+    absum = torch.einsum("bto,b->o", G.double().abs(), f) / (B * T)
+    _close_to_sum(db, want, absum, B * T / 8 + T * n / 256 + 20, 2.0 ** -23)
