@@ -44,12 +44,16 @@ def build_host(force=False):
     import torch
     from torch.utils import cpp_extension
     header = os.path.join(os.path.dirname(PKG), "include", "fdp_b200.h")
+    tag = f"fdp_host for torch {torch.__version__}"      # the module carries it: another torch needs another build
     if not force and os.path.exists(HOST_LIB) and all(
             os.path.getmtime(d) <= os.path.getmtime(HOST_LIB) for d in (HOST_SOURCE, header)):
-        return HOST_LIB
+        with open(HOST_LIB, "rb") as f:
+            if tag.encode() + b"\0" in f.read():
+                return HOST_LIB
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     includes = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-DTORCH_EXTENSION_NAME=_fdp_host",
+           f'-DFDP_HOST_TAG="{tag}"',
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", HOST_SOURCE, "-o", HOST_LIB]
     cmd += ["-isystem" + d for d in includes]
     cmd += ["-L" + d for d in cpp_extension.library_paths()]

@@ -233,6 +233,7 @@ py::tuple layernorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, cons
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.attr("built_for") = FDP_HOST_TAG;      // the build compares it with the torch it finds
   m.def("bind", &bind);
   m.def("linear_wgrad", &linear_wgrad);
   m.def("bias_grad", &bias_grad);

@@ -304,3 +304,20 @@ def test_input_gradient_of_a_whole_backward_needs_its_own_flag():
         plain = w(B, T, n_in, n_out, _lib.FDP_F32, wide)
         assert q(B, T, n_in, n_out, _lib.FDP_F32, wide, 3) == plain
         assert q(B, T, n_in, n_out, _lib.FDP_F32, both, 3) > w(B, T, n_in, n_out, _lib.FDP_F32, both)
+
+
+def test_call_layer_is_rebuilt_for_another_torch(monkeypatch, tmp_path):
+    """_fdp_host.so fits the torch that it was built against only: newer sources or another torch rebuild it."""
+    import shutil
+    import types
+    from flashdp4review_b200 import build
+    copy = tmp_path / "_fdp_host.so"
+    shutil.copy(build.HOST_LIB, copy)           # (a new time of modification)
+    compiled = []
+    monkeypatch.setattr(build, "HOST_LIB", str(copy))
+    monkeypatch.setattr(build.subprocess, "run", lambda cmd, **kw: compiled.append(cmd) or types.SimpleNamespace(returncode=0, stderr=""))
+    build.build_host()
+    assert not compiled
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    build.build_host()
+    assert len(compiled) == 1 and str(copy) in compiled[0]
