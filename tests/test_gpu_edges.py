@@ -311,3 +311,60 @@ def test_bias_gradient_of_short_samples_with_long_rows(ops, dtype, B, T, n, shor
     want = torch.einsum("bto,b->o", G.double(), f) / (B * T)
     absum = torch.einsum("bto,b->o", G.double().abs(), f) / (B * T)
     _close_to_sum(db, want, absum, B * T / 8 + T * n / 256 + 20, 2.0 ** -23)
+
+
+def _parts(v):
+    """the three bf16 parts of an fp32 number"""
+    v, out = torch.tensor(v, dtype=torch.float32), []
+    for _ in range(3):
+        p = v.to(torch.bfloat16).float()
+        out.append(float(p))
+        v = v - p
+    assert float(v) == 0.0
+    return out
+
+
+# every one of the six products is there, in the gradient and in the norms: with constant operands what a product
+# contributes adds up over all elements instead of averaging out
+@pytest.mark.parametrize("B,T,n_in,n_out", [(2, 64, 72, 130), (1, 65, 257, 100), (3, 127, 64, 300), (2, 192, 136, 264)])
+@pytest.mark.parametrize("layout", ["out_in", "in_out"])
+def test_fp32_six_products_are_six(ops, B, T, n_in, n_out, layout):
+    g = 1.0 + 2.0 ** -9 + 2.0 ** -10 + 2.0 ** -18 + 2.0 ** -19 + 2.0 ** -20
+    x = 1.0 + 2.0 ** -9 + 2.0 ** -11 + 2.0 ** -18 + 2.0 ** -19 + 2.0 ** -21
+    G, X = torch.full((B, T, n_out), g, device=dev()), torch.full((B, T, n_in), x, device=dev())
+    assert float(G[0, 0, 0]) == g and float(X[0, 0, 0]) == x
+    dW, norms, _ = ops.dp_linear_weight_grad(X, G, 1e9, 1.0, batch_divisor=1, layout=layout, return_norms=True, fp32_tensor=True)
+    # steps on a large accumulator (4 of the 24 of a hand-off; 2 of the norm pass) truncate up to a unit each, the
+    # additions of the hand-offs in registers round up to half a unit each; the norm's sums of squares 8 more
+    n = (T + 63) // 64
+    bound = (4 + B * n / 2 + 2) * 2.0 ** -23
+    bound_n = (2 + 2 * n / 2 + 8) * 2.0 ** -23
+    rel = ((dW.double() - B * T * g * x).abs() / (B * T * g * x)).max()
+    want_n = T * g * x * (n_in * n_out) ** 0.5
+    rel_n = ((norms.double() - want_n).abs() / want_n).max()
+    assert float(rel) < bound and float(rel_n) < bound_n, (float(rel), float(rel_n))
+    # what a missing product would make of it: further off than the bounds allow, each of the six
+    pg, px = _parts(g), _parts(x)
+    for i in range(3):
+        for j in range(3 - i):
+            assert pg[i] * px[j] / (g * x) > 2 * max(bound, bound_n), (i, j)
+
+
+# the FMA kernels on the same ragged shapes: the path of "exact" mode and of a card without room for the split copies
+@pytest.mark.parametrize("B,T,n_in,n_out", [(1, 64, 64, 64), (2, 65, 72, 328), (3, 127, 257, 130), (5, 197, 520, 64),
+                                            (64, 1, 65, 129), (9, 63, 333, 100), (2, 1000, 300, 515), (400, 70, 66, 66)])
+@pytest.mark.parametrize("layout", ["out_in", "in_out"])
+def test_fp32_ragged_shapes_on_fma_kernels(ops, B, T, n_in, n_out, layout):
+    X = _randn(B, T, n_in, seed=1, dtype=torch.float32)
+    G = _randn(B, T, n_out, seed=2, dtype=torch.float32, scale=1e-2)
+    G[0] *= 30.0
+    dW, norms, _ = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, layout=layout, return_norms=True, fp32_tensor=False)
+    per = torch.einsum("bto,bti->boi", G.double(), X.double())
+    want_n = per.flatten(1).norm(dim=1)
+    assert float(((norms.double() - want_n) / want_n).abs().max()) < 1e-5
+    f = (1.0 / (want_n + 1e-10)).clamp(max=1.0)
+    want = torch.einsum("boi,b->oi", per, f) / B
+    absum = torch.einsum("bto,bti,b->oi", G.double().abs(), X.double().abs(), f) / B
+    if layout == "in_out":
+        want, absum = want.t(), absum.t()
+    _close_to_sum(dW, want, absum, B * T + 100, 2.0 ** -23)      # one chain over all rows; 1e-5 of the factor is 84 units
