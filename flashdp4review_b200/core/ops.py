@@ -103,8 +103,10 @@ def dp_linear_weight_grad(input, grad_output, C, clamp_value, *, batch_divisor=N
     `fp32_tensor` (default: runtime.fp32_mode() == "tensor", which is the package default): fp32 inputs
     with 64-aligned shapes run on the tensor cores as three bf16 products with short accumulation
     chains -- about six times faster than the fp32-FMA kernels and within the same 1e-5 of float64;
-    other shapes (widths of at least 64, at least 128 rows) as six products, as close to float64 as the
-    FMA kernels.  False forces the FMA kernels.
+    other shapes (widths of at least 64; T of at least 64, or at least 128 rows in all) as six products, as
+    close to float64 as the FMA kernels.  False forces the FMA kernels.  Six products need 1.5 times the
+    inputs and 38.8 MB beside them; where that cannot be allocated the FMA kernels take the call, so two runs
+    of which one was short of memory may differ in the last bits.
     """
     host = _lib.host()
     _require_cuda(input, grad_output)

@@ -702,7 +702,8 @@ static void ln_bwd_launch(const void* dy, const void* x, const void* gamma, cons
   // ring of up to FDP_LN_BWD_STAGES stages within FDP_LN_BWD_RING_KB (five stages in 160 KiB measured
   // no faster than three in 96 KiB: 36.1 against 35.3 us per call at B=16, T=1024, d=1024, bf16; the
   // 64 KiB stages of wide fp32 rows need 192 KiB for three: with one stage, hence without the ring, B=8,
-  // T=1024, d=1024 took 31.2 us in this kernel, now 16.8, and B=4, T=512, d=8192 205, now 54.8); needs 16-byte rows, i.e. the vector path
+  // T=1024, d=1024 took 31.2 us in this kernel, now 16.8, and B=4, T=512, d=8192 205, now 54.8); needs 16-byte
+  // rows, i.e. the vector path
   const size_t stage_bytes = static_cast<size_t>(2) * (CW / pl.tpr) * d * sizeof(Tin);
   int n_stages = static_cast<int>((static_cast<size_t>(FDP_LN_BWD_RING_KB) * 1024) / stage_bytes);
   if (n_stages > FDP_LN_BWD_STAGES) n_stages = FDP_LN_BWD_STAGES;

@@ -87,7 +87,8 @@ struct TcArgs {
   // sums then sit on the critical path of a few warps instead of spreading over the whole GPU.)
   int units_full, split;
   float* split_ws;
-  // EPI_STORE_SCALED: K is `segs` segments (samples; 0: the factors are in the operand, one segment) of `seg_stages` stages; every segment has its own
+  // EPI_STORE_SCALED: K is `segs` segments (samples; 0: the factors are in the operand, one segment) of
+  // `seg_stages` stages; every segment has its own
   // accumulator, scaled by that sample's clip factor when it is drained.  The factors come either from
   // `factors` (global, computed by an earlier kernel) or, when norm_partials != null, from the norm
   // pass's partial sums: the epilogue warps reduce them into shared memory while the first main loop
@@ -263,10 +264,10 @@ __device__ __forceinline__ void add_bias32(const TcArgs& args, int n, float v[32
 // ---- output boxes ------------------------------------------------------------------------------------
 // After tcgen05.ld a lane holds one row of the tile, so direct stores put the 32 lanes of an instruction
 // on 32 different rows: half-used sectors, 32 lines per request (16384 rows, 1024 -> 3072, bf16 forward with
-// bias: 171 us, tensor pipe 27 % busy; 86 us with the boxes and add_bias32).  Instead every epilogue warp writes boxes of 32 rows x 128 bytes into its own
-// 4 KB of shared memory, in the 128-byte swizzle of the tensor map (16-byte chunk j of row r at slot
-// j ^ (r & 7): no bank conflicts), and one lane hands each box to the copy engine, which also clips what
-// lies past the matrix.
+// bias: 171 us, tensor pipe 27 % busy; 86 us with the boxes and add_bias32).  Instead every epilogue warp
+// writes boxes of 32 rows x 128 bytes into its own 4 KB of shared memory, in the 128-byte swizzle of the
+// tensor map (16-byte chunk j of row r at slot j ^ (r & 7): no bank conflicts), and one lane hands each box
+// to the copy engine, which also clips what lies past the matrix.
 __device__ __forceinline__ void box_wait(int lane) {      // the previous box has been read out
   if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
   __syncwarp();
@@ -481,9 +482,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     slot = v;
   };
   // chained epilogues: end of the hand-off that contains stage ks -- sub_stages further, cut at the
-  // sample's and at the unit's end.  (With fp32 inputs it is a few stages only: the tensor cores add into the TMEM accumulator by truncation, about one unit in the
-  // last place per K = 16 step and all of one sign, so a long chain drifts; short chains summed in
-  // registers with round-to-nearest do not.)
+  // sample's and at the unit's end.  (With fp32 inputs it is a few stages only: the tensor cores add into the
+  // TMEM accumulator by truncation, about one unit in the last place per K = 16 step and all of one sign, so a
+  // long chain drifts; short chains summed in registers with round-to-nearest do not.)
   auto segment_end = [&](int ks, int ks1) {
     const int s0 = ks / args.seg_stages * args.seg_stages;
     const int sub = ((ks - s0) / args.sub_stages + 1) * args.sub_stages;
@@ -1308,8 +1309,10 @@ static bool three_products_ok(int T, int n_in, int n_out) {
 // ... and of FDP_FP32_WIDE's six
 static bool wide_ok(int B, int T, int n_in, int n_out, int norm_algo) {
   if (n_in < 64 || n_out < 64) return false;
-  // (below 128 rows in all the FMA kernels' K loop is shorter than the extra launches: 64 samples of one row,
-  // 256 -> 256, 43 us a call against 52; 210 rows, 1024 -> 4096, 122 against 77)
+  // T >= 64: the FMA kernels lose at every size, one sample of 64 rows included (whole call, 64 -> 64: 24.7 us, six
+  // products 15.8; 1024 -> 1000: 219 / 18.5; 8192 -> 8200: 1945 / 152).  Shorter sequences have no norm pass on the tensor
+  // cores to gain from, and below 128 rows in all the FMA kernels' K loop is shorter than the extra launches: 64 samples
+  // of one row, 256 -> 256, 43 us a call against 52; 210 rows, 1024 -> 4096, 122 against 77.
   return T >= SHORT_SEQ || (norm_algo != FDP_NORM_DIRECT && static_cast<long long>(B) * T >= 128);
 }
 

@@ -1,9 +1,9 @@
 """DPLinear: nn.Linear whose backward yields per-sample-clipped, noised parameter gradients.
 
 Same constructor and attributes as the reference's DPLinear (flashdp/layers/linear.py:11-32).
-Backward = `_DPLinearFunc.backward` (flashdp/layers/linear.py:49-104): grad_input, then one
-library call for the weight gradient (norms -> clip factors -> clipped sum / B -> noise) and one
-for the bias gradient.  Unlike the reference, 2-D and >3-D inputs get a grad_input of the
+Backward = `_DPLinearFunc.backward` (flashdp/layers/linear.py:49-104) in one library call: grad_input (or, where no
+kernel of the library takes the shape, by torch before it), the weight gradient (norms -> clip factors -> clipped
+sum / B -> noise) and the bias gradient.  Unlike the reference, 2-D and >3-D inputs get a grad_input of the
 input's own shape, and grad_output is left unmodified.
 """
 import torch

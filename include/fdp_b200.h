@@ -77,10 +77,11 @@ enum fdp_norm_algo {
    * (runtime.set_fp32_mode). */
   FDP_FP32_TENSOR = 16,
   /* flag, OR-ed into the same arguments: fp32 inputs of other shapes (any widths of at least 64; T of at least 64,
-   * or T shorter than 64 with at least 128 rows in all) run on the tensor cores as six bf16 products (x = hi + mid + lo, dropping
-   * what lies below 2^-26 of a product).  Norms and gradients are as close to float64 as those of the FMA
-   * kernels.  Operands and output need no alignment.  The workspace grows by 1.5 times the size of the
-   * inputs. */
+   * or T shorter than 64 with at least 128 rows in all) run on the tensor cores as six bf16 products (x = hi + mid
+   * + lo, dropping what lies below 2^-26 of a product).  Norms and gradients are as close to float64 as those of the
+   * FMA kernels (for operands of at least 2^-100 in magnitude; the parts of smaller ones run into bf16's smallest
+   * numbers).  Operands and output need no alignment.  The workspace grows by 1.5 times the size of the inputs and
+   * the 38.8 MB in which the parts of a K split are parked. */
   FDP_FP32_WIDE = 32
 };
 
@@ -114,7 +115,8 @@ int fdp_check_device(int device);
 
 /* Waits for `stream`, then reports whether a bounded wait ran out: reads the status word at the start
  * of `workspace` (of fdp_linear_wgrad / fdp_linear_dgrad / fdp_linear_fwd; may be NULL) and the
- * device's host-visible word.  Returns FDP_OK, FDP_ERR_TIMEOUT or FDP_ERR_LAUNCH. */
+ * device's host-visible word.  (The workspace of fdp_linear_bwd has no status word, other data may lie there: pass
+ * NULL after it.)  Returns FDP_OK, FDP_ERR_TIMEOUT or FDP_ERR_LAUNCH. */
 int fdp_device_status(const void* workspace, fdp_stream_t stream);
 
 /* Non-blocking poll / reset of the host-visible status word of `device` (-1: the current device).

@@ -32,7 +32,7 @@ def test_wgrad_fuzz(B, T, n_in, n_out, dtype, layout, C, clamp):
 def test_fp32_tensor_mode_fuzz(B, T, n_in, n_out, layout, algo, C):
     """fp32 inputs with `fp32_tensor=True`: shapes on both sides of what the three-product tensor-core
     path takes (64-aligned features of at least 128, T a multiple of 64 and at least 128); the others
-    fall back to the fp32-FMA kernels.  The fp32 tolerance 1e-5 either way."""
+    run as six products.  The fp32 tolerance 1e-5 either way."""
     from flashdp4review_b200.core import ops
     from conftest import rel_err, norm_err
     from gpu_util import dev
