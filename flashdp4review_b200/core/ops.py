@@ -34,13 +34,6 @@ def _require_cuda(*tensors):
                                "there is no CPU path")
 
 
-def _check_weight(weight, n_in, n_out, layout, device):
-    """The kernels take a weight as a bare pointer and its sizes from the other operands."""
-    shape = (n_out, n_in) if layout == "out_in" else (n_in, n_out)
-    if tuple(weight.shape) != shape or weight.device != device:
-        raise RuntimeError(f"weight must be a {shape} tensor ({layout}) on {device}, got {tuple(weight.shape)} on {weight.device}")
-
-
 def _ptr(t):
     return None if t is None else t.data_ptr()
 
@@ -235,9 +228,6 @@ def linear_input_grad(grad_output, weight, w_layout="out_in", out_dtype=None, fp
     `fp32_tensor` as in dp_linear_weight_grad: fp32 operands as three bf16 tensor-core products."""
     host = _lib.host()
     _require_cuda(grad_output, weight)
-    contracted = 0 if w_layout == "out_in" else 1
-    if weight.dim() != 2 or weight.shape[contracted] != grad_output.shape[-1]:
-        raise RuntimeError(f"grad_output {tuple(grad_output.shape)} and weight {tuple(weight.shape)} ({w_layout}) do not fit")
     G = _aligned(grad_output.contiguous())
     W = _aligned(weight.to(G.dtype).contiguous())         # AMP: weight follows the grad dtype (linear.py:66)
     n_out = G.shape[-1]
@@ -258,10 +248,6 @@ def dp_linear_backward(input, grad_output, weight, C, clamp_value, *, need_dx=Tr
     _require_cuda(input, grad_output, weight if need_dx else None)
     if input.dim() != 3 or grad_output.dim() != 3 or input.shape[:2] != grad_output.shape[:2]:
         raise RuntimeError(f"expected (B,T,in) and (B,T,out), got {tuple(input.shape)} and {tuple(grad_output.shape)}")
-    if input.device != grad_output.device:
-        raise RuntimeError(f"input is on {input.device}, grad_output on {grad_output.device}")
-    if need_dx:
-        _check_weight(weight, input.shape[-1], grad_output.shape[-1], layout, grad_output.device)
     n_in = input.shape[-1]
     G = grad_output.contiguous()
     if need_dx or need_dw:
@@ -292,11 +278,6 @@ def linear_forward(input, weight, bias=None, w_layout="out_in", out_dtype=None, 
     [in,out]) -- flashdp/layers/linear.py:41-46, transformers_conv1d.py:40-43."""
     host = _lib.host()
     _require_cuda(input, weight, bias)
-    contracted, columns = (1, 0) if w_layout == "out_in" else (0, 1)
-    if weight.dim() != 2 or weight.shape[contracted] != input.shape[-1]:
-        raise RuntimeError(f"input {tuple(input.shape)} and weight {tuple(weight.shape)} ({w_layout}) do not fit")
-    if bias is not None and bias.numel() != weight.shape[columns]:
-        raise RuntimeError(f"bias has {bias.numel()} elements, the output {weight.shape[columns]} columns")
     X = _aligned(input.contiguous())
     W = _aligned(weight.to(X.dtype).contiguous())
     b = None if bias is None else _aligned(bias.to(X.dtype).contiguous())

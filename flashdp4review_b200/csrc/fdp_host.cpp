@@ -1,8 +1,11 @@
 // Host side of the operator layer: allocates a call's outputs and workspace with torch's caching allocator and
-// enters the C ABI.  The checks on shapes, dtypes and devices, and all choices, stay in core/ops.py; what is
-// here is what every call pays for -- device guard, current stream, two to five allocations, argument
+// enters the C ABI.  The checks on arguments and dtypes, and all choices, stay in core/ops.py; what is
+// here, beside the checks that operands fit each other (5 us a layer in Python, under 1 here), is what every call pays for -- device guard, current stream, two to five allocations, argument
 // marshalling -- which through ctypes and torch's Python functions took 20 us an operator, more than the kernels
 // of a small layer.  Every function returns (status, outputs...).
+#include <stdexcept>
+#include <string>
+
 #include <torch/extension.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -63,6 +66,22 @@ Tensor algo_workspace(const Tensor& like, int& algo, Query query) {
     return workspace(like, query(algo));
   }
 }
+// The kernels take bare pointers and their sizes from one operand each: what does not fit would be misread, or read past
+// its end.  Raised as RuntimeError before anything is allocated or launched.
+void refuse(const char* what, const Tensor& t) {
+  // (no stream: the module may carry a C++ library of its own beside torch's, whose locales do not mix)
+  std::string s(what);
+  s += ": got (";
+  for (int64_t d = 0; d < t.dim(); ++d) s += (d ? ", " : "") + std::to_string(t.size(d));
+  s += ") on " + std::string(c10::DeviceTypeName(t.device().type(), true)) + (t.device().has_index() ? ":" + std::to_string(t.device().index()) : "");
+  throw std::runtime_error(s);
+}
+// weight of a product that contracts `k` columns: [n, k] or, with k_rows, [k, n] (n < 0: any)
+void check_weight(const Tensor& W, int64_t k, int64_t n, bool k_rows, const Tensor& like) {
+  if (W.dim() != 2 || W.size(k_rows ? 0 : 1) != k || (n >= 0 && W.size(k_rows ? 1 : 0) != n)) refuse("weight does not fit the other operands", W);
+  if (W.device() != like.device()) refuse("weight is on another device", W);
+}
+
 void* ptr(const Tensor& t) { return t.data_ptr(); }
 void* ptr(const OptTensor& t) { return t.has_value() ? t->data_ptr() : nullptr; }
 fdp_stream_t stream(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
@@ -123,6 +142,7 @@ Tensor with_columns(const Tensor& a, int64_t cols, int dt) {
 }
 
 py::tuple linear_dgrad(const Tensor& G, const Tensor& W, int rows, int code, int out_dt, int w_layout) {
+  check_weight(W, G.size(-1), -1, w_layout == FDP_OUT_IN, G);
   const c10::cuda::CUDAGuard guard(G.device());
   const int n_out = static_cast<int>(G.size(-1)), n_in = static_cast<int>(W.size(w_layout == FDP_OUT_IN ? 1 : 0));
   const Tensor dX = with_columns(G, n_in, out_dt);
@@ -138,6 +158,8 @@ py::tuple linear_dgrad(const Tensor& G, const Tensor& W, int rows, int code, int
 // G, X as (B, T, .); X only where dW is wanted, W only where dX is
 py::tuple linear_bwd(const Tensor& G, const OptTensor& X, const OptTensor& W, const OptTensor& out, int n_in, int in_dt, int dx_dt, int dw_dt, int db_dt,
                      int layout, int algo, const py::tuple& p, const py::tuple& p_bias, bool need_dx, bool need_dw, bool need_db) {
+  if (need_dx) check_weight(W.value(), G.size(2), n_in, layout == FDP_OUT_IN, G);
+  if (X.has_value() && X->device() != G.device()) refuse("input is on another device than grad_output", *X);
   const fdp_dp_params q = params(p), qb = params(p_bias);
   const c10::cuda::CUDAGuard guard(G.device());
   const int B = static_cast<int>(G.size(0)), T = static_cast<int>(G.size(1)), n_out = static_cast<int>(G.size(2));
@@ -183,6 +205,9 @@ py::tuple linear_bwd(const Tensor& G, const OptTensor& X, const OptTensor& W, co
 }
 
 py::tuple linear_fwd(const Tensor& X, const Tensor& W, const OptTensor& bias, int rows, int code, int out_dt, int w_layout) {
+  check_weight(W, X.size(-1), -1, w_layout != FDP_OUT_IN, X);
+  if (bias.has_value() && (bias->numel() != W.size(w_layout == FDP_OUT_IN ? 0 : 1) || bias->device() != X.device()))
+    refuse("bias does not fit the output's columns", *bias);
   const c10::cuda::CUDAGuard guard(X.device());
   const int n_in = static_cast<int>(X.size(-1)), n_out = static_cast<int>(W.size(w_layout == FDP_OUT_IN ? 0 : 1));
   const Tensor Y = with_columns(X, n_out, out_dt);

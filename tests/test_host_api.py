@@ -231,36 +231,35 @@ def no_launch(monkeypatch):
 
 
 @pytest.mark.parametrize("layout", ["out_in", "in_out"])
-def test_operands_that_do_not_fit_are_refused_before_a_launch(no_launch, layout):
+def test_operands_that_do_not_fit_are_refused_before_a_launch(monkeypatch, layout):
     """The kernels take the weight as a bare pointer: another shape than (out, in) or (in, out) would be misread, a
-    smaller one read past its end."""
-    ops, Launched = no_launch
+    smaller one read past its end.  (On CPU tensors: the call layer looks before it touches a device.)"""
+    from flashdp4review_b200.core import ops
+    monkeypatch.setattr(ops, "_require_cuda", lambda *tensors: None)
     X, G = torch.zeros(2, 3, 16), torch.zeros(2, 3, 8)
     right = (8, 16) if layout == "out_in" else (16, 8)
     shapes = [right[::-1], (right[0], right[1] + 1), (right[0] + 1, right[1]), (right[0] - 1, right[1]), (4, 4), right + (1,), (128,)]
+    refused = "weight does not fit"
     for shape in shapes:
-        with pytest.raises(RuntimeError, match="weight"):
+        with pytest.raises(RuntimeError, match=refused):
             ops.dp_linear_backward(X, G, torch.zeros(shape), 1.0, 1.0, layout=layout)
         if len(shape) != 2 or shape[0 if layout == "out_in" else 1] != 8:
-            with pytest.raises(RuntimeError, match="weight"):
+            with pytest.raises(RuntimeError, match=refused):
                 ops.linear_input_grad(G, torch.zeros(shape), layout)
         if len(shape) != 2 or shape[1 if layout == "out_in" else 0] != 16:
-            with pytest.raises(RuntimeError, match="weight"):
+            with pytest.raises(RuntimeError, match=refused):
                 ops.linear_forward(X, torch.zeros(shape), None, layout)
     W = torch.zeros(right)
-    with pytest.raises(RuntimeError, match="weight"):
-        ops.dp_linear_backward(X, G, W.to("meta"), 1.0, 1.0, layout=layout)
-    with pytest.raises(RuntimeError, match="input is on"):
-        ops.dp_linear_backward(X.to("meta"), G, W, 1.0, 1.0, layout=layout)
-    with pytest.raises(RuntimeError, match="bias"):
-        ops.linear_forward(X, W, torch.zeros(7), layout)
-    # what fits goes through, and a weight that is not needed is not looked at
-    for call in (lambda: ops.dp_linear_backward(X, G, W, 1.0, 1.0, layout=layout),
-                 lambda: ops.dp_linear_backward(X, G, None, 1.0, 1.0, layout=layout, need_dx=False),
-                 lambda: ops.linear_input_grad(G, W, layout), lambda: ops.linear_forward(X, W, torch.zeros(8), layout),
-                 lambda: ops.linear_forward(X, W, None, layout)):
-        with pytest.raises(Launched):
+    monkeypatch.setattr(ops, "_aligned", lambda t: t)          # (a meta tensor has no address to look at)
+    for call in (lambda: ops.dp_linear_backward(X, G, W.to("meta"), 1.0, 1.0, layout=layout),
+                 lambda: ops.linear_input_grad(G, W.to("meta"), layout), lambda: ops.linear_forward(X, W.to("meta"), None, layout)):
+        with pytest.raises(RuntimeError, match="weight is on another device"):
             call()
+    with pytest.raises(RuntimeError, match="input is on another device"):
+        ops.dp_linear_backward(X.to("meta"), G, W, 1.0, 1.0, layout=layout)
+    for bias in (torch.zeros(7), torch.zeros(8).to("meta")):
+        with pytest.raises(RuntimeError, match="bias does not fit"):
+            ops.linear_forward(X, W, bias, layout)
 
 
 def test_partial_backward_takes_only_what_it_needs(no_launch):
