@@ -1,8 +1,9 @@
 // Host side of the operator layer: allocates a call's outputs and workspace with torch's caching allocator and
-// enters the C ABI.  The checks on arguments and dtypes, and all choices, stay in core/ops.py; what is
-// here, beside the checks that operands fit each other (5 us a layer in Python, under 1 here), is what every call pays for -- device guard, current stream, two to five allocations, argument
-// marshalling -- which through ctypes and torch's Python functions took 20 us an operator, more than the kernels
-// of a small layer.  Every function returns (status, outputs...).
+// enters the C ABI.  The checks on arguments and dtypes, and all choices, stay in core/ops.py; what is here,
+// beside the checks that operands fit each other (5 us a layer in Python, under 1 here), is what every call pays
+// for -- device guard, current stream, two to five allocations, argument marshalling -- which through ctypes and
+// torch's Python functions took 20 us an operator, more than the kernels of a small layer.  Every function
+// returns (status, outputs...).
 #include <stdexcept>
 #include <string>
 
