@@ -9,7 +9,7 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 # FDP_B200_LIB points at another build of the same ABI (used to compare builds on one GPU)
 LIB_PATH = os.environ.get("FDP_B200_LIB") or os.path.join(PKG, "libfdp_b200.so")
 
-ABI_VERSION = 4
+ABI_VERSION = 5
 FDP_OK = 0
 FDP_ERR_ARG, FDP_ERR_DTYPE, FDP_ERR_SHAPE, FDP_ERR_ALIGN = -1, -2, -3, -4
 FDP_ERR_WORKSPACE, FDP_ERR_ARCH, FDP_ERR_LAUNCH, FDP_ERR_TIMEOUT = -5, -6, -7, -8
@@ -18,7 +18,7 @@ FDP_STATIC_SCRATCH_BYTES = 8 << 20
 FDP_F32, FDP_BF16, FDP_F16 = 0, 1, 2
 FDP_OUT_IN, FDP_IN_OUT = 0, 1
 FDP_NORM_AUTO, FDP_NORM_DIRECT, FDP_NORM_GRAM = 0, 1, 2
-FDP_FP32_TENSOR, FDP_FP32_WIDE = 16, 32
+FDP_FP32_TENSOR, FDP_FP32_WIDE, FDP_KEEP_PRODUCTS = 16, 32, 64
 
 c_void_p, c_int, c_size_t, c_float = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t, ctypes.c_float
 

@@ -116,7 +116,7 @@ def dp_linear_weight_grad(input, grad_output, C, clamp_value, *, batch_divisor=N
         out_dtype = out.dtype
     else:
         out_dtype = out_dtype or G.dtype
-    algo = NORM_ALGOS[norm_algo]
+    algo = NORM_ALGOS[norm_algo] | _lib.FDP_KEEP_PRODUCTS
     if fp32_tensor is None:
         fp32_tensor = runtime.fp32_mode() == "tensor"
     if fp32_tensor and G.dtype == torch.float32:
@@ -256,7 +256,7 @@ def dp_linear_backward(input, grad_output, weight, C, clamp_value, *, need_dx=Tr
     X = _aligned(input.to(dt).contiguous()) if need_dw else None
     W = _aligned(weight.to(dt).contiguous()) if need_dx else None
     code = _dt(dt)
-    algo = NORM_ALGOS[norm_algo]
+    algo = NORM_ALGOS[norm_algo] | _lib.FDP_KEEP_PRODUCTS
     if dt == torch.float32 and runtime.fp32_mode() == "tensor":
         algo |= _lib.FDP_FP32_TENSOR | _lib.FDP_FP32_WIDE
     if out is not None:

@@ -250,7 +250,8 @@ static int wgrad_run(const void* G, const void* X, void* dW, float* norms_out, f
   if (!w.tc.ok || w.short_seq) FDP_CUDA_OK(cudaMemsetAsync(w.status, 0, sizeof(int), s));
 
   // the scaled epilogue of the clipped-sum GEMM reduces the norm partials itself: no clip-factor launch
-  const bool fused_factors = w.tc.ok && w.tc.scaled_epilogue && tc_fused_factors_ok(B);
+  if (w.tc.keep) w.nparts = tc_keep_partials(n_in, n_out, layout);
+  const bool fused_factors = w.tc.keep ? tc_keep_fused_factors_ok(B, w.nparts) : w.tc.ok && w.tc.scaled_epilogue && tc_fused_factors_ok(B);
   prof_mark(0, s);
   // fp32 inputs on the tensor cores: split G and X into bf16 halves first, then run as bf16
   const void* Gt = G;
@@ -268,15 +269,27 @@ static int wgrad_run(const void* G, const void* X, void* dW, float* norms_out, f
   if (w.short_seq) {
     simt_norm_gram_small(G, X, w.partials, B, T, n_in, n_out, in_dtype, s);
   } else if (w.tc.ok) {
-    if ((st = tc_norms(Gt, Xt, w.partials, w.status, B, T, n_in, n_out, tdt, w.tc, s)) != FDP_OK) return st;
+    if ((st = tc_norms(Gt, Xt, w.partials, w.status, B, T, n_in, n_out, tdt, w.tc, s,
+                       w.tc.keep ? static_cast<float*>(w.tc_extra) : nullptr, layout)) != FDP_OK) return st;
   } else {
     w.nparts = simt_norm_direct(G, X, w.partials, B, T, n_in, n_out, in_dtype, norm_algo & FDP_NORM_MASK, s);
   }
   prof_mark(1, s);
   if (!fused_factors)
-    clip_factors(w.partials, w.nparts, B, p->C, p->clamp_value, w.norms, w.factors, norms_out, factors_out, s);
+    clip_factors(w.partials, w.nparts, B, p->C, p->clamp_value, w.norms, w.factors, norms_out, factors_out, s, w.tc.keep);
   prof_mark(2, s);
-  if (w.tc.ok) {
+  TcFactorSource fs{};
+  if (fused_factors) {
+    fs.norm_partials = w.partials; fs.nparts = w.nparts; fs.C = p->C; fs.clamp = p->clamp_value;
+    fs.norms_out = norms_out; fs.factors_out = factors_out;
+  } else {
+    fs.factors = w.factors;
+  }
+  if (w.tc.keep) {
+    prof_mark(3, s);
+    if ((st = tc_weighted_sum(static_cast<const float*>(w.tc_extra), fs, dW, B, n_in, n_out, out_dtype, layout, inv_div, nk, s)) != FDP_OK)
+      return st;
+  } else if (w.tc.ok) {
     float* split_ws = static_cast<float*>(w.tc_extra);
     char* gs = static_cast<char*>(w.tc_extra) + w.tc.split_bytes;
     if (split && w.short_seq) {     // c_b G in fp32, then its parts
@@ -287,13 +300,6 @@ static int wgrad_run(const void* G, const void* X, void* dW, float* norms_out, f
       if ((st = tc_prescale(G, w.factors, gs, B, T, n_out, in_dtype, s)) != FDP_OK) return st;
     }
     prof_mark(3, s);
-    TcFactorSource fs{};
-    if (fused_factors) {
-      fs.norm_partials = w.partials; fs.nparts = w.nparts; fs.C = p->C; fs.clamp = p->clamp_value;
-      fs.norms_out = norms_out; fs.factors_out = factors_out;
-    } else {
-      fs.factors = w.factors;
-    }
     if ((st = tc_clipped_wgrad(w.tc.scaled_epilogue ? Gt : gs, Xt, w.tc.scaled_epilogue ? &fs : nullptr, split_ws,
                                dW, w.status, B, T, n_in, n_out, tdt, out_dtype, layout, inv_div, nk,
                                s, w.tc.planes)) != FDP_OK) return st;
@@ -314,7 +320,7 @@ int fdp_linear_wgrad(const void* G, const void* X, void* dW, float* norms_out, f
   if (G == nullptr || X == nullptr || dW == nullptr) return FDP_ERR_ARG;
   if (B <= 0 || T <= 0 || n_in <= 0 || n_out <= 0) return FDP_ERR_ARG;
   if (layout != FDP_OUT_IN && layout != FDP_IN_OUT) return FDP_ERR_ARG;
-  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
+  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE | FDP_KEEP_PRODUCTS)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
     return FDP_ERR_ARG;
   if (!valid_dtype(in_dtype) || !valid_dtype(out_dtype)) return FDP_ERR_DTYPE;
   if (static_cast<long long>(B) * T >= (1ll << 31) / 2) return FDP_ERR_SHAPE;   // row indices are 32-bit
@@ -523,7 +529,7 @@ int fdp_linear_bwd(const void* G, const void* X, const void* W, void* dX, void* 
   if (B <= 0 || T <= 0 || n_in <= 0 || n_out <= 0) return FDP_ERR_ARG;
   if (static_cast<long long>(B) * T >= (1ll << 31) / 2) return FDP_ERR_SHAPE;   // row indices are 32-bit
   if (!valid_dtype(in_dtype)) return FDP_ERR_DTYPE;
-  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
+  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE | FDP_KEEP_PRODUCTS)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
     return FDP_ERR_ARG;
   const int outputs = (dX ? FDP_BWD_DX : 0) | (dW ? FDP_BWD_DW : 0) | (db ? FDP_BWD_DB : 0);
   if (outputs == 0) return FDP_ERR_ARG;

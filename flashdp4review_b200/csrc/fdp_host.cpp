@@ -54,18 +54,20 @@ Tensor new_tensor(const Tensor& like, at::IntArrayRef sizes, at::ScalarType t) {
 Tensor workspace(const Tensor& like, size_t bytes) {
   return new_tensor(like, {static_cast<int64_t>(bytes < 256 ? 256 : bytes)}, at::kByte);
 }
-// The workspace of a weight gradient with `algo`.  The split copies of fp32 operands (1.5 times the inputs with
-// FDP_FP32_WIDE) and the 38.8 MB parking area may not fit the card: the shapes of FDP_FP32_WIDE then stay on the FMA
-// kernels, which need next to nothing.
+// The workspace of a weight gradient with `algo`.  Where it does not fit the card, what asks for most is given up first:
+// the per-sample products (FDP_KEEP_PRODUCTS, up to 512 MiB), then the split copies of fp32 operands (1.5 times the inputs
+// with FDP_FP32_WIDE) and the 38.8 MB parking area -- those shapes then stay on the FMA kernels, which need next to nothing.
 template <typename Query>
 Tensor algo_workspace(const Tensor& like, int& algo, Query query) {
-  try {
-    return workspace(like, query(algo));
-  } catch (const c10::OutOfMemoryError&) {
-    if ((algo & FDP_FP32_WIDE) == 0) throw;
-    algo &= ~FDP_FP32_WIDE;
-    return workspace(like, query(algo));
+  for (const int flag : {FDP_KEEP_PRODUCTS, FDP_FP32_WIDE}) {
+    try {
+      return workspace(like, query(algo));
+    } catch (const c10::OutOfMemoryError&) {
+      if ((algo & (FDP_KEEP_PRODUCTS | FDP_FP32_WIDE)) == 0) throw;
+      algo &= ~flag;
+    }
   }
+  return workspace(like, query(algo));
 }
 // The kernels take bare pointers and their sizes from one operand each: what does not fit would be misread, or read past
 // its end.  Raised as RuntimeError before anything is allocated or launched.
@@ -182,18 +184,24 @@ py::tuple linear_bwd(const Tensor& G, const OptTensor& X, const OptTensor& W, co
   const int outputs = (need_dx ? FDP_BWD_DX : 0) | (need_dw ? FDP_BWD_DW : 0) | (need_db ? FDP_BWD_DB : 0);
   int st = FDP_OK;
   OptTensor ws;
-  try {
-    allocate(outputs);
-    ws = workspace(G, bytes(outputs, algo));
-  } catch (const c10::OutOfMemoryError&) {
-    // below
+  const auto take = [&] {
+    try {
+      allocate(outputs);
+      ws = workspace(G, bytes(outputs, algo));
+    } catch (const c10::OutOfMemoryError&) {
+      dX.reset(); dW.reset(); db.reset();
+    }
+    return ws.has_value();
+  };
+  if (!take() && bytes(outputs, algo & ~FDP_KEEP_PRODUCTS) < bytes(outputs, algo)) {
+    algo &= ~FDP_KEEP_PRODUCTS;
+    take();
   }
   if (ws.has_value()) {
     st = call(outputs, algo, *ws);
   } else {
     // One output at a time: the same results from less memory.  The workspaces follow one another, and no parts of W
     // and no statistics lie beside the parts of G and X.
-    dX.reset(); dW.reset(); db.reset();
     for (const int one : {FDP_BWD_DX, FDP_BWD_DW, FDP_BWD_DB}) {
       if ((outputs & one) == 0 || st != FDP_OK) continue;
       allocate(one);

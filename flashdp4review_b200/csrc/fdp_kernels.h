@@ -59,7 +59,7 @@ void simt_norm_gram_small(const void* G, const void* X, float* sumsq, int B, int
                           int dt, cudaStream_t s);
 // sumsq_b = fixed-order sum of partials[b, 0..nparts); norm = sqrt; factor = clip_factor(norm)
 void clip_factors(const float* partials, int nparts, int B, float C, float clamp, float* norms,
-                  float* factors, float* norms_out, float* factors_out, cudaStream_t s);
+                  float* factors, float* norms_out, float* factors_out, cudaStream_t s, bool dependent = false);
 // the same for 2B entries (two tensors of B samples): factors[2B]; norms go to two outputs
 void clip_factors_pair(const float* partials, int nparts, int B, float C, float clamp, float* factors,
                        float* norms_out_first, float* norms_out_second, cudaStream_t s);
@@ -131,6 +131,7 @@ struct TcPlan {
   int nparts;       // norm partials per sample
   bool scaled_epilogue;  // clip factors applied per sample in the GEMM epilogue, no pre-scale pass
   bool short_seq;        // T < SHORT_SEQ: norms by simt_norm_gram_small, clipped sum over the pre-scaled G
+  bool keep;             // per-sample products kept in the workspace (at its start; split_bytes), no second contraction
   bool any_align;        // takes operands and outputs of any alignment
   // fp32 inputs (planes > 1): G and X are first split into 2 or 3 bf16 parts ([rows, planes * n] each, n
   // rounded up to a multiple of 8, behind the parking area in the workspace), and every contraction runs as
@@ -145,7 +146,7 @@ struct SplitJob { const void* src; void* dst; size_t rows; int n; const float* f
 int tc_split(const SplitJob* jobs, int njobs, int planes, int* zero_status, cudaStream_t s);
 // With pl.planes > 1, G and X are the split matrices and dt is FDP_BF16.
 int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int B, int T, int n_in,
-             int n_out, int dt, const TcPlan& pl, cudaStream_t s);
+             int n_out, int dt, const TcPlan& pl, cudaStream_t s, float* keep = nullptr, int layout = FDP_OUT_IN);
 // Gs[r,:] = factors[r / T] * G[r,:]
 int tc_prescale(const void* G, const float* factors, void* Gs, int B, int T, int n_out, int dt,
                 cudaStream_t s);
@@ -159,6 +160,13 @@ struct TcFactorSource {
   float* norms_out; float* factors_out;
 };
 bool tc_fused_factors_ok(int B);
+// pl.keep: tc_norms leaves every sample's product in `keep` (fp32, in the orientation of `layout`, tile by tile), and
+// the clipped sum is their weighted sum: dW = inv_div * sum_b c_b P_b + noise (factors from partials where
+// tc_keep_fused_factors_ok)
+int tc_keep_partials(int n_in, int n_out, int layout);    // norm partials per sample
+bool tc_keep_fused_factors_ok(int B, int nparts);
+int tc_weighted_sum(const float* keep, const TcFactorSource& fs, void* dW, int B, int n_in, int n_out, int out_dt, int layout,
+                    float inv_div, NoiseKey nk, cudaStream_t s);
 // dW = inv_div * sum_b c_b G_b^T X_b + noise over K = B*T.  fs == nullptr: Gs is the pre-scaled copy;
 // otherwise Gs is G itself and c_b is applied per sample in the epilogue.  planes > 1: G and X are split.
 int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, float* split_ws,

@@ -40,6 +40,10 @@ constexpr int SMEM_BYTES_STORE = SMEM_BYTES + 8 * BOX_BYTES;
 constexpr int SMEM_BYTES_SCALED = SMEM_BYTES_STORE + MAX_SMEM_FACTORS * 4;
 static_assert(SMEM_BYTES_SCALED <= 227 * 1024, "shared memory of one CTA");
 constexpr int TMEM_COLS = 512;
+// Per-sample products kept in a call's workspace.  Beyond that there is nothing to gain: 4 x 2048 rows, 4096 -> 11008 bf16,
+// 721 MB of products, a layer's forward and backward 2148 us against 2157.
+constexpr size_t KEEP_LIMIT = static_cast<size_t>(512) << 20;
+constexpr int KEEP_SMEM_FACTORS = 128;
 constexpr int MAX_SMS = 148;           // workers the split-K parking area is sized for
 
 // EPI_STORE_SCALED: the accumulator of each sample (K segment) is drained on its own and added, times
@@ -47,16 +51,20 @@ constexpr int MAX_SMS = 148;           // workers the split-K parking area is si
 // EPI_SPLIT_*: fp32 inputs as bf16 halves, three products per K stage (see TcArgs::plane_a): the clipped sum,
 // a plain product (+ bias), and one sample's product tile squared and summed.
 // EPI_SPLIT6_*: the same with bf16 thirds and six products.
+// EPI_KEEP: one sample's product tile squared and summed, and kept in HBM for weighted_sum_kernel (the SPLIT_SUMSQ
+// ones keep it too when TcArgs::keep is set).
 enum { EPI_STORE = 0, EPI_SUMSQ = 1, EPI_GRAM = 2, EPI_STORE_SCALED = 3, EPI_SPLIT_SCALED = 4, EPI_SPLIT_STORE = 5,
-       EPI_SPLIT_SUMSQ = 6, EPI_SPLIT6_SCALED = 7, EPI_SPLIT6_SUMSQ = 8 };
-__host__ __device__ constexpr bool epi_chained(int epi) { return epi >= EPI_STORE_SCALED; }
+       EPI_SPLIT_SUMSQ = 6, EPI_SPLIT6_SCALED = 7, EPI_SPLIT6_SUMSQ = 8, EPI_KEEP = 9 };
+__host__ __device__ constexpr bool epi_chained(int epi) { return epi >= EPI_STORE_SCALED && epi != EPI_KEEP; }
 // bf16 parts of an operand
-__host__ __device__ constexpr int epi_planes(int epi) { return epi >= EPI_SPLIT6_SCALED ? 3 : epi >= EPI_SPLIT_SCALED ? 2 : 1; }
+__host__ __device__ constexpr int epi_planes(int epi) {
+  return epi == EPI_SPLIT6_SCALED || epi == EPI_SPLIT6_SUMSQ ? 3 : epi_chained(epi) && epi != EPI_STORE_SCALED ? 2 : 1;
+}
 __host__ __device__ constexpr bool epi_scaled(int epi) { return epi == EPI_STORE_SCALED || epi == EPI_SPLIT_SCALED || epi == EPI_SPLIT6_SCALED; }
 __host__ __device__ constexpr bool epi_sumsq(int epi) { return epi == EPI_SPLIT_SUMSQ || epi == EPI_SPLIT6_SUMSQ; }
 __host__ __device__ constexpr bool epi_stores(int epi) { return epi == EPI_STORE || epi_scaled(epi) || epi == EPI_SPLIT_STORE; }
 // eight epilogue warps (two per TMEM lane quarter, 128 columns each) for the store epilogues, four for the norms
-__host__ __device__ constexpr int epi_warps_for(int epi) { return (epi == EPI_STORE || epi_chained(epi)) ? 8 : 4; }
+__host__ __device__ constexpr int epi_warps_for(int epi) { return (epi == EPI_STORE || epi == EPI_KEEP || epi_chained(epi)) ? 8 : 4; }
 constexpr int threads_for(int epi) { return 64 + 32 * epi_warps_for(epi); }
 constexpr int smem_for(int epi) {
   return epi_scaled(epi) ? SMEM_BYTES_SCALED : epi_stores(epi) ? SMEM_BYTES_STORE : SMEM_BYTES;
@@ -118,6 +126,7 @@ struct TcArgs {
   int m_group;
   // the output cannot be written by the copy engine (row pitch or base not a multiple of 16 bytes)
   int direct_out;
+  float* keep;          // EPI_KEEP, EPI_SPLIT*_SUMSQ (may be null there): the product tiles, [tile][CTA of the pair][box]
 };
 
 // ---- PTX wrappers (mbarrier helpers live in fdp_async.cuh) --------------------------------------------
@@ -297,6 +306,15 @@ __device__ __forceinline__ void store_f32x32(uint32_t box, const CUtensorMap* ma
             __float_as_uint(v[4 * j + 3]));
   box_send(box, map, col, row, lane);
 }
+// A kept product leaves straight from the registers, 32 x 32 elements at a time in the order that suits them: element
+// group j (four columns) of all 32 rows, then the next, so that every store of a warp is 512 contiguous bytes.  Through
+// shared memory and the copy engine, as an output goes, the stores compete with the operands for shared memory
+// (16 x 512 rows, 4096 -> 4096 bf16: 336 us with tensor stores, 298 with whole boxes, 273 so).  weighted_sum_kernel knows the order.
+__device__ __forceinline__ void keep_f32x32(float* dst, const float v[32], int lane) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    reinterpret_cast<float4*>(dst)[j * 32 + lane] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+}
 // chunk c4 (32 columns) of a warp's 128 columns, in the output type; 16-bit types fill a box with two chunks
 __device__ __forceinline__ void store_out32(const TcArgs& args, uint32_t box, const CUtensorMap* map, const float v[32], int c4,
                                             int col0, int row, int lane) {
@@ -373,7 +391,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   constexpr int BN_CTA = BN / CTAS;                      // B columns (rows if K-major) loaded by this CTA
   constexpr int EPI_WARPS = epi_warps_for(EPI);
   static_assert(NST * STG <= STAGES * STAGE_BYTES, "ring size");
-  static_assert(CTAS == 1 || EPI == EPI_STORE || epi_chained(EPI), "pairs: store and chained epilogues only");
+  static_assert(CTAS == 1 || EPI_WARPS == 8, "pairs: eight epilogue warps");
   const uint32_t cta_rank = (CTAS == 2) ? cluster_ctarank() : 0u;
   const bool is_leader = cta_rank == 0;
   extern __shared__ uint8_t smem_raw[];
@@ -691,6 +709,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int row = quarter * 32 + lane;
     const int ew = warp - 2;
     const uint32_t box = base + NST * STG + ew * BOX_BYTES;
+    // where box c4 of this warp's part of a kept tile goes
+    auto kept_box = [&](int tile, int c4) {
+      return args.keep + (((static_cast<size_t>(tile) * CTAS + cta_rank) * EPI_WARPS + ew) * 4 + c4) * 1024;
+    };
     int it = 0;
     bool ok = true;
     if (epi_scaled(EPI) && args.norm_partials != nullptr) {
@@ -781,6 +803,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
           part = warp_sum(part);
           if (lane == 0) args.partials[(static_cast<size_t>(tile) * CTAS + cta_rank) * EPI_WARPS + ew] = part;
+          if (args.keep != nullptr && m0 + quarter * 32 < args.M) {
+#pragma unroll
+            for (int c4 = 0; c4 < 4; ++c4)
+              if (nb + c4 * 32 < args.N) keep_f32x32(kept_box(tile, c4), accr + c4 * 32, lane);
+          }
         } else if (slot < 0) {
           if (m0 + quarter * 32 < args.M) {
 #pragma unroll
@@ -805,7 +832,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       tc_fence_after();
       const uint32_t tbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + (EPI == EPI_GRAM ? 0 : acc * BN);
       float part = 0.f;
-      if (EPI == EPI_STORE) {
+      if constexpr (EPI == EPI_STORE || EPI == EPI_KEEP) {
         // this warp's 128 columns into registers, then the accumulator goes back to the MMA warp at once
         const int col0 = (ew >> 2) * 128;
         float v[128];
@@ -819,6 +846,22 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           else mbar_arrive_cluster(mapa_u32(tempty_bar(acc), 0));
         }
         ++it;
+        if constexpr (EPI == EPI_KEEP) {
+          // (rows and columns outside the matrix were zero-filled by the loads)
+          float sq[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int i = 0; i < 128; ++i) sq[i & 3] = fmaf(v[i], v[i], sq[i & 3]);
+          part = warp_sum((sq[0] + sq[1]) + (sq[2] + sq[3]));
+          if (lane == 0) args.partials[(static_cast<size_t>(tile) * CTAS + cta_rank) * EPI_WARPS + ew] = part;
+          if (m0 + quarter * 32 < args.M) {
+#pragma unroll
+            for (int c4 = 0; c4 < 4; ++c4) {
+              const int n = n0 + col0 + c4 * 32;
+              if (n < args.N) keep_f32x32(kept_box(tile, c4), v + c4 * 32, lane);
+            }
+          }
+          continue;
+        }
         if (slot >= 0) {   // K-split unit: park the raw accumulator for the fix-up kernel
 #pragma unroll
           for (int c4 = 0; c4 < 4; ++c4)
@@ -946,6 +989,92 @@ __global__ void __launch_bounds__(256) splitk_fixup_kernel(const float* __restri
   }
   for (int j = 0; j < 4; ++j)
     if (n + j < N) store_as(out, out_dt, idx0 + j, v[j]);
+}
+
+// ---- the clipped sum of kept products: out = sum_b (c_b scale) P_b + noise ----------------------------------------
+// HBM-bound: B fp32 tiles read once, one written.  A block takes one 32 x 32 box of every sample as an epilogue warp
+// left it (keep_f32x32): four adjacent elements a thread, eight samples' loads under way, and the sum goes through
+// shared memory so that rows are written in whole.  Eight samples are summed
+// among themselves and then added to the rest, so the chain of the sum is an eighth of B.
+__global__ void __launch_bounds__(256) weighted_sum_kernel(const float* __restrict__ P, const TcFactorSource fs, int B, int ctas,
+                                                           int tiles_m, size_t sample_stride, int M, int N,
+                                                           void* __restrict__ out, int out_dt, int vec_out, float scale, NoiseKey nk) {
+  // box -> tile, CTA of the pair, epilogue warp (lane quarter, column half), 32 columns
+  const int c4 = blockIdx.x & 3, ew = (blockIdx.x >> 2) & 7, rank = ctas == 2 ? (blockIdx.x >> 5) & 1 : 0;
+  const int tile = blockIdx.x / (32 * ctas);
+  const int mi = tile % tiles_m, ni = tile / tiles_m;
+  const int m0 = (mi * ctas + rank) * BM + ((ew + 2) & 3) * 32, n0 = ni * BN + (ew >> 2) * 128 + c4 * 32;
+  if (m0 >= M || n0 >= N) return;
+  __shared__ float4 box[8][33];
+  __shared__ float sfac[KEEP_SMEM_FACTORS];
+  pdl_wait();
+  if (fs.factors == nullptr) {     // few partials: every block derives the factors, as the per-sample epilogue does
+    for (int b = threadIdx.x >> 5; b < B; b += 8) {
+      const float* pp = fs.norm_partials + static_cast<size_t>(b) * fs.nparts;
+      float sq = 0.f;
+      for (int i = threadIdx.x & 31; i < fs.nparts; i += 32) sq += pp[i];
+      sq = warp_sum(sq);
+      if ((threadIdx.x & 31) == 0) {
+        const float n = norm_of_sumsq(sq), f = clip_factor(n, fs.C, fs.clamp);
+        sfac[b] = f;
+        if (blockIdx.x == 8) {     // the box at row 0 and column 0, which every matrix has
+          if (fs.norms_out != nullptr) fs.norms_out[b] = n;
+          if (fs.factors_out != nullptr) fs.factors_out[b] = f;
+        }
+      }
+    }
+    __syncthreads();
+  }
+  const float* factors = fs.factors != nullptr ? fs.factors : sfac;
+  const float4* p = reinterpret_cast<const float4*>(P) + static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x;
+  const size_t stride = sample_stride / 4;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto add = [&](float4& a, float c, const float4& v) {
+    a.x = fmaf(c, v.x, a.x); a.y = fmaf(c, v.y, a.y); a.z = fmaf(c, v.z, a.z); a.w = fmaf(c, v.w, a.w);
+  };
+  constexpr int U = 8;
+  int b = 0;
+  for (; b + U <= B; b += U, p += U * stride) {
+    float4 v[U], t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < U; ++k) v[k] = __ldcs(p + k * stride);
+#pragma unroll
+    for (int k = 0; k < U; ++k) add(t, factors[b + k] * scale, v[k]);
+    acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
+  }
+  for (; b < B; ++b, p += stride) add(acc, factors[b] * scale, __ldcs(p));
+  box[threadIdx.x >> 5][threadIdx.x & 31] = acc;
+  __syncthreads();
+  acc = box[threadIdx.x & 7][threadIdx.x >> 3];
+  const int m = m0 + (threadIdx.x >> 3), n = n0 + (threadIdx.x & 7) * 4;
+  if (m >= M || n >= N) return;
+  const size_t idx = static_cast<size_t>(m) * N + n;
+  float r[4] = {acc.x, acc.y, acc.z, acc.w};
+  if (nk.std != 0.f) {
+    if ((idx & 3) == 0) {
+      float z[4];
+      noise_group(nk, idx >> 2, z);
+      r[0] += z[0]; r[1] += z[1]; r[2] += z[2]; r[3] += z[3];
+    } else {     // a row pitch that is no multiple of four
+#pragma unroll
+      for (int j = 0; j < 4; ++j) r[j] += noise_at(nk, idx + j);
+    }
+  }
+  if (vec_out) {     // N a multiple of four, `out` aligned to four elements
+    if (out_dt == FDP_F32) {
+      reinterpret_cast<float4*>(out)[idx >> 2] = make_float4(r[0], r[1], r[2], r[3]);
+    } else if (out_dt == FDP_BF16) {
+      const __nv_bfloat162 a = __floats2bfloat162_rn(r[0], r[1]), c = __floats2bfloat162_rn(r[2], r[3]);
+      reinterpret_cast<uint2*>(out)[idx >> 2] = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&c));
+    } else {
+      const __half2 a = __floats2half2_rn(r[0], r[1]), c = __floats2half2_rn(r[2], r[3]);
+      reinterpret_cast<uint2*>(out)[idx >> 2] = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&c));
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (n + j < N) store_as(out, out_dt, idx + j, r[j]);
+  }
 }
 
 // ---- c_b pre-scale: Gs[r,:] = c[r / T] * G[r,:] (HBM-bound, 16-byte vectors) ------------------------
@@ -1318,11 +1447,65 @@ static bool wide_ok(int B, int T, int n_in, int n_out, int norm_algo) {
 
 // The tensor-core path needs 16-bit inputs, row pitches that are multiples of 16 bytes, and
 // matrices large enough that the 128x256 tile is not mostly padding.
+// tiles of a sample's product, in the orientation that has more (the workspace query does not know the layout)
+static int most_product_tiles(int n_in, int n_out) {
+  const int ctas = ctas_per_tile();
+  const int a = ceil_div(n_out, BM * ctas) * ceil_div(n_in, BN), b = ceil_div(n_in, BM * ctas) * ceil_div(n_out, BN);
+  return a > b ? a : b;
+}
+static size_t keep_bytes(int B, int n_in, int n_out) {
+  return static_cast<size_t>(B) * most_product_tiles(n_in, n_out) * ctas_per_tile() * BM * BN * sizeof(float);
+}
+// Whether keeping the per-sample products beats the plan `p` that contracts twice, by estimates in us of both.  Fitted to
+// 36 shapes, B 1 to 64, T 64 to 4096, widths 64 to 11008, both sides timed (within 10 % but for the smallest); they part
+// where B n_in n_out fp32 elements written and read cost what a norm pass costs: 8 x 1024 rows 1024 -> 3072 bf16 70 us
+// kept, 82 contracted twice; 12 x 500, 1024 -> 4096 94 / 80; 16 x 512, 4096 -> 4096 539 / 331; 4 x 2048, 4096 -> 11008
+// 690 / 735; fp32 (three products) 8 x 1024, 1024 -> 3072 182 / 270.
+// The SM count is a constant here: the workspace query and the launch must pick the same plan.
+static bool keep_wins(int B, int T, int n_in, int n_out, const TcPlan& p) {
+  if (keep_bytes(B, n_in, n_out) > KEEP_LIMIT) return false;
+  // 16-bit samples of few rows leave faster than they can be written (64 x 128 rows, 1024 -> 1024: 101 us kept, 47; 48 x 64,
+  // 768 -> 3072: 160 / 53); only calls of a few launches gain there (5 x 92, 512 -> 512: 12.6 / 18.6), which the host bounds.
+  if (p.planes == 1 && T < 256) return false;
+  const int i = p.planes - 1, workers = MAX_SMS / 2;
+  const int tiles = most_product_tiles(n_in, n_out), stages = ceil_div(T, BK);
+  const auto rounds = [](long long units, int on) { return static_cast<double>((units + on - 1) / on); };
+  const double elements = static_cast<double>(n_in) * n_out, launch = 6.0;
+  const double product_rounds = rounds(static_cast<long long>(B) * tiles, workers);
+  constexpr double KEEP_STAGE[3] = {0.38, 1.22, 2.9}, KEEP_FIXED[3] = {1.8, 2.2, 2.2}, KEEP_LEAST[3] = {3.5, 5.0, 5.0};
+  const double round = stages * KEEP_STAGE[i] + KEEP_FIXED[i];
+  const double keep = launch + product_rounds * (round > KEEP_LEAST[i] ? round : KEEP_LEAST[i]) + 3.5 + 4.0 * elements * (B + 1) / 6.4e6;
+
+  double norm;
+  if (p.planes > 1) {
+    constexpr double STAGE[3] = {0.0, 1.05, 2.45}, FIXED[3] = {0.0, 0.5, 1.5};
+    norm = launch + product_rounds * (stages * STAGE[i] + FIXED[i]);
+  } else if (p.algo == FDP_NORM_DIRECT) {
+    norm = 4.0 + rounds(static_cast<long long>(B) * ceil_div(n_out, BM) * ceil_div(n_in, BN), MAX_SMS) * (stages * 0.42 + 1.0);
+  } else {
+    norm = 4.0 + rounds(static_cast<long long>(B) * gram_tiles(T), MAX_SMS) * ((ceil_div(n_in, BK) + ceil_div(n_out, BK)) * 0.40 + 1.0);
+  }
+  const int k = p.scaled_epilogue ? B * stages : ceil_div(B * T, BK);
+  const int split = plan_tail_split(tiles, k, workers, p.planes == 3 ? 6 : p.planes == 2 ? 3 : 1);
+  const int rem = tiles <= workers ? tiles : tiles % workers;
+  const double waves = (tiles - rem) / workers + rounds(static_cast<long long>(rem) * split, workers) / split;
+  constexpr double SUM_STAGE[3] = {0.40, 1.2, 2.2};
+  double sum = launch + waves * (k * SUM_STAGE[i] + (p.scaled_epilogue && p.planes == 1 ? 0.5 * B : 0.0));
+  if (split > 1) sum += 4.0 + 0.04 * rem * split;
+  if (!p.scaled_epilogue) sum += 4.5 + 4.0 * B * T * n_out / 5e6;
+  // Six products are to be no further from float64 than before: a K split cuts the chain of a long sample's sum, which
+  // keeping does not (one sample of 2816 rows 1.8e-7 against 0.9e-7 in four parts).
+  if (p.planes == 3 && stages > 16 && B < split) return false;
+  // (fp32 calls hold the parts of both operands already: a tenth has to be gained for more)
+  return keep < (p.planes > 1 ? 0.9 : 0.97) * (norm + sum);
+}
+
 TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
   TcPlan p; p.ok = false; p.algo = FDP_NORM_DIRECT; p.ws_bytes = 0; p.nparts = 0; p.scaled_epilogue = false;
-  p.short_seq = false; p.any_align = false; p.split_bytes = 0;
+  p.short_seq = false; p.any_align = false; p.keep = false; p.split_bytes = 0;
   p.planes = 1; p.split_g_bytes = p.split_x_bytes = 0;
   const bool fp32_tensor = (norm_algo & FDP_FP32_TENSOR) != 0, fp32_wide = (norm_algo & FDP_FP32_WIDE) != 0;
+  const bool may_keep = (norm_algo & (FDP_KEEP_PRODUCTS | FDP_NORM_MASK)) == (FDP_KEEP_PRODUCTS | FDP_NORM_AUTO);
   norm_algo &= FDP_NORM_MASK;
   if (dt == FDP_F32) {
     // fp32 on the tensor cores, when the caller asks for it.  FDP_FP32_TENSOR: three bf16 products (hi*hi +
@@ -1351,6 +1534,14 @@ TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
     const int ctas = ctas_per_tile();
     p.ok = true; p.algo = FDP_NORM_DIRECT; p.scaled_epilogue = true;
     p.nparts = ceil_div(n_out, BM * ctas) * ceil_div(n_in, BN) * ctas * epi_warps_for(EPI_STORE_SCALED);
+    if (may_keep && keep_wins(B, T, n_in, n_out, p)) {
+      p.keep = true; p.scaled_epilogue = false;
+      p.nparts = most_product_tiles(n_in, n_out) * ctas_per_tile() * epi_warps_for(EPI_KEEP);
+      // never less than the parking area: a call that is short of memory gives way where it did before
+      const size_t kept = keep_bytes(B, n_in, n_out);
+      if (kept > p.split_bytes) p.split_bytes = kept;
+      p.ws_bytes = p.split_bytes + p.split_g_bytes + p.split_x_bytes;
+    }
     return p;
   }
   if (dt != FDP_BF16 && dt != FDP_F16) return p;
@@ -1390,6 +1581,11 @@ TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
   // the parked accumulators of the split-K tail, then (pre-scale path only) the c_b-scaled copy of G
   p.split_bytes = split_ws_bytes();
   p.ws_bytes = p.split_bytes + (p.scaled_epilogue ? 0 : align256(static_cast<size_t>(B) * T * n_out * 2));
+  if (may_keep && keep_wins(B, T, n_in, n_out, p)) {
+    p.keep = true; p.scaled_epilogue = false; p.algo = FDP_NORM_DIRECT;
+    p.nparts = most_product_tiles(n_in, n_out) * ctas_per_tile() * epi_warps_for(EPI_KEEP);
+    p.split_bytes = p.ws_bytes = keep_bytes(B, n_in, n_out);
+  }
   return p;
 }
 
@@ -1441,7 +1637,7 @@ int tc_split_stats(const void* G, void* dst, float* colsum_part, float* sq_part,
 }
 
 int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int B, int T, int n_in,
-             int n_out, int dt, const TcPlan& pl, cudaStream_t s) {
+             int n_out, int dt, const TcPlan& pl, cudaStream_t s, float* keep, int layout) {
   const uint64_t rows = static_cast<uint64_t>(B) * T;
   CUtensorMap a, b, a2, b2;
   TcArgs args{};
@@ -1452,22 +1648,39 @@ int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int
     // clipped-sum GEMM, handed to the epilogue every few K stages and summed there in registers; a
     // unit is (sample, tile) and ends with the sum of its squares instead of a store
     const int po = pitch8(n_out), pi = pitch8(n_in);
-    if (!make_rows_map(&a, G, B, T, pl.planes * po, dt) || !make_rows_map(&b, X, B, T, pl.planes * pi, dt)) return FDP_ERR_LAUNCH;
+    const bool oi = keep == nullptr || layout == FDP_OUT_IN;     // products that are kept have the output's orientation
+    if (!make_rows_map(oi ? &a : &b, G, B, T, pl.planes * po, dt) || !make_rows_map(oi ? &b : &a, X, B, T, pl.planes * pi, dt))
+      return FDP_ERR_LAUNCH;
     const int ctas = ctas_per_tile();
-    args.M = n_out; args.N = n_in; args.ld_out = n_in;
-    args.tiles_m = ceil_div(n_out, BM * ctas); args.tiles_n = ceil_div(n_in, BN);
+    args.M = oi ? n_out : n_in; args.N = oi ? n_in : n_out; args.ld_out = args.N;
+    args.tiles_m = ceil_div(args.M, BM * ctas); args.tiles_n = ceil_div(args.N, BN);
     args.tiles_per_batch = args.tiles_m * args.tiles_n;
     args.k_stages = ceil_div(T, BK);
-    args.plane_a = po; args.plane_b = pi;
+    args.plane_a = oi ? po : pi; args.plane_b = oi ? pi : po;
     args.idesc = make_idesc(dt, true, true, ctas);
     args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = chain_stages(args.seg_stages, pl.planes);
     args.scale = 1.0f; args.nk = NoiseKey{};
     args.zero_status = 0; args.dependent = 1;      // follows the split kernel, which has cleared the status word
+    args.keep = keep;
     if (pl.planes == 3)
       return ctas == 2 ? launch<true, true, EPI_SPLIT6_SUMSQ, 2>(a, b, a, b, a, args, s)
                        : launch<true, true, EPI_SPLIT6_SUMSQ, 1>(a, b, a, b, a, args, s);
     return ctas == 2 ? launch<true, true, EPI_SPLIT_SUMSQ, 2>(a, b, a, b, a, args, s)
                      : launch<true, true, EPI_SPLIT_SUMSQ, 1>(a, b, a, b, a, args, s);
+  }
+  if (keep != nullptr) {
+    const bool oi = layout == FDP_OUT_IN;
+    const int ctas = ctas_per_tile();
+    args.M = oi ? n_out : n_in; args.N = oi ? n_in : n_out;
+    if (!make_rows_map(oi ? &a : &b, G, B, T, n_out, dt) || !make_rows_map(oi ? &b : &a, X, B, T, n_in, dt))
+      return FDP_ERR_LAUNCH;
+    args.keep = keep;
+    args.tiles_m = ceil_div(args.M, BM * ctas); args.tiles_n = ceil_div(args.N, BN);
+    args.tiles_per_batch = args.tiles_m * args.tiles_n;
+    args.k_stages = ceil_div(T, BK); args.seg_stages = args.k_stages;
+    args.idesc = make_idesc(dt, true, true, ctas);
+    return ctas == 2 ? launch<true, true, EPI_KEEP, 2>(a, b, a, b, a, args, s)
+                     : launch<true, true, EPI_KEEP, 1>(a, b, a, b, a, args, s);
   }
   if (pl.algo == FDP_NORM_DIRECT) {
     if (!make_rows_map(&a, G, B, T, n_out, dt) || !make_rows_map(&b, X, B, T, n_in, dt)) return FDP_ERR_LAUNCH;
@@ -1500,6 +1713,22 @@ int tc_prescale(const void* G, const float* factors, void* Gs, int B, int T, int
     prescale_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)G, factors, (__nv_bfloat16*)Gs, nvec, vps);
   else
     prescale_kernel<__half><<<grid, 256, 0, s>>>((const __half*)G, factors, (__half*)Gs, nvec, vps);
+  note_launch();
+  return FDP_OK;
+}
+
+static int product_tiles(int M, int N) { return ceil_div(M, BM * ctas_per_tile()) * ceil_div(N, BN); }
+int tc_keep_partials(int n_in, int n_out, int layout) {
+  return product_tiles(layout == FDP_OUT_IN ? n_out : n_in, layout == FDP_OUT_IN ? n_in : n_out) * ctas_per_tile() * epi_warps_for(EPI_KEEP);
+}
+bool tc_keep_fused_factors_ok(int B, int nparts) { return B <= KEEP_SMEM_FACTORS && B * nparts <= 2048; }
+int tc_weighted_sum(const float* keep, const TcFactorSource& fs, void* dW, int B, int n_in, int n_out, int out_dt, int layout,
+                    float inv_div, NoiseKey nk, cudaStream_t s) {
+  const int M = layout == FDP_OUT_IN ? n_out : n_in, N = layout == FDP_OUT_IN ? n_in : n_out;
+  const int ctas = ctas_per_tile(), tiles = product_tiles(M, N);
+  const int vec_out = N % 4 == 0 && reinterpret_cast<uintptr_t>(dW) % (4 * dtype_size(out_dt)) == 0;
+  launch_dependent(weighted_sum_kernel, dim3(tiles * ctas * 32), dim3(256), 0, s, keep, fs, B, ctas, ceil_div(M, BM * ctas),
+                   static_cast<size_t>(tiles) * ctas * BM * BN, M, N, dW, out_dt, vec_out, inv_div, nk);
   note_launch();
   return FDP_OK;
 }

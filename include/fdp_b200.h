@@ -32,8 +32,9 @@ extern "C" {
 /* 2: asynchronous status word, SM reservation, saturating LayerNorm mode, FDP_FP32_TENSOR.
  * 3: fdp_dp_params.step_device (appended; earlier fields keep their offsets); FDP_FP32_TENSOR also
  *    accepted in the dtype of fdp_linear_dgrad / fdp_linear_fwd.
- * 4: FDP_FP32_WIDE, fdp_linear_bwd. */
-#define FDP_ABI_VERSION 4
+ * 4: FDP_FP32_WIDE, fdp_linear_bwd.
+ * 5: FDP_KEEP_PRODUCTS. */
+#define FDP_ABI_VERSION 5
 
 typedef void* fdp_stream_t; /* a cudaStream_t */
 
@@ -82,7 +83,12 @@ enum fdp_norm_algo {
    * FMA kernels (for operands of at least 2^-100 in magnitude; the parts of smaller ones run into bf16's smallest
    * numbers).  Operands and output need no alignment.  The workspace grows by 1.5 times the size of the inputs and
    * the 38.8 MB in which the parts of a K split are parked. */
-  FDP_FP32_WIDE = 32
+  FDP_FP32_WIDE = 32,
+  /* flag, OR-ed into the same arguments: with FDP_NORM_AUTO the tensor-core path may keep every sample's product
+   * G_b^T X_b in the workspace (fp32, B * n_in * n_out elements, at most 512 MiB) where that is expected to be faster
+   * than contracting twice: the norms come from the tiles as they leave, the clipped sum is their weighted sum.
+   * fp32 accumulation throughout, as without the flag. */
+  FDP_KEEP_PRODUCTS = 64
 };
 
 /* DP hyper-parameters of one call.  C / clamp_value are the arguments of

@@ -1,0 +1,87 @@
+"""Weight gradients whose per-sample products are kept and summed: tile edges, every input form, noise, against float64."""
+import pytest
+import torch
+
+from gpu_util import dev
+from test_gpu_edges import UNIT, _close_to_sum, _randn, ops  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def _kept(call):
+    """whether `call` sums kept products"""
+    call()
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    return any("weighted_sum_kernel" in e.name for e in p.events())
+
+
+# edges of the 256 x 256 tiles and their 32 x 32 boxes, one tile and several, samples that end inside a K stage, 8 and
+# more samples to a sum, three and six products
+@pytest.mark.parametrize("B,T,n_in,n_out,dtype", [
+    (1, 256, 128, 128, torch.bfloat16), (3, 270, 200, 264, torch.float16), (9, 319, 520, 136, torch.bfloat16),
+    (17, 300, 264, 776, torch.bfloat16), (2, 1000, 256, 512, torch.float16), (4, 128, 256, 320, torch.float32),
+    (9, 192, 512, 256, torch.float32), (2, 64, 64, 64, torch.float32), (3, 100, 130, 1001, torch.float32),
+    (11, 70, 259, 97, torch.float32)])
+@pytest.mark.parametrize("layout", ["out_in", "in_out"])
+def test_kept_products(ops, B, T, n_in, n_out, dtype, layout):  # noqa: F811
+    X, G = _randn(B, T, n_in, seed=1, dtype=dtype), _randn(B, T, n_out, seed=2, dtype=dtype, scale=1e-2)
+    G[0] *= 30.0
+    assert _kept(lambda: ops.dp_linear_weight_grad(X, G, 1.0, 1.0, layout=layout))
+    per = torch.einsum("bto,bti->boi", G.double(), X.double())
+    want_n = per.flatten(1).norm(dim=1)
+    f = (1.0 / (want_n + 1e-10)).clamp(max=1.0)
+    want = (f.view(-1, 1, 1) * per).sum(0) / B
+    absum = (f.view(-1, 1, 1) * torch.einsum("bto,bti->boi", G.double().abs(), X.double().abs())).sum(0) / B
+    if layout == "in_out":
+        want, absum = want.t(), absum.t()
+    # three products leave out what lies below 2^-16 of a product of two elements (2^-8 of each), the others nothing
+    dropped = 2.0 ** -16 if dtype == torch.float32 and n_in % 64 == 0 and n_out % 64 == 0 and T % 64 == 0 and T >= 128 else 0.0
+    for out_dtype in (torch.float32, torch.bfloat16):
+        dW, norms, factors = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, layout=layout, out_dtype=out_dtype, return_norms=True)
+        k = T // 16 + B + 8        # additions on the way to an element: one a K step, one a sample, the factor's roundings
+        _close_to_sum(dW, want, absum * (1 + dropped * 2 ** 23 / k), k, UNIT[out_dtype])
+        assert float(((norms.double() - want_n) / want_n).abs().max()) < (T / 16 + 8) * 2.0 ** -23 + dropped
+        assert float(((factors.double() - f) / f).abs().max()) < (T / 16 + 12) * 2.0 ** -23 + dropped
+
+
+def test_kept_products_noise_and_infinities(ops):  # noqa: F811
+    """A zero gradient returns the noise stream of the direct form bit for bit, with rows of any pitch; a sample that is
+    not finite has norm inf and factor 0 and leaves the others' elements alone."""
+    spec = ops.NoiseSpec(std=0.5, seed=77, param_id=3, step=2, rank=1, world=2)
+    for (n_in, n_out, dtype) in ((264, 200, torch.bfloat16), (259, 97, torch.float32)):
+        T = 256 if dtype == torch.bfloat16 else 128
+        X, G = _randn(4, T, n_in, seed=1, dtype=dtype), torch.zeros(4, T, n_out, device=dev(), dtype=dtype)
+        assert _kept(lambda: ops.dp_linear_weight_grad(X, G, 1.0, 1.0))
+        kw = dict(batch_divisor=8, noise=spec, out_dtype=torch.float32)
+        assert torch.equal(ops.dp_linear_weight_grad(X, G, 1.0, 1.0, **kw),
+                           ops.dp_linear_weight_grad(X, G, 1.0, 1.0, norm_algo="direct", **kw))
+        G = _randn(4, T, n_out, seed=2, dtype=dtype, scale=1e-2)
+        clean = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, out_dtype=torch.float32)
+        G[2, 5, 7] = float("inf")
+        dW, norms, factors = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, out_dtype=torch.float32, return_norms=True)
+        assert norms[2] == float("inf") and factors[2] == 0 and bool(torch.isfinite(norms[[0, 1, 3]]).all())
+        rows = torch.arange(n_out, device=dev()) != 7
+        G[2] = 0.0
+        rest = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, out_dtype=torch.float32)
+        assert torch.equal(dW[rows], rest[rows]) and not torch.equal(dW[rows], clean[rows])
+
+
+def test_kept_products_give_way(ops):  # noqa: F811
+    """Where the products do not fit the card the call contracts twice."""
+    B, T, n = 8, 2048, 2048                      # 134 MB of products
+    X, G = _randn(B, T, n, seed=1, dtype=torch.bfloat16), _randn(B, T, n, seed=2, dtype=torch.bfloat16, scale=1e-2)
+    call = lambda: ops.dp_linear_weight_grad(X, G, 1.0, 1.0, out_dtype=torch.float32)   # noqa: E731
+    assert _kept(call)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        # the result and the parking area (38.8 MB) have room, the products have not
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (96 << 20)) / total)
+        got = call()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.equal(got, ops.dp_linear_weight_grad(X, G, 1.0, 1.0, out_dtype=torch.float32, norm_algo="direct"))
