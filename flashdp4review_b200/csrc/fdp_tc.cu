@@ -176,24 +176,10 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
 }
-__device__ __forceinline__ void tc_mma_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t r[32]) {
   asm volatile(
@@ -209,24 +195,43 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t r[32]) {
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // shared-memory matrix descriptor (sm_100 format): start address, leading / stride byte offsets in
-// 16-byte units, version 1, 128-byte swizzle
-__device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr >> 4) & 0x3FFF);
-  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= static_cast<uint64_t>(1) << 46;  // descriptor version of sm_100
-  d |= static_cast<uint64_t>(2) << 61;  // SWIZZLE_128B
+// 16-byte units, version 1, 128-byte swizzle.  The low word holds the address (and the leading offset), so that what
+// moves with the stage and the K slice is one 32-bit addition.
+struct Desc { uint32_t lo, hi; };
+__device__ __forceinline__ Desc make_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  Desc d;
+  d.lo = ((saddr >> 4) & 0x3FFF) | (((lbo_bytes >> 4) & 0x3FFF) << 16);
+  d.hi = ((sbo_bytes >> 4) & 0x3FFF) | (1u << 14) /* descriptor version of sm_100 */ | (2u << 29) /* SWIZZLE_128B */;
   return d;
 }
-// Descriptor of the k16-th UMMA_K slice of an operand stage.
+// Descriptor of an operand whose first stage is at `saddr`, and the step of its low word to the k16-th UMMA_K slice.
 //  MN-major: 64-element (128 B) MN chunks of BK rows each, chunk stride BK*128 B (leading offset),
 //            8-row groups 1024 B apart (stride offset); a K=16 slice is 16 rows = 2048 B further.
 //  K-major : rows of 128 B (64 K elements), 8-row groups 1024 B apart; a K=16 slice is 32 B further.
 template <bool MN_MAJOR>
-__device__ __forceinline__ uint64_t operand_desc(uint32_t stage_base, int k16) {
-  if (MN_MAJOR) return make_desc(stage_base + k16 * (UMMA_K * 128), BK * 128, 1024);
-  return make_desc(stage_base + k16 * (UMMA_K * 2), 0, 1024);
+__device__ __forceinline__ Desc operand_desc(uint32_t saddr) { return make_desc(saddr, MN_MAJOR ? BK * 128 : 0, 1024); }
+template <bool MN_MAJOR>
+__device__ __forceinline__ constexpr uint32_t slice_step(int k16) { return (k16 * UMMA_K * (MN_MAJOR ? 128 : 2)) >> 4; }
+template <int CTAS>
+__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                       uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "mov.b64 a, {%1, %2};\n\t"
+      "mov.b64 b, {%3, %4};\n\t"
+      "tcgen05.mma.cta_group::%7.kind::f16 [%0], a, b, %5, p;\n\t}"
+      ::"r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "n"(CTAS) : "memory");
+}
+// one lane of the warp, the same one every time
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
 }
 
 // The Gaussian noise of 32 adjacent output elements starting at flat index idx0 (a multiple of 4: the
@@ -416,7 +421,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   // six products: accumulator hand-offs per K stage.  In the norm pass the truncation of the accumulators does not
   // average out over the elements (it shrinks all of them), so its chains hold two large steps instead of four.
   constexpr int SUBS = (EPI == EPI_SPLIT6_SUMSQ) ? 2 : 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (uniform, and known to be)
   const int total_tiles = args.batch * args.tiles_per_batch;
   const int kst_total = args.k_stages + (EPI == EPI_GRAM ? args.k_stages2 : 0);
   const int total_units = args.units_full + (total_tiles - args.units_full) * args.split;
@@ -516,8 +521,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   };
 
   if (warp == 0) {
-    // ================= TMA producer =================
-    if (lane == 0) {
+    // ================= TMA producer (the warp walks the loop, one elected lane issues) =================
+    {
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
       for (int u = wid; u < total_units && ok; u += wstep) {
@@ -530,12 +535,13 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         int z = 0, t = 0;
         if (A_MN && B_MN) { z = b + ks0 / args.seg_stages; t = ks0 % args.seg_stages * BK; }
         for (int ks = ks0; ks < ks1; ++ks) {
-          if (!mbar_wait(empty_bar(stage), phase ^ 1u, wctx, 1)) { ok = false; break; }
+          if (!mbar_wait_warp(empty_bar(stage), phase ^ 1u, wctx, 1)) { ok = false; break; }
           const bool second = (EPI == EPI_GRAM) && ks >= args.k_stages;
           const CUtensorMap* ma = second ? &tmA2 : &tmA;
           const CUtensorMap* mb = second ? &tmB2 : &tmB;
           const int k0 = (second ? ks - args.k_stages : ks) * BK;
           const uint32_t sa = base + stage * STG, sb = sa + A_BYTES;
+          if (elect_one()) {
           if (EPI == EPI_GRAM) {
             // A: the t-block; B: two independent 128-row s-blocks, one per half of the stage
             // (a unit that contains the diagonal block (i, i) has its t-block in the B stage already:
@@ -577,15 +583,17 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 load(db, mb, k0 + cb, nb0);
               }
             }
-            if (A_MN && B_MN) {
-              t += BK;
-              if (t >= args.seg_stages * BK) { t = 0; ++z; }
-            }
+          }
+          }
+          __syncwarp();
+          if (A_MN && B_MN) {
+            t += BK;
+            if (t >= args.seg_stages * BK) { t = 0; ++z; }
           }
           if (++stage == NST) { stage = 0; phase ^= 1u; }
         }
       }
-      if (!ok) {
+      if (!ok && lane == 0) {
         // wait (bounded) for the copies already in flight before the CTA may leave
         for (int s = 0; s < NST; ++s) {
           const long long t0 = clock64();
@@ -596,27 +604,42 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
   } else if (warp == 1) {
     // ================= MMA issuer (the leader CTA of a pair issues for both) =================
+    // The whole warp walks the loop and one elected lane issues, so that addresses and descriptors stay in uniform
+    // registers: issued from a branch of one lane, an instruction took about 130 cycles, as long as the 256 x 256 x 16
+    // product itself, and every wait of the loop held the tensor cores up (one pair alone, 256 x 256 tile: 0.30 us a K stage
+    // whatever the ring's depth, now 0.19; 16384 rows, 1024 -> 3072 bf16: 83 us, now 74; 32768 x 4096 x 4096 clipped sum
+    // with its norms 1007 -> 897).
     auto commit = [&](uint32_t bar) {   // signals `bar` (in both CTAs of a pair) when the MMAs issued so far are done
       if (CTAS == 1) tc_commit(bar); else tc_commit_pair(bar);
     };
-    // The six products of K slices [k0, k1) of a stage, smallest first: the accumulator is added to by truncation,
-    // one unit in its last place per step, so the steps that come before it is large cost nothing.
-    auto issue_six = [&](uint32_t d, uint32_t sa, uint32_t idesc, int k0, int k1, bool fresh) {
-      constexpr int PA[6] = {0, 2, 1, 0, 1, 0}, PB[6] = {2, 0, 1, 1, 0, 0};   // hi*lo, lo*hi, mid*mid, hi*mid, mid*hi, hi*hi
-      const uint32_t sb = sa + A_BYTES;
-#pragma unroll
-      for (int q = 0; q < 6; ++q)
-        for (int k16 = k0; k16 < k1; ++k16) {
-          const uint64_t da = operand_desc<A_MN>(sa + PA[q] * A_STAGE_BYTES, k16);
-          const uint64_t db = operand_desc<B_MN>(sb + PB[q] * B_BYTES, k16);
-          const uint32_t acc_in = (fresh && k16 == k0 && q == 0) ? 0u : 1u;
-          if (CTAS == 1) tc_mma(d, da, db, idesc, acc_in); else tc_mma_pair(d, da, db, idesc, acc_in);
-        }
-    };
-    if (lane == 0 && is_leader) {
+    if (is_leader) {
       int stage = 0; uint32_t phase = 0;
       int it = 0;
       bool ok = true;
+      const Desc a0 = operand_desc<A_MN>(base), b0 = operand_desc<B_MN>(base + A_BYTES);
+      // products of a K slice, by the parts of A and B they take.  Three: hi*lo, lo*hi, hi*hi.  Six, smallest first (the
+      // accumulator is added to by truncation, one unit in its last place per step, so the steps that come before it is
+      // large cost nothing): hi*lo, lo*hi, mid*mid, hi*mid, mid*hi, hi*hi.
+      constexpr int PRODUCTS = PLANES == 3 ? 6 : PLANES == 2 ? 3 : 1;
+      constexpr int PA[3][6] = {{0}, {0, 1, 0}, {0, 2, 1, 0, 1, 0}}, PB[3][6] = {{0}, {1, 0, 0}, {2, 0, 1, 1, 0, 0}};
+      // issues the products of K slices [k0, k1) of the stage at offset `so`, in slices or product by product
+      auto issue = [&](uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, auto k0, auto k1, bool fresh) {
+        auto one = [&](int q, int k16, bool first) {
+          tc_mma<CTAS>(d, a_lo + PA[PLANES - 1][q] * (A_STAGE_BYTES >> 4) + slice_step<A_MN>(k16), a0.hi,
+                       b_lo + PB[PLANES - 1][q] * (B_BYTES >> 4) + slice_step<B_MN>(k16), b0.hi, idesc, first && fresh ? 0u : 1u);
+        };
+        if constexpr (PLANES == 3) {
+#pragma unroll
+          for (int q = 0; q < PRODUCTS; ++q)
+#pragma unroll
+            for (int k16 = k0; k16 < k1; ++k16) one(q, k16, q == 0 && k16 == k0);
+        } else {
+#pragma unroll
+          for (int k16 = k0; k16 < k1; ++k16)
+#pragma unroll
+            for (int q = 0; q < PRODUCTS; ++q) one(q, k16, q == 0 && k16 == k0);
+        }
+      };
       for (int u = wid; u < total_units && ok; u += wstep) {
         int tile, ks0, ks1, slot, tb, tm0, tn0, half;
         decode_unit(u, tile, ks0, ks1, slot);
@@ -633,16 +656,21 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // one accumulator per segment: the whole unit, or one sample's share of it for EPI_STORE_SCALED
         if constexpr (SUBS > 1) {
           for (; ks < ks1 && ok; ++ks) {
-            if (!mbar_wait(full_bar(stage), phase, wctx, 3)) { ok = false; break; }
+            if (!mbar_wait_warp(full_bar(stage), phase, wctx, 3)) { ok = false; break; }
+            const uint32_t so = static_cast<uint32_t>(stage * STG) >> 4;
+#pragma unroll
             for (int sub = 0; sub < SUBS; ++sub, ++it) {
               const int acc = it % NUM_ACC;
-              if (!mbar_wait(tempty_bar(acc), ((it / NUM_ACC) & 1u) ^ 1u, wctx, 2)) { ok = false; break; }
+              if (!mbar_wait_warp(tempty_bar(acc), ((it / NUM_ACC) & 1u) ^ 1u, wctx, 2)) { ok = false; break; }
               tc_fence_after();
-              issue_six(tmem_base + acc * BN, base + stage * STG, idesc, sub * (4 / SUBS), (sub + 1) * (4 / SUBS), true);
-              commit(tfull_bar(acc));
+              if (elect_one()) {
+                issue(tmem_base + acc * BN, a0.lo + so, b0.lo + so, idesc, sub * (4 / SUBS), (sub + 1) * (4 / SUBS), true);
+                commit(tfull_bar(acc));
+                if (sub == SUBS - 1) commit(empty_bar(stage));
+              }
+              __syncwarp();
             }
             if (!ok) break;
-            commit(empty_bar(stage));
             if (++stage == NST) { stage = 0; phase ^= 1u; }
           }
         }
@@ -658,45 +686,34 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
           const int acc = it % NUM_ACC;
           const uint32_t acc_phase = (it / NUM_ACC) & 1u;
-          if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, wctx, 2)) { ok = false; break; }
+          if (!mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, wctx, 2)) { ok = false; break; }
           tc_fence_after();
           for (; ks < seg_end; ++ks) {
-            if (!mbar_wait(full_bar(stage), phase, wctx, 3)) { ok = false; break; }
+            if (!mbar_wait_warp(full_bar(stage), phase, wctx, 3)) { ok = false; break; }
             tc_fence_after();
             const bool second = (EPI == EPI_GRAM) && ks >= args.k_stages;
             const uint32_t d = tmem_base + (EPI == EPI_GRAM ? (second ? BN : 0) : acc * BN);
             const bool first_stage = second ? (ks == args.k_stages) : (ks == seg_begin);
-            uint32_t sa = base + stage * STG;
-            const uint32_t sb = sa + A_BYTES;
+            const uint32_t so = static_cast<uint32_t>(stage * STG) >> 4;
+            uint32_t a_lo = a0.lo + so;
+            const uint32_t b_lo = b0.lo + so;
             if (EPI == EPI_GRAM) {   // diagonal block in this unit: A is the matching half of the B stage
-              if (tn0 == tm0) sa = sb;
-              else if (gram_n1 == tm0) sa = sb + B_STAGE_BYTES / 2;
+              if (tn0 == tm0) a_lo = b_lo;
+              else if (gram_n1 == tm0) a_lo = b_lo + (B_STAGE_BYTES / 2 >> 4);
             }
-            if constexpr (PLANES == 3) {
-              issue_six(d, sa, idesc, 0, BK / UMMA_K, first_stage);
-            } else {
-#pragma unroll
-              for (int k16 = 0; k16 < BK / UMMA_K; ++k16) {
-#pragma unroll
-                for (int q = 0; q < (PLANES == 2 ? 3 : 1); ++q) {   // hi*lo, lo*hi, hi*hi
-                  const uint64_t da = operand_desc<A_MN>(sa + (PLANES == 2 && q == 1 ? A_STAGE_BYTES : 0), k16);
-                  const uint64_t db = operand_desc<B_MN>(sb + (PLANES == 2 && q == 0 ? B_BYTES : 0), k16);
-                  const uint32_t acc_in = (first_stage && k16 == 0 && q == 0) ? 0u : 1u;
-                  if (CTAS == 1) tc_mma(d, da, db, idesc, acc_in); else tc_mma_pair(d, da, db, idesc, acc_in);
-                }
-              }
+            if (elect_one()) {
+              issue(d, a_lo, b_lo, idesc, 0, BK / UMMA_K, first_stage);
+              // frees the stage (in both CTAs of a pair) once these MMAs have read it
+              commit(empty_bar(stage));
+              if (ks + 1 == seg_end) commit(tfull_bar(acc));
             }
-            // frees the stage (in both CTAs of a pair) once these MMAs have read it
-            commit(empty_bar(stage));
+            __syncwarp();
             if (++stage == NST) { stage = 0; phase ^= 1u; }
           }
-          if (ok) {
-            commit(tfull_bar(acc));
-            ++it;
-          }
+          if (ok) ++it;
         }
       }
-      if (!ok) {
+      if (!ok && elect_one()) {
         // let MMAs already issued finish before TMEM is released
         commit(drain_bar);
         const long long t0 = clock64();
