@@ -85,3 +85,23 @@ def test_kept_products_give_way(ops):  # noqa: F811
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert torch.equal(got, ops.dp_linear_weight_grad(X, G, 1.0, 1.0, out_dtype=torch.float32, norm_algo="direct"))
+
+
+# products whose last round of tiles is cut in two along N: behind full rounds, alone, with halves that overhang or miss
+# the matrix, K-major and MN-major weights, 16-bit and fp32 (three products)
+@pytest.mark.parametrize("rows,K,N", [(256 * 80, 64, 256), (256 * 25 + 3, 128, 776), (200, 320, 264), (130, 128, 136)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("layout", ["out_in", "in_out"])
+def test_cut_tiles(ops, rows, K, N, dtype, layout):  # noqa: F811
+    if dtype == torch.float32 and K < 128:
+        K = 128
+    X, W = _randn(rows, K, seed=1, dtype=dtype), _randn(*((N, K) if layout == "out_in" else (K, N)), seed=2, dtype=dtype, scale=0.1)
+    b = _randn(N, seed=3, dtype=dtype)
+    w = W if layout == "in_out" else W.t()
+    want, absum = X.double() @ w.double() + b.double(), X.double().abs() @ w.double().abs() + b.double().abs()
+    # three products leave out what lies below 2^-16 of a product of two elements
+    k = K / 16 + 8 + (2.0 ** 7 if dtype == torch.float32 else 0)
+    _close_to_sum(ops.linear_forward(X, W, b, layout), want, absum, k, UNIT[dtype])
+    G = _randn(rows, N, seed=4, dtype=dtype)
+    _close_to_sum(ops.linear_input_grad(G, W, layout), G.double() @ w.double().t(), G.double().abs() @ w.double().abs().t(),
+                  N / 16 + 8 + (2.0 ** 7 if dtype == torch.float32 else 0), UNIT[dtype])
