@@ -159,8 +159,12 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// Hands an accumulator back to the leader's MMA warp.  Relaxed: no memory is handed over with it, the accumulator's loads
+// have completed (tcgen05.wait::ld) and tcgen05.fence orders the rest.  A release at cluster scope waits for the warp's
+// own earlier stores and took 1300 to 2500 cycles, in which the pair's tensor cores ran dry (weight gradients in six products,
+// 16 x 197 rows 768 -> 3072: 151 us, now 134; 5 x 704, 64 -> 7928: 153 / 121; one pair alone in three products, 8192 deep: 89 / 64).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t leader_bar) {
   asm volatile(
@@ -513,16 +517,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     ks1 = static_cast<int>(static_cast<long long>(kst_total) * (part + 1) / args.split);
     slot = v;
   };
-  // chained epilogues: end of the hand-off that contains stage ks -- sub_stages further, cut at the
-  // sample's and at the unit's end.  (With fp32 inputs it is a few stages only: the tensor cores add into the
+  // Chained epilogues hand an accumulator over every sub_stages stages, counted from the sample's start, and at the
+  // sample's and the unit's end.  (With fp32 inputs it is a few stages only: the tensor cores add into the
   // TMEM accumulator by truncation, about one unit in the last place per K = 16 step and all of one sign, so a
   // long chain drifts; short chains summed in registers with round-to-nearest do not.)
-  auto segment_end = [&](int ks, int ks1) {
-    const int s0 = ks / args.seg_stages * args.seg_stages;
-    const int sub = ((ks - s0) / args.sub_stages + 1) * args.sub_stages;
-    const int e = s0 + (sub < args.seg_stages ? sub : args.seg_stages);
-    return e < ks1 ? e : ks1;
-  };
   // running number of the hand-off that contains stage ks
   auto segment_index = [&](int ks) {
     const int sg = ks / args.seg_stages;
@@ -689,7 +687,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         while (ks < ks1 && ok) {
           const int seg_begin = ks;
           int seg_end = ks1;
-          if (epi_chained(EPI)) {      // segment_end(ks, ks1) without its divisions
+          if (epi_chained(EPI)) {
             const int len = min(args.sub_stages - sub_off, sample_left);
             sub_off = 0;
             seg_end = min(ks + len, ks1);
@@ -784,16 +782,27 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const bool pre_noise = epi_scaled(EPI) && slot < 0 && args.nk.std != 0.f && m < args.M && !args.direct_out;
         const uint64_t g0 = (static_cast<uint64_t>(m) * args.ld_out + n0 + chalf * 128) >> 2;
         const int nseg = segment_index(ks1 - 1) - segment_index(ks0) + 1;
-        int ng = 0, seg = 0;
+        // (no divisions from here on: what a hand-off takes between the commit and the arrival is time the tensor cores
+        // wait when its MMAs are few)
+        int ng = 0, noise_due = 0;
+        int sample = ks0 / args.seg_stages, sample_left = (sample + 1) * args.seg_stages - ks0;
+        int sub_off = (args.seg_stages - sample_left) % args.sub_stages;
         for (int ks = ks0, sub = 0; ks < ks1 && ok; ++it) {
           const int acc = it % NUM_ACC;
           const uint32_t acc_phase = (it / NUM_ACC) & 1u;
-          if (!mbar_wait_warp(tfull_bar(acc), acc_phase, wctx, 4)) { ok = false; break; }
-          tc_fence_after();
-          const int sample = ks / args.seg_stages;
           // the divisor goes into the factor, so the noise is added as it is drawn
           const float cbs = !epi_scaled(EPI) || args.segs == 0 ? args.scale
                           : (args.norm_partials != nullptr ? sfac[sample] : __ldg(args.factors + sample)) * args.scale;
+          if (++sub == SUBS) {     // on to the next hand-off's first stage, as the MMA warp goes
+            sub = 0;
+            const int len = min(args.sub_stages - sub_off, sample_left);
+            sub_off = 0;
+            ks += len;
+            sample_left -= len;
+            if (sample_left == 0) { sample_left = args.seg_stages; ++sample; }
+          }
+          if (!mbar_wait_warp(tfull_bar(acc), acc_phase, wctx, 4)) { ok = false; break; }
+          tc_fence_after();
           const uint32_t tb = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN + chalf * warp_cols;
 #pragma unroll
           for (int c4 = 0; c4 < 4; ++c4) {
@@ -801,20 +810,19 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             uint32_t r[32];
             tc_ld32(tb + c4 * 32, r);
             tc_wait_ld();
+            if (c4 == 3 || (narrow && c4 == 1)) {     // the accumulator has been read: back to the MMA warp
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) {
+                if (CTAS == 1 || is_leader) mbar_arrive(tempty_bar(acc));
+                else mbar_arrive_cluster(mapa_u32(tempty_bar(acc), 0));
+              }
+            }
 #pragma unroll
             for (int j = 0; j < 32; ++j) accr[c4 * 32 + j] = fmaf(cbs, __uint_as_float(r[j]), accr[c4 * 32 + j]);
           }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            if (CTAS == 1 || is_leader) mbar_arrive(tempty_bar(acc));
-            else mbar_arrive_cluster(mapa_u32(tempty_bar(acc), 0));
-          }
-          if (++sub == SUBS) { sub = 0; ks = segment_end(ks, ks1); }
-          ++seg;
           if (epi_scaled(EPI) && pre_noise) {
-            const int target = (32 * seg) / nseg;
-            for (; ng < target; ++ng) {
+            for (noise_due += 32; noise_due >= nseg; noise_due -= nseg, ++ng) {
               float z[4];
               noise_group(args.nk, g0 + ng, z);
               add_group(accr, ng, z, 1.0f);
