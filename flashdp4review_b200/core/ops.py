@@ -210,14 +210,29 @@ def native_product_ok(dtype, rows, K, N):
     return mode == "native" or (K % 8 == 0 and N % 8 == 0 and N >= 128 and K >= 64 and rows >= 128)
 
 
+def wide_product_ok(dtype, rows, K, N):
+    """Whether a product outside native_product_ok runs on this library's tensor-core kernels all the same, through
+    copies of the operands with padded rows: fp32 in mode "tensor" as six bf16 products over three parts, as close to
+    float64 as cuBLAS's fp32 kernels.  Never under input_grad_impl() == "library"."""
+    if runtime.input_grad_impl() == "library" or dtype != torch.float32:
+        return False
+    # (measured: 2^26 multiply-adds are where the split of the operands has paid off against cuBLAS)
+    return runtime.fp32_mode() == "tensor" and rows >= 128 and K >= 64 and N >= 64 and rows * K * N >= 1 << 26
+
+
+def library_product_ok(dtype, rows, K, N):
+    """Whether a DP layer leaves the product [rows, K] x [K, N] to this library rather than to torch."""
+    return native_product_ok(dtype, rows, K, N) or wide_product_ok(dtype, rows, K, N)
+
+
 def _gemm_dtype_code(dtype, fp32_tensor):
-    """dtype code of the forward / input-gradient entry points, with the fp32 tensor-core flag"""
-    code = _dt(dtype)
+    """dtype code of the forward / input-gradient entry points, with the fp32 tensor-core flags"""
+    code = _dt(dtype) | _lib.FDP_GEMM_SPLIT_K
     if dtype == torch.float32:
         if fp32_tensor is None:
             fp32_tensor = runtime.fp32_mode() == "tensor"
         if fp32_tensor:
-            code |= _lib.FDP_FP32_TENSOR
+            code |= _lib.FDP_FP32_TENSOR | _lib.FDP_FP32_WIDE_GEMM
     return code
 
 
@@ -225,7 +240,8 @@ def linear_input_grad(grad_output, weight, w_layout="out_in", out_dtype=None, fp
     """grad_output @ weight (nn.Linear, weight [out,in]) or grad_output @ weight.t() (Conv1D,
     weight [in,out]) -- flashdp/layers/linear.py:62-67, transformers_conv1d.py:70-75.
     `out_dtype` (default: grad_output's) lets the kernel write the dtype autograd wants directly.
-    `fp32_tensor` as in dp_linear_weight_grad: fp32 operands as three bf16 tensor-core products."""
+    `fp32_tensor` as in dp_linear_weight_grad: fp32 operands as three bf16 tensor-core products, or six (see
+    wide_product_ok)."""
     host = _lib.host()
     _require_cuda(grad_output, weight)
     G = _aligned(grad_output.contiguous())
@@ -256,9 +272,9 @@ def dp_linear_backward(input, grad_output, weight, C, clamp_value, *, need_dx=Tr
     X = _aligned(input.to(dt).contiguous()) if need_dw else None
     W = _aligned(weight.to(dt).contiguous()) if need_dx else None
     code = _dt(dt)
-    algo = NORM_ALGOS[norm_algo] | _lib.FDP_KEEP_PRODUCTS
+    algo = NORM_ALGOS[norm_algo] | _lib.FDP_KEEP_PRODUCTS | _lib.FDP_GEMM_SPLIT_K
     if dt == torch.float32 and runtime.fp32_mode() == "tensor":
-        algo |= _lib.FDP_FP32_TENSOR | _lib.FDP_FP32_WIDE
+        algo |= _lib.FDP_FP32_TENSOR | _lib.FDP_FP32_WIDE | _lib.FDP_FP32_WIDE_GEMM
     if out is not None:
         shape = (G.shape[-1], n_in) if layout == "out_in" else (n_in, G.shape[-1])
         if tuple(out.shape) != shape or not out.is_contiguous() or out.device != G.device:

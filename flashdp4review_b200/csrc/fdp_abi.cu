@@ -320,7 +320,7 @@ int fdp_linear_wgrad(const void* G, const void* X, void* dW, float* norms_out, f
   if (G == nullptr || X == nullptr || dW == nullptr) return FDP_ERR_ARG;
   if (B <= 0 || T <= 0 || n_in <= 0 || n_out <= 0) return FDP_ERR_ARG;
   if (layout != FDP_OUT_IN && layout != FDP_IN_OUT) return FDP_ERR_ARG;
-  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE | FDP_KEEP_PRODUCTS)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
+  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE | FDP_KEEP_PRODUCTS | FDP_FP32_WIDE_GEMM | FDP_GEMM_SPLIT_K)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
     return FDP_ERR_ARG;
   if (!valid_dtype(in_dtype) || !valid_dtype(out_dtype)) return FDP_ERR_DTYPE;
   if (static_cast<long long>(B) * T >= (1ll << 31) / 2) return FDP_ERR_SHAPE;   // row indices are 32-bit
@@ -386,30 +386,52 @@ int fdp_bias_grad(const void* G, void* db, float* norms_out, float* factors_out,
 }
 
 // ---- input gradient ---------------------------------------------------------------------------------
-// fp32 with FDP_FP32_TENSOR in `dtype`: whether the product [rows, K] x [K, N] takes the three-product path
-static bool gemm3_wanted(int dtype, int rows, int K, int N) {
-  return dtype == (FDP_F32 | FDP_FP32_TENSOR) && tc_gemm3_ok(rows, K, N);
+constexpr int GEMM_FLAGS = FDP_FP32_TENSOR | FDP_FP32_WIDE_GEMM | FDP_GEMM_SPLIT_K;
+// `dtype` of a forward or input-gradient product without its flags (fp32's with 16-bit types are left in: no such dtype)
+static int gemm_dtype(int dtype) { return dtype & ~((dtype & ~GEMM_FLAGS) == FDP_F32 ? GEMM_FLAGS : FDP_GEMM_SPLIT_K); }
+// fp32 with FDP_FP32_TENSOR / FDP_FP32_WIDE_GEMM in `dtype`: how many parts the operands of [rows, K] x [K, N] are split
+// into -- two (three products), three (six) or none
+static int gemm_parts(int dtype, int rows, int K, int N) {
+  if (gemm_dtype(dtype) != FDP_F32) return 0;
+  if ((dtype & FDP_FP32_TENSOR) != 0 && tc_gemm3_ok(rows, K, N)) return 2;
+  return (dtype & FDP_FP32_WIDE_GEMM) != 0 && tc_gemm6_ok(rows, K, N) ? 3 : 0;
+}
+static size_t gemm_ws_bytes(int parts, int rows, int K, int N) {
+  return parts == 2 ? tc_gemm3_ws_bytes(rows, K, N) : parts == 3 ? tc_gemm6_ws_bytes(rows, K, N) : 0;
+}
+// the workspace of a product: the status word, the split copies of the two operands when fp32 runs on the tensor cores,
+// and with FDP_GEMM_SPLIT_K the place for a K split's parts
+static size_t gemm_park_bytes(int dtype, int parts, int rows, int K, int N) {
+  if ((dtype & FDP_GEMM_SPLIT_K) == 0 || (parts == 0 && !tc_dgrad_ok(rows, N, K, gemm_dtype(dtype)))) return 0;
+  return tc_gemm_park_bytes(rows, K, N, parts == 3 ? 6 : parts == 2 ? 3 : 1);
+}
+static GemmPark gemm_park(void* workspace, size_t workspace_bytes, int parts, int rows, int K, int N) {
+  const size_t off = 256 + gemm_ws_bytes(parts, rows, K, N);
+  if (workspace_bytes <= off) return GemmPark{nullptr, 0};
+  return GemmPark{reinterpret_cast<float*>(static_cast<char*>(workspace) + off), workspace_bytes - off};
 }
 
 size_t fdp_linear_dgrad_workspace_bytes(int rows, int n_in, int n_out, int dtype) {
-  // the status word, then the split copies of the two operands when fp32 runs on the tensor cores
   // (K = n_out, N = n_in; the forward product queries with the two exchanged)
-  return 256 + (gemm3_wanted(dtype, rows, n_out, n_in) ? tc_gemm3_ws_bytes(rows, n_out, n_in) : 0);
+  const int parts = gemm_parts(dtype, rows, n_out, n_in);
+  return 256 + gemm_ws_bytes(parts, rows, n_out, n_in) + gemm_park_bytes(dtype, parts, rows, n_out, n_in);
 }
 
-// Y[rows, N] = A[rows, K] * W (+ bias), fp32 in and out, as three bf16 products: split, then one GEMM
-static int gemm3_call(const void* A, const void* W, const void* bias, void* Y, int rows, int K, int N, int out_dtype,
-                      bool w_kn, void* workspace, size_t workspace_bytes, cudaStream_t s) {
-  if (workspace_bytes < 256 + tc_gemm3_ws_bytes(rows, K, N)) return FDP_ERR_WORKSPACE;
+// Y[rows, N] = A[rows, K] * W (+ bias), fp32 in and out, as three or six bf16 products: split, then one GEMM
+static int gemm_split_call(int parts, const void* A, const void* W, const void* bias, void* Y, int rows, int K, int N, int out_dtype,
+                           bool w_kn, void* workspace, size_t workspace_bytes, cudaStream_t s, const GemmPark& park) {
+  if (workspace_bytes < 256 + gemm_ws_bytes(parts, rows, K, N)) return FDP_ERR_WORKSPACE;
   int* status = static_cast<int*>(workspace);
   char* a3 = static_cast<char*>(workspace) + 256;
-  char* w3 = a3 + ((static_cast<size_t>(rows) * K * 4 + 255) & ~static_cast<size_t>(255));
+  // (the copy of W lies at the end, whatever its orientation needs)
+  char* w3 = a3 + gemm_ws_bytes(parts, rows, K, N) - (parts == 2 ? tc_gemm3_w_bytes(K, N, 2) : tc_gemm6_w_bytes(K, N));
   // W is [K, N] (w_kn) or [N, K]: either way its rows are split along their own columns
   const SplitJob jobs[2] = {{A, a3, static_cast<size_t>(rows), K, nullptr, 1},
                             {W, w3, static_cast<size_t>(w_kn ? K : N), w_kn ? N : K, nullptr, 1}};
-  const int st = tc_split(jobs, 2, 2, status, s);
+  const int st = tc_split(jobs, 2, parts, status, s);
   if (st != FDP_OK) return st;
-  return tc_gemm3(a3, w3, bias, Y, status, rows, K, N, out_dtype, w_kn, s);
+  return parts == 2 ? tc_gemm3(a3, w3, bias, Y, status, rows, K, N, out_dtype, w_kn, s, park)
+                    : tc_gemm6(a3, w3, bias, Y, status, rows, K, N, out_dtype, w_kn, s, park);
 }
 
 int fdp_linear_dgrad(const void* G, const void* W, void* dX, int rows, int n_in, int n_out,
@@ -419,20 +441,22 @@ int fdp_linear_dgrad(const void* G, const void* W, void* dX, int rows, int n_in,
   if (G == nullptr || W == nullptr || dX == nullptr) return FDP_ERR_ARG;
   if (rows <= 0 || n_in <= 0 || n_out <= 0) return FDP_ERR_ARG;
   if (w_layout != FDP_OUT_IN && w_layout != FDP_IN_OUT) return FDP_ERR_ARG;
-  const bool want3 = gemm3_wanted(dtype, rows, n_out, n_in);
-  if ((dtype & FDP_FP32_TENSOR) != 0 && (dtype & ~FDP_FP32_TENSOR) == FDP_F32) dtype = FDP_F32;
+  const int parts = gemm_parts(dtype, rows, n_out, n_in);
+  const bool split_k = (dtype & FDP_GEMM_SPLIT_K) != 0;
+  dtype = gemm_dtype(dtype);
   if (!valid_dtype(dtype) || !valid_dtype(out_dtype)) return FDP_ERR_DTYPE;
   int st = current_device_ok();
   if (st != FDP_OK) return st;
   if (workspace == nullptr || workspace_bytes < 256 || !aligned16(workspace)) return FDP_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int* status = static_cast<int*>(workspace);
-  if (want3 && aligned16(G) && aligned16(W) && aligned16(dX)) {
+  const GemmPark park = split_k ? gemm_park(workspace, workspace_bytes, parts, rows, n_out, n_in) : GemmPark{nullptr, 0};
+  if (parts == 3 || (parts == 2 && aligned16(G) && aligned16(W) && aligned16(dX))) {
     // dX = G [rows, n_out] * W: W is [n_out, n_in] = [K, N] for nn.Linear, [n_in, n_out] = [N, K] for Conv1D
-    if ((st = gemm3_call(G, W, nullptr, dX, rows, n_out, n_in, out_dtype, w_layout == FDP_OUT_IN, workspace,
-                         workspace_bytes, s)) != FDP_OK) return st;
+    if ((st = gemm_split_call(parts, G, W, nullptr, dX, rows, n_out, n_in, out_dtype, w_layout == FDP_OUT_IN, workspace,
+                              workspace_bytes, s, park)) != FDP_OK) return st;
   } else if (tc_dgrad_ok(rows, n_in, n_out, dtype) && aligned16(G) && aligned16(W) && aligned16(dX)) {
-    if ((st = tc_dgrad(G, W, dX, status, rows, n_in, n_out, dtype, out_dtype, w_layout, s)) != FDP_OK) return st;
+    if ((st = tc_dgrad(G, W, dX, status, rows, n_in, n_out, dtype, out_dtype, w_layout, s, park)) != FDP_OK) return st;
   } else {
     FDP_CUDA_OK(cudaMemsetAsync(status, 0, sizeof(int), s));
     simt_dgrad(G, W, dX, rows, n_in, n_out, dtype, out_dtype, w_layout, s);
@@ -449,22 +473,24 @@ int fdp_linear_fwd(const void* X, const void* W, const void* bias, void* Y, int 
   if (X == nullptr || W == nullptr || Y == nullptr) return FDP_ERR_ARG;
   if (rows <= 0 || n_in <= 0 || n_out <= 0) return FDP_ERR_ARG;
   if (w_layout != FDP_OUT_IN && w_layout != FDP_IN_OUT) return FDP_ERR_ARG;
-  const bool want3 = gemm3_wanted(dtype, rows, n_in, n_out);
-  if ((dtype & FDP_FP32_TENSOR) != 0 && (dtype & ~FDP_FP32_TENSOR) == FDP_F32) dtype = FDP_F32;
+  const int parts = gemm_parts(dtype, rows, n_in, n_out);
+  const bool split_k = (dtype & FDP_GEMM_SPLIT_K) != 0;
+  dtype = gemm_dtype(dtype);
   if (!valid_dtype(dtype) || !valid_dtype(out_dtype)) return FDP_ERR_DTYPE;
   int st = current_device_ok();
   if (st != FDP_OK) return st;
   if (workspace == nullptr || workspace_bytes < 256 || !aligned16(workspace)) return FDP_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int* status = static_cast<int*>(workspace);
-  if (want3 && aligned16(X) && aligned16(W) && aligned16(Y) && (bias == nullptr || aligned16(bias))) {
+  const GemmPark park = split_k ? gemm_park(workspace, workspace_bytes, parts, rows, n_in, n_out) : GemmPark{nullptr, 0};
+  if (parts == 3 || (parts == 2 && aligned16(X) && aligned16(W) && aligned16(Y) && (bias == nullptr || aligned16(bias)))) {
     // Y = X [rows, n_in] * W^T: W is [n_out, n_in] = [N, K] for nn.Linear, [n_in, n_out] = [K, N] for Conv1D
-    if ((st = gemm3_call(X, W, bias, Y, rows, n_in, n_out, out_dtype, w_layout == FDP_IN_OUT, workspace,
-                         workspace_bytes, s)) != FDP_OK) return st;
+    if ((st = gemm_split_call(parts, X, W, bias, Y, rows, n_in, n_out, out_dtype, w_layout == FDP_IN_OUT, workspace,
+                              workspace_bytes, s, park)) != FDP_OK) return st;
   } else
   // same shape rules as the input gradient with the roles of n_in and n_out exchanged
   if (tc_dgrad_ok(rows, n_out, n_in, dtype) && aligned16(X) && aligned16(W) && aligned16(Y)) {
-    if ((st = tc_fwd(X, W, bias, Y, status, rows, n_in, n_out, dtype, out_dtype, w_layout, s)) != FDP_OK) return st;
+    if ((st = tc_fwd(X, W, bias, Y, status, rows, n_in, n_out, dtype, out_dtype, w_layout, s, park)) != FDP_OK) return st;
   } else {
     FDP_CUDA_OK(cudaMemsetAsync(status, 0, sizeof(int), s));
     simt_fwd(X, W, bias, Y, rows, n_in, n_out, dtype, out_dtype, w_layout, s);
@@ -475,11 +501,14 @@ int fdp_linear_fwd(const void* X, const void* W, const void* bias, void* Y, int 
 
 // ---- the whole backward of a Linear / Conv1D layer ----------------------------------------------------------
 namespace {
+// the input gradient's dtype with the flags that came in norm_algo
+int gemm_code(int dtype, int norm_algo) { return dtype | (norm_algo & (dtype == FDP_F32 ? GEMM_FLAGS : FDP_GEMM_SPLIT_K)); }
 // Whether one set of split copies can serve both products: fp32 on the tensor cores with the parts made before the
 // norms, and an input gradient that takes them too.
 struct LinearBwdWs {
   WgradWs w;
   bool shared;
+  int dx_parts;       // parts that the input gradient's product takes
   char* w_parts;      // split copy of W
   GstatsPlan pl;
   float* factors; float* sq_part; float* colsum_part;
@@ -491,14 +520,15 @@ LinearBwdWs linear_bwd_ws(void* base, int B, int T, int n_in, int n_out, int dty
   const bool dx = (outputs & FDP_BWD_DX) != 0, dw = (outputs & FDP_BWD_DW) != 0, db = (outputs & FDP_BWD_DB) != 0;
   if (dw) {
     q.w = wgrad_ws(base, B, T, n_in, n_out, dtype, norm_algo);
-    // (the input gradient takes part as three products, which is FDP_FP32_TENSOR's to allow)
-    q.shared = (dx || db) && q.w.tc.ok && q.w.tc.planes > 1 && !q.w.short_seq &&
-               (!dx || ((norm_algo & FDP_FP32_TENSOR) != 0 && tc_gemm3_ok(rows, n_out, n_in)));
+    // (the input gradient takes part as three products, which is FDP_FP32_TENSOR's to allow, or as six, which is
+    // FDP_FP32_WIDE_GEMM's)
+    q.dx_parts = dx ? gemm_parts(gemm_code(dtype, norm_algo), rows, n_out, n_in) : 0;
+    q.shared = (dx || db) && q.w.tc.ok && q.w.tc.planes > 1 && !q.w.short_seq && (!dx || (q.dx_parts > 0 && q.dx_parts <= q.w.tc.planes));
   }
   if (!q.shared) {
     // one output after another in the same memory: what the hungriest of those that are wanted takes
     size_t most = q.w.bytes;
-    const size_t d = dx ? fdp_linear_dgrad_workspace_bytes(rows, n_in, n_out, dtype == FDP_F32 ? dtype | (norm_algo & FDP_FP32_TENSOR) : dtype) : 0;
+    const size_t d = dx ? fdp_linear_dgrad_workspace_bytes(rows, n_in, n_out, gemm_code(dtype, norm_algo)) : 0;
     const size_t g = db ? fdp_bias_grad_workspace_bytes(B, T, n_out, dtype) : 0;
     if (d > most) most = d;
     if (g > most) most = g;
@@ -507,7 +537,7 @@ LinearBwdWs linear_bwd_ws(void* base, int B, int T, int n_in, int n_out, int dty
   }
   Carver c(base);
   c.off = q.w.bytes;
-  q.w_parts = c.take<char>(dx ? tc_gemm3_w_bytes(n_out, n_in, q.w.tc.planes) : 0);
+  q.w_parts = c.take<char>(!dx ? 0 : q.dx_parts == 3 ? tc_gemm6_w_bytes(n_out, n_in) : tc_gemm3_w_bytes(n_out, n_in, q.w.tc.planes));
   q.pl = gstats_plan(B, T, n_out, dtype);
   q.factors = c.take<float>(B);
   q.sq_part = c.take<float>(static_cast<size_t>(B) * q.pl.row_chunks * q.pl.col_chunks);
@@ -529,7 +559,7 @@ int fdp_linear_bwd(const void* G, const void* X, const void* W, void* dX, void* 
   if (B <= 0 || T <= 0 || n_in <= 0 || n_out <= 0) return FDP_ERR_ARG;
   if (static_cast<long long>(B) * T >= (1ll << 31) / 2) return FDP_ERR_SHAPE;   // row indices are 32-bit
   if (!valid_dtype(in_dtype)) return FDP_ERR_DTYPE;
-  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE | FDP_KEEP_PRODUCTS)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
+  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE | FDP_KEEP_PRODUCTS | FDP_FP32_WIDE_GEMM | FDP_GEMM_SPLIT_K)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
     return FDP_ERR_ARG;
   const int outputs = (dX ? FDP_BWD_DX : 0) | (dW ? FDP_BWD_DW : 0) | (db ? FDP_BWD_DB : 0);
   if (outputs == 0) return FDP_ERR_ARG;
@@ -565,9 +595,13 @@ int fdp_linear_bwd(const void* G, const void* X, const void* W, void* dX, void* 
     if ((st = tc_split(jobs, dX != nullptr ? 2 : 1, planes, q.w.status, s)) != FDP_OK) return st;
     if ((st = wgrad_run(G, X, dW, nullptr, nullptr, B, T, n_in, n_out, in_dtype, dw_dtype, layout, norm_algo, p, q.w, true, s)) != FDP_OK)
       return st;
-    if (dX != nullptr &&
-        (st = tc_gemm3(sg, q.w_parts, nullptr, dX, q.w.status, rows, n_out, n_in, dx_dtype, w_kn, s, planes)) != FDP_OK)
-      return st;
+    if (dX != nullptr) {
+      // (the weight gradient is through with its parking area, or kept products, at the workspace's start)
+      const GemmPark park = (norm_algo & FDP_GEMM_SPLIT_K) != 0 ? GemmPark{static_cast<float*>(q.w.tc_extra), q.w.tc.split_bytes} : GemmPark{nullptr, 0};
+      st = q.dx_parts == 3 ? tc_gemm6(sg, q.w_parts, nullptr, dX, q.w.status, rows, n_out, n_in, dx_dtype, w_kn, s, park)
+                           : tc_gemm3(sg, q.w_parts, nullptr, dX, q.w.status, rows, n_out, n_in, dx_dtype, w_kn, s, park, planes);
+      if (st != FDP_OK) return st;
+    }
     if (db != nullptr) {
       const int div = p_bias->batch_divisor > 0 ? p_bias->batch_divisor : B;
       bias_clip_finalize(q.colsum_part, q.sq_part, q.pl.row_chunks * q.pl.col_chunks, p_bias->C, p_bias->clamp_value, q.factors,
@@ -579,7 +613,7 @@ int fdp_linear_bwd(const void* G, const void* X, const void* W, void* dX, void* 
   }
   int st = FDP_OK;
   if (dX != nullptr)
-    st = fdp_linear_dgrad(G, W, dX, rows, n_in, n_out, in_dtype == FDP_F32 ? in_dtype | (norm_algo & FDP_FP32_TENSOR) : in_dtype,
+    st = fdp_linear_dgrad(G, W, dX, rows, n_in, n_out, gemm_code(in_dtype, norm_algo),
                           dx_dtype, layout, workspace, workspace_bytes, stream);
   if (st == FDP_OK && dW != nullptr)
     st = fdp_linear_wgrad(G, X, dW, nullptr, nullptr, B, T, n_in, n_out, in_dtype, dw_dtype, layout, norm_algo, p, workspace,

@@ -54,20 +54,22 @@ Tensor new_tensor(const Tensor& like, at::IntArrayRef sizes, at::ScalarType t) {
 Tensor workspace(const Tensor& like, size_t bytes) {
   return new_tensor(like, {static_cast<int64_t>(bytes < 256 ? 256 : bytes)}, at::kByte);
 }
-// The workspace of a weight gradient with `algo`.  Where it does not fit the card, what asks for most is given up first:
-// the per-sample products (FDP_KEEP_PRODUCTS, up to 512 MiB), then the split copies of fp32 operands (1.5 times the inputs
-// with FDP_FP32_WIDE) and the 38.8 MB parking area -- those shapes then stay on the FMA kernels, which need next to nothing.
+// The workspace that `query` asks for under the flags of `code`.  Where it does not fit the card, what asks for most is given
+// up first: the per-sample products (up to 512 MiB) and the parts of a K split (38.8 MB); then the split copies of fp32
+// operands in six products (1.5 times the operands, and 38.8 MB for a weight gradient), whose shapes then stay on the FMA
+// kernels, which need next to nothing.
 template <typename Query>
-Tensor algo_workspace(const Tensor& like, int& algo, Query query) {
-  for (const int flag : {FDP_KEEP_PRODUCTS, FDP_FP32_WIDE}) {
+Tensor workspace_or_less(const Tensor& like, int& code, Query query) {
+  constexpr int SPEED = FDP_KEEP_PRODUCTS | FDP_GEMM_SPLIT_K, COPIES = FDP_FP32_WIDE | FDP_FP32_WIDE_GEMM;
+  for (const int flags : {SPEED, COPIES}) {
     try {
-      return workspace(like, query(algo));
+      return workspace(like, query(code));
     } catch (const c10::OutOfMemoryError&) {
-      if ((algo & (FDP_KEEP_PRODUCTS | FDP_FP32_WIDE)) == 0) throw;
-      algo &= ~flag;
+      if ((code & (SPEED | COPIES)) == 0) throw;
+      code &= ~flags;
     }
   }
-  return workspace(like, query(algo));
+  return workspace(like, query(code));
 }
 // The kernels take bare pointers and their sizes from one operand each: what does not fit would be misread, or read past
 // its end.  Raised as RuntimeError before anything is allocated or launched.
@@ -110,7 +112,7 @@ py::tuple linear_wgrad(const Tensor& G, const Tensor& X, const OptTensor& out, i
               : layout == FDP_OUT_IN ? new_tensor(G, {n_out, n_in}, scalar_type(out_dt)) : new_tensor(G, {n_in, n_out}, scalar_type(out_dt));
   OptTensor norms, factors;
   if (want_norms) { norms = new_tensor(G, {B}, at::kFloat); factors = new_tensor(G, {B}, at::kFloat); }
-  const Tensor ws = algo_workspace(G, algo, [&](int a) { return abi.linear_wgrad_workspace_bytes(B, T, n_in, n_out, in_dt, a); });
+  const Tensor ws = workspace_or_less(G, algo, [&](int a) { return abi.linear_wgrad_workspace_bytes(B, T, n_in, n_out, in_dt, a); });
   int st;
   {
     py::gil_scoped_release nogil;
@@ -149,7 +151,7 @@ py::tuple linear_dgrad(const Tensor& G, const Tensor& W, int rows, int code, int
   const c10::cuda::CUDAGuard guard(G.device());
   const int n_out = static_cast<int>(G.size(-1)), n_in = static_cast<int>(W.size(w_layout == FDP_OUT_IN ? 1 : 0));
   const Tensor dX = with_columns(G, n_in, out_dt);
-  const Tensor ws = workspace(G, abi.linear_dgrad_workspace_bytes(rows, n_in, n_out, code));
+  const Tensor ws = workspace_or_less(G, code, [&](int c) { return abi.linear_dgrad_workspace_bytes(rows, n_in, n_out, c); });
   int st;
   {
     py::gil_scoped_release nogil;
@@ -193,8 +195,9 @@ py::tuple linear_bwd(const Tensor& G, const OptTensor& X, const OptTensor& W, co
     }
     return ws.has_value();
   };
-  if (!take() && bytes(outputs, algo & ~FDP_KEEP_PRODUCTS) < bytes(outputs, algo)) {
-    algo &= ~FDP_KEEP_PRODUCTS;
+  constexpr int SPEED = FDP_KEEP_PRODUCTS | FDP_GEMM_SPLIT_K;
+  if (!take() && bytes(outputs, algo & ~SPEED) < bytes(outputs, algo)) {
+    algo &= ~SPEED;
     take();
   }
   if (ws.has_value()) {
@@ -206,7 +209,7 @@ py::tuple linear_bwd(const Tensor& G, const OptTensor& X, const OptTensor& W, co
       if ((outputs & one) == 0 || st != FDP_OK) continue;
       allocate(one);
       int a = algo;
-      const Tensor own = algo_workspace(G, a, [&](int b) { return bytes(one, b); });
+      const Tensor own = workspace_or_less(G, a, [&](int b) { return bytes(one, b); });
       st = call(one, a, own);
     }
   }
@@ -220,7 +223,7 @@ py::tuple linear_fwd(const Tensor& X, const Tensor& W, const OptTensor& bias, in
   const c10::cuda::CUDAGuard guard(X.device());
   const int n_in = static_cast<int>(X.size(-1)), n_out = static_cast<int>(W.size(w_layout == FDP_OUT_IN ? 0 : 1));
   const Tensor Y = with_columns(X, n_out, out_dt);
-  const Tensor ws = workspace(X, abi.linear_dgrad_workspace_bytes(rows, n_out, n_in, code));
+  const Tensor ws = workspace_or_less(X, code, [&](int c) { return abi.linear_dgrad_workspace_bytes(rows, n_out, n_in, c); });
   int st;
   {
     py::gil_scoped_release nogil;

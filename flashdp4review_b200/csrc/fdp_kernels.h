@@ -174,6 +174,10 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
                      int layout, float inv_div, NoiseKey nk, cudaStream_t s, int planes = 1);
 // test aid: one warp waits `limit_cycles` on a barrier nobody arrives on and reports the timeout
 int tc_wait_selftest(int* status, long long limit_cycles, cudaStream_t s);
+// Where a product [rows, K] x [K, N] of `products` bf16 products may park the parts of a K split: what the plan needs, 0
+// for none.  Without it (or with less) the product runs unsplit.
+struct GemmPark { float* ws; size_t bytes; };
+size_t tc_gemm_park_bytes(int rows, int K, int N, int products);
 bool tc_dgrad_ok(int rows, int n_in, int n_out, int dt);
 // fp32 product Y[rows, N] = A[rows, K] * W (+ bias) as three bf16 tensor-core products over operands split
 // by tc_split (A3 [rows, 2K]; W3 [K, 2N] if w_kn, else [N, 2K]); workspace for the two split copies
@@ -181,10 +185,16 @@ bool tc_gemm3_ok(int rows, int K, int N);
 size_t tc_gemm3_ws_bytes(int rows, int K, int N);
 size_t tc_gemm3_w_bytes(int K, int N, int planes);     // the split copy of W alone
 int tc_gemm3(const void* A3, const void* W3, const void* bias, void* Y, int* dev_status, int rows, int K, int N,
-             int out_dt, bool w_kn, cudaStream_t s, int planes = 2);
+             int out_dt, bool w_kn, cudaStream_t s, const GemmPark& park, int planes = 2);
+// the same as six products over three parts, any K and N (A3 [rows, 3 pitch8(K)]; W3 [K, 3 pitch8(N)] or [N, 3 pitch8(K)])
+bool tc_gemm6_ok(int rows, int K, int N);
+size_t tc_gemm6_ws_bytes(int rows, int K, int N);
+size_t tc_gemm6_w_bytes(int K, int N);
+int tc_gemm6(const void* A3, const void* W3, const void* bias, void* Y, int* dev_status, int rows, int K, int N,
+             int out_dt, bool w_kn, cudaStream_t s, const GemmPark& park);
 int tc_fwd(const void* X, const void* W, const void* bias, void* Y, int* dev_status, int rows, int n_in,
-           int n_out, int dt, int out_dt, int w_layout, cudaStream_t s);
+           int n_out, int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park);
 int tc_dgrad(const void* G, const void* W, void* dX, int* dev_status, int rows, int n_in, int n_out,
-             int dt, int out_dt, int w_layout, cudaStream_t s);
+             int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park);
 
 }  // namespace fdp

@@ -54,15 +54,15 @@ constexpr int MAX_SMS = 148;           // workers the split-K parking area is si
 // EPI_KEEP: one sample's product tile squared and summed, and kept in HBM for weighted_sum_kernel (the SPLIT_SUMSQ
 // ones keep it too when TcArgs::keep is set).
 enum { EPI_STORE = 0, EPI_SUMSQ = 1, EPI_GRAM = 2, EPI_STORE_SCALED = 3, EPI_SPLIT_SCALED = 4, EPI_SPLIT_STORE = 5,
-       EPI_SPLIT_SUMSQ = 6, EPI_SPLIT6_SCALED = 7, EPI_SPLIT6_SUMSQ = 8, EPI_KEEP = 9 };
+       EPI_SPLIT_SUMSQ = 6, EPI_SPLIT6_SCALED = 7, EPI_SPLIT6_SUMSQ = 8, EPI_KEEP = 9, EPI_SPLIT6_STORE = 10 };
 __host__ __device__ constexpr bool epi_chained(int epi) { return epi >= EPI_STORE_SCALED && epi != EPI_KEEP; }
 // bf16 parts of an operand
 __host__ __device__ constexpr int epi_planes(int epi) {
-  return epi == EPI_SPLIT6_SCALED || epi == EPI_SPLIT6_SUMSQ ? 3 : epi_chained(epi) && epi != EPI_STORE_SCALED ? 2 : 1;
+  return epi == EPI_SPLIT6_SCALED || epi == EPI_SPLIT6_SUMSQ || epi == EPI_SPLIT6_STORE ? 3 : epi_chained(epi) && epi != EPI_STORE_SCALED ? 2 : 1;
 }
 __host__ __device__ constexpr bool epi_scaled(int epi) { return epi == EPI_STORE_SCALED || epi == EPI_SPLIT_SCALED || epi == EPI_SPLIT6_SCALED; }
 __host__ __device__ constexpr bool epi_sumsq(int epi) { return epi == EPI_SPLIT_SUMSQ || epi == EPI_SPLIT6_SUMSQ; }
-__host__ __device__ constexpr bool epi_stores(int epi) { return epi == EPI_STORE || epi_scaled(epi) || epi == EPI_SPLIT_STORE; }
+__host__ __device__ constexpr bool epi_stores(int epi) { return epi == EPI_STORE || epi_scaled(epi) || epi == EPI_SPLIT_STORE || epi == EPI_SPLIT6_STORE; }
 // eight epilogue warps (two per TMEM lane quarter, 128 columns each) for the store epilogues, four for the norms
 __host__ __device__ constexpr int epi_warps_for(int epi) { return (epi == EPI_STORE || epi == EPI_KEEP || epi_chained(epi)) ? 8 : 4; }
 constexpr int threads_for(int epi) { return 64 + 32 * epi_warps_for(epi); }
@@ -401,7 +401,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   constexpr int STG = A_BYTES + PLANES * B_BYTES;
   constexpr int BN_CTA = BN / CTAS;                      // B columns (rows if K-major) loaded by this CTA
   constexpr int EPI_WARPS = epi_warps_for(EPI);
-  constexpr bool CUTS = EPI == EPI_STORE || EPI == EPI_SPLIT_STORE;   // may have units of half a tile's columns
+  constexpr bool CUTS = EPI == EPI_STORE || EPI == EPI_SPLIT_STORE || EPI == EPI_SPLIT6_STORE;   // may have units of half a tile's columns
   static_assert(NST * STG <= STAGES * STAGE_BYTES, "ring size");
   static_assert(CTAS == 1 || EPI_WARPS == 8, "pairs: eight epilogue warps");
   const uint32_t cta_rank = (CTAS == 2) ? cluster_ctarank() : 0u;
@@ -579,6 +579,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               if (A_MN) {
 #pragma unroll
                 for (int i = 0; i < BM / 64; ++i) load3(da + i * (BK * 128), ma, m0 + 64 * i + ca, t, z);
+              } else if (EPI == EPI_SPLIT6_STORE) {     // (column, part, row): a K stage that ends past the last column reads zeros
+                load3(da, ma, k0, pl, m0);
               } else {
                 load(da, ma, k0 + ca, m0);
               }
@@ -587,8 +589,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 for (int j = 0; j < BN_CTA / 64; ++j) {
                   if (narrow && j >= BN_CTA / 128) break;
                   if (A_MN) load3(db + j * (BK * 128), mb, nb0 + 64 * j + cb, t, z);
+                  else if (EPI == EPI_SPLIT6_STORE) load3(db + j * (BK * 128), mb, nb0 + 64 * j, pl, k0);
                   else load(db + j * (BK * 128), mb, nb0 + 64 * j + cb, k0);
                 }
+              } else if (EPI == EPI_SPLIT6_STORE) {
+                load3(db, narrow ? &tmB2 : mb, k0, pl, nb0);
               } else {
                 load(db, narrow ? &tmB2 : mb, k0 + cb, nb0);    // tmB2: boxes of half the rows
               }
@@ -855,7 +860,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             for (int c4 = 0; c4 < 4; ++c4) {
               if (narrow && c4 >= 2) break;
               const int n = n0 + chalf * warp_cols + c4 * 32;
-              if (EPI == EPI_SPLIT_STORE && args.bias != nullptr && n < args.N) add_bias32(args, n, accr + c4 * 32);
+              if ((EPI == EPI_SPLIT_STORE || EPI == EPI_SPLIT6_STORE) && args.bias != nullptr && n < args.N) add_bias32(args, n, accr + c4 * 32);
               if (args.direct_out) store_rows32(args, box, accr + c4 * 32, n, m0 + quarter * 32, lane, epi_scaled(EPI) && args.nk.std != 0.f);
               else store_out32(args, box, &tmOut, accr + c4 * 32, c4, n0 + chalf * warp_cols, m0 + quarter * 32, lane);
             }
@@ -996,7 +1001,7 @@ __global__ void __launch_bounds__(256) splitk_fixup_kernel(const float* __restri
                                                            int tile_rows, int M, int N, int tiles_m, int tiles_n, int n_fastest,
                                                            int m_group,
                                                            void* __restrict__ out, int out_dt, long long ld_out,
-                                                           float scale, NoiseKey nk) {
+                                                           float scale, NoiseKey nk, const void* __restrict__ bias, int bias_dt) {
   pdl_wait();
   const int t = blockIdx.y;  // index among the split tiles
   const int q = first_tile + t;
@@ -1023,6 +1028,10 @@ __global__ void __launch_bounds__(256) splitk_fixup_kernel(const float* __restri
   }
   float v[4] = {acc.x * scale, acc.y * scale, acc.z * scale, acc.w * scale};
   const size_t idx0 = static_cast<size_t>(m) * ld_out + n;
+  if (bias != nullptr)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (n + j < N) v[j] += load_as(bias, bias_dt, n + j);
   if (nk.std != 0.f) {
     if ((idx0 & 3) == 0) {
       float z[4];
@@ -1294,6 +1303,19 @@ bool make_rows_map(CUtensorMap* m, const void* base, int B, uint64_t T, uint64_t
   return r == CUDA_SUCCESS;
 }
 int pitch8(int n) { return (n + 7) & ~7; }     // columns of one part in a split copy
+// three parts of [rows, cols] as (column, part, row), for products whose K range runs over the columns or over the rows
+// of any number: what lies past the last of either reads as zeros
+bool make_parts_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return false;
+  const uint64_t pitch = pitch8(static_cast<int>(cols));
+  const cuuint64_t dims[3] = {cols, 3, rows};
+  const cuuint64_t strides[2] = {pitch * 2, 3 * pitch * 2};
+  const cuuint32_t box[3] = {64, 1, box_rows};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 // Map of an output matrix [rows, cols] for the epilogue warps' boxes of 32 rows x 128 bytes.  The row pitch
 // has to be a multiple of 16 bytes and the base 16-byte aligned.
@@ -1415,17 +1437,18 @@ int ctas_per_tile() { return forced_ctas() == 1 ? 1 : 2; }
 // (256 KB), 4 for each further round.  Measured, GEMM + fix-up: 48 pair tiles of 256 stages for 74 pairs 110 us
 // unsplit, 117 in two parts, 91 in three; 16 tiles of 128 stages 54 / 37 / 30 / 26 us in one to four parts; 64 tiles
 // of 128 stages 62 us unsplit, 72 in two parts.
-int plan_tail_split(int total_tiles, int k_stages, int workers, int products) {
+int plan_tail_split(int total_tiles, int k_stages, int workers, int products, double whole = 1.0, double least_gain = 0.03,
+                    int most_rounds = 2) {
   const int rem = total_tiles <= workers ? total_tiles : total_tiles % workers;
   // stages are counted by their work: with split fp32 operands one holds three or six products
   const int min_stages = products == 6 ? 2 : products == 3 ? 3 : 8;      // shortest part
   if (rem == 0 || k_stages < 4 * min_stages) return 1;
   // FDP_TC_SPLIT=n forces the number of parts (measurements), within the same limits
   static const int forced = [] { const char* e = getenv("FDP_TC_SPLIT"); return e ? atoi(e) : 0; }();
-  if (forced >= 1) return (rem * forced > 2 * workers || k_stages / forced < min_stages) ? 1 : forced;
-  int best_s = 1; double best = 1.0;
+  if (forced >= 1) return (rem * forced > most_rounds * workers || k_stages / forced < min_stages) ? 1 : forced;
+  int best_s = 1; double best = whole - least_gain + 0.03;     // `whole`: tile-times of the round without a split
   for (int sp = 2; sp <= 16; ++sp) {
-    if (rem * sp > 2 * workers || k_stages / sp < min_stages) break;
+    if (rem * sp > most_rounds * workers || k_stages / sp < min_stages) break;
     const int rounds = (rem * sp + workers - 1) / workers;
     const double cost = static_cast<double>(rounds) / sp +
                         (6.0 + 0.11 * rem * sp + 4.0 * (rounds - 1)) / (static_cast<double>(k_stages) * products);
@@ -1433,15 +1456,49 @@ int plan_tail_split(int total_tiles, int k_stages, int workers, int products) {
   }
   return best_s;
 }
-// The forward and input-gradient products have no parking area: tiles that fill less than half of the last round (all of
-// them where there are fewer than half the workers) are cut in two along N, so that the round takes
-// less: 6000 rows 4096 -> 1024 fp16, 96 tiles for 74 pairs, 46.2 -> 41.6 us; 192 rows 1216 -> 384 bf16, 2 tiles, 13.0 -> 8.8;
-// 512 rows 768 -> 768 fp32, 6 tiles, 19.6 -> 14.9.
-void plan_cut(TcArgs& a, int ctas, uint32_t idesc_half) {
-  const int workers = launch_sms() / ctas, total = a.tiles_per_batch;
+// The last round of the forward and input-gradient products.  Tiles that fill less than half of it (all of them where
+// there are fewer than half the workers) are cut in two along N, so that the round takes less: 6000 rows 4096 -> 1024 fp16,
+// 96 tiles for 74 pairs, 46.2 -> 41.6 us; 192 rows 1216 -> 384 bf16, 2 tiles, 13.0 -> 8.8; 512 rows 768 -> 768 fp32,
+// 6 tiles, 19.6 -> 14.9.  Or, with a place to park the parts, the tiles are cut along K where that takes less still:
+// a narrow stage takes 0.7 of a whole one (its copies are 0.75), another launch is worth ten stages, and
+// parts of more than one round gain nothing (3152 rows 3072 -> 768 fp32, 39 tiles in three parts: 61.2 / 60.3 us).  972 rows 3480 -> 688
+// bf16, 12 tiles of 55 stages, 22.3 -> 15.5 us; 300 rows 8192 -> 264 30.2 -> 21.2; fp32 in six products 2816 rows 3888 -> 64
+// 86 -> 48, 128 rows 8190 -> 70 119 -> 34.
+int plan_gemm_split(int total, int k_stages, int workers, int products) {
   const int rem = total <= workers ? total : total % workers;
-  if (ctas != 2 || rem == 0 || 2 * rem > workers) return;
+  return plan_tail_split(total, k_stages, workers, products, 2 * rem <= workers ? 0.7 : 1.0, 10.0 / (static_cast<double>(k_stages) * products), 1);
+}
+// parking space of a product; a constant SM count, like every plan that a workspace query shares with the launch
+size_t gemm_park_bytes(int rows, int K, int N, int products) {
+  const int ctas = ctas_per_tile(), workers = MAX_SMS / ctas;
+  const int total = ceil_div(rows, BM * ctas) * ceil_div(N, BN), rem = total <= workers ? total : total % workers;
+  const int split = plan_gemm_split(total, ceil_div(K, BK), workers, products);
+  return split <= 1 ? 0 : static_cast<size_t>(rem) * split * ctas * BM * BN * sizeof(float);
+}
+// `mp`: map of the parking space, where it is used
+bool plan_last_round(TcArgs& a, int ctas, uint32_t idesc_half, int K, int products, const GemmPark& park, CUtensorMap* mp) {
+  const int total = a.tiles_per_batch;
+  const size_t bytes = gemm_park_bytes(a.M, K, a.N, products);
+  if (bytes > 0 && park.ws != nullptr && park.bytes >= bytes) {
+    const int workers = MAX_SMS / ctas, rem = total <= workers ? total : total % workers;
+    a.split = plan_gemm_split(total, a.k_stages, workers, products);
+    a.units_full = total - rem;
+    a.split_ws = park.ws;
+    return make_out_map(mp, park.ws, bytes / (BN * sizeof(float)), BN, FDP_F32);
+  }
+  const int workers = launch_sms() / ctas, rem = total <= workers ? total : total % workers;
+  if (ctas != 2 || rem == 0 || 2 * rem > workers) return true;
   a.cut = 2; a.units_full = total - rem; a.idesc_half = idesc_half;
+  return true;
+}
+// the parts of a K split into their tiles
+int gemm_fixup(int st, const TcArgs& a, int ctas, cudaStream_t s) {
+  if (st != FDP_OK || a.split <= 1) return st;
+  launch_dependent(splitk_fixup_kernel, dim3(BM * ctas * BN / (256 * 4), a.tiles_per_batch - a.units_full), dim3(256), 0, s, a.split_ws,
+                   a.units_full, a.split, BM * ctas, a.M, a.N, a.tiles_m, a.tiles_n, a.n_fastest, a.m_group, a.out, a.out_dt, a.ld_out,
+                   1.0f, a.nk, a.bias, a.bias_dt);
+  note_launch();
+  return cudaPeekAtLastError() == cudaSuccess ? FDP_OK : (cudaGetLastError(), FDP_ERR_LAUNCH);
 }
 // parked accumulators: up to 2 * MAX_SMS parts of 128 x 256 fp32 (a CTA pair parks two per part)
 size_t split_ws_bytes() { return static_cast<size_t>(2) * MAX_SMS * BM * BN * sizeof(float); }
@@ -1861,7 +1918,7 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
   dim3 grid(BM * ctas * BN / (256 * 4), n_split_tiles);
   launch_dependent(splitk_fixup_kernel, grid, dim3(256), 0, s, args.split_ws, args.units_full, split, BM * ctas, args.M,
                    args.N, args.tiles_m, args.tiles_n, args.n_fastest, args.m_group, dW, out_dt, args.ld_out,
-                   scaled || planes > 1 ? 1.0f : inv_div, nk);
+                   scaled || planes > 1 ? 1.0f : inv_div, nk, nullptr, 0);
   note_launch();
   return FDP_OK;
 }
@@ -1870,8 +1927,10 @@ bool tc_dgrad_ok(int rows, int n_in, int n_out, int dt) {
   return (dt == FDP_BF16 || dt == FDP_F16) && n_in % 8 == 0 && n_out % 8 == 0 && n_in >= 128 && n_out >= 64 && rows >= 128;
 }
 
+size_t tc_gemm_park_bytes(int rows, int K, int N, int products) { return gemm_park_bytes(rows, K, N, products); }
+
 int tc_dgrad(const void* G, const void* W, void* dX, int* dev_status, int rows, int n_in, int n_out,
-             int dt, int out_dt, int w_layout, cudaStream_t s) {
+             int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park) {
   CUtensorMap mg, mw, mo;
   const int ctas = ctas_per_tile();
   if (!make_map(&mg, G, rows, n_out, BK, BM, dt) || !make_out_map(&mo, dX, rows, n_in, out_dt)) return FDP_ERR_LAUNCH;
@@ -1888,23 +1947,25 @@ int tc_dgrad(const void* G, const void* W, void* dX, int* dev_status, int rows, 
   if (w_layout == FDP_OUT_IN) {  // W [n_out, n_in]: rows are K, N contiguous
     if (!make_map(&mw, W, n_out, n_in, 64, BK, dt)) return FDP_ERR_LAUNCH;
     args.idesc = make_idesc(dt, false, true, ctas);
-    plan_cut(args, ctas, make_idesc(dt, false, true, ctas, BN / 2));
-    return ctas == 2 ? launch<false, true, EPI_STORE, 2>(mg, mw, mg, mw, mo, args, s)
-                     : launch<false, true, EPI_STORE, 1>(mg, mw, mg, mw, mo, args, s);
+    CUtensorMap mp = mg;
+    if (!plan_last_round(args, ctas, make_idesc(dt, false, true, ctas, BN / 2), n_out, 1, park, &mp)) return FDP_ERR_LAUNCH;
+    return gemm_fixup(ctas == 2 ? launch<false, true, EPI_STORE, 2>(mg, mw, mp, mw, mo, args, s)
+                                : launch<false, true, EPI_STORE, 1>(mg, mw, mp, mw, mo, args, s), args, ctas, s);
   }
   // W [n_in, n_out]: K contiguous; a CTA of a pair loads half of the 256 B rows
   CUtensorMap mh;
   if (!make_map(&mw, W, n_in, n_out, BK, BN / ctas, dt) || !make_map(&mh, W, n_in, n_out, BK, BN / 2 / ctas, dt)) return FDP_ERR_LAUNCH;
   args.idesc = make_idesc(dt, false, false, ctas);
-  plan_cut(args, ctas, make_idesc(dt, false, false, ctas, BN / 2));
-  return ctas == 2 ? launch<false, false, EPI_STORE, 2>(mg, mw, mg, mh, mo, args, s)
-                   : launch<false, false, EPI_STORE, 1>(mg, mw, mg, mh, mo, args, s);
+  CUtensorMap mp = mg;
+  if (!plan_last_round(args, ctas, make_idesc(dt, false, false, ctas, BN / 2), n_out, 1, park, &mp)) return FDP_ERR_LAUNCH;
+  return gemm_fixup(ctas == 2 ? launch<false, false, EPI_STORE, 2>(mg, mw, mp, mh, mo, args, s)
+                              : launch<false, false, EPI_STORE, 1>(mg, mw, mp, mh, mo, args, s), args, ctas, s);
 }
 
 // forward: A = X [rows, n_in] K-major; B = W, K-major for [n_out, n_in] (Linear), MN-major for
 // [n_in, n_out] (Conv1D); bias added in the epilogue
 int tc_fwd(const void* X, const void* W, const void* bias, void* Y, int* dev_status, int rows, int n_in,
-           int n_out, int dt, int out_dt, int w_layout, cudaStream_t s) {
+           int n_out, int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park) {
   CUtensorMap mx, mw, mo;
   const int ctas = ctas_per_tile();
   if (!make_map(&mx, X, rows, n_in, BK, BM, dt) || !make_out_map(&mo, Y, rows, n_out, out_dt)) return FDP_ERR_LAUNCH;
@@ -1921,15 +1982,17 @@ int tc_fwd(const void* X, const void* W, const void* bias, void* Y, int* dev_sta
     CUtensorMap mh;
     if (!make_map(&mw, W, n_out, n_in, BK, BN / ctas, dt) || !make_map(&mh, W, n_out, n_in, BK, BN / 2 / ctas, dt)) return FDP_ERR_LAUNCH;
     args.idesc = make_idesc(dt, false, false, ctas);
-    plan_cut(args, ctas, make_idesc(dt, false, false, ctas, BN / 2));
-    return ctas == 2 ? launch<false, false, EPI_STORE, 2>(mx, mw, mx, mh, mo, args, s)
-                     : launch<false, false, EPI_STORE, 1>(mx, mw, mx, mh, mo, args, s);
+    CUtensorMap mp = mx;
+    if (!plan_last_round(args, ctas, make_idesc(dt, false, false, ctas, BN / 2), n_in, 1, park, &mp)) return FDP_ERR_LAUNCH;
+    return gemm_fixup(ctas == 2 ? launch<false, false, EPI_STORE, 2>(mx, mw, mp, mh, mo, args, s)
+                                : launch<false, false, EPI_STORE, 1>(mx, mw, mp, mh, mo, args, s), args, ctas, s);
   }
   if (!make_map(&mw, W, n_in, n_out, 64, BK, dt)) return FDP_ERR_LAUNCH;  // W [n_in, n_out]: N contiguous
   args.idesc = make_idesc(dt, false, true, ctas);
-  plan_cut(args, ctas, make_idesc(dt, false, true, ctas, BN / 2));
-  return ctas == 2 ? launch<false, true, EPI_STORE, 2>(mx, mw, mx, mw, mo, args, s)
-                   : launch<false, true, EPI_STORE, 1>(mx, mw, mx, mw, mo, args, s);
+  CUtensorMap mp = mx;
+  if (!plan_last_round(args, ctas, make_idesc(dt, false, true, ctas, BN / 2), n_in, 1, park, &mp)) return FDP_ERR_LAUNCH;
+  return gemm_fixup(ctas == 2 ? launch<false, true, EPI_STORE, 2>(mx, mw, mp, mw, mo, args, s)
+                              : launch<false, true, EPI_STORE, 1>(mx, mw, mp, mw, mo, args, s), args, ctas, s);
 }
 
 // ---- fp32 products on the tensor cores: Y[rows, N] = A[rows, K] * W (+ bias) --------------------------
@@ -1945,7 +2008,7 @@ size_t tc_gemm3_ws_bytes(int rows, int K, int N) {
   return align256(static_cast<size_t>(rows) * K * 4) + align256(static_cast<size_t>(K) * N * 4);
 }
 int tc_gemm3(const void* A3, const void* W3, const void* bias, void* Y, int* dev_status, int rows, int K, int N,
-             int out_dt, bool w_kn, cudaStream_t s, int planes) {
+             int out_dt, bool w_kn, cudaStream_t s, const GemmPark& park, int planes) {
   CUtensorMap ma, mw, mo;
   const int ctas = ctas_per_tile();
   if (!make_map(&ma, A3, rows, static_cast<uint64_t>(planes) * K, BK, BM, FDP_BF16) || !make_out_map(&mo, Y, rows, N, out_dt)) return FDP_ERR_LAUNCH;
@@ -1964,17 +2027,64 @@ int tc_gemm3(const void* A3, const void* W3, const void* bias, void* Y, int* dev
   if (w_kn) {   // rows of W3 are K, N contiguous
     if (!make_map(&mw, W3, K, static_cast<uint64_t>(planes) * N, 64, BK, FDP_BF16)) return FDP_ERR_LAUNCH;
     args.idesc = make_idesc(FDP_BF16, false, true, ctas);
-    plan_cut(args, ctas, make_idesc(FDP_BF16, false, true, ctas, BN / 2));
-    return ctas == 2 ? launch<false, true, EPI_SPLIT_STORE, 2>(ma, mw, ma, mw, mo, args, s)
-                     : launch<false, true, EPI_SPLIT_STORE, 1>(ma, mw, ma, mw, mo, args, s);
+    CUtensorMap mp = ma;
+    if (!plan_last_round(args, ctas, make_idesc(FDP_BF16, false, true, ctas, BN / 2), K, 3, park, &mp)) return FDP_ERR_LAUNCH;
+    return gemm_fixup(ctas == 2 ? launch<false, true, EPI_SPLIT_STORE, 2>(ma, mw, mp, mw, mo, args, s)
+                                : launch<false, true, EPI_SPLIT_STORE, 1>(ma, mw, mp, mw, mo, args, s), args, ctas, s);
   }
   CUtensorMap mh;
   if (!make_map(&mw, W3, N, static_cast<uint64_t>(planes) * K, BK, BN / ctas, FDP_BF16) ||                        // K contiguous
       !make_map(&mh, W3, N, static_cast<uint64_t>(planes) * K, BK, BN / 2 / ctas, FDP_BF16)) return FDP_ERR_LAUNCH;
   args.idesc = make_idesc(FDP_BF16, false, false, ctas);
-  plan_cut(args, ctas, make_idesc(FDP_BF16, false, false, ctas, BN / 2));
-  return ctas == 2 ? launch<false, false, EPI_SPLIT_STORE, 2>(ma, mw, ma, mh, mo, args, s)
-                   : launch<false, false, EPI_SPLIT_STORE, 1>(ma, mw, ma, mh, mo, args, s);
+  CUtensorMap mp = ma;
+  if (!plan_last_round(args, ctas, make_idesc(FDP_BF16, false, false, ctas, BN / 2), K, 3, park, &mp)) return FDP_ERR_LAUNCH;
+  return gemm_fixup(ctas == 2 ? launch<false, false, EPI_SPLIT_STORE, 2>(ma, mw, mp, mh, mo, args, s)
+                              : launch<false, false, EPI_SPLIT_STORE, 1>(ma, mw, mp, mh, mo, args, s), args, ctas, s);
+}
+
+// The same as six products, for the shapes that three do not take: K and N of any number (the copies' rows are padded,
+// their maps end at the last column), an output of any alignment.  These ran on cuBLAS's or this library's fp32 FMA
+// kernels and are to be no further from float64.  Against cuBLAS (bias added): 1024 rows 1000 -> 1024 21.9 / 43.1 us, error
+// 1.0e-7 / 5.7e-7; 2376 rows 1168 -> 312 27.6 / 54; 5000 rows 900 -> 900 56 / 195; 128 rows 8190 -> 8191 243 / 333; 128 rows
+// 1001 -> 4097 26 / 32; 130 rows 72 -> 100 9.6 / 6.1, which is why the Python layer asks for it from 2^26 multiply-adds on.
+bool tc_gemm6_ok(int rows, int K, int N) { return rows >= 128 && K >= 64 && N >= 64; }
+size_t tc_gemm6_w_bytes(int K, int N) {      // in either orientation
+  const size_t a = static_cast<size_t>(K) * pitch8(N), b = static_cast<size_t>(N) * pitch8(K);
+  return align256((a > b ? a : b) * 6);
+}
+size_t tc_gemm6_ws_bytes(int rows, int K, int N) {
+  return align256(static_cast<size_t>(rows) * pitch8(K) * 6) + tc_gemm6_w_bytes(K, N);
+}
+int tc_gemm6(const void* A3, const void* W3, const void* bias, void* Y, int* dev_status, int rows, int K, int N,
+             int out_dt, bool w_kn, cudaStream_t s, const GemmPark& park) {
+  CUtensorMap ma, mw, mh, mo;
+  const int ctas = ctas_per_tile();
+  TcArgs args{};
+  args.direct_out = !aligned16(Y) || N * dtype_size(out_dt) % 16 != 0;
+  if (!make_parts_map(&ma, A3, rows, K, BM)) return FDP_ERR_LAUNCH;
+  if (args.direct_out) mo = ma;   // not used
+  else if (!make_out_map(&mo, Y, rows, N, out_dt)) return FDP_ERR_LAUNCH;
+  args.batch = 1; args.batch_rows = 0; args.status = dev_status;
+  args.dependent = 1;            // follows the split kernels of the same call
+  args.M = rows; args.N = N; args.ld_out = N;
+  args.tiles_m = ceil_div(rows, BM * ctas); args.tiles_n = ceil_div(N, BN);
+  args.tiles_per_batch = args.tiles_m * args.tiles_n;
+  args.k_stages = ceil_div(K, BK);
+  args.n_fastest = 1;
+  args.out = Y; args.out_dt = out_dt; args.scale = 1.0f; args.nk = NoiseKey{};
+  args.bias = bias; args.bias_dt = FDP_F32; args.bias_vec = aligned16(bias);
+  args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = chain_stages(args.seg_stages, 3);
+  args.idesc = make_idesc(FDP_BF16, false, w_kn, ctas);
+  CUtensorMap mp = ma;
+  if (!plan_last_round(args, ctas, make_idesc(FDP_BF16, false, w_kn, ctas, BN / 2), K, 6, park, &mp)) return FDP_ERR_LAUNCH;
+  if (w_kn) {   // rows of W3 are K, N contiguous
+    if (!make_parts_map(&mw, W3, K, N, BK)) return FDP_ERR_LAUNCH;
+    return gemm_fixup(ctas == 2 ? launch<false, true, EPI_SPLIT6_STORE, 2>(ma, mw, mp, mw, mo, args, s)
+                                : launch<false, true, EPI_SPLIT6_STORE, 1>(ma, mw, mp, mw, mo, args, s), args, ctas, s);
+  }
+  if (!make_parts_map(&mw, W3, N, K, BN / ctas) || !make_parts_map(&mh, W3, N, K, BN / 2 / ctas)) return FDP_ERR_LAUNCH;
+  return gemm_fixup(ctas == 2 ? launch<false, false, EPI_SPLIT6_STORE, 2>(ma, mw, mp, mh, mo, args, s)
+                              : launch<false, false, EPI_SPLIT6_STORE, 1>(ma, mw, mp, mh, mo, args, s), args, ctas, s);
 }
 
 }  // namespace fdp

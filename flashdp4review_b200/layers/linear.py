@@ -27,7 +27,7 @@ class _DPLinearFunc(Function):
         ctx.save_for_backward(x, weight, bias, w if dt is not None else None)
         ctx.layer = layer
         ctx.input_dtype = input.dtype
-        if x.is_cuda and ops.native_product_ok(
+        if x.is_cuda and ops.library_product_ok(
                 x.dtype, x.numel() // x.shape[-1], w.shape[1], w.shape[0]):
             return ops.linear_forward(x, w, bias, "out_in")     # library GEMM, bias added in its epilogue
         output = x @ w.t()
@@ -47,7 +47,7 @@ class _DPLinearFunc(Function):
         need_dx, need_dw = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
         need_db = bias is not None and ctx.needs_input_grad[2]
 
-        native_dx = need_dx and ops.native_product_ok(
+        native_dx = need_dx and ops.library_product_ok(
             g3.dtype, g3.numel() // g3.shape[-1], w_for_dx.shape[0], w_for_dx.shape[1])
         if need_dx and not native_dx:
             grad_input = g3 @ w_for_dx.to(g3.dtype)

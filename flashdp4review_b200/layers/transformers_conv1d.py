@@ -44,7 +44,7 @@ class _DPConv1DFunc(Function):
         ctx.save_for_backward(bias, x, weight, w if dt is not None else None)
         ctx.layer = layer
         ctx.input_dtype = input.dtype
-        if x.is_cuda and ops.native_product_ok(
+        if x.is_cuda and ops.library_product_ok(
                 x.dtype, x.numel() // x.shape[-1], w.shape[0], w.shape[1]):
             return ops.linear_forward(x, w, bias, "in_out")     # library GEMM, bias added in its epilogue
         return x @ w + (bias if dt is None else bias.to(dt))
@@ -69,7 +69,7 @@ class _DPConv1DFunc(Function):
                 grad_bias = None
             need_db = False
 
-        native_dx = need_dx and ops.native_product_ok(
+        native_dx = need_dx and ops.library_product_ok(
             g3.dtype, g3.numel() // g3.shape[-1], w_for_dx.shape[1], w_for_dx.shape[0])
         if need_dx and not native_dx:
             grad_input = g3 @ w_for_dx.to(g3.dtype).t()

@@ -33,7 +33,7 @@ extern "C" {
  * 3: fdp_dp_params.step_device (appended; earlier fields keep their offsets); FDP_FP32_TENSOR also
  *    accepted in the dtype of fdp_linear_dgrad / fdp_linear_fwd.
  * 4: FDP_FP32_WIDE, fdp_linear_bwd.
- * 5: FDP_KEEP_PRODUCTS. */
+ * 5: FDP_KEEP_PRODUCTS, FDP_FP32_WIDE_GEMM, FDP_GEMM_SPLIT_K. */
 #define FDP_ABI_VERSION 5
 
 typedef void* fdp_stream_t; /* a cudaStream_t */
@@ -88,7 +88,15 @@ enum fdp_norm_algo {
    * G_b^T X_b in the workspace (fp32, B * n_in * n_out elements, at most 512 MiB) where that is expected to be faster
    * than contracting twice: the norms come from the tiles as they leave, the clipped sum is their weighted sum.
    * fp32 accumulation throughout, as without the flag. */
-  FDP_KEEP_PRODUCTS = 64
+  FDP_KEEP_PRODUCTS = 64,
+  /* flag, OR-ed into the dtype of fdp_linear_dgrad / fdp_linear_fwd and into fdp_linear_bwd's norm_algo (and those of
+   * their workspace queries): fp32 forward and input-gradient products that FDP_FP32_TENSOR's three products do not
+   * take, with at least 128 rows and 64 columns on either side, run as six bf16 products, as close to float64 as an
+   * fp32 FMA kernel.  Operands and output need no alignment.  The workspace holds 1.5 times both operands. */
+  FDP_FP32_WIDE_GEMM = 128,
+  /* flag, OR-ed into the same arguments, of any dtype: products of few output tiles and a long contraction are cut along
+   * it.  The workspace then has room for the fp32 parts, at most 38.8 MB; in a smaller one the product runs uncut. */
+  FDP_GEMM_SPLIT_K = 256
 };
 
 /* DP hyper-parameters of one call.  C / clamp_value are the arguments of
@@ -220,7 +228,7 @@ int fdp_bias_grad_static(const void* G, void* db, float* norms_out, float* facto
  *   the call (also of fdp_linear_fwd).  Where the contracted dimension is a multiple of 64 and rows,
  *   n_in and n_out are at least 128 the product runs as three bf16 products with chained accumulation,
  *   within 1e-5 of float64 and about five times cuBLAS's fp32 GEMM; the workspace then also holds the
- *   bf16 halves of both operands.  Other shapes ignore the flag.
+ *   bf16 halves of both operands.  Other shapes ignore the flag; FDP_FP32_WIDE_GEMM is for them.
  */
 size_t fdp_linear_dgrad_workspace_bytes(int rows, int n_in, int n_out, int dtype);
 int fdp_linear_dgrad(const void* G, const void* W, void* dX, int rows, int n_in, int n_out,
@@ -233,7 +241,7 @@ int fdp_linear_dgrad(const void* G, const void* W, void* dX, int rows, int n_in,
  * dW needs none of the weight gradient's.  `layout` is that of W and of dW.  p belongs to the weight, p_bias to the bias.
  * fp32 inputs with FDP_FP32_TENSOR / FDP_FP32_WIDE in norm_algo: G is split into its bf16 parts once for both
  * products, in the pass that also takes the bias gradient's statistics.  dX runs on the tensor cores with
- * FDP_FP32_TENSOR only, as in fdp_linear_dgrad. */
+ * FDP_FP32_TENSOR or FDP_FP32_WIDE_GEMM only, as in fdp_linear_dgrad. */
 enum fdp_bwd_outputs { FDP_BWD_DX = 1, FDP_BWD_DW = 2, FDP_BWD_DB = 4 };
 size_t fdp_linear_bwd_workspace_bytes(int B, int T, int n_in, int n_out, int in_dtype, int norm_algo, int outputs);
 int fdp_linear_bwd(const void* G, const void* X, const void* W, void* dX, void* dW, void* db, int B, int T,

@@ -105,3 +105,55 @@ def test_cut_tiles(ops, rows, K, N, dtype, layout):  # noqa: F811
     G = _randn(rows, N, seed=4, dtype=dtype)
     _close_to_sum(ops.linear_input_grad(G, W, layout), G.double() @ w.double().t(), G.double().abs() @ w.double().abs().t(),
                   N / 16 + 8 + (2.0 ** 7 if dtype == torch.float32 else 0), UNIT[dtype])
+
+
+# fp32 forward and input gradient in six products: widths of any number (rows that are no multiple of 16 bytes, K stages and
+# tiles that end past the last column), the smallest sizes, cut along K and not, misaligned operands
+@pytest.mark.parametrize("rows,K,N", [(128, 64, 65), (130, 65, 64), (129, 100, 257), (200, 1999, 70), (1000, 333, 515), (300, 2000, 100)])
+@pytest.mark.parametrize("layout", ["out_in", "in_out"])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_fp32_products_in_six(ops, rows, K, N, layout, offset):  # noqa: F811
+    def tensor(*shape, seed, scale=1.0):
+        n = 1
+        for d in shape:
+            n *= d
+        return _randn(n + offset, seed=seed, dtype=torch.float32, scale=scale)[offset:].view(*shape)
+    X, G, b = tensor(rows, K, seed=1), tensor(rows, N, seed=2), tensor(N, seed=3)
+    W = tensor(*((N, K) if layout == "out_in" else (K, N)), seed=4, scale=0.1)
+    w = W if layout == "in_out" else W.t()
+    # each hand-off of 24 steps of which four meet a large accumulator, then one rounded addition a stage, and the parts
+    bound = lambda k: k / 64 * 2 + 8        # noqa: E731
+    _close_to_sum(ops.linear_forward(X, W, b, layout), X.double() @ w.double() + b.double(),
+                  X.double().abs() @ w.double().abs() + b.double().abs(), bound(K), UNIT[torch.float32])
+    _close_to_sum(ops.linear_input_grad(G, W, layout), G.double() @ w.double().t(), G.double().abs() @ w.double().abs().t(),
+                  bound(N), UNIT[torch.float32])
+
+
+@pytest.mark.parametrize("layout", ["out_in", "in_out"])
+def test_whole_backward_in_six_products(ops, layout):  # noqa: F811
+    """One split of G serves the weight gradient and an input gradient in six products: the same bits as the calls alone."""
+    B, T, n_in, n_out = 3, 100, 330, 1001
+    X, G = _randn(B, T, n_in, seed=1, dtype=torch.float32), _randn(B, T, n_out, seed=2, dtype=torch.float32, scale=1e-2)
+    W = _randn(*((n_out, n_in) if layout == "out_in" else (n_in, n_out)), seed=3, dtype=torch.float32, scale=0.1)
+    dX, dW, db = ops.dp_linear_backward(X, G, W, 1.0, 1.0, layout=layout)
+    assert torch.equal(dX, ops.linear_input_grad(G, W, layout))
+    assert torch.equal(dW, ops.dp_linear_weight_grad(X, G, 1.0, 1.0, layout=layout))
+    assert torch.allclose(db, ops.dp_bias_grad(G, 1.0, 1.0), rtol=1e-5, atol=1e-9)
+
+
+# 16-bit and three-product outputs whose parts are parked and added, with and without bias
+@pytest.mark.parametrize("rows,K,N", [(300, 8192, 264), (972, 3520, 688), (128, 4096, 128)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("layout", ["out_in", "in_out"])
+def test_products_cut_along_k(ops, rows, K, N, dtype, layout):  # noqa: F811
+    from flashdp4review_b200 import _lib
+    q = _lib.load().fdp_linear_dgrad_workspace_bytes
+    code = {torch.bfloat16: _lib.FDP_BF16, torch.float32: _lib.FDP_F32 | _lib.FDP_FP32_TENSOR}[dtype]
+    assert q(rows, N, K, code | _lib.FDP_GEMM_SPLIT_K) > q(rows, N, K, code)
+    X, W = _randn(rows, K, seed=1, dtype=dtype), _randn(*((N, K) if layout == "out_in" else (K, N)), seed=2, dtype=dtype, scale=0.1)
+    w = W if layout == "in_out" else W.t()
+    want, absum = X.double() @ w.double(), X.double().abs() @ w.double().abs()
+    k = K / 16 + 8 + (2.0 ** 7 if dtype == torch.float32 else 0)     # (as in test_cut_tiles)
+    for b in (None, _randn(N, seed=3, dtype=dtype)):
+        bd = 0.0 if b is None else b.double()
+        _close_to_sum(ops.linear_forward(X, W, b, layout), want + bd, absum + (0.0 if b is None else bd.abs()), k, UNIT[dtype])
