@@ -225,6 +225,12 @@ def library_product_ok(dtype, rows, K, N):
     return native_product_ok(dtype, rows, K, N) or wide_product_ok(dtype, rows, K, N)
 
 
+def fp32_product_flags():
+    """flags of a layer's forward product, of which fp32 takes all"""
+    flags = _lib.FDP_GEMM_SPLIT_K
+    return flags | _lib.FDP_FP32_TENSOR | _lib.FDP_FP32_WIDE_GEMM if runtime.fp32_mode() == "tensor" else flags
+
+
 def _gemm_dtype_code(dtype, fp32_tensor):
     """dtype code of the forward / input-gradient entry points, with the fp32 tensor-core flags"""
     code = _dt(dtype) | _lib.FDP_GEMM_SPLIT_K
@@ -253,6 +259,14 @@ def linear_input_grad(grad_output, weight, w_layout="out_in", out_dtype=None, fp
     return dX
 
 
+def backward_algo(code, norm_algo):
+    """norm_algo argument of a whole backward: the algorithm and the flags of what the modes allow"""
+    algo = NORM_ALGOS[norm_algo] | _lib.FDP_KEEP_PRODUCTS | _lib.FDP_GEMM_SPLIT_K
+    if code == _lib.FDP_F32 and runtime.fp32_mode() == "tensor":
+        algo |= _lib.FDP_FP32_TENSOR | _lib.FDP_FP32_WIDE | _lib.FDP_FP32_WIDE_GEMM
+    return algo
+
+
 def dp_linear_backward(input, grad_output, weight, C, clamp_value, *, need_dx=True, need_dw=True, need_db=True,
                        batch_divisor=None, noise=None, noise_bias=None, layout="out_in", dx_dtype=None, dw_dtype=None,
                        db_dtype=None, norm_algo="auto", out=None):
@@ -272,9 +286,7 @@ def dp_linear_backward(input, grad_output, weight, C, clamp_value, *, need_dx=Tr
     X = _aligned(input.to(dt).contiguous()) if need_dw else None
     W = _aligned(weight.to(dt).contiguous()) if need_dx else None
     code = _dt(dt)
-    algo = NORM_ALGOS[norm_algo] | _lib.FDP_KEEP_PRODUCTS | _lib.FDP_GEMM_SPLIT_K
-    if dt == torch.float32 and runtime.fp32_mode() == "tensor":
-        algo |= _lib.FDP_FP32_TENSOR | _lib.FDP_FP32_WIDE | _lib.FDP_FP32_WIDE_GEMM
+    algo = backward_algo(code, norm_algo)
     if out is not None:
         shape = (G.shape[-1], n_in) if layout == "out_in" else (n_in, G.shape[-1])
         if tuple(out.shape) != shape or not out.is_contiguous() or out.device != G.device:

@@ -8,6 +8,9 @@
 #include <string>
 
 #include <torch/extension.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 
@@ -160,12 +163,12 @@ py::tuple linear_dgrad(const Tensor& G, const Tensor& W, int rows, int code, int
   return py::make_tuple(st, dX);
 }
 
+struct Bwd { int st; OptTensor dX, dW, db; };
 // G, X as (B, T, .); X only where dW is wanted, W only where dX is
-py::tuple linear_bwd(const Tensor& G, const OptTensor& X, const OptTensor& W, const OptTensor& out, int n_in, int in_dt, int dx_dt, int dw_dt, int db_dt,
-                     int layout, int algo, const py::tuple& p, const py::tuple& p_bias, bool need_dx, bool need_dw, bool need_db) {
+Bwd linear_bwd_call(const Tensor& G, const OptTensor& X, const OptTensor& W, const OptTensor& out, int n_in, int in_dt, int dx_dt, int dw_dt, int db_dt,
+                     int layout, int algo, const fdp_dp_params& q, const fdp_dp_params& qb, bool need_dx, bool need_dw, bool need_db) {
   if (need_dx) check_weight(W.value(), G.size(2), n_in, layout == FDP_OUT_IN, G);
   if (X.has_value() && X->device() != G.device()) refuse("input is on another device than grad_output", *X);
-  const fdp_dp_params q = params(p), qb = params(p_bias);
   const c10::cuda::CUDAGuard guard(G.device());
   const int B = static_cast<int>(G.size(0)), T = static_cast<int>(G.size(1)), n_out = static_cast<int>(G.size(2));
   OptTensor dX, dW, db;
@@ -177,7 +180,6 @@ py::tuple linear_bwd(const Tensor& G, const OptTensor& X, const OptTensor& W, co
   };
   // one call for the outputs that are named, in the workspace `ws`
   const auto call = [&](int outputs, int a, const Tensor& ws) {
-    py::gil_scoped_release nogil;
     return abi.linear_bwd(ptr(G), ptr(X), ptr(W), (outputs & FDP_BWD_DX) ? ptr(dX) : nullptr, (outputs & FDP_BWD_DW) ? ptr(dW) : nullptr,
                           (outputs & FDP_BWD_DB) ? ptr(db) : nullptr, B, T, n_in, n_out, in_dt, dx_dt, dw_dt, db_dt, layout, a,
                           &q, &qb, ptr(ws), ws.numel(), stream(G));
@@ -213,10 +215,20 @@ py::tuple linear_bwd(const Tensor& G, const OptTensor& X, const OptTensor& W, co
       st = call(one, a, own);
     }
   }
-  return py::make_tuple(st, dX, dW, db);
+  return {st, dX, dW, db};
+}
+py::tuple linear_bwd(const Tensor& G, const OptTensor& X, const OptTensor& W, const OptTensor& out, int n_in, int in_dt, int dx_dt, int dw_dt, int db_dt,
+                     int layout, int algo, const py::tuple& p, const py::tuple& p_bias, bool need_dx, bool need_dw, bool need_db) {
+  const fdp_dp_params q = params(p), qb = params(p_bias);
+  Bwd r;
+  {
+    py::gil_scoped_release nogil;
+    r = linear_bwd_call(G, X, W, out, n_in, in_dt, dx_dt, dw_dt, db_dt, layout, algo, q, qb, need_dx, need_dw, need_db);
+  }
+  return py::make_tuple(r.st, r.dX, r.dW, r.db);
 }
 
-py::tuple linear_fwd(const Tensor& X, const Tensor& W, const OptTensor& bias, int rows, int code, int out_dt, int w_layout) {
+std::pair<int, Tensor> linear_fwd_call(const Tensor& X, const Tensor& W, const OptTensor& bias, int rows, int code, int out_dt, int w_layout) {
   check_weight(W, X.size(-1), -1, w_layout != FDP_OUT_IN, X);
   if (bias.has_value() && (bias->numel() != W.size(w_layout == FDP_OUT_IN ? 0 : 1) || bias->device() != X.device()))
     refuse("bias does not fit the output's columns", *bias);
@@ -224,30 +236,40 @@ py::tuple linear_fwd(const Tensor& X, const Tensor& W, const OptTensor& bias, in
   const int n_in = static_cast<int>(X.size(-1)), n_out = static_cast<int>(W.size(w_layout == FDP_OUT_IN ? 0 : 1));
   const Tensor Y = with_columns(X, n_out, out_dt);
   const Tensor ws = workspace_or_less(X, code, [&](int c) { return abi.linear_dgrad_workspace_bytes(rows, n_out, n_in, c); });
-  int st;
+  const int st = abi.linear_fwd(ptr(X), ptr(W), ptr(bias), ptr(Y), rows, n_in, n_out, code, out_dt, w_layout, ptr(ws), ws.numel(), stream(X));
+  return {st, Y};
+}
+py::tuple linear_fwd(const Tensor& X, const Tensor& W, const OptTensor& bias, int rows, int code, int out_dt, int w_layout) {
+  std::pair<int, Tensor> r;
   {
     py::gil_scoped_release nogil;
-    st = abi.linear_fwd(ptr(X), ptr(W), ptr(bias), ptr(Y), rows, n_in, n_out, code, out_dt, w_layout, ptr(ws), ws.numel(), stream(X));
+    r = linear_fwd_call(X, W, bias, rows, code, out_dt, w_layout);
   }
-  return py::make_tuple(st, Y);
+  return py::make_tuple(r.first, r.second);
 }
 
-py::tuple layernorm_fwd(const Tensor& x, const Tensor& w, const Tensor& b, double eps, int rows, int dt, int pdt) {
+
+struct LnFwd { int st; Tensor y, mean, rstd; };
+LnFwd layernorm_fwd_call(const Tensor& x, const Tensor& w, const Tensor& b, double eps, int rows, int dt, int pdt) {
   const c10::cuda::CUDAGuard guard(x.device());
   const Tensor y = new_tensor(x, x.sizes(), x.scalar_type());
   const Tensor mean = new_tensor(x, {rows}, at::kFloat), rstd = new_tensor(x, {rows}, at::kFloat);
-  int st;
+  const int st = abi.layernorm_fwd(ptr(x), ptr(w), ptr(b), ptr(y), static_cast<float*>(ptr(mean)), static_cast<float*>(ptr(rstd)), rows,
+                                   static_cast<int>(x.size(-1)), static_cast<float>(eps), dt, pdt, stream(x));
+  return {st, y, mean, rstd};
+}
+py::tuple layernorm_fwd(const Tensor& x, const Tensor& w, const Tensor& b, double eps, int rows, int dt, int pdt) {
+  LnFwd r;
   {
     py::gil_scoped_release nogil;
-    st = abi.layernorm_fwd(ptr(x), ptr(w), ptr(b), ptr(y), static_cast<float*>(ptr(mean)), static_cast<float*>(ptr(rstd)), rows,
-                           static_cast<int>(x.size(-1)), static_cast<float>(eps), dt, pdt, stream(x));
+    r = layernorm_fwd_call(x, w, b, eps, rows, dt, pdt);
   }
-  return py::make_tuple(st, y, mean, rstd);
+  return py::make_tuple(r.st, r.y, r.mean, r.rstd);
 }
 
-py::tuple layernorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd, int B, int T,
-                        int dt, int pdt, const py::tuple& p, bool need_dx, bool need_dbeta, bool want_norms) {
-  const fdp_dp_params q = params(p);
+struct LnBwd { int st; OptTensor dx; Tensor dgamma; OptTensor dbeta, ng, nb; };
+LnBwd layernorm_bwd_call(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd, int B, int T,
+                         int dt, int pdt, const fdp_dp_params& q, bool need_dx, bool need_dbeta, bool want_norms) {
   const c10::cuda::CUDAGuard guard(x.device());
   const int d = static_cast<int>(x.size(-1));
   OptTensor dx, dbeta, ng, nb;
@@ -257,14 +279,228 @@ py::tuple layernorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, cons
   if (want_norms) ng = new_tensor(x, {B}, at::kFloat);
   if (want_norms && need_dbeta) nb = new_tensor(x, {B}, at::kFloat);
   const Tensor ws = workspace(x, abi.layernorm_bwd_workspace_bytes(B, T, d));
-  int st;
+  const int st = abi.layernorm_bwd(ptr(dy), ptr(x), ptr(w), static_cast<const float*>(ptr(mean)), static_cast<const float*>(ptr(rstd)), ptr(dx),
+                                   ptr(dgamma), ptr(dbeta), static_cast<float*>(ptr(ng)), static_cast<float*>(ptr(nb)), B, T, d, dt, pdt, &q,
+                                   ptr(ws), ws.numel(), stream(x));
+  return {st, dx, dgamma, dbeta, ng, nb};
+}
+py::tuple layernorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd, int B, int T,
+                        int dt, int pdt, const py::tuple& p, bool need_dx, bool need_dbeta, bool want_norms) {
+  const fdp_dp_params q = params(p);
+  LnBwd r;
   {
     py::gil_scoped_release nogil;
-    st = abi.layernorm_bwd(ptr(dy), ptr(x), ptr(w), static_cast<const float*>(ptr(mean)), static_cast<const float*>(ptr(rstd)), ptr(dx),
-                           ptr(dgamma), ptr(dbeta), static_cast<float*>(ptr(ng)), static_cast<float*>(ptr(nb)), B, T, d, dt, pdt, &q,
-                           ptr(ws), ws.numel(), stream(x));
+    r = layernorm_bwd_call(dy, x, w, mean, rstd, B, T, dt, pdt, q, need_dx, need_dbeta, want_norms);
   }
-  return py::make_tuple(st, dx, dgamma, dbeta, ng, nb);
+  return py::make_tuple(r.st, r.dx, r.dgamma, r.dbeta, r.ng, r.nb);
+}
+
+// ---- the layers' autograd nodes --------------------------------------------------------------------------------------
+// What the Function classes of layers/*.py do, without a Python frame per tensor operation: a pass of a small layer is
+// bound by the host, and of its 120 to 160 us those classes took a third.  Choices and noise bookkeeping stay in
+// Python: one call a backward (`layers/_common.py`) takes the step and returns the parameters.  Both are tested to give
+// the same bits.
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+struct PyCalls { py::object product, linear, layernorm, direct_done, check, dtype; }* py_calls = nullptr;    // (outlives the interpreter)
+
+void bind_layers(const py::dict& f) {
+  if (py_calls == nullptr) py_calls = new PyCalls;
+  py_calls->product = f["product"]; py_calls->linear = f["linear"]; py_calls->layernorm = f["layernorm"];
+  py_calls->direct_done = f["direct_done"]; py_calls->check = f["check"]; py_calls->dtype = f["dtype"];
+}
+// A Python exception on its way through the autograd engine, which knows python_error.
+template <typename F>
+auto python(F f) -> decltype(f()) {
+  try {
+    return f();
+  } catch (py::error_already_set& e) {
+    e.restore();
+    python_error err;
+    err.persist();
+    throw err;
+  }
+}
+// ... and back at the boundary to Python
+template <typename F>
+auto boundary(F f) -> decltype(f()) {
+  try {
+    return f();
+  } catch (python_error& e) {
+    e.restore();
+    throw py::error_already_set();
+  }
+}
+void check_status(int st, const char* what) {
+  if (st == FDP_OK) return;
+  py::gil_scoped_acquire gil;
+  python([&] { py_calls->check(st, what); });
+}
+int dtype_code(const Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kFloat: return FDP_F32;
+    case at::kBFloat16: return FDP_BF16;
+    case at::kHalf: return FDP_F16;
+    default: break;
+  }
+  py::gil_scoped_acquire gil;
+  return python([&] { return py_calls->dtype(t).cast<int>(); });     // raises
+}
+Tensor aligned(const Tensor& t) {
+  return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone(at::MemoryFormat::Contiguous);
+}
+// a Python object in a node's saved data
+struct Holder final : c10::ivalue::PyObjectHolder {
+  explicit Holder(PyObject* o) : o_(o) { Py_INCREF(o_); }
+  ~Holder() override {
+    if (!Py_IsInitialized()) return;
+    py::gil_scoped_acquire gil;
+    Py_DECREF(o_);
+  }
+  PyObject* getPyObject() override { return o_; }
+  c10::InferredType tryToInferType() override { return c10::InferredType(std::string("a Python object")); }
+  c10::IValue toIValue(const c10::TypePtr&, std::optional<int32_t>) override { return c10::IValue(); }
+  std::string toStr() override { return "a Python object"; }
+  std::vector<at::Tensor> extractTensors() override { return {}; }
+
+ private:
+  PyObject* o_;
+};
+c10::IValue hold(const py::object& o) { return c10::IValue(c10::intrusive_ptr<c10::ivalue::PyObjectHolder>(c10::make_intrusive<Holder>(o.ptr()))); }
+py::object held(const c10::IValue& v) { return py::reinterpret_borrow<py::object>(v.toPyObject()); }
+at::ScalarType autocast_type(const Tensor& input, const Tensor& weight) {
+  if (!at::autocast::is_autocast_enabled(at::kCUDA) || !input.is_cuda() || !weight.is_cuda()) return at::ScalarType::Undefined;
+  return at::autocast::get_autocast_dtype(at::kCUDA);
+}
+bool product_ok(const Tensor& a, int64_t rows, int64_t K, int64_t N) {
+  const auto t = a.scalar_type();
+  if (t != at::kFloat && t != at::kBFloat16 && t != at::kHalf) return false;
+  return python([&] { return py_calls->product(dtype_code(a), rows, K, N).cast<bool>(); });
+}
+
+struct DpLinear : torch::autograd::Function<DpLinear> {
+  // code: flags that an fp32 product takes; in_out: weight (in, out), as Conv1D's
+  static Tensor forward(AutogradContext* ctx, const Tensor& input, const Tensor& weight, const OptTensor& bias, const c10::IValue& layer,
+                        bool in_out, int64_t code) {
+    const at::ScalarType dt = autocast_type(input, weight);
+    const bool cast = dt != at::ScalarType::Undefined;
+    const Tensor x = cast ? input.to(dt) : input, w = cast ? weight.to(dt) : weight;
+    ctx->save_for_backward({x, weight, bias.has_value() ? *bias : Tensor(), cast ? w : Tensor()});
+    ctx->saved_data["layer"] = layer;
+    ctx->saved_data["in_out"] = in_out;
+    ctx->saved_data["dtype"] = static_cast<int64_t>(input.scalar_type());
+    const int64_t K = x.size(-1);
+    if (K > 0 && w.dim() == 2 && product_ok(x, x.numel() / K, w.size(in_out ? 0 : 1), w.size(in_out ? 1 : 0))) {
+      const Tensor X = aligned(x.contiguous()), W = aligned(w.to(x.scalar_type()).contiguous());
+      OptTensor b;
+      if (bias.has_value()) b = aligned(bias->to(x.scalar_type()).contiguous());
+      const int t = dtype_code(x);
+      const auto r = linear_fwd_call(X, W, b, static_cast<int>(X.numel() / K), t == FDP_F32 ? t | static_cast<int>(code) : t | FDP_GEMM_SPLIT_K, t,
+                                     in_out ? FDP_IN_OUT : FDP_OUT_IN);
+      check_status(r.first, "fdp_linear_fwd");
+      return r.second;
+    }
+    Tensor y = at::matmul(x, in_out ? w : w.t());
+    if (!bias.has_value()) return y;
+    const Tensor b = cast ? bias->to(dt) : *bias;
+    return in_out ? y + b : y.add_(b);
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &weight = saved[1], &bias = saved[2], &w = saved[3].defined() ? saved[3] : saved[1];
+    const bool in_out = ctx->saved_data["in_out"].toBool();
+    const bool need_dx = ctx->needs_input_grad(0), need_dw = ctx->needs_input_grad(1);
+    const bool need_db = bias.defined() && ctx->needs_input_grad(2);
+    Tensor x3 = x, g3 = grads[0];
+    if (x.dim() == 2) {
+      x3 = x.unsqueeze(1); g3 = g3.unsqueeze(1);
+    } else if (x.dim() > 3) {
+      x3 = x.reshape({x.size(0), -1, x.size(-1)}); g3 = g3.reshape({x.size(0), -1, g3.size(-1)});
+    }
+    const int64_t B = x3.size(0), K = w.size(in_out ? 1 : 0), N = w.size(in_out ? 0 : 1);
+    const int t = dtype_code(g3);
+    bool native_dx = false;
+    OptTensor target;
+    fdp_dp_params p{}, pb{};
+    int algo = 0;
+    {
+      py::gil_scoped_acquire gil;
+      python([&] {
+        const py::tuple c = py_calls->linear(held(ctx->saved_data["layer"]), weight, B, t, K > 0 ? g3.numel() / K : 0, K, N, need_dx, need_dw);
+        native_dx = c[0].cast<bool>();
+        p = params(c[1]); pb = params(c[2]);
+        algo = c[3].cast<int>();
+        if (!c[4].is_none()) target = c[4].cast<Tensor>();
+      });
+    }
+    Tensor dX;
+    if (need_dx && !native_dx) {
+      const Tensor wg = w.to(g3.scalar_type());
+      dX = at::matmul(g3, in_out ? wg.t() : wg);
+    }
+    Tensor dW, db;
+    if (native_dx || need_dw || need_db) {
+      if (x3.dim() != 3 || g3.dim() != 3 || x3.size(0) != g3.size(0) || x3.size(1) != g3.size(1)) refuse("expected (B,T,in) and (B,T,out)", g3);
+      Tensor G = g3.contiguous();
+      if (native_dx || need_dw) G = aligned(G);
+      OptTensor X, W;
+      if (need_dw) X = aligned(x3.to(G.scalar_type()).contiguous());
+      if (native_dx) W = aligned(w.to(G.scalar_type()).contiguous());
+      if (target.has_value() && (target->sizes() != weight.sizes() || !target->is_contiguous() || target->device() != G.device()))
+        refuse("out must be a contiguous tensor of the weight's shape on its device", *target);
+      const auto input_type = static_cast<at::ScalarType>(ctx->saved_data["dtype"].toInt());
+      const int dx_dt = input_type == at::kFloat ? FDP_F32 : input_type == at::kBFloat16 ? FDP_BF16 : FDP_F16;
+      const Bwd r = linear_bwd_call(G, X, W, target, static_cast<int>(x3.size(-1)), t, dx_dt, need_dw ? dtype_code(target.has_value() ? *target : weight) : t,
+                                    need_db ? dtype_code(bias) : t, in_out ? FDP_IN_OUT : FDP_OUT_IN, algo, p, pb, native_dx, need_dw, need_db);
+      check_status(r.st, "fdp_linear_bwd");
+      if (native_dx) dX = *r.dX;
+      if (need_dw && !target.has_value()) dW = *r.dW;       // else it is where the optimizer and the all-reduce read it
+      if (need_db) db = *r.db;
+      if (target.has_value()) {
+        py::gil_scoped_acquire gil;
+        python([&] { py_calls->direct_done(weight); });
+      }
+    }
+    if (need_dx) dX = dX.reshape(x.sizes());
+    return {dX, dW, db, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+struct DpLayerNorm : torch::autograd::Function<DpLayerNorm> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& input, const Tensor& weight, const Tensor& bias, const c10::IValue& layer, double eps) {
+    const Tensor x = input.contiguous(), w = weight.contiguous(), b = bias.to(w.scalar_type()).contiguous();
+    const int64_t d = x.size(-1);
+    if (d * x.element_size() >= 65536) throw std::runtime_error("This layer norm doesn't support feature dim >= 64KB.");
+    const LnFwd r = layernorm_fwd_call(x, w, b, eps, d > 0 ? static_cast<int>(x.numel() / d) : 0, dtype_code(x), dtype_code(w));
+    check_status(r.st, "fdp_layernorm_fwd");
+    ctx->save_for_backward({input, weight, r.mean, r.rstd});
+    ctx->saved_data["layer"] = layer;
+    return r.y;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list saved = ctx->get_saved_variables();
+    const Tensor x = saved[0].contiguous(), w = saved[1].contiguous(), dy = grads[0].contiguous();
+    const int64_t d = x.size(-1), B = x.dim() > 1 ? x.size(0) : 1;
+    const bool need_dx = ctx->needs_input_grad(0), need_dw = ctx->needs_input_grad(1), need_db = ctx->needs_input_grad(2);
+    fdp_dp_params p{};
+    {
+      py::gil_scoped_acquire gil;
+      python([&] { p = params(py_calls->layernorm(held(ctx->saved_data["layer"]), B)); });
+    }
+    const LnBwd r = layernorm_bwd_call(dy, x, w, saved[2], saved[3], static_cast<int>(B), static_cast<int>(x.numel() / (B * d)), dtype_code(x),
+                                       dtype_code(w), p, need_dx, need_db, false);
+    check_status(r.st, "fdp_layernorm_bwd");
+    return {need_dx ? *r.dx : Tensor(), need_dw ? r.dgamma : Tensor(), need_db ? *r.dbeta : Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor dp_linear(const Tensor& input, const Tensor& weight, const OptTensor& bias, const py::object& layer, bool in_out, int64_t code) {
+  return boundary([&] { return DpLinear::apply(input, weight, bias, hold(layer), in_out, code); });
+}
+Tensor dp_layernorm(const Tensor& input, const Tensor& weight, const Tensor& bias, const py::object& layer, double eps) {
+  return boundary([&] { return DpLayerNorm::apply(input, weight, bias, hold(layer), eps); });
 }
 
 }  // namespace
@@ -279,4 +515,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("linear_fwd", &linear_fwd);
   m.def("layernorm_fwd", &layernorm_fwd);
   m.def("layernorm_bwd", &layernorm_bwd);
+  m.def("bind_layers", &bind_layers);
+  m.def("dp_linear", &dp_linear);
+  m.def("dp_layernorm", &dp_layernorm);
 }

@@ -1,5 +1,8 @@
 """Shared pieces of the DP layer backward passes."""
-from .. import runtime
+import torch
+
+from .. import _lib, runtime
+from ..core import ops
 from ..core.ops import NoiseSpec, noise_std
 from ..distributed import direct_reducer
 
@@ -69,7 +72,47 @@ def autocast_dtype(*tensors):
     reference the Conv1D forward adds an fp32 bias to the bf16 product, the output and hence the
     whole backward become fp32 -- flashdp/layers/transformers_conv1d.py:40-43.)
     """
-    import torch
     if torch.is_autocast_enabled("cuda") and all(t is None or t.is_cuda for t in tensors):
         return torch.get_autocast_dtype("cuda")
     return None
+
+
+# ---- the native autograd nodes (csrc/fdp_host.cpp) and what they ask Python for ------------------------------------
+_CODES = {code: dtype for dtype, code in ops._DT.items()}
+_native = None
+
+
+def native_nodes(input):
+    """The call layer with the layers' autograd nodes, or None where the Function classes take the call: tensors that
+    are not on a GPU, and torch.jit.trace, which records a Function but would take a node's output for a constant."""
+    global _native
+    if not input.is_cuda or torch._C._get_tracing_state() is not None:
+        return None
+    if _native is None:
+        host = _lib.host()
+        host.bind_layers({"product": _product, "linear": _linear_call, "layernorm": _layernorm_call,
+                          "direct_done": direct_grad_done, "check": _lib.check, "dtype": lambda t: ops._dt(t.dtype)})
+        _native = host
+    return _native
+
+
+def _product(code, rows, K, N):
+    return ops.library_product_ok(_CODES[code], rows, K, N)
+
+
+def _linear_call(layer, weight, B, code, rows, K, N, need_dx, need_dw):
+    """One backward of a Linear / Conv1D layer: whether the input gradient is the library's, the parameters of the
+    weight's and of the bias's gradient, the flags of the call, and the bucket slice the weight gradient goes to."""
+    step = layer._next_step()
+    native_dx = need_dx and ops.library_product_ok(_CODES[code], rows, K, N)
+    w_id, b_id = layer._dp_param_ids
+    div, noise = dp_scalars(B, layer.noise_multiplier, w_id, step)
+    p = ops._params(layer.C, layer.clamp_value, div, noise)
+    bias = p[:5] + (int(b_id) & 0xFFFFFFFF,) + p[6:]
+    return native_dx, p, bias, ops.backward_algo(code, layer.norm_algo), direct_grad_target(weight) if need_dw else None
+
+
+def _layernorm_call(layer, B):
+    g_id, b_id = layer._dp_param_ids
+    div, noise = dp_scalars(B, layer.noise_multiplier, g_id, layer._next_step(), param_id2=b_id)
+    return ops._params(layer.C, layer.clamp_value, div, noise)

@@ -22,7 +22,7 @@ from torch.autograd.function import Function
 
 from ..core import ops
 from .utils import DPParameter as Parameter
-from ._common import DPLayerMixin, dp_scalars
+from ._common import DPLayerMixin, dp_scalars, native_nodes
 
 
 class _DPLayerNormFunc(Function):
@@ -87,4 +87,7 @@ class DPLayerNorm(nn.LayerNorm, DPLayerMixin):
         if not self.elementwise_affine:
             return torch.nn.functional.layer_norm(input, self.normalized_shape, None, None, self.eps)
         bias = self.bias if self.bias is not None else torch.zeros_like(self.weight)
+        native = None if self.compat_fused_saturation else native_nodes(input)
+        if native is not None:
+            return native.dp_layernorm(input, self.weight, bias, self, float(self.eps))
         return _DPLayerNormFunc.apply(input, self.weight, bias, self)

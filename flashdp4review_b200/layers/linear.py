@@ -15,7 +15,7 @@ from ..core import ops
 from ..core.ops import RuntimeAutoTuner
 from .utils import DPParameter as Parameter
 from ._common import (DPLayerMixin, reshape_to_3d, dp_scalars, autocast_dtype, direct_grad_target,
-                      direct_grad_done)
+                      direct_grad_done, native_nodes)
 
 
 class _DPLinearFunc(Function):
@@ -91,4 +91,7 @@ class DPLinear(nn.Linear, DPLayerMixin):
             self.bias = Parameter(self.bias.data)
 
     def forward(self, input):
+        native = native_nodes(input)
+        if native is not None:
+            return native.dp_linear(input, self.weight, self.bias, self, False, ops.fp32_product_flags())
         return _DPLinearFunc.apply(input, self.weight, self.bias, self)
