@@ -19,6 +19,7 @@ FDP_F32, FDP_BF16, FDP_F16 = 0, 1, 2
 FDP_OUT_IN, FDP_IN_OUT = 0, 1
 FDP_NORM_AUTO, FDP_NORM_DIRECT, FDP_NORM_GRAM = 0, 1, 2
 FDP_FP32_TENSOR, FDP_FP32_WIDE, FDP_KEEP_PRODUCTS, FDP_FP32_WIDE_GEMM, FDP_GEMM_SPLIT_K = 16, 32, 64, 128, 256
+FDP_PAD_16BIT = 512
 
 c_void_p, c_int, c_size_t, c_float = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t, ctypes.c_float
 

@@ -116,7 +116,7 @@ def dp_linear_weight_grad(input, grad_output, C, clamp_value, *, batch_divisor=N
         out_dtype = out.dtype
     else:
         out_dtype = out_dtype or G.dtype
-    algo = NORM_ALGOS[norm_algo] | _lib.FDP_KEEP_PRODUCTS
+    algo = NORM_ALGOS[norm_algo] | _lib.FDP_KEEP_PRODUCTS | _lib.FDP_PAD_16BIT
     if fp32_tensor is None:
         fp32_tensor = runtime.fp32_mode() == "tensor"
     if fp32_tensor and G.dtype == torch.float32:
@@ -212,12 +212,17 @@ def native_product_ok(dtype, rows, K, N):
 
 def wide_product_ok(dtype, rows, K, N):
     """Whether a product outside native_product_ok runs on this library's tensor-core kernels all the same, through
-    copies of the operands with padded rows: fp32 in mode "tensor" as six bf16 products over three parts, as close to
-    float64 as cuBLAS's fp32 kernels.  Never under input_grad_impl() == "library"."""
-    if runtime.input_grad_impl() == "library" or dtype != torch.float32:
+    copies of the operands with padded rows: 16-bit with a width that is no multiple of 8 (cuBLAS then falls back to
+    kernels of an older generation) and at least 128 rows and 64 columns on either side; fp32 in mode
+    "tensor" as six bf16 products over three parts, as close to float64 as cuBLAS's fp32 kernels.  Never under
+    input_grad_impl() == "library"."""
+    if runtime.input_grad_impl() == "library" or rows < 128 or K < 64 or N < 64:
         return False
-    # (measured: 2^26 multiply-adds are where the split of the operands has paid off against cuBLAS)
-    return runtime.fp32_mode() == "tensor" and rows >= 128 and K >= 64 and N >= 64 and rows * K * N >= 1 << 26
+    if dtype == torch.float32:
+        # (measured: 2^26 multiply-adds are where the split of the operands has paid off against cuBLAS)
+        return runtime.fp32_mode() == "tensor" and rows * K * N >= 1 << 26
+    # (measured: 1000 rows 999 -> 999 18 us against 45, 128 rows 65 -> 65 11 against 6)
+    return dtype in (torch.bfloat16, torch.float16) and (K % 8 != 0 or N % 8 != 0) and rows * K * N >= 1 << 24
 
 
 def library_product_ok(dtype, rows, K, N):
@@ -227,13 +232,13 @@ def library_product_ok(dtype, rows, K, N):
 
 def fp32_product_flags():
     """flags of a layer's forward product, of which fp32 takes all"""
-    flags = _lib.FDP_GEMM_SPLIT_K
+    flags = _lib.FDP_GEMM_SPLIT_K | _lib.FDP_PAD_16BIT
     return flags | _lib.FDP_FP32_TENSOR | _lib.FDP_FP32_WIDE_GEMM if runtime.fp32_mode() == "tensor" else flags
 
 
 def _gemm_dtype_code(dtype, fp32_tensor):
     """dtype code of the forward / input-gradient entry points, with the fp32 tensor-core flags"""
-    code = _dt(dtype) | _lib.FDP_GEMM_SPLIT_K
+    code = _dt(dtype) | _lib.FDP_GEMM_SPLIT_K | _lib.FDP_PAD_16BIT
     if dtype == torch.float32:
         if fp32_tensor is None:
             fp32_tensor = runtime.fp32_mode() == "tensor"
@@ -261,7 +266,7 @@ def linear_input_grad(grad_output, weight, w_layout="out_in", out_dtype=None, fp
 
 def backward_algo(code, norm_algo):
     """norm_algo argument of a whole backward: the algorithm and the flags of what the modes allow"""
-    algo = NORM_ALGOS[norm_algo] | _lib.FDP_KEEP_PRODUCTS | _lib.FDP_GEMM_SPLIT_K
+    algo = NORM_ALGOS[norm_algo] | _lib.FDP_KEEP_PRODUCTS | _lib.FDP_GEMM_SPLIT_K | _lib.FDP_PAD_16BIT
     if code == _lib.FDP_F32 and runtime.fp32_mode() == "tensor":
         algo |= _lib.FDP_FP32_TENSOR | _lib.FDP_FP32_WIDE | _lib.FDP_FP32_WIDE_GEMM
     return algo

@@ -114,7 +114,7 @@ struct WgradWs {
 WgradWs wgrad_ws(void* base, int B, int T, int n_in, int n_out, int dt, int norm_algo) {
   WgradWs w;
   w.tc = tc_plan(B, T, n_in, n_out, dt, norm_algo);
-  w.short_seq = T < SHORT_SEQ && (norm_algo & FDP_NORM_MASK) != FDP_NORM_DIRECT;
+  w.short_seq = w.tc.ok ? w.tc.short_seq : T < SHORT_SEQ && (norm_algo & FDP_NORM_MASK) != FDP_NORM_DIRECT;
   w.nparts = w.tc.ok ? w.tc.nparts : (w.short_seq ? 1 : simt_norm_tiles(n_in, n_out));
   Carver c(base);
   w.status = c.take<int>(64);
@@ -266,11 +266,27 @@ static int wgrad_run(const void* G, const void* X, void* dW, float* norms_out, f
     if (!w.short_seq && !presplit && (st = tc_split(jobs, 2, w.tc.planes, w.status, s)) != FDP_OK) return st;
     Gt = sg; Xt = sx; tdt = FDP_BF16;
   }
+  // 16-bit operands whose rows or pointers the copy engine cannot take: copies with padded rows
+  int pitch_g = 0, pitch_x = 0;
+  if (w.tc.ok && w.tc.pad) {
+    char* pg = static_cast<char*>(w.tc_extra) + w.tc.split_bytes;
+    SplitJob jobs[2];
+    int n = 0;
+    if (n_out % 8 != 0 || !aligned16(G)) {
+      jobs[n++] = SplitJob{G, pg, static_cast<size_t>(B) * T, n_out, nullptr, T};
+      Gt = pg; pitch_g = tc_pitch(n_out);
+    }
+    if (n_in % 8 != 0 || !aligned16(X)) {
+      jobs[n++] = SplitJob{X, pg + w.tc.pad_g_bytes, static_cast<size_t>(B) * T, n_in, nullptr, T};
+      Xt = pg + w.tc.pad_g_bytes; pitch_x = tc_pitch(n_in);
+    }
+    if (n > 0 && (st = tc_split(jobs, n, 0, nullptr, s)) != FDP_OK) return st;
+  }
   if (w.short_seq) {
     simt_norm_gram_small(G, X, w.partials, B, T, n_in, n_out, in_dtype, s);
   } else if (w.tc.ok) {
     if ((st = tc_norms(Gt, Xt, w.partials, w.status, B, T, n_in, n_out, tdt, w.tc, s,
-                       w.tc.keep ? static_cast<float*>(w.tc_extra) : nullptr, layout)) != FDP_OK) return st;
+                       w.tc.keep ? static_cast<float*>(w.tc_extra) : nullptr, layout, pitch_g, pitch_x)) != FDP_OK) return st;
   } else {
     w.nparts = simt_norm_direct(G, X, w.partials, B, T, n_in, n_out, in_dtype, norm_algo & FDP_NORM_MASK, s);
   }
@@ -302,7 +318,7 @@ static int wgrad_run(const void* G, const void* X, void* dW, float* norms_out, f
     prof_mark(3, s);
     if ((st = tc_clipped_wgrad(w.tc.scaled_epilogue ? Gt : gs, Xt, w.tc.scaled_epilogue ? &fs : nullptr, split_ws,
                                dW, w.status, B, T, n_in, n_out, tdt, out_dtype, layout, inv_div, nk,
-                               s, w.tc.planes)) != FDP_OK) return st;
+                               s, w.tc.planes, w.tc.pad, pitch_g, pitch_x)) != FDP_OK) return st;
   } else {
     prof_mark(3, s);
     simt_clipped_wgrad(G, X, w.factors, dW, B, T, n_in, n_out, in_dtype, out_dtype, layout, inv_div, nk, s);
@@ -320,7 +336,7 @@ int fdp_linear_wgrad(const void* G, const void* X, void* dW, float* norms_out, f
   if (G == nullptr || X == nullptr || dW == nullptr) return FDP_ERR_ARG;
   if (B <= 0 || T <= 0 || n_in <= 0 || n_out <= 0) return FDP_ERR_ARG;
   if (layout != FDP_OUT_IN && layout != FDP_IN_OUT) return FDP_ERR_ARG;
-  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE | FDP_KEEP_PRODUCTS | FDP_FP32_WIDE_GEMM | FDP_GEMM_SPLIT_K)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
+  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE | FDP_KEEP_PRODUCTS | FDP_FP32_WIDE_GEMM | FDP_GEMM_SPLIT_K | FDP_PAD_16BIT)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
     return FDP_ERR_ARG;
   if (!valid_dtype(in_dtype) || !valid_dtype(out_dtype)) return FDP_ERR_DTYPE;
   if (static_cast<long long>(B) * T >= (1ll << 31) / 2) return FDP_ERR_SHAPE;   // row indices are 32-bit
@@ -386,9 +402,17 @@ int fdp_bias_grad(const void* G, void* db, float* norms_out, float* factors_out,
 }
 
 // ---- input gradient ---------------------------------------------------------------------------------
-constexpr int GEMM_FLAGS = FDP_FP32_TENSOR | FDP_FP32_WIDE_GEMM | FDP_GEMM_SPLIT_K;
+constexpr int GEMM_FLAGS = FDP_FP32_TENSOR | FDP_FP32_WIDE_GEMM | FDP_GEMM_SPLIT_K | FDP_PAD_16BIT, GEMM_FLAGS_16 = FDP_GEMM_SPLIT_K | FDP_PAD_16BIT;
 // `dtype` of a forward or input-gradient product without its flags (fp32's with 16-bit types are left in: no such dtype)
-static int gemm_dtype(int dtype) { return dtype & ~((dtype & ~GEMM_FLAGS) == FDP_F32 ? GEMM_FLAGS : FDP_GEMM_SPLIT_K); }
+static int gemm_dtype(int dtype) { return dtype & ~((dtype & ~GEMM_FLAGS) == FDP_F32 ? GEMM_FLAGS : GEMM_FLAGS_16); }
+// 16-bit shapes that the tensor cores take with FDP_PAD_16BIT only, and the copies of [rows, K] and of W
+static bool gemm_pad(int dtype, int rows, int K, int N) {
+  return (dtype & FDP_PAD_16BIT) != 0 && !tc_dgrad_ok(rows, N, K, gemm_dtype(dtype)) && tc_pad_gemm_ok(rows, N, K, gemm_dtype(dtype));
+}
+static size_t gemm_pad_bytes(int rows, int K, int N) {
+  const size_t wk = tc_pad_bytes(K, N), wn = tc_pad_bytes(N, K);      // the query does not know W's orientation
+  return tc_pad_bytes(rows, K) + (wk > wn ? wk : wn);
+}
 // fp32 with FDP_FP32_TENSOR / FDP_FP32_WIDE_GEMM in `dtype`: how many parts the operands of [rows, K] x [K, N] are split
 // into -- two (three products), three (six) or none
 static int gemm_parts(int dtype, int rows, int K, int N) {
@@ -402,11 +426,11 @@ static size_t gemm_ws_bytes(int parts, int rows, int K, int N) {
 // the workspace of a product: the status word, the split copies of the two operands when fp32 runs on the tensor cores,
 // and with FDP_GEMM_SPLIT_K the place for a K split's parts
 static size_t gemm_park_bytes(int dtype, int parts, int rows, int K, int N) {
-  if ((dtype & FDP_GEMM_SPLIT_K) == 0 || (parts == 0 && !tc_dgrad_ok(rows, N, K, gemm_dtype(dtype)))) return 0;
+  if ((dtype & FDP_GEMM_SPLIT_K) == 0 || (parts == 0 && !tc_dgrad_ok(rows, N, K, gemm_dtype(dtype)) && !gemm_pad(dtype, rows, K, N))) return 0;
   return tc_gemm_park_bytes(rows, K, N, parts == 3 ? 6 : parts == 2 ? 3 : 1);
 }
-static GemmPark gemm_park(void* workspace, size_t workspace_bytes, int parts, int rows, int K, int N) {
-  const size_t off = 256 + gemm_ws_bytes(parts, rows, K, N);
+static GemmPark gemm_park(void* workspace, size_t workspace_bytes, int parts, bool pad, int rows, int K, int N) {
+  const size_t off = 256 + gemm_ws_bytes(parts, rows, K, N) + (pad ? gemm_pad_bytes(rows, K, N) : 0);
   if (workspace_bytes <= off) return GemmPark{nullptr, 0};
   return GemmPark{reinterpret_cast<float*>(static_cast<char*>(workspace) + off), workspace_bytes - off};
 }
@@ -414,7 +438,29 @@ static GemmPark gemm_park(void* workspace, size_t workspace_bytes, int parts, in
 size_t fdp_linear_dgrad_workspace_bytes(int rows, int n_in, int n_out, int dtype) {
   // (K = n_out, N = n_in; the forward product queries with the two exchanged)
   const int parts = gemm_parts(dtype, rows, n_out, n_in);
-  return 256 + gemm_ws_bytes(parts, rows, n_out, n_in) + gemm_park_bytes(dtype, parts, rows, n_out, n_in);
+  return 256 + gemm_ws_bytes(parts, rows, n_out, n_in) + (gemm_pad(dtype, rows, n_out, n_in) ? gemm_pad_bytes(rows, n_out, n_in) : 0) +
+         gemm_park_bytes(dtype, parts, rows, n_out, n_in);
+}
+
+// The operands of a padded product: A [rows, K] and W [w_rows, w_cols], copied behind the status word where their rows are
+// no multiple of 16 bytes (pitch 0: used as they are).
+struct PaddedOperands { const void* A; const void* W; int pitch_a, pitch_w, st; };
+static PaddedOperands pad_operands(const void* A, const void* W, int rows, int K, int w_rows, int w_cols, void* workspace, cudaStream_t s) {
+  PaddedOperands o{A, W, 0, 0, FDP_OK};
+  char* c = static_cast<char*>(workspace) + 256;
+  SplitJob jobs[2];
+  int n = 0;
+  if (K % 8 != 0) {
+    jobs[n++] = SplitJob{A, c, static_cast<size_t>(rows), K, nullptr, 1};
+    o.A = c; o.pitch_a = tc_pitch(K);
+    c += tc_pad_bytes(rows, K);
+  }
+  if (w_cols % 8 != 0) {
+    jobs[n++] = SplitJob{W, c, static_cast<size_t>(w_rows), w_cols, nullptr, 1};
+    o.W = c; o.pitch_w = tc_pitch(w_cols);
+  }
+  if (n > 0) o.st = tc_split(jobs, n, 0, nullptr, s);
+  return o;
 }
 
 // Y[rows, N] = A[rows, K] * W (+ bias), fp32 in and out, as three or six bf16 products: split, then one GEMM
@@ -443,6 +489,8 @@ int fdp_linear_dgrad(const void* G, const void* W, void* dX, int rows, int n_in,
   if (w_layout != FDP_OUT_IN && w_layout != FDP_IN_OUT) return FDP_ERR_ARG;
   const int parts = gemm_parts(dtype, rows, n_out, n_in);
   const bool split_k = (dtype & FDP_GEMM_SPLIT_K) != 0;
+  // (in a workspace without room for the copies the generic kernels take the call)
+  const bool pad = gemm_pad(dtype, rows, n_out, n_in) && workspace_bytes >= 256 + gemm_pad_bytes(rows, n_out, n_in);
   dtype = gemm_dtype(dtype);
   if (!valid_dtype(dtype) || !valid_dtype(out_dtype)) return FDP_ERR_DTYPE;
   int st = current_device_ok();
@@ -450,13 +498,18 @@ int fdp_linear_dgrad(const void* G, const void* W, void* dX, int rows, int n_in,
   if (workspace == nullptr || workspace_bytes < 256 || !aligned16(workspace)) return FDP_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int* status = static_cast<int*>(workspace);
-  const GemmPark park = split_k ? gemm_park(workspace, workspace_bytes, parts, rows, n_out, n_in) : GemmPark{nullptr, 0};
+  const GemmPark park = split_k ? gemm_park(workspace, workspace_bytes, parts, pad, rows, n_out, n_in) : GemmPark{nullptr, 0};
   if (parts == 3 || (parts == 2 && aligned16(G) && aligned16(W) && aligned16(dX))) {
     // dX = G [rows, n_out] * W: W is [n_out, n_in] = [K, N] for nn.Linear, [n_in, n_out] = [N, K] for Conv1D
     if ((st = gemm_split_call(parts, G, W, nullptr, dX, rows, n_out, n_in, out_dtype, w_layout == FDP_OUT_IN, workspace,
                               workspace_bytes, s, park)) != FDP_OK) return st;
   } else if (tc_dgrad_ok(rows, n_in, n_out, dtype) && aligned16(G) && aligned16(W) && aligned16(dX)) {
     if ((st = tc_dgrad(G, W, dX, status, rows, n_in, n_out, dtype, out_dtype, w_layout, s, park)) != FDP_OK) return st;
+  } else if (pad && (aligned16(G) || n_out % 8 != 0) && (aligned16(W) || (w_layout == FDP_OUT_IN ? n_in : n_out) % 8 != 0)) {
+    const bool oi = w_layout == FDP_OUT_IN;
+    const PaddedOperands o = pad_operands(G, W, rows, n_out, oi ? n_out : n_in, oi ? n_in : n_out, workspace, s);
+    if (o.st != FDP_OK) return o.st;
+    if ((st = tc_dgrad(o.A, o.W, dX, status, rows, n_in, n_out, dtype, out_dtype, w_layout, s, park, o.pitch_a, o.pitch_w)) != FDP_OK) return st;
   } else {
     FDP_CUDA_OK(cudaMemsetAsync(status, 0, sizeof(int), s));
     simt_dgrad(G, W, dX, rows, n_in, n_out, dtype, out_dtype, w_layout, s);
@@ -475,6 +528,7 @@ int fdp_linear_fwd(const void* X, const void* W, const void* bias, void* Y, int 
   if (w_layout != FDP_OUT_IN && w_layout != FDP_IN_OUT) return FDP_ERR_ARG;
   const int parts = gemm_parts(dtype, rows, n_in, n_out);
   const bool split_k = (dtype & FDP_GEMM_SPLIT_K) != 0;
+  const bool pad = gemm_pad(dtype, rows, n_in, n_out) && workspace_bytes >= 256 + gemm_pad_bytes(rows, n_in, n_out);
   dtype = gemm_dtype(dtype);
   if (!valid_dtype(dtype) || !valid_dtype(out_dtype)) return FDP_ERR_DTYPE;
   int st = current_device_ok();
@@ -482,7 +536,7 @@ int fdp_linear_fwd(const void* X, const void* W, const void* bias, void* Y, int 
   if (workspace == nullptr || workspace_bytes < 256 || !aligned16(workspace)) return FDP_ERR_WORKSPACE;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int* status = static_cast<int*>(workspace);
-  const GemmPark park = split_k ? gemm_park(workspace, workspace_bytes, parts, rows, n_in, n_out) : GemmPark{nullptr, 0};
+  const GemmPark park = split_k ? gemm_park(workspace, workspace_bytes, parts, pad, rows, n_in, n_out) : GemmPark{nullptr, 0};
   if (parts == 3 || (parts == 2 && aligned16(X) && aligned16(W) && aligned16(Y) && (bias == nullptr || aligned16(bias)))) {
     // Y = X [rows, n_in] * W^T: W is [n_out, n_in] = [N, K] for nn.Linear, [n_in, n_out] = [K, N] for Conv1D
     if ((st = gemm_split_call(parts, X, W, bias, Y, rows, n_in, n_out, out_dtype, w_layout == FDP_IN_OUT, workspace,
@@ -491,6 +545,11 @@ int fdp_linear_fwd(const void* X, const void* W, const void* bias, void* Y, int 
   // same shape rules as the input gradient with the roles of n_in and n_out exchanged
   if (tc_dgrad_ok(rows, n_out, n_in, dtype) && aligned16(X) && aligned16(W) && aligned16(Y)) {
     if ((st = tc_fwd(X, W, bias, Y, status, rows, n_in, n_out, dtype, out_dtype, w_layout, s, park)) != FDP_OK) return st;
+  } else if (pad && (aligned16(X) || n_in % 8 != 0) && (aligned16(W) || (w_layout == FDP_OUT_IN ? n_in : n_out) % 8 != 0)) {
+    const bool oi = w_layout == FDP_OUT_IN;
+    const PaddedOperands o = pad_operands(X, W, rows, n_in, oi ? n_out : n_in, oi ? n_in : n_out, workspace, s);
+    if (o.st != FDP_OK) return o.st;
+    if ((st = tc_fwd(o.A, o.W, bias, Y, status, rows, n_in, n_out, dtype, out_dtype, w_layout, s, park, o.pitch_a, o.pitch_w)) != FDP_OK) return st;
   } else {
     FDP_CUDA_OK(cudaMemsetAsync(status, 0, sizeof(int), s));
     simt_fwd(X, W, bias, Y, rows, n_in, n_out, dtype, out_dtype, w_layout, s);
@@ -502,7 +561,7 @@ int fdp_linear_fwd(const void* X, const void* W, const void* bias, void* Y, int 
 // ---- the whole backward of a Linear / Conv1D layer ----------------------------------------------------------
 namespace {
 // the input gradient's dtype with the flags that came in norm_algo
-int gemm_code(int dtype, int norm_algo) { return dtype | (norm_algo & (dtype == FDP_F32 ? GEMM_FLAGS : FDP_GEMM_SPLIT_K)); }
+int gemm_code(int dtype, int norm_algo) { return dtype | (norm_algo & (dtype == FDP_F32 ? GEMM_FLAGS : GEMM_FLAGS_16)); }
 // Whether one set of split copies can serve both products: fp32 on the tensor cores with the parts made before the
 // norms, and an input gradient that takes them too.
 struct LinearBwdWs {
@@ -559,7 +618,7 @@ int fdp_linear_bwd(const void* G, const void* X, const void* W, void* dX, void* 
   if (B <= 0 || T <= 0 || n_in <= 0 || n_out <= 0) return FDP_ERR_ARG;
   if (static_cast<long long>(B) * T >= (1ll << 31) / 2) return FDP_ERR_SHAPE;   // row indices are 32-bit
   if (!valid_dtype(in_dtype)) return FDP_ERR_DTYPE;
-  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE | FDP_KEEP_PRODUCTS | FDP_FP32_WIDE_GEMM | FDP_GEMM_SPLIT_K)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
+  if (norm_algo < 0 || (norm_algo & ~(FDP_NORM_MASK | FDP_FP32_TENSOR | FDP_FP32_WIDE | FDP_KEEP_PRODUCTS | FDP_FP32_WIDE_GEMM | FDP_GEMM_SPLIT_K | FDP_PAD_16BIT)) != 0 || (norm_algo & FDP_NORM_MASK) > FDP_NORM_GRAM)
     return FDP_ERR_ARG;
   const int outputs = (dX ? FDP_BWD_DX : 0) | (dW ? FDP_BWD_DW : 0) | (db ? FDP_BWD_DB : 0);
   if (outputs == 0) return FDP_ERR_ARG;

@@ -59,11 +59,11 @@ Tensor workspace(const Tensor& like, size_t bytes) {
 }
 // The workspace that `query` asks for under the flags of `code`.  Where it does not fit the card, what asks for most is given
 // up first: the per-sample products (up to 512 MiB) and the parts of a K split (38.8 MB); then the split copies of fp32
-// operands in six products (1.5 times the operands, and 38.8 MB for a weight gradient), whose shapes then stay on the FMA
-// kernels, which need next to nothing.
+// operands in six products (1.5 times the operands, and 38.8 MB for a weight gradient) and the padded ones of 16-bit
+// operands, whose shapes then stay on the FMA kernels, which need next to nothing.
 template <typename Query>
 Tensor workspace_or_less(const Tensor& like, int& code, Query query) {
-  constexpr int SPEED = FDP_KEEP_PRODUCTS | FDP_GEMM_SPLIT_K, COPIES = FDP_FP32_WIDE | FDP_FP32_WIDE_GEMM;
+  constexpr int SPEED = FDP_KEEP_PRODUCTS | FDP_GEMM_SPLIT_K, COPIES = FDP_FP32_WIDE | FDP_FP32_WIDE_GEMM | FDP_PAD_16BIT;
   for (const int flags : {SPEED, COPIES}) {
     try {
       return workspace(like, query(code));
@@ -395,7 +395,7 @@ struct DpLinear : torch::autograd::Function<DpLinear> {
       OptTensor b;
       if (bias.has_value()) b = aligned(bias->to(x.scalar_type()).contiguous());
       const int t = dtype_code(x);
-      const auto r = linear_fwd_call(X, W, b, static_cast<int>(X.numel() / K), t == FDP_F32 ? t | static_cast<int>(code) : t | FDP_GEMM_SPLIT_K, t,
+      const auto r = linear_fwd_call(X, W, b, static_cast<int>(X.numel() / K), t | (static_cast<int>(code) & (t == FDP_F32 ? ~0 : FDP_GEMM_SPLIT_K | FDP_PAD_16BIT)), t,
                                      in_out ? FDP_IN_OUT : FDP_OUT_IN);
       check_status(r.first, "fdp_linear_fwd");
       return r.second;

@@ -138,6 +138,9 @@ struct TcPlan {
   // three or six bf16 products
   int planes;
   size_t split_g_bytes, split_x_bytes;
+  // 16-bit inputs of any width: copies with padded rows, in the same place, of the operands that need one
+  bool pad;
+  size_t pad_g_bytes, pad_x_bytes;
 };
 TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo);
 // fp32 [rows, n] -> bf16 [rows, planes, n rounded up to 8]: high parts, then what is left of them, ...; row r is
@@ -146,7 +149,8 @@ struct SplitJob { const void* src; void* dst; size_t rows; int n; const float* f
 int tc_split(const SplitJob* jobs, int njobs, int planes, int* zero_status, cudaStream_t s);
 // With pl.planes > 1, G and X are the split matrices and dt is FDP_BF16.
 int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int B, int T, int n_in,
-             int n_out, int dt, const TcPlan& pl, cudaStream_t s, float* keep = nullptr, int layout = FDP_OUT_IN);
+             int n_out, int dt, const TcPlan& pl, cudaStream_t s, float* keep = nullptr, int layout = FDP_OUT_IN,
+             int pitch_g = 0, int pitch_x = 0);
 // Gs[r,:] = factors[r / T] * G[r,:]
 int tc_prescale(const void* G, const float* factors, void* Gs, int B, int T, int n_out, int dt,
                 cudaStream_t s);
@@ -171,7 +175,7 @@ int tc_weighted_sum(const float* keep, const TcFactorSource& fs, void* dW, int B
 // otherwise Gs is G itself and c_b is applied per sample in the epilogue.  planes > 1: G and X are split.
 int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, float* split_ws,
                      void* dW, int* dev_status, int B, int T, int n_in, int n_out, int dt, int out_dt,
-                     int layout, float inv_div, NoiseKey nk, cudaStream_t s, int planes = 1);
+                     int layout, float inv_div, NoiseKey nk, cudaStream_t s, int planes = 1, bool chained = false, int pitch_g = 0, int pitch_x = 0);
 // test aid: one warp waits `limit_cycles` on a barrier nobody arrives on and reports the timeout
 int tc_wait_selftest(int* status, long long limit_cycles, cudaStream_t s);
 // Where a product [rows, K] x [K, N] of `products` bf16 products may park the parts of a K split: what the plan needs, 0
@@ -193,8 +197,13 @@ size_t tc_gemm6_w_bytes(int K, int N);
 int tc_gemm6(const void* A3, const void* W3, const void* bias, void* Y, int* dev_status, int rows, int K, int N,
              int out_dt, bool w_kn, cudaStream_t s, const GemmPark& park);
 int tc_fwd(const void* X, const void* W, const void* bias, void* Y, int* dev_status, int rows, int n_in,
-           int n_out, int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park);
+           int n_out, int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park, int pitch_x = 0, int pitch_w = 0);
 int tc_dgrad(const void* G, const void* W, void* dX, int* dev_status, int rows, int n_in, int n_out,
-             int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park);
+             int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park, int pitch_g = 0, int pitch_w = 0);
+// the same for 16-bit operands of any width from 64 on, given as copies with rows of tc_pitch(n) elements where n is no
+// multiple of 8 (tc_split with planes 0; tc_pad_bytes each)
+bool tc_pad_gemm_ok(int rows, int N, int K, int dt);
+size_t tc_pad_bytes(size_t rows, int n);
+int tc_pitch(int n);
 
 }  // namespace fdp

@@ -53,15 +53,17 @@ constexpr int MAX_SMS = 148;           // workers the split-K parking area is si
 // EPI_SPLIT6_*: the same with bf16 thirds and six products.
 // EPI_KEEP: one sample's product tile squared and summed, and kept in HBM for weighted_sum_kernel (the SPLIT_SUMSQ
 // ones keep it too when TcArgs::keep is set).
+// EPI_CHAIN_SUMSQ: the same for 16-bit operands whose norms came from FMA kernels before: an accumulator runs for one K
+// stage only, as with split operands (one for all of a sample's stages drifts: 768 rows 6.8e-7, 4000 3.8e-6).
 enum { EPI_STORE = 0, EPI_SUMSQ = 1, EPI_GRAM = 2, EPI_STORE_SCALED = 3, EPI_SPLIT_SCALED = 4, EPI_SPLIT_STORE = 5,
-       EPI_SPLIT_SUMSQ = 6, EPI_SPLIT6_SCALED = 7, EPI_SPLIT6_SUMSQ = 8, EPI_KEEP = 9, EPI_SPLIT6_STORE = 10 };
+       EPI_SPLIT_SUMSQ = 6, EPI_SPLIT6_SCALED = 7, EPI_SPLIT6_SUMSQ = 8, EPI_KEEP = 9, EPI_SPLIT6_STORE = 10, EPI_CHAIN_SUMSQ = 11 };
 __host__ __device__ constexpr bool epi_chained(int epi) { return epi >= EPI_STORE_SCALED && epi != EPI_KEEP; }
 // bf16 parts of an operand
 __host__ __device__ constexpr int epi_planes(int epi) {
-  return epi == EPI_SPLIT6_SCALED || epi == EPI_SPLIT6_SUMSQ || epi == EPI_SPLIT6_STORE ? 3 : epi_chained(epi) && epi != EPI_STORE_SCALED ? 2 : 1;
+  return epi == EPI_SPLIT6_SCALED || epi == EPI_SPLIT6_SUMSQ || epi == EPI_SPLIT6_STORE ? 3 : epi_chained(epi) && epi != EPI_STORE_SCALED && epi != EPI_CHAIN_SUMSQ ? 2 : 1;
 }
 __host__ __device__ constexpr bool epi_scaled(int epi) { return epi == EPI_STORE_SCALED || epi == EPI_SPLIT_SCALED || epi == EPI_SPLIT6_SCALED; }
-__host__ __device__ constexpr bool epi_sumsq(int epi) { return epi == EPI_SPLIT_SUMSQ || epi == EPI_SPLIT6_SUMSQ; }
+__host__ __device__ constexpr bool epi_sumsq(int epi) { return epi == EPI_SPLIT_SUMSQ || epi == EPI_SPLIT6_SUMSQ || epi == EPI_CHAIN_SUMSQ; }
 __host__ __device__ constexpr bool epi_stores(int epi) { return epi == EPI_STORE || epi_scaled(epi) || epi == EPI_SPLIT_STORE || epi == EPI_SPLIT6_STORE; }
 // eight epilogue warps (two per TMEM lane quarter, 128 columns each) for the store epilogues, four for the norms
 __host__ __device__ constexpr int epi_warps_for(int epi) { return (epi == EPI_STORE || epi == EPI_KEEP || epi_chained(epi)) ? 8 : 4; }
@@ -94,6 +96,7 @@ struct TcArgs {
   // At B=16, T=1024, 1024->3072 that took 0.19 ms against 0.10 ms with the separate launch: the
   // sums then sit on the critical path of a few warps instead of spreading over the whole GPU.)
   int units_full, split;
+  int park_whole;       // host side: the tiles from units_full on are parked even with split = 1
   // store GEMMs without a K split: the tiles from units_full on are cut into `cut` column parts (1 or 2)
   int cut;
   float* split_ws;
@@ -128,7 +131,7 @@ struct TcArgs {
   int m_group;
   // the output cannot be written by the copy engine (row pitch or base not a multiple of 16 bytes)
   int direct_out;
-  float* keep;          // EPI_KEEP, EPI_SPLIT*_SUMSQ (may be null there): the product tiles, [tile][CTA of the pair][box]
+  float* keep;          // EPI_KEEP, EPI_*_SUMSQ (may be null there): the product tiles, [tile][CTA of the pair][box]
 };
 
 // ---- PTX wrappers (mbarrier helpers live in fdp_async.cuh) --------------------------------------------
@@ -927,7 +930,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (args.bias != nullptr && n < args.N) add_bias32(args, n, w);
             if (args.nk.std != 0.f && m < args.M && n < args.N)
               add_noise32(args.nk, static_cast<size_t>(m) * args.ld_out + n, w);
-            store_out32(args, box, &tmOut, w, c4, n0 + col0, m0 + quarter * 32, lane);
+            if (args.direct_out) store_rows32(args, box, w, n, m0 + quarter * 32, lane, false);
+            else store_out32(args, box, &tmOut, w, c4, n0 + col0, m0 + quarter * 32, lane);
           }
         }
         continue;
@@ -1194,7 +1198,36 @@ __global__ void __launch_bounds__(256) split_kernel(const SplitRun j0, const Spl
   }
 }
 
-// ---- the same for G, with the bias gradient's statistics taken from the pass (grid and partials of gstats_kernel) ---
+// ---- 16-bit operands whose rows are no multiple of 16 bytes: copies with padded rows (zeros), one or two in a launch --
+// HBM-bound: one read, one write.  Eight elements a thread; a row's elements sit at any even address, so they are read
+// as words where the columns are even in number and one by one otherwise (the lines come from L1).
+__global__ void __launch_bounds__(256) pad_kernel(const SplitRun j0, const SplitRun j1, unsigned first, int* zero_status) {
+  pdl_trigger();
+  if (zero_status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *zero_status = 0;
+  const bool second = blockIdx.x >= first;
+  const SplitRun& j = second ? j1 : j0;
+  const unsigned block = second ? blockIdx.x - first : blockIdx.x, blocks = second ? gridDim.x - first : first;
+  const uint16_t* src = reinterpret_cast<const uint16_t*>(j.src);
+  for (unsigned i = block * 256u + threadIdx.x; i < j.nvec; i += blocks * 256u) {
+    const unsigned row = i / j.vec_per_row, cv = i - row * j.vec_per_row;
+    const int c0 = static_cast<int>(cv) * 8;
+    const uint16_t* p = src + static_cast<size_t>(row) * j.n + c0;
+    uint32_t w[4];
+    if (j.vec) {      // an even number of columns, 4-byte aligned
+#pragma unroll
+      for (int e = 0; e < 4; ++e) w[e] = c0 + 2 * e < j.n ? __ldg(reinterpret_cast<const uint32_t*>(p) + e) : 0u;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t lo = c0 + 2 * e < j.n ? __ldg(p + 2 * e) : 0u, hi = c0 + 2 * e + 1 < j.n ? __ldg(p + 2 * e + 1) : 0u;
+        w[e] = lo | (hi << 16);
+      }
+    }
+    j.dst[i] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+// ---- the split of G, with the bias gradient's statistics taken from the pass (grid and partials of gstats_kernel) ---
 // In a whole backward G is split once for both products, and the column sums and sums of squares cost no read of
 // their own: 8192 x 3072 fp32, G 33 + 33 + 23 us (two splits and the statistics) as separate passes, one pass here.
 template <int PLANES>
@@ -1273,12 +1306,13 @@ EncodeTiledFn encode_fn() {
 }
 
 // 2-D map over a row-major [rows, cols] matrix of 16-bit elements, 128-byte swizzle, zero fill
+// (rows of `pitch` elements, 0: as many as there are columns)
 bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t box_cols,
-              uint32_t box_rows, int dt) {
+              uint32_t box_rows, int dt, uint64_t pitch = 0) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return false;
   const cuuint64_t dims[2] = {cols, rows};
-  const cuuint64_t strides[1] = {cols * 2};
+  const cuuint64_t strides[1] = {(pitch != 0 ? pitch : cols) * 2};
   const cuuint32_t box[2] = {box_cols, box_rows};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = fn(m, dt == FDP_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
@@ -1289,11 +1323,12 @@ bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, ui
 }
 
 // [B * T, cols] as (column, row of the sample, sample), for K ranges that run over the rows: boxes of 64 x BK
-bool make_rows_map(CUtensorMap* m, const void* base, int B, uint64_t T, uint64_t cols, int dt) {
+bool make_rows_map(CUtensorMap* m, const void* base, int B, uint64_t T, uint64_t cols, int dt, uint64_t pitch = 0) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return false;
   const cuuint64_t dims[3] = {cols, T, static_cast<cuuint64_t>(B)};
-  const cuuint64_t strides[2] = {cols * 2, cols * 2 * T};
+  if (pitch == 0) pitch = cols;
+  const cuuint64_t strides[2] = {pitch * 2, pitch * 2 * T};
   const cuuint32_t box[3] = {64, BK, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = fn(m, dt == FDP_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
@@ -1384,7 +1419,7 @@ int launch(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& a2, co
   la.sticky = sticky_status_slot();
   const int total = la.batch * la.tiles_per_batch;
   if (la.cut != 2) la.cut = 1;
-  if (la.split <= 1) { la.split = 1; if (la.cut == 1) la.units_full = total; }
+  if (la.split <= 1) { la.split = 1; if (la.cut == 1 && !la.park_whole) la.units_full = total; }
   int units = la.units_full + (total - la.units_full) * la.split * la.cut;
   const int workers = launch_sms() / CTAS;   // CTAs, or CTA pairs
   const int grid = CTAS * (units < workers ? units : workers);
@@ -1570,55 +1605,110 @@ static int most_product_tiles(int n_in, int n_out) {
 static size_t keep_bytes(int B, int n_in, int n_out) {
   return static_cast<size_t>(B) * most_product_tiles(n_in, n_out) * ctas_per_tile() * BM * BN * sizeof(float);
 }
-// Whether keeping the per-sample products beats the plan `p` that contracts twice, by estimates in us of both.  Fitted to
-// 36 shapes, B 1 to 64, T 64 to 4096, widths 64 to 11008, both sides timed (within 10 % but for the smallest); they part
-// where B n_in n_out fp32 elements written and read cost what a norm pass costs: 8 x 1024 rows 1024 -> 3072 bf16 70 us
-// kept, 82 contracted twice; 12 x 500, 1024 -> 4096 94 / 80; 16 x 512, 4096 -> 4096 539 / 331; 4 x 2048, 4096 -> 11008
-// 690 / 735; fp32 (three products) 8 x 1024, 1024 -> 3072 182 / 270.
-// The SM count is a constant here: the workspace query and the launch must pick the same plan.
+// ---- estimates in us by which weight-gradient plans are chosen -----------------------------------------------------
+// Fitted to 36 shapes, B 1 to 64, T 64 to 4096, widths 64 to 11008, every side timed (within 10 % but for the smallest).
+// The SM count is a constant: the workspace query and the launch must pick the same plan.
+namespace {
+constexpr int PLAN_PAIRS = MAX_SMS / 2;
+double rounds(long long units, int on) { return static_cast<double>((units + on - 1) / on); }
+// every sample's product once, kept, and their weighted sum
+double keep_us(int B, int T, int n_in, int n_out, int planes) {
+  constexpr double STAGE[3] = {0.38, 1.22, 2.9}, FIXED[3] = {1.8, 2.2, 2.2}, LEAST[3] = {3.5, 5.0, 5.0};
+  const double r = ceil_div(T, BK) * STAGE[planes - 1] + FIXED[planes - 1], least = LEAST[planes - 1];
+  return 9.5 + rounds(static_cast<long long>(B) * most_product_tiles(n_in, n_out), PLAN_PAIRS) * (r > least ? r : least) +
+         4.0 * n_in * n_out * (B + 1.0) / 6.4e6;
+}
+// a norm pass over product tiles or Gram blocks
+double norm_us(int B, int T, int n_in, int n_out, int planes, int algo) {
+  const int stages = ceil_div(T, BK);
+  if (planes > 1) {
+    constexpr double STAGE[3] = {0.0, 1.05, 2.45}, FIXED[3] = {0.0, 0.5, 1.5};
+    return 6.0 + rounds(static_cast<long long>(B) * most_product_tiles(n_in, n_out), PLAN_PAIRS) * (stages * STAGE[planes - 1] + FIXED[planes - 1]);
+  }
+  if (algo == FDP_NORM_DIRECT)
+    return 4.0 + rounds(static_cast<long long>(B) * ceil_div(n_out, BM) * ceil_div(n_in, BN), MAX_SMS) * (stages * 0.42 + 1.0);
+  return 4.0 + rounds(static_cast<long long>(B) * gram_tiles(T), MAX_SMS) * ((ceil_div(n_in, BK) + ceil_div(n_out, BK)) * 0.40 + 1.0);
+}
+// the clipped sum as one contraction, factors per sample in the epilogue (`scaled`) or in a copy of G
+double sum_us(int B, int T, int n_in, int n_out, int planes, bool scaled) {
+  constexpr double STAGE[3] = {0.40, 1.2, 2.2};
+  const int tiles = most_product_tiles(n_in, n_out);
+  const int k = scaled ? B * ceil_div(T, BK) : static_cast<int>((static_cast<long long>(B) * T + BK - 1) / BK);
+  const int split = plan_tail_split(tiles, k, PLAN_PAIRS, planes == 3 ? 6 : planes == 2 ? 3 : 1);
+  const int rem = tiles <= PLAN_PAIRS ? tiles : tiles % PLAN_PAIRS;
+  const double waves = (tiles - rem) / PLAN_PAIRS + rounds(static_cast<long long>(rem) * split, PLAN_PAIRS) / split;
+  double us = 6.0 + waves * (k * STAGE[planes - 1] + (scaled && planes == 1 ? 0.5 * B : 0.0));
+  if (split > 1) us += 4.0 + 0.04 * rem * split;
+  if (!scaled) us += 4.5 + 4.0 * B * T * n_out / 5e6;
+  return us;
+}
+// norms of short samples by the T x T blocks of simt_norm_gram_small, one block a sample: 4 x 10 rows, 7400 + 72 columns
+// 129 us, 46 x 27, 6272 + 176 309, 2 x 40, 7248 + 256 391, 2 x 3, 6848 + 123 105
+double small_norm_us(int B, int T, int cols) {
+  if (T == 1) return 4.0;
+  const double waves = B > 400 ? B / 400.0 : 1.0;
+  return 3.0 + waves * cols * (0.015 + T * T / 31000.0);
+}
+// the clipped sum on FMA kernels: 42 rows 1472 -> 2496 34 us, 40 rows 7400 -> 72 20, 17 rows 6904 -> 2308 64
+double fma_sum_us(long long rows, int n_in, int n_out) {
+  const double waves = static_cast<double>(ceil_div(n_in, 64)) * ceil_div(n_out, 64) / MAX_SMS;
+  return 5.0 + rows * 0.14 * (waves > 1.0 ? waves : 1.0);
+}
+}  // namespace
+
+// Whether keeping the per-sample products beats the plan `p` that contracts twice.  They part where B n_in n_out fp32
+// elements written and read cost what a norm pass costs: 8 x 1024 rows 1024 -> 3072 bf16 70 us kept, 82 contracted twice;
+// 12 x 500, 1024 -> 4096 94 / 80; 16 x 512, 4096 -> 4096 539 / 331; fp32 (three products) 8 x 1024, 1024 -> 3072 182 / 270.
 static bool keep_wins(int B, int T, int n_in, int n_out, const TcPlan& p) {
   if (keep_bytes(B, n_in, n_out) > KEEP_LIMIT) return false;
   // 16-bit samples of few rows leave faster than they can be written (64 x 128 rows, 1024 -> 1024: 101 us kept, 47; 48 x 64,
   // 768 -> 3072: 160 / 53); only calls of a few launches gain there (5 x 92, 512 -> 512: 12.6 / 18.6), which the host bounds.
-  if (p.planes == 1 && T < 256) return false;
-  const int i = p.planes - 1, workers = MAX_SMS / 2;
-  const int tiles = most_product_tiles(n_in, n_out), stages = ceil_div(T, BK);
-  const auto rounds = [](long long units, int on) { return static_cast<double>((units + on - 1) / on); };
-  const double elements = static_cast<double>(n_in) * n_out, launch = 6.0;
-  const double product_rounds = rounds(static_cast<long long>(B) * tiles, workers);
-  constexpr double KEEP_STAGE[3] = {0.38, 1.22, 2.9}, KEEP_FIXED[3] = {1.8, 2.2, 2.2}, KEEP_LEAST[3] = {3.5, 5.0, 5.0};
-  const double round = stages * KEEP_STAGE[i] + KEEP_FIXED[i];
-  const double keep = launch + product_rounds * (round > KEEP_LEAST[i] ? round : KEEP_LEAST[i]) + 3.5 + 4.0 * elements * (B + 1) / 6.4e6;
-
-  double norm;
-  if (p.planes > 1) {
-    constexpr double STAGE[3] = {0.0, 1.05, 2.45}, FIXED[3] = {0.0, 0.5, 1.5};
-    norm = launch + product_rounds * (stages * STAGE[i] + FIXED[i]);
-  } else if (p.algo == FDP_NORM_DIRECT) {
-    norm = 4.0 + rounds(static_cast<long long>(B) * ceil_div(n_out, BM) * ceil_div(n_in, BN), MAX_SMS) * (stages * 0.42 + 1.0);
-  } else {
-    norm = 4.0 + rounds(static_cast<long long>(B) * gram_tiles(T), MAX_SMS) * ((ceil_div(n_in, BK) + ceil_div(n_out, BK)) * 0.40 + 1.0);
-  }
-  const int k = p.scaled_epilogue ? B * stages : ceil_div(B * T, BK);
-  const int split = plan_tail_split(tiles, k, workers, p.planes == 3 ? 6 : p.planes == 2 ? 3 : 1);
-  const int rem = tiles <= workers ? tiles : tiles % workers;
-  const double waves = (tiles - rem) / workers + rounds(static_cast<long long>(rem) * split, workers) / split;
-  constexpr double SUM_STAGE[3] = {0.40, 1.2, 2.2};
-  double sum = launch + waves * (k * SUM_STAGE[i] + (p.scaled_epilogue && p.planes == 1 ? 0.5 * B : 0.0));
-  if (split > 1) sum += 4.0 + 0.04 * rem * split;
-  if (!p.scaled_epilogue) sum += 4.5 + 4.0 * B * T * n_out / 5e6;
+  if (p.planes == 1 && !p.pad && T < 256) return false;
   // Six products are to be no further from float64 than before: a K split cuts the chain of a long sample's sum, which
   // keeping does not (one sample of 2816 rows 1.8e-7 against 0.9e-7 in four parts).
-  if (p.planes == 3 && stages > 16 && B < split) return false;
+  const int stages = ceil_div(T, BK);
+  if (p.planes == 3 && stages > 16 && B < plan_tail_split(most_product_tiles(n_in, n_out), B * stages, PLAN_PAIRS, 6)) return false;
   // (fp32 calls hold the parts of both operands already: a tenth has to be gained for more)
-  return keep < (p.planes > 1 ? 0.9 : 0.97) * (norm + sum);
+  return keep_us(B, T, n_in, n_out, p.planes) < (p.planes > 1 ? 0.9 : 0.97) * (norm_us(B, T, n_in, n_out, p.planes, p.algo) +
+                                                                             sum_us(B, T, n_in, n_out, p.planes, p.scaled_epilogue));
+}
+
+// Turns `p` into a plan that keeps the products.  With split fp32 operands never in less than the parking area: a call that
+// is short of memory gives way where it did before.
+static void plan_keep(TcPlan& p, int B, int n_in, int n_out) {
+  p.ok = true; p.keep = true; p.short_seq = false; p.scaled_epilogue = false; p.algo = FDP_NORM_DIRECT;
+  p.nparts = most_product_tiles(n_in, n_out) * ctas_per_tile() * epi_warps_for(EPI_KEEP);
+  p.split_bytes = keep_bytes(B, n_in, n_out);
+  if (p.planes > 1 && p.split_bytes < split_ws_bytes()) p.split_bytes = split_ws_bytes();
+  p.ws_bytes = p.split_bytes + p.split_g_bytes + p.split_x_bytes + p.pad_g_bytes + p.pad_x_bytes;
+}
+
+// Short samples (T < SHORT_SEQ): `p` has norms by T x T blocks and a pre-scaled contraction, or nothing (p.ok unset: the FMA
+// kernels).  Both are slow for few samples of wide layers, one block a sample: instead the product form of longer samples,
+// their one K stage filled up with zeros, kept or contracted twice, where that is expected to take less.  3 x 44 rows,
+// 1024 -> 3072 bf16: 266 us, now 14; 40 x 20, 1000 -> 1000 fp32 85 / 58; 64 x 16, 1024 -> 1024 bf16 47 / 41; 1000 x 30,
+// 768 -> 768 stays (282).
+static void plan_short(TcPlan& p, int B, int T, int n_in, int n_out) {
+  const double before = small_norm_us(B, T, n_in + n_out) + 2.0 +
+                        (p.ok ? sum_us(B, T, n_in, n_out, p.planes, false) : fma_sum_us(static_cast<long long>(B) * T, n_in, n_out));
+  const double kept = keep_bytes(B, n_in, n_out) <= KEEP_LIMIT ? keep_us(B, T, n_in, n_out, p.planes) : 1e30;
+  const double twice = norm_us(B, T, n_in, n_out, p.planes, FDP_NORM_DIRECT) + sum_us(B, T, n_in, n_out, p.planes, true);
+  if ((kept < twice ? kept : twice) > 0.9 * before) return;
+  if (kept < twice) { plan_keep(p, B, n_in, n_out); return; }
+  p.ok = true; p.short_seq = false; p.scaled_epilogue = true; p.algo = FDP_NORM_DIRECT;
+  p.nparts = p.planes > 1 || p.pad ? most_product_tiles(n_in, n_out) * ctas_per_tile() * epi_warps_for(EPI_STORE_SCALED)
+                                   : 4 * ceil_div(n_out, BM) * ceil_div(n_in, BN);
+  p.split_bytes = split_ws_bytes();
+  p.ws_bytes = p.split_bytes + p.split_g_bytes + p.split_x_bytes + p.pad_g_bytes + p.pad_x_bytes;
 }
 
 TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
   TcPlan p; p.ok = false; p.algo = FDP_NORM_DIRECT; p.ws_bytes = 0; p.nparts = 0; p.scaled_epilogue = false;
   p.short_seq = false; p.any_align = false; p.keep = false; p.split_bytes = 0;
   p.planes = 1; p.split_g_bytes = p.split_x_bytes = 0;
+  p.pad = false; p.pad_g_bytes = p.pad_x_bytes = 0;
   const bool fp32_tensor = (norm_algo & FDP_FP32_TENSOR) != 0, fp32_wide = (norm_algo & FDP_FP32_WIDE) != 0;
+  const bool may_pad = (norm_algo & FDP_PAD_16BIT) != 0;
   const bool may_keep = (norm_algo & (FDP_KEEP_PRODUCTS | FDP_NORM_MASK)) == (FDP_KEEP_PRODUCTS | FDP_NORM_AUTO);
   norm_algo &= FDP_NORM_MASK;
   if (dt == FDP_F32) {
@@ -1630,8 +1720,9 @@ TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
     // more than a few K stages: it is handed to the epilogue warps, which add it to registers with
     // round-to-nearest (chain_stages).  The clip factors are applied there per sample (or, for short
     // sequences, in fp32 before the split: a pre-scaled bf16 copy would round c_b * G).
+    const bool wide = fp32_wide && wide_ok(B, T, n_in, n_out, norm_algo);
     if (fp32_tensor && three_products_ok(T, n_in, n_out)) p.planes = 2;
-    else if (fp32_wide && wide_ok(B, T, n_in, n_out, norm_algo)) p.planes = 3;
+    else if (wide || (fp32_wide && may_keep && T < SHORT_SEQ && n_in >= 64 && n_out >= 64)) p.planes = 3;
     else return p;
     p.any_align = p.planes == 3;
     p.split_g_bytes = align256(static_cast<size_t>(B) * T * pitch8(n_out) * 2 * p.planes);
@@ -1639,7 +1730,9 @@ TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
     p.split_bytes = split_ws_bytes();
     p.ws_bytes = p.split_bytes + p.split_g_bytes + p.split_x_bytes;
     if (T < SHORT_SEQ) {
-      p.ok = true; p.algo = FDP_NORM_GRAM; p.short_seq = true; p.nparts = 1;
+      p.algo = FDP_NORM_GRAM; p.short_seq = true; p.nparts = 1;
+      p.ok = wide;
+      if (may_keep) plan_short(p, B, T, n_in, n_out);
       return p;
     }
     // always the product form, accumulated in short chains (tc_norms); the Gram form needs both T x T tiles
@@ -1648,25 +1741,30 @@ TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
     const int ctas = ctas_per_tile();
     p.ok = true; p.algo = FDP_NORM_DIRECT; p.scaled_epilogue = true;
     p.nparts = ceil_div(n_out, BM * ctas) * ceil_div(n_in, BN) * ctas * epi_warps_for(EPI_STORE_SCALED);
-    if (may_keep && keep_wins(B, T, n_in, n_out, p)) {
-      p.keep = true; p.scaled_epilogue = false;
-      p.nparts = most_product_tiles(n_in, n_out) * ctas_per_tile() * epi_warps_for(EPI_KEEP);
-      // never less than the parking area: a call that is short of memory gives way where it did before
-      const size_t kept = keep_bytes(B, n_in, n_out);
-      if (kept > p.split_bytes) p.split_bytes = kept;
-      p.ws_bytes = p.split_bytes + p.split_g_bytes + p.split_x_bytes;
-    }
+    if (may_keep && keep_wins(B, T, n_in, n_out, p)) plan_keep(p, B, n_in, n_out);
     return p;
   }
   if (dt != FDP_BF16 && dt != FDP_F16) return p;
-  if (n_in % 8 != 0 || n_out % 8 != 0 || n_in < 128 || n_out < 128) return p;
+  if (n_in % 8 != 0 || n_out % 8 != 0 || n_in < 128 || n_out < 128) {
+    // Any width from 64 on with FDP_PAD_16BIT: operands whose rows (or pointers) are no multiple of 16 bytes are copied.
+    // The FMA kernels that these shapes ran on apply the factors in fp32 and add in short chains, so G is never pre-scaled
+    // here and no accumulator runs for more than a stage.  Whole weight gradients, error of dW and of the norms against
+    // float64: 30 x 768 rows 5952 -> 64 bf16 5124 us, 2.7e-6, 7e-8 before, now 85 us, 1.3e-7, 1.0e-7; 16 x 1024, 1023 -> 3071
+    // 10168 / 220 us; 64 x 256, 65 -> 66 2063 / 28; 3 x 300, 129 -> 1001 fp16 144 / 15; 2 x 64, 64 -> 64 30 / 9.
+    if (!may_pad || n_in < 64 || n_out < 64) return p;
+    p.pad = true; p.any_align = true;
+    p.pad_g_bytes = align256(static_cast<size_t>(B) * T * pitch8(n_out) * 2);
+    p.pad_x_bytes = align256(static_cast<size_t>(B) * T * pitch8(n_in) * 2);
+  }
   if (T < SHORT_SEQ) {
     // short sequences: the norms come from the small Gram kernel (one partial per sample); the
     // clipped sum is still one GEMM with K = B*T over the pre-scaled copy of G, if K is worth a tile
-    if (norm_algo == FDP_NORM_DIRECT || static_cast<long long>(B) * T < 4 * BK) return p;
-    p.ok = true; p.algo = FDP_NORM_GRAM; p.short_seq = true; p.nparts = 1;
+    if (norm_algo == FDP_NORM_DIRECT) return p;
+    p.algo = FDP_NORM_GRAM; p.short_seq = true; p.nparts = 1;
+    p.ok = !p.pad && static_cast<long long>(B) * T >= 4 * BK;
     p.split_bytes = split_ws_bytes();
     p.ws_bytes = p.split_bytes + align256(static_cast<size_t>(B) * T * n_out * 2);
+    if (may_keep) plan_short(p, B, T, n_in, n_out);
     return p;
   }
   // Cost of the two norm algorithms in K stages on the critical path: both kernels deal equal work
@@ -1681,6 +1779,7 @@ TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
                       (ceil_div(n_in, BK) + ceil_div(n_out, BK) + UNIT_FIXED_STAGES);
   int algo = norm_algo;
   if (algo == FDP_NORM_AUTO) algo = direct <= gram ? FDP_NORM_DIRECT : FDP_NORM_GRAM;
+  if (p.pad) algo = FDP_NORM_DIRECT;      // in chains of one stage, over the tiles of the clipped sum
   p.ok = true;
   p.algo = algo;
   // clip factors applied in the GEMM epilogue (no scaled copy of G) when a sample's main loop is long
@@ -1689,17 +1788,14 @@ TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
   // 400 multiply-adds' time each.  FDP_WGRAD_PRESCALE=1 forces the pre-scale pass (for A/B measurements)
   static const bool force_prescale = [] { const char* e = getenv("FDP_WGRAD_PRESCALE"); return e && e[0] == '1'; }();
   const long long pad = static_cast<long long>(ceil_div(T, BK)) * BK - T;
-  p.scaled_epilogue = !force_prescale && T >= 256 && pad * n_in <= 400ll * T;
+  p.scaled_epilogue = p.pad || (!force_prescale && T >= 256 && pad * n_in <= 400ll * T);
   // one partial per work unit and epilogue warp
-  p.nparts = 4 * ((algo == FDP_NORM_DIRECT) ? ceil_div(n_out, BM) * ceil_div(n_in, BN) : gram_tiles(T));
+  p.nparts = p.pad ? most_product_tiles(n_in, n_out) * ctas_per_tile() * epi_warps_for(EPI_CHAIN_SUMSQ)
+                   : 4 * ((algo == FDP_NORM_DIRECT) ? ceil_div(n_out, BM) * ceil_div(n_in, BN) : gram_tiles(T));
   // the parked accumulators of the split-K tail, then (pre-scale path only) the c_b-scaled copy of G
   p.split_bytes = split_ws_bytes();
-  p.ws_bytes = p.split_bytes + (p.scaled_epilogue ? 0 : align256(static_cast<size_t>(B) * T * n_out * 2));
-  if (may_keep && keep_wins(B, T, n_in, n_out, p)) {
-    p.keep = true; p.scaled_epilogue = false; p.algo = FDP_NORM_DIRECT;
-    p.nparts = most_product_tiles(n_in, n_out) * ctas_per_tile() * epi_warps_for(EPI_KEEP);
-    p.split_bytes = p.ws_bytes = keep_bytes(B, n_in, n_out);
-  }
+  p.ws_bytes = p.split_bytes + (p.scaled_epilogue ? 0 : align256(static_cast<size_t>(B) * T * n_out * 2)) + p.pad_g_bytes + p.pad_x_bytes;
+  if (may_keep && keep_wins(B, T, n_in, n_out, p)) plan_keep(p, B, n_in, n_out);
   return p;
 }
 
@@ -1716,11 +1812,12 @@ int tc_split(const SplitJob* jobs, int njobs, int planes, int* zero_status, cuda
       const unsigned vpr = pitch8(j.n) / 8;
       const size_t most = (1u << 31) / vpr, left = j.rows - done[k], nr = left < most ? left : most;
       if (nr < j.rows && j.factors != nullptr) return FDP_ERR_SHAPE;   // (factors come with short sequences only)
-      r[k].src = static_cast<const float*>(j.src) + done[k] * j.n;
-      r[k].dst = static_cast<uint4*>(j.dst) + done[k] * vpr * planes;
+      // (planes 0: a 16-bit operand is copied as it is)
+      r[k].src = reinterpret_cast<const float*>(static_cast<const char*>(j.src) + done[k] * j.n * (planes > 0 ? 4 : 2));
+      r[k].dst = static_cast<uint4*>(j.dst) + done[k] * vpr * (planes > 0 ? planes : 1);
       r[k].factors = j.factors; r[k].T = j.T; r[k].n = j.n; r[k].vec_per_row = vpr;
       r[k].nvec = static_cast<unsigned>(nr * vpr);
-      r[k].vec = j.n % 4 == 0 && aligned16(r[k].src);
+      r[k].vec = planes > 0 ? j.n % 4 == 0 && aligned16(r[k].src) : j.n % 2 == 0 && reinterpret_cast<uintptr_t>(r[k].src) % 4 == 0;
       blocks[k] = (r[k].nvec + 255) / 256;
       done[k] += nr;
     }
@@ -1732,7 +1829,8 @@ int tc_split(const SplitJob* jobs, int njobs, int planes, int* zero_status, cuda
       for (int k = 0; k < 2; ++k)
         if (blocks[k] > 0) blocks[k] = static_cast<unsigned>(blocks[k] * static_cast<unsigned long long>(cap) / all) + 1;
     }
-    if (planes == 2) split_kernel<2><<<blocks[0] + blocks[1], 256, 0, s>>>(r[0], r[1], blocks[0], zero_status);
+    if (planes == 0) pad_kernel<<<blocks[0] + blocks[1], 256, 0, s>>>(r[0], r[1], blocks[0], zero_status);
+    else if (planes == 2) split_kernel<2><<<blocks[0] + blocks[1], 256, 0, s>>>(r[0], r[1], blocks[0], zero_status);
     else split_kernel<3><<<blocks[0] + blocks[1], 256, 0, s>>>(r[0], r[1], blocks[0], zero_status);
     note_launch();
   }
@@ -1751,19 +1849,20 @@ int tc_split_stats(const void* G, void* dst, float* colsum_part, float* sq_part,
 }
 
 int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int B, int T, int n_in,
-             int n_out, int dt, const TcPlan& pl, cudaStream_t s, float* keep, int layout) {
+             int n_out, int dt, const TcPlan& pl, cudaStream_t s, float* keep, int layout, int pitch_g, int pitch_x) {
   const uint64_t rows = static_cast<uint64_t>(B) * T;
   CUtensorMap a, b, a2, b2;
   TcArgs args{};
   args.batch = B; args.batch_rows = T; args.partials = partials; args.status = dev_status; args.T = T;
   args.zero_status = 1;      // the norm pass is the first launch of a weight-gradient call
-  if (pl.planes > 1) {
-    // fp32 inputs: the per-sample products G_b^T X_b themselves, on the tiles and CTA pairs of the
+  if (pl.planes > 1 || pl.pad) {
+    // fp32 inputs (and 16-bit ones that come as padded copies): the per-sample products G_b^T X_b themselves, on the tiles and CTA pairs of the
     // clipped-sum GEMM, handed to the epilogue every few K stages and summed there in registers; a
     // unit is (sample, tile) and ends with the sum of its squares instead of a store
-    const int po = pitch8(n_out), pi = pitch8(n_in);
+    const int po = pl.pad ? n_out : pitch8(n_out), pi = pl.pad ? n_in : pitch8(n_in);
     const bool oi = keep == nullptr || layout == FDP_OUT_IN;     // products that are kept have the output's orientation
-    if (!make_rows_map(oi ? &a : &b, G, B, T, pl.planes * po, dt) || !make_rows_map(oi ? &b : &a, X, B, T, pl.planes * pi, dt))
+    if (!make_rows_map(oi ? &a : &b, G, B, T, pl.planes * po, dt, pitch_g) ||
+        !make_rows_map(oi ? &b : &a, X, B, T, pl.planes * pi, dt, pitch_x))
       return FDP_ERR_LAUNCH;
     const int ctas = ctas_per_tile();
     args.M = oi ? n_out : n_in; args.N = oi ? n_in : n_out; args.ld_out = args.N;
@@ -1772,10 +1871,13 @@ int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int
     args.k_stages = ceil_div(T, BK);
     args.plane_a = oi ? po : pi; args.plane_b = oi ? pi : po;
     args.idesc = make_idesc(dt, true, true, ctas);
-    args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = chain_stages(args.seg_stages, pl.planes);
+    args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = pl.pad ? 1 : chain_stages(args.seg_stages, pl.planes);
     args.scale = 1.0f; args.nk = NoiseKey{};
-    args.zero_status = 0; args.dependent = 1;      // follows the split kernel, which has cleared the status word
+    if (!pl.pad) { args.zero_status = 0; args.dependent = 1; }     // follows the split kernel, which has cleared the status word
     args.keep = keep;
+    if (pl.pad)
+      return ctas == 2 ? launch<true, true, EPI_CHAIN_SUMSQ, 2>(a, b, a, b, a, args, s)
+                       : launch<true, true, EPI_CHAIN_SUMSQ, 1>(a, b, a, b, a, args, s);
     if (pl.planes == 3)
       return ctas == 2 ? launch<true, true, EPI_SPLIT6_SUMSQ, 2>(a, b, a, b, a, args, s)
                        : launch<true, true, EPI_SPLIT6_SUMSQ, 1>(a, b, a, b, a, args, s);
@@ -1786,7 +1888,7 @@ int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int
     const bool oi = layout == FDP_OUT_IN;
     const int ctas = ctas_per_tile();
     args.M = oi ? n_out : n_in; args.N = oi ? n_in : n_out;
-    if (!make_rows_map(oi ? &a : &b, G, B, T, n_out, dt) || !make_rows_map(oi ? &b : &a, X, B, T, n_in, dt))
+    if (!make_rows_map(oi ? &a : &b, G, B, T, n_out, dt, pitch_g) || !make_rows_map(oi ? &b : &a, X, B, T, n_in, dt, pitch_x))
       return FDP_ERR_LAUNCH;
     args.keep = keep;
     args.tiles_m = ceil_div(args.M, BM * ctas); args.tiles_n = ceil_div(args.N, BN);
@@ -1797,7 +1899,7 @@ int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int
                      : launch<true, true, EPI_KEEP, 1>(a, b, a, b, a, args, s);
   }
   if (pl.algo == FDP_NORM_DIRECT) {
-    if (!make_rows_map(&a, G, B, T, n_out, dt) || !make_rows_map(&b, X, B, T, n_in, dt)) return FDP_ERR_LAUNCH;
+    if (!make_rows_map(&a, G, B, T, n_out, dt, pitch_g) || !make_rows_map(&b, X, B, T, n_in, dt, pitch_x)) return FDP_ERR_LAUNCH;
     args.M = n_out; args.N = n_in;
     args.tiles_m = ceil_div(n_out, BM); args.tiles_n = ceil_div(n_in, BN);
     args.tiles_per_batch = args.tiles_m * args.tiles_n;
@@ -1806,8 +1908,8 @@ int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int
     return launch<true, true, EPI_SUMSQ>(a, b, a, b, a, args, s);
   }
   // A and B boxes are both 128 rows: a B stage is filled by two independent copies
-  if (!make_map(&a, G, rows, n_out, BK, BM, dt) || !make_map(&b, G, rows, n_out, BK, BN / 2, dt) ||
-      !make_map(&a2, X, rows, n_in, BK, BM, dt) || !make_map(&b2, X, rows, n_in, BK, BN / 2, dt))
+  if (!make_map(&a, G, rows, n_out, BK, BM, dt, pitch_g) || !make_map(&b, G, rows, n_out, BK, BN / 2, dt, pitch_g) ||
+      !make_map(&a2, X, rows, n_in, BK, BM, dt, pitch_x) || !make_map(&b2, X, rows, n_in, BK, BN / 2, dt, pitch_x))
     return FDP_ERR_LAUNCH;
   args.M = T; args.N = T;
   args.gram_nb = ceil_div(T, BM);
@@ -1851,7 +1953,7 @@ bool tc_fused_factors_ok(int B) { return B <= MAX_SMEM_FACTORS; }
 
 int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, float* split_ws,
                      void* dW, int* dev_status, int B, int T, int n_in, int n_out, int dt, int out_dt,
-                     int layout, float inv_div, NoiseKey nk, cudaStream_t s, int planes) {
+                     int layout, float inv_div, NoiseKey nk, cudaStream_t s, int planes, bool chained, int pitch_g, int pitch_x) {
   const uint64_t rows = static_cast<uint64_t>(B) * T;
   const bool scaled = fs != nullptr;  // Gs is then the unscaled G
   if (planes == 2 && !scaled) return FDP_ERR_ARG;
@@ -1860,14 +1962,14 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
   const int segs = scaled ? B : 1;
   const uint64_t seg_rows = scaled ? T : rows;
   const int po = planes > 1 ? pitch8(n_out) : n_out, pi = planes > 1 ? pitch8(n_in) : n_in;
-  if (!make_rows_map(&mg, Gs, segs, seg_rows, static_cast<uint64_t>(planes) * po, dt) ||
-      !make_rows_map(&mx, X, segs, seg_rows, static_cast<uint64_t>(planes) * pi, dt)) return FDP_ERR_LAUNCH;
+  if (!make_rows_map(&mg, Gs, segs, seg_rows, static_cast<uint64_t>(planes) * po, dt, pitch_g) ||
+      !make_rows_map(&mx, X, segs, seg_rows, static_cast<uint64_t>(planes) * pi, dt, pitch_x)) return FDP_ERR_LAUNCH;
   TcArgs args{};
   args.batch = 1; args.batch_rows = 0; args.status = dev_status;
   args.dependent = 1;             // always follows a kernel of the same call (norm pass, clip factors or pre-scale)
   args.seg_stages = static_cast<int>((seg_rows + BK - 1) / BK);
   args.k_stages = segs * args.seg_stages;
-  args.sub_stages = planes > 1 ? chain_stages(args.seg_stages, planes) : args.seg_stages;
+  args.sub_stages = planes > 1 ? chain_stages(args.seg_stages, planes) : chained ? 1 : args.seg_stages;
   args.out = dW; args.out_dt = out_dt; args.scale = inv_div; args.nk = nk;
   // [out,in]: A = G (M = n_out), B = X (N = n_in); [in,out]: operands swap roles, no transpose pass
   const bool oi = (layout == FDP_OUT_IN);
@@ -1894,8 +1996,13 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
   // workspace and summed in fixed order by the fix-up kernel (deterministic, no waits)
   const int total = args.tiles_per_batch, workers = launch_sms() / ctas;
   const int split = plan_tail_split(total, args.k_stages, workers, planes == 3 ? 6 : planes == 2 ? 3 : 1);
+  // Noise in the epilogue hides behind the main loop of the next tile or of the tile itself (drawn sample by sample).  Where
+  // there is one round of short main loops, tiles go to the fix-up kernel as they are and it draws the noise on all SMs:
+  // 2 x 71 rows, 576 -> 1472 fp16, 12 tiles of 3 stages, whole call 41 us, parked 21; 5 x 92, 512 -> 512 42 / 20.
+  const bool park_whole = nk.std != 0.f && split <= 1 && total <= workers && args.k_stages * (planes == 3 ? 6 : planes == 2 ? 3 : 1) <= 96;
   int n_split_tiles = 0;
-  if (split > 1) {
+  if (split > 1 || park_whole) {
+    args.park_whole = park_whole;
     n_split_tiles = total <= workers ? total : total % workers;
     args.split = split;
     args.units_full = total - n_split_tiles;
@@ -1913,7 +2020,7 @@ int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, fl
   else if (scaled) st = ctas == 2 ? FDP_WGRAD_LAUNCH(EPI_STORE_SCALED, 2) : FDP_WGRAD_LAUNCH(EPI_STORE_SCALED, 1);
   else st = ctas == 2 ? FDP_WGRAD_LAUNCH(EPI_STORE, 2) : FDP_WGRAD_LAUNCH(EPI_STORE, 1);
 #undef FDP_WGRAD_LAUNCH
-  if (st != FDP_OK || split <= 1) return st;
+  if (st != FDP_OK || n_split_tiles == 0) return st;
   // the scaled epilogue parks its parts already divided by the batch
   dim3 grid(BM * ctas * BN / (256 * 4), n_split_tiles);
   launch_dependent(splitk_fixup_kernel, grid, dim3(256), 0, s, args.split_ws, args.units_full, split, BM * ctas, args.M,
@@ -1929,12 +2036,21 @@ bool tc_dgrad_ok(int rows, int n_in, int n_out, int dt) {
 
 size_t tc_gemm_park_bytes(int rows, int K, int N, int products) { return gemm_park_bytes(rows, K, N, products); }
 
+// 16-bit products of any width from 64 on.  Operands whose rows are no multiple of 16 bytes are copied first
+// (tc_pad_bytes each).
+bool tc_pad_gemm_ok(int rows, int N, int K, int dt) { return (dt == FDP_BF16 || dt == FDP_F16) && rows >= 128 && N >= 64 && K >= 64; }
+size_t tc_pad_bytes(size_t rows, int n) { return n % 8 == 0 ? 0 : align256(rows * pitch8(n) * 2); }
+int tc_pitch(int n) { return pitch8(n); }
+
 int tc_dgrad(const void* G, const void* W, void* dX, int* dev_status, int rows, int n_in, int n_out,
-             int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park) {
+             int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park, int pitch_g, int pitch_w) {
   CUtensorMap mg, mw, mo;
   const int ctas = ctas_per_tile();
-  if (!make_map(&mg, G, rows, n_out, BK, BM, dt) || !make_out_map(&mo, dX, rows, n_in, out_dt)) return FDP_ERR_LAUNCH;
   TcArgs args{};
+  args.direct_out = !aligned16(dX) || n_in * dtype_size(out_dt) % 16 != 0;
+  if (!make_map(&mg, G, rows, n_out, BK, BM, dt, pitch_g)) return FDP_ERR_LAUNCH;
+  if (args.direct_out) mo = mg;   // not used
+  else if (!make_out_map(&mo, dX, rows, n_in, out_dt)) return FDP_ERR_LAUNCH;
   args.batch = 1; args.batch_rows = 0; args.status = dev_status; args.zero_status = 1;
   args.M = rows; args.N = n_in; args.ld_out = n_in;
   args.tiles_m = ceil_div(rows, BM * ctas); args.tiles_n = ceil_div(n_in, BN);
@@ -1945,7 +2061,7 @@ int tc_dgrad(const void* G, const void* W, void* dX, int* dev_status, int rows, 
   args.n_fastest = 1;
   args.out = dX; args.out_dt = out_dt; args.scale = 1.0f; args.nk = NoiseKey{};
   if (w_layout == FDP_OUT_IN) {  // W [n_out, n_in]: rows are K, N contiguous
-    if (!make_map(&mw, W, n_out, n_in, 64, BK, dt)) return FDP_ERR_LAUNCH;
+    if (!make_map(&mw, W, n_out, n_in, 64, BK, dt, pitch_w)) return FDP_ERR_LAUNCH;
     args.idesc = make_idesc(dt, false, true, ctas);
     CUtensorMap mp = mg;
     if (!plan_last_round(args, ctas, make_idesc(dt, false, true, ctas, BN / 2), n_out, 1, park, &mp)) return FDP_ERR_LAUNCH;
@@ -1954,7 +2070,7 @@ int tc_dgrad(const void* G, const void* W, void* dX, int* dev_status, int rows, 
   }
   // W [n_in, n_out]: K contiguous; a CTA of a pair loads half of the 256 B rows
   CUtensorMap mh;
-  if (!make_map(&mw, W, n_in, n_out, BK, BN / ctas, dt) || !make_map(&mh, W, n_in, n_out, BK, BN / 2 / ctas, dt)) return FDP_ERR_LAUNCH;
+  if (!make_map(&mw, W, n_in, n_out, BK, BN / ctas, dt, pitch_w) || !make_map(&mh, W, n_in, n_out, BK, BN / 2 / ctas, dt, pitch_w)) return FDP_ERR_LAUNCH;
   args.idesc = make_idesc(dt, false, false, ctas);
   CUtensorMap mp = mg;
   if (!plan_last_round(args, ctas, make_idesc(dt, false, false, ctas, BN / 2), n_out, 1, park, &mp)) return FDP_ERR_LAUNCH;
@@ -1965,11 +2081,14 @@ int tc_dgrad(const void* G, const void* W, void* dX, int* dev_status, int rows, 
 // forward: A = X [rows, n_in] K-major; B = W, K-major for [n_out, n_in] (Linear), MN-major for
 // [n_in, n_out] (Conv1D); bias added in the epilogue
 int tc_fwd(const void* X, const void* W, const void* bias, void* Y, int* dev_status, int rows, int n_in,
-           int n_out, int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park) {
+           int n_out, int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park, int pitch_x, int pitch_w) {
   CUtensorMap mx, mw, mo;
   const int ctas = ctas_per_tile();
-  if (!make_map(&mx, X, rows, n_in, BK, BM, dt) || !make_out_map(&mo, Y, rows, n_out, out_dt)) return FDP_ERR_LAUNCH;
   TcArgs args{};
+  args.direct_out = !aligned16(Y) || n_out * dtype_size(out_dt) % 16 != 0;
+  if (!make_map(&mx, X, rows, n_in, BK, BM, dt, pitch_x)) return FDP_ERR_LAUNCH;
+  if (args.direct_out) mo = mx;   // not used
+  else if (!make_out_map(&mo, Y, rows, n_out, out_dt)) return FDP_ERR_LAUNCH;
   args.batch = 1; args.batch_rows = 0; args.status = dev_status; args.zero_status = 1;
   args.M = rows; args.N = n_out; args.ld_out = n_out;
   args.tiles_m = ceil_div(rows, BM * ctas); args.tiles_n = ceil_div(n_out, BN);
@@ -1980,14 +2099,14 @@ int tc_fwd(const void* X, const void* W, const void* bias, void* Y, int* dev_sta
   args.bias = bias; args.bias_dt = dt; args.bias_vec = aligned16(bias);
   if (w_layout == FDP_OUT_IN) {  // W [n_out, n_in]: K contiguous
     CUtensorMap mh;
-    if (!make_map(&mw, W, n_out, n_in, BK, BN / ctas, dt) || !make_map(&mh, W, n_out, n_in, BK, BN / 2 / ctas, dt)) return FDP_ERR_LAUNCH;
+    if (!make_map(&mw, W, n_out, n_in, BK, BN / ctas, dt, pitch_w) || !make_map(&mh, W, n_out, n_in, BK, BN / 2 / ctas, dt, pitch_w)) return FDP_ERR_LAUNCH;
     args.idesc = make_idesc(dt, false, false, ctas);
     CUtensorMap mp = mx;
     if (!plan_last_round(args, ctas, make_idesc(dt, false, false, ctas, BN / 2), n_in, 1, park, &mp)) return FDP_ERR_LAUNCH;
     return gemm_fixup(ctas == 2 ? launch<false, false, EPI_STORE, 2>(mx, mw, mp, mh, mo, args, s)
                                 : launch<false, false, EPI_STORE, 1>(mx, mw, mp, mh, mo, args, s), args, ctas, s);
   }
-  if (!make_map(&mw, W, n_in, n_out, 64, BK, dt)) return FDP_ERR_LAUNCH;  // W [n_in, n_out]: N contiguous
+  if (!make_map(&mw, W, n_in, n_out, 64, BK, dt, pitch_w)) return FDP_ERR_LAUNCH;  // W [n_in, n_out]: N contiguous
   args.idesc = make_idesc(dt, false, true, ctas);
   CUtensorMap mp = mx;
   if (!plan_last_round(args, ctas, make_idesc(dt, false, true, ctas, BN / 2), n_in, 1, park, &mp)) return FDP_ERR_LAUNCH;

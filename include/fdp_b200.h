@@ -33,7 +33,7 @@ extern "C" {
  * 3: fdp_dp_params.step_device (appended; earlier fields keep their offsets); FDP_FP32_TENSOR also
  *    accepted in the dtype of fdp_linear_dgrad / fdp_linear_fwd.
  * 4: FDP_FP32_WIDE, fdp_linear_bwd.
- * 5: FDP_KEEP_PRODUCTS, FDP_FP32_WIDE_GEMM, FDP_GEMM_SPLIT_K. */
+ * 5: FDP_KEEP_PRODUCTS, FDP_FP32_WIDE_GEMM, FDP_GEMM_SPLIT_K, FDP_PAD_16BIT. */
 #define FDP_ABI_VERSION 5
 
 typedef void* fdp_stream_t; /* a cudaStream_t */
@@ -96,7 +96,11 @@ enum fdp_norm_algo {
   FDP_FP32_WIDE_GEMM = 128,
   /* flag, OR-ed into the same arguments, of any dtype: products of few output tiles and a long contraction are cut along
    * it.  The workspace then has room for the fp32 parts, at most 38.8 MB; in a smaller one the product runs uncut. */
-  FDP_GEMM_SPLIT_K = 256
+  FDP_GEMM_SPLIT_K = 256,
+  /* flag, OR-ed into the same arguments and into fdp_linear_wgrad's norm_algo: 16-bit inputs of widths from 64 on, of any
+   * number, run on the tensor cores (without it: multiples of 8 from 128 on).  Operands whose rows are no multiple of 16
+   * bytes are copied into the workspace with padded rows; operands and outputs need no alignment. */
+  FDP_PAD_16BIT = 512
 };
 
 /* DP hyper-parameters of one call.  C / clamp_value are the arguments of

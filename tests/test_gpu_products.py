@@ -157,3 +157,73 @@ def test_products_cut_along_k(ops, rows, K, N, dtype, layout):  # noqa: F811
     for b in (None, _randn(N, seed=3, dtype=dtype)):
         bd = 0.0 if b is None else b.double()
         _close_to_sum(ops.linear_forward(X, W, b, layout), want + bd, absum + (0.0 if b is None else bd.abs()), k, UNIT[dtype])
+
+
+# 16-bit layers of any width from 64 on: rows that are no multiple of 16 bytes (one operand, both, none), samples that end
+# inside a K stage, samples of one row, kept and contracted twice, noise with rows of any pitch
+@pytest.mark.parametrize("B,T,n_in,n_out", [(2, 64, 64, 64), (3, 300, 129, 1001), (5, 100, 72, 65), (1, 700, 333, 128), (40, 65, 130, 66),
+                                            (9, 20, 515, 70), (3, 2, 600, 100), (30, 1, 257, 129), (200, 1, 100, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("layout", ["out_in", "in_out"])
+def test_16bit_of_any_width(ops, B, T, n_in, n_out, dtype, layout):  # noqa: F811
+    X, G = _randn(B, T, n_in, seed=1, dtype=dtype), _randn(B, T, n_out, seed=2, dtype=dtype, scale=1e-2)
+    G[0] *= 30.0
+    per = torch.einsum("bto,bti->boi", G.double(), X.double())
+    want_n = per.flatten(1).norm(dim=1)
+    f = (1.0 / (want_n + 1e-10)).clamp(max=1.0)
+    want = (f.view(-1, 1, 1) * per).sum(0) / B
+    absum = (f.view(-1, 1, 1) * torch.einsum("bto,bti->boi", G.double().abs(), X.double().abs())).sum(0) / B
+    if layout == "in_out":
+        want, absum = want.t(), absum.t()
+    k = 4 + B * (T + 63) // 64 + 8        # four steps an accumulator, one addition a stage, the factor's roundings
+    for out_dtype in (torch.float32, dtype):
+        dW, norms, _ = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, layout=layout, out_dtype=out_dtype, return_norms=True)
+        # below 2^-14 an fp16 result is rounded to a multiple of 2^-24, whatever its size
+        steps = absum + (2.0 ** -25 / (k * 2.0 ** -23) if out_dtype == torch.float16 else 0.0)
+        _close_to_sum(dW, want, steps, k, UNIT[out_dtype])
+        assert float(((norms.double() - want_n) / want_n).abs().max()) < 8 * 2.0 ** -23
+    zero = torch.zeros_like(G)
+    spec = ops.NoiseSpec(std=0.5, seed=77, param_id=3, step=2)
+    kw = dict(layout=layout, noise=spec, out_dtype=torch.float32)
+    stream = ops.dp_linear_weight_grad(X.float(), zero.float(), 1.0, 1.0, fp32_tensor=False, **kw)      # of the FMA kernels
+    assert torch.equal(ops.dp_linear_weight_grad(X, zero, 1.0, 1.0, **kw), stream)
+
+
+@pytest.mark.parametrize("rows,K,N", [(128, 65, 64), (130, 64, 65), (300, 999, 130), (1000, 515, 1001), (129, 72, 100), (256, 4001, 72)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("layout", ["out_in", "in_out"])
+def test_16bit_products_of_any_width(ops, rows, K, N, dtype, layout):  # noqa: F811
+    X, W = _randn(rows, K, seed=1, dtype=dtype), _randn(*((N, K) if layout == "out_in" else (K, N)), seed=2, dtype=dtype, scale=0.1)
+    G, b = _randn(rows, N, seed=3, dtype=dtype), _randn(N, seed=4, dtype=dtype)
+    w = W if layout == "in_out" else W.t()
+    _close_to_sum(ops.linear_forward(X, W, b, layout), X.double() @ w.double() + b.double(),
+                  X.double().abs() @ w.double().abs() + b.double().abs(), K / 16 + 8, UNIT[dtype])
+    for out_dtype in (dtype, torch.float32):
+        _close_to_sum(ops.linear_input_grad(G, W, layout, out_dtype=out_dtype), G.double() @ w.double().t(),
+                      G.double().abs() @ w.double().abs().t(), N / 16 + 8, UNIT[out_dtype])
+
+
+# few short samples of wide layers in the product form, every type; and noise drawn by the fix-up kernel
+@pytest.mark.parametrize("B,T,n_in,n_out,dtype", [(3, 44, 1024, 512, torch.bfloat16), (2, 2, 2000, 136, torch.float16), (8, 63, 256, 768, torch.bfloat16),
+                                                  (3, 44, 512, 260, torch.float32), (2, 3, 1200, 123, torch.float32), (40, 20, 300, 300, torch.float32)])
+def test_short_samples_as_products(ops, B, T, n_in, n_out, dtype):  # noqa: F811
+    X, G = _randn(B, T, n_in, seed=1, dtype=dtype), _randn(B, T, n_out, seed=2, dtype=dtype, scale=1e-1)
+    G[0] *= 30.0
+    per = torch.einsum("bto,bti->boi", G.double(), X.double())
+    want_n = per.flatten(1).norm(dim=1)
+    f = (1.0 / (want_n + 1e-10)).clamp(max=1.0)
+    dW, norms, _ = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, out_dtype=torch.float32, return_norms=True)
+    absum = (f.view(-1, 1, 1) * torch.einsum("bto,bti->boi", G.double().abs(), X.double().abs())).sum(0) / B
+    _close_to_sum(dW, (f.view(-1, 1, 1) * per).sum(0) / B, absum, 4 + B + 8, 2.0 ** -23)
+    assert float(((norms.double() - want_n) / want_n).abs().max()) < 8 * 2.0 ** -23
+
+
+@pytest.mark.parametrize("B,T,n_in,n_out", [(2, 71, 576, 1472), (5, 92, 512, 512), (300, 4, 256, 136)])
+def test_noise_of_short_contractions(ops, B, T, n_in, n_out):  # noqa: F811
+    X, G = _randn(B, T, n_in, seed=1, dtype=torch.bfloat16), _randn(B, T, n_out, seed=2, dtype=torch.bfloat16, scale=1e-2)
+    spec = ops.NoiseSpec(std=0.5, seed=77, param_id=3, step=2)
+    stream = ops.dp_linear_weight_grad(X.float(), torch.zeros_like(G).float(), 1.0, 1.0, fp32_tensor=False, noise=spec)
+    kw = dict(out_dtype=torch.float32)
+    assert torch.equal(ops.dp_linear_weight_grad(X, torch.zeros_like(G), 1.0, 1.0, noise=spec, **kw), stream)
+    plain, noisy = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, **kw), ops.dp_linear_weight_grad(X, G, 1.0, 1.0, noise=spec, **kw)
+    assert float((noisy - (plain + stream)).abs().max()) <= 2.0 ** -23 * float(noisy.abs().max())
