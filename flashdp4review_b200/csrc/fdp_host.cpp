@@ -90,6 +90,17 @@ void check_weight(const Tensor& W, int64_t k, int64_t n, bool k_rows, const Tens
   if (W.device() != like.device()) refuse("weight is on another device", W);
 }
 
+// parameters and statistics of a layer norm over the last dimension of `x`, and what has its shape (dy)
+void check_layernorm(const Tensor& x, const Tensor& w, const OptTensor& b, const OptTensor& mean, const OptTensor& rstd, const OptTensor& dy) {
+  if (x.dim() < 1) refuse("input has no last dimension", x);
+  const int64_t d = x.size(-1), rows = d > 0 ? x.numel() / d : 0;
+  if (w.device() != x.device() || (b.has_value() && b->device() != x.device())) refuse("layer norm: input and parameters are not on one device", w);
+  if (w.numel() != d || (b.has_value() && b->numel() != d)) refuse("layer norm: parameters do not fit the input's last dimension", w);
+  for (const OptTensor& t : {mean, rstd})
+    if (t.has_value() && (t->device() != x.device() || t->numel() != rows || t->scalar_type() != at::kFloat)) refuse("layer norm: statistics do not fit the input", *t);
+  if (dy.has_value() && (dy->device() != x.device() || dy->numel() != x.numel())) refuse("layer norm: grad_output does not fit the input", *dy);
+}
+
 void* ptr(const Tensor& t) { return t.data_ptr(); }
 void* ptr(const OptTensor& t) { return t.has_value() ? t->data_ptr() : nullptr; }
 fdp_stream_t stream(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
@@ -251,6 +262,7 @@ py::tuple linear_fwd(const Tensor& X, const Tensor& W, const OptTensor& bias, in
 
 struct LnFwd { int st; Tensor y, mean, rstd; };
 LnFwd layernorm_fwd_call(const Tensor& x, const Tensor& w, const Tensor& b, double eps, int rows, int dt, int pdt) {
+  check_layernorm(x, w, b, {}, {}, {});
   const c10::cuda::CUDAGuard guard(x.device());
   const Tensor y = new_tensor(x, x.sizes(), x.scalar_type());
   const Tensor mean = new_tensor(x, {rows}, at::kFloat), rstd = new_tensor(x, {rows}, at::kFloat);
@@ -270,6 +282,7 @@ py::tuple layernorm_fwd(const Tensor& x, const Tensor& w, const Tensor& b, doubl
 struct LnBwd { int st; OptTensor dx; Tensor dgamma; OptTensor dbeta, ng, nb; };
 LnBwd layernorm_bwd_call(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd, int B, int T,
                          int dt, int pdt, const fdp_dp_params& q, bool need_dx, bool need_dbeta, bool want_norms) {
+  check_layernorm(x, w, {}, mean, rstd, dy);
   const c10::cuda::CUDAGuard guard(x.device());
   const int d = static_cast<int>(x.size(-1));
   OptTensor dx, dbeta, ng, nb;

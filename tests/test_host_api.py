@@ -262,6 +262,31 @@ def test_operands_that_do_not_fit_are_refused_before_a_launch(monkeypatch, layou
             ops.linear_forward(X, W, bias, layout)
 
 
+def test_layernorm_operands_that_do_not_fit_are_refused_before_a_launch(monkeypatch):
+    """Parameters, statistics and upstream gradient of a layer norm go to the kernels as bare pointers too: a layer that
+    was never moved to the input's device, or another size, stops in the call layer, through the layers' nodes and
+    through the operators.  (On CPU tensors, as above; the other device is torch's meta device.)"""
+    from flashdp4review_b200 import _lib
+    from flashdp4review_b200.core import ops
+    monkeypatch.setattr(ops, "_require_cuda", lambda *tensors: None)
+    host = _lib.host()
+    x, w, b = torch.zeros(2, 3, 16), torch.ones(16), torch.zeros(16)
+    for fwd in (lambda *a: ops.layernorm_fwd_fused(*a, 1e-5), lambda *a: host.dp_layernorm(*a, None, 1e-5)):
+        for args in ((x, w.to("meta"), b), (x, w, b.to("meta")), (x.to("meta"), w, b)):
+            with pytest.raises(RuntimeError, match="not on one device"):
+                fwd(*args)
+        for args in ((x, torch.ones(15), b), (x, w, torch.zeros(8)), (x, torch.ones(17), torch.zeros(17))):
+            with pytest.raises(RuntimeError, match="parameters do not fit"):
+                fwd(*args)
+    mean, rstd = torch.zeros(6), torch.ones(6)
+    for args, refused in (((x, x, w.to("meta"), mean, rstd), "not on one device"), ((x, x, torch.ones(8), mean, rstd), "parameters do not fit"),
+                          ((x, x, w, mean.to("meta"), rstd), "statistics"), ((x, x, w, mean, torch.ones(5)), "statistics"),
+                          ((x, x, w, mean.double(), rstd), "statistics"), ((torch.zeros(2, 2, 16), x, w, mean, rstd), "grad_output"),
+                          ((x.to("meta"), x, w, mean, rstd), "grad_output")):
+        with pytest.raises(RuntimeError, match=refused):
+            ops.dp_layernorm_backward(*args, 1.0, 1.0)
+
+
 def test_partial_backward_takes_only_what_it_needs(no_launch):
     """Without the weight gradient (a frozen weight, a bias alone) the workspace of a whole backward is that of the
     remaining outputs, and the layer input stays out of the call: no cast, no copy."""
