@@ -1617,6 +1617,11 @@ static int most_product_tiles(int n_in, int n_out) {
   const int a = ceil_div(n_out, BM * ctas) * ceil_div(n_in, BN), b = ceil_div(n_in, BM * ctas) * ceil_div(n_out, BN);
   return a > b ? a : b;
 }
+// norm partials per sample of a product pass that keeps nothing: always in the orientation [out, in] (tc_norms)
+static int product_partials(int n_in, int n_out) {
+  const int ctas = ctas_per_tile();
+  return ceil_div(n_out, BM * ctas) * ceil_div(n_in, BN) * ctas * epi_warps_for(EPI_STORE_SCALED);
+}
 static size_t keep_bytes(int B, int n_in, int n_out) {
   return static_cast<size_t>(B) * most_product_tiles(n_in, n_out) * ctas_per_tile() * BM * BN * sizeof(float);
 }
@@ -1711,7 +1716,7 @@ static void plan_short(TcPlan& p, int B, int T, int n_in, int n_out) {
   if ((kept < twice ? kept : twice) > 0.9 * before) return;
   if (kept < twice) { plan_keep(p, B, n_in, n_out); return; }
   p.ok = true; p.short_seq = false; p.scaled_epilogue = true; p.algo = FDP_NORM_DIRECT;
-  p.nparts = p.planes > 1 || p.pad ? most_product_tiles(n_in, n_out) * ctas_per_tile() * epi_warps_for(EPI_STORE_SCALED)
+  p.nparts = p.planes > 1 || p.pad ? product_partials(n_in, n_out)
                                    : 4 * ceil_div(n_out, BM) * ceil_div(n_in, BN);
   p.split_bytes = split_ws_bytes();
   p.ws_bytes = p.split_bytes + p.split_g_bytes + p.split_x_bytes + p.pad_g_bytes + p.pad_x_bytes;
@@ -1753,9 +1758,8 @@ TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
     // always the product form, accumulated in short chains (tc_norms); the Gram form needs both T x T tiles
     // complete in TMEM before its epilogue can multiply them, i.e. one chain of 3 * (in + out) / 16
     // truncating additions.  The chained norm pass: tiles of the clipped-sum GEMM, eight epilogue warps per CTA
-    const int ctas = ctas_per_tile();
     p.ok = true; p.algo = FDP_NORM_DIRECT; p.scaled_epilogue = true;
-    p.nparts = ceil_div(n_out, BM * ctas) * ceil_div(n_in, BN) * ctas * epi_warps_for(EPI_STORE_SCALED);
+    p.nparts = product_partials(n_in, n_out);
     if (may_keep && keep_wins(B, T, n_in, n_out, p)) plan_keep(p, B, n_in, n_out);
     return p;
   }
@@ -1805,7 +1809,7 @@ TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
   const long long pad = static_cast<long long>(ceil_div(T, BK)) * BK - T;
   p.scaled_epilogue = p.pad || (!force_prescale && T >= 256 && pad * n_in <= 400ll * T);
   // one partial per work unit and epilogue warp
-  p.nparts = p.pad ? most_product_tiles(n_in, n_out) * ctas_per_tile() * epi_warps_for(EPI_CHAIN_SUMSQ)
+  p.nparts = p.pad ? product_partials(n_in, n_out)
                    : 4 * ((algo == FDP_NORM_DIRECT) ? ceil_div(n_out, BM) * ceil_div(n_in, BN) : gram_tiles(T));
   // the parked accumulators of the split-K tail, then (pre-scale path only) the c_b-scaled copy of G
   p.split_bytes = split_ws_bytes();

@@ -227,3 +227,45 @@ def test_noise_of_short_contractions(ops, B, T, n_in, n_out):  # noqa: F811
     assert torch.equal(ops.dp_linear_weight_grad(X, torch.zeros_like(G), 1.0, 1.0, noise=spec, **kw), stream)
     plain, noisy = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, **kw), ops.dp_linear_weight_grad(X, G, 1.0, 1.0, noise=spec, **kw)
     assert float((noisy - (plain + stream)).abs().max()) <= 2.0 ** -23 * float(noisy.abs().max())
+
+
+_SINGLE_CTA_CHILD = r"""
+import sys, torch
+sys.path.insert(0, %r)
+from flashdp4review_b200.core import ops
+worst = 0.0
+# padded 16-bit widths, samples of one K stage, fp32 parts: more tiles along the input's columns than along the output's, and
+# the reverse; enough samples that the products are not kept
+for (B, T, n_in, n_out, dtype) in [(200, 128, 520, 72, torch.bfloat16), (100, 128, 72, 520, torch.float16), (150, 100, 300, 65, torch.bfloat16),
+                                   (300, 20, 600, 100, torch.float16), (2, 50, 2000, 136, torch.bfloat16), (3, 40, 1400, 260, torch.float32),
+                                   (150, 70, 600, 72, torch.float32), (4, 300, 200, 648, torch.bfloat16)]:
+    gen = torch.Generator(device="cuda").manual_seed(B)
+    X = torch.randn(B, T, n_in, device="cuda", generator=gen).to(dtype)
+    G = (torch.randn(B, T, n_out, device="cuda", generator=gen) * torch.linspace(1e-3, 1e-1, B, device="cuda").view(B, 1, 1)).to(dtype)
+    per = torch.einsum("bto,bti->boi", G.double(), X.double())
+    n = per.flatten(1).norm(dim=1)
+    f = (1.0 / (n + 1e-10)).clamp(max=1.0)
+    want = (f.view(-1, 1, 1) * per).sum(0) / B
+    for layout in ("out_in", "in_out"):
+        dW, norms, factors = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, layout=layout, out_dtype=torch.float32, return_norms=True)
+        w = want if layout == "out_in" else want.t()
+        worst = max(worst, float(((norms.double() - n) / n).abs().max()), float(((factors.double() - f) / f).abs().max()),
+                    float((dW.double() - w).norm() / w.norm()) * 1e-3 if dtype != torch.float32 else float((dW.double() - w).norm() / w.norm()))
+torch.cuda.synchronize()
+print("WORST", worst)
+"""
+
+
+def test_single_cta_tiles_of_any_width():
+    """FDP_TC_CTAS=1 (tiles of 128 x 256, whose number depends on the orientation) on the plans for any width and for short
+    samples: norms and factors within the truncation of their chains (300 rows at most: 20 steps of half a unit), dW likewise or, where G is
+    rounded once more to 16 bits, within 2^-9."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _SINGLE_CTA_CHILD % root], env={**os.environ, "FDP_TC_CTAS": "1"},
+                       capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
+    worst = float(r.stdout.strip().split("WORST")[-1])
+    assert worst < 20 * 2.0 ** -23, worst
