@@ -347,43 +347,66 @@ __device__ __forceinline__ void store_out32(const TcArgs& args, uint32_t box, co
   if ((c4 & 1) == 1) box_send(box, map, col0 + 64 * (c4 >> 1), row, lane);
 }
 
-// 32 columns of an output that the copy engine cannot write: through the box all the same, then row by row, so
-// that an instruction writes 32 adjacent elements; eight rows at a time, or each row would wait for its own trip
-// through shared memory (16960 rows 79 -> 5597 fp32 229 us, now 207; 65502 rows 208 -> 494 fp16 95 / 81).  The noise is drawn per element here: a row pitch that is no multiple of four
-// puts an element group across rows.
-template <typename T>
-__device__ __forceinline__ void store_box_rows(const TcArgs& args, uint32_t box, int n, int row, int rows, int lane, bool noise) {
-  const size_t ld = static_cast<size_t>(args.ld_out);
-  const size_t idx = static_cast<size_t>(row) * ld + n + lane;
-  T* out = static_cast<T*>(args.out) + idx;
-  const bool in = n + lane < args.N;
-  for (int r0 = 0; r0 < rows; r0 += 8) {
-    float x[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k)      // (the box holds 32 rows, whatever the matrix has)
-      asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x[k])
-                   : "r"(box + (r0 + k) * 128 + (((lane >> 2) ^ k) << 4) + (lane & 3) * 4) : "memory");
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (in && r0 + k < rows) {
-        if (noise) x[k] += noise_at(args.nk, idx + (r0 + k) * ld);
-        out[(r0 + k) * ld] = from_f32<T>(x[k]);
-      }
-  }
-}
-__device__ __forceinline__ void store_rows32(const TcArgs& args, uint32_t box, const float v[32], int n, int row, int lane,
-                                             bool noise) {
-  box_wait(lane);       // a parked part may still be on its way out of the box
+// An epilogue warp's columns of an output that the copy engine cannot write: 32 at a time through the box all the same,
+// then row by row, so that an instruction writes 32 adjacent elements; eight rows at a time, or each row would wait for its
+// own trip through shared memory (16960 rows 79 -> 5597 fp32 229 us one by one, 175 now; 65502 rows 208 -> 494 fp16 95 / 60).  The noise
+// is drawn per element here: a row pitch that is no multiple of four puts an element group across rows.  All of this is
+// one loop, whose only part that depends on the registers' numbers is the filling of the box: unrolled over columns, types
+// and rows it held 96 copies of the noise generator, and a warp that skipped them waited for instructions all the way
+// (weight gradient of 39 x 21 rows, 5730 -> 1152 fp32, without noise 538 us, now 472, with it 773 / 555; 2 x 5, 642 -> 296 bf16 43 / 16).
+__device__ __forceinline__ void box_fill(uint32_t box, const float v[32], int lane) {
 #pragma unroll
   for (int j = 0; j < 8; ++j)
     box_put(box, lane, j, __float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]), __float_as_uint(v[4 * j + 2]),
             __float_as_uint(v[4 * j + 3]));
-  __syncwarp();
+}
+__device__ __forceinline__ float box_at(uint32_t box, int r, int lane) {
+  float x;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(box + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4) : "memory");
+  return x;
+}
+template <typename T>
+__device__ __forceinline__ void store_box_rows(T* out, size_t ld, uint32_t box, int rows, int lane, bool in) {
+#pragma unroll 1
+  for (int r0 = 0; r0 < rows; r0 += 8, out += 8 * ld) {
+    float x[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = box_at(box, r0 + k, lane);      // (the box holds 32 rows, whatever the matrix has)
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (in && r0 + k < rows) out[k * ld] = from_f32<T>(x[k]);
+  }
+}
+__device__ __forceinline__ void store_rows(const TcArgs& args, uint32_t box, const float v[128], int chunks, int n0, int row,
+                                           int lane, bool noise) {
   const int rows = min(BOX_ROWS, args.M - row);
-  if (args.out_dt == FDP_F32) store_box_rows<float>(args, box, n, row, rows, lane, noise);
-  else if (args.out_dt == FDP_BF16) store_box_rows<__nv_bfloat16>(args, box, n, row, rows, lane, noise);
-  else store_box_rows<__half>(args, box, n, row, rows, lane, noise);
-  __syncwarp();         // the box may be filled again
+  const size_t ld = static_cast<size_t>(args.ld_out);
+#pragma unroll 1
+  for (int c4 = 0; c4 < chunks && n0 + c4 * 32 < args.N; ++c4) {
+    box_wait(lane);       // a parked part may still be on its way out of the box
+    switch (c4) {
+      case 0: box_fill(box, v, lane); break;
+      case 1: box_fill(box, v + 32, lane); break;
+      case 2: box_fill(box, v + 64, lane); break;
+      default: box_fill(box, v + 96, lane); break;
+    }
+    __syncwarp();
+    const int n = n0 + c4 * 32 + lane;
+    const bool in = n < args.N;
+    const size_t idx = static_cast<size_t>(row) * ld + n;
+    if (noise) {
+#pragma unroll 2
+      for (int r = 0; r < rows; ++r)
+        if (in) store_as(args.out, args.out_dt, idx + r * ld, box_at(box, r, lane) + noise_at(args.nk, idx + r * ld));
+    } else if (args.out_dt == FDP_F32) {
+      store_box_rows(static_cast<float*>(args.out) + idx, ld, box, rows, lane, in);
+    } else if (args.out_dt == FDP_BF16) {
+      store_box_rows(static_cast<__nv_bfloat16*>(args.out) + idx, ld, box, rows, lane, in);
+    } else {
+      store_box_rows(static_cast<__half*>(args.out) + idx, ld, box, rows, lane, in);
+    }
+    __syncwarp();         // the box may be filled again
+  }
 }
 
 // accr[4g .. 4g+3] += z * f with g known only at run time: a switch keeps every index static, so
@@ -879,9 +902,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               if (narrow && c4 >= 2) break;
               const int n = n0 + chalf * warp_cols + c4 * 32;
               if ((EPI == EPI_SPLIT_STORE || EPI == EPI_SPLIT6_STORE) && args.bias != nullptr && n < args.N) add_bias32(args, n, accr + c4 * 32);
-              if (args.direct_out) store_rows32(args, box, accr + c4 * 32, n, m0 + quarter * 32, lane, epi_scaled(EPI) && args.nk.std != 0.f);
-              else store_out32(args, box, &tmOut, accr + c4 * 32, c4, n0 + chalf * warp_cols, m0 + quarter * 32, lane);
+              if (EPI == EPI_SPLIT_STORE || !args.direct_out) store_out32(args, box, &tmOut, accr + c4 * 32, c4, n0 + chalf * warp_cols, m0 + quarter * 32, lane);
             }
+            if (EPI != EPI_SPLIT_STORE && args.direct_out)       // (three products: rows and pointers of 16 bytes only)
+              store_rows(args, box, accr, narrow ? 2 : 4, n0 + chalf * warp_cols, m0 + quarter * 32, lane, epi_scaled(EPI) && args.nk.std != 0.f);
           }
         } else {
           // park this part (already divided by the batch) for the fix-up kernel
@@ -945,9 +969,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (args.bias != nullptr && n < args.N) add_bias32(args, n, w);
             if (args.nk.std != 0.f && m < args.M && n < args.N)
               add_noise32(args.nk, static_cast<size_t>(m) * args.ld_out + n, w);
-            if (args.direct_out) store_rows32(args, box, w, n, m0 + quarter * 32, lane, false);
-            else store_out32(args, box, &tmOut, w, c4, n0 + col0, m0 + quarter * 32, lane);
+            if (!args.direct_out) store_out32(args, box, &tmOut, w, c4, n0 + col0, m0 + quarter * 32, lane);
           }
+          if (args.direct_out) store_rows(args, box, v, narrow ? 2 : 4, n0 + col0, m0 + quarter * 32, lane, false);
         }
         continue;
       } else if (EPI == EPI_SUMSQ) {
