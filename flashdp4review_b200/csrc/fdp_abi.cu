@@ -509,7 +509,7 @@ int fdp_linear_dgrad(const void* G, const void* W, void* dX, int rows, int n_in,
     const bool oi = w_layout == FDP_OUT_IN;
     const PaddedOperands o = pad_operands(G, W, rows, n_out, oi ? n_out : n_in, oi ? n_in : n_out, workspace, s);
     if (o.st != FDP_OK) return o.st;
-    if ((st = tc_dgrad(o.A, o.W, dX, status, rows, n_in, n_out, dtype, out_dtype, w_layout, s, park, o.pitch_a, o.pitch_w)) != FDP_OK) return st;
+    if ((st = tc_dgrad(o.A, o.W, dX, status, rows, n_in, n_out, dtype, out_dtype, w_layout, s, park, o.pitch_a, o.pitch_w, out_dtype == FDP_F32)) != FDP_OK) return st;
   } else {
     FDP_CUDA_OK(cudaMemsetAsync(status, 0, sizeof(int), s));
     simt_dgrad(G, W, dX, rows, n_in, n_out, dtype, out_dtype, w_layout, s);
@@ -549,7 +549,7 @@ int fdp_linear_fwd(const void* X, const void* W, const void* bias, void* Y, int 
     const bool oi = w_layout == FDP_OUT_IN;
     const PaddedOperands o = pad_operands(X, W, rows, n_in, oi ? n_out : n_in, oi ? n_in : n_out, workspace, s);
     if (o.st != FDP_OK) return o.st;
-    if ((st = tc_fwd(o.A, o.W, bias, Y, status, rows, n_in, n_out, dtype, out_dtype, w_layout, s, park, o.pitch_a, o.pitch_w)) != FDP_OK) return st;
+    if ((st = tc_fwd(o.A, o.W, bias, Y, status, rows, n_in, n_out, dtype, out_dtype, w_layout, s, park, o.pitch_a, o.pitch_w, out_dtype == FDP_F32)) != FDP_OK) return st;
   } else {
     FDP_CUDA_OK(cudaMemsetAsync(status, 0, sizeof(int), s));
     simt_fwd(X, W, bias, Y, rows, n_in, n_out, dtype, out_dtype, w_layout, s);

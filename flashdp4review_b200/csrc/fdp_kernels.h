@@ -197,11 +197,13 @@ size_t tc_gemm6_w_bytes(int K, int N);
 int tc_gemm6(const void* A3, const void* W3, const void* bias, void* Y, int* dev_status, int rows, int K, int N,
              int out_dt, bool w_kn, cudaStream_t s, const GemmPark& park);
 int tc_fwd(const void* X, const void* W, const void* bias, void* Y, int* dev_status, int rows, int n_in,
-           int n_out, int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park, int pitch_x = 0, int pitch_w = 0);
+           int n_out, int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park, int pitch_x = 0, int pitch_w = 0,
+           bool chained = false);
 int tc_dgrad(const void* G, const void* W, void* dX, int* dev_status, int rows, int n_in, int n_out,
-             int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park, int pitch_g = 0, int pitch_w = 0);
+             int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park, int pitch_g = 0, int pitch_w = 0,
+             bool chained = false);
 // the same for 16-bit operands of any width from 64 on, given as copies with rows of tc_pitch(n) elements where n is no
-// multiple of 8 (tc_split with planes 0; tc_pad_bytes each)
+// multiple of 8 (tc_split with planes 0; tc_pad_bytes each); chained: an accumulator runs for one K stage only
 bool tc_pad_gemm_ok(int rows, int N, int K, int dt);
 size_t tc_pad_bytes(size_t rows, int n);
 int tc_pitch(int n);

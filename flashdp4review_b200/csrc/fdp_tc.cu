@@ -55,16 +55,20 @@ constexpr int MAX_SMS = 148;           // workers the split-K parking area is si
 // ones keep it too when TcArgs::keep is set).
 // EPI_CHAIN_SUMSQ: the same for 16-bit operands whose norms came from FMA kernels before: an accumulator runs for one K
 // stage only, as with split operands (one for all of a sample's stages drifts: 768 rows 6.8e-7, 4000 3.8e-6).
+// EPI_CHAIN_STORE: a plain 16-bit product with an fp32 output that FMA kernels computed before, in the same chains.
 enum { EPI_STORE = 0, EPI_SUMSQ = 1, EPI_GRAM = 2, EPI_STORE_SCALED = 3, EPI_SPLIT_SCALED = 4, EPI_SPLIT_STORE = 5,
-       EPI_SPLIT_SUMSQ = 6, EPI_SPLIT6_SCALED = 7, EPI_SPLIT6_SUMSQ = 8, EPI_KEEP = 9, EPI_SPLIT6_STORE = 10, EPI_CHAIN_SUMSQ = 11 };
+       EPI_SPLIT_SUMSQ = 6, EPI_SPLIT6_SCALED = 7, EPI_SPLIT6_SUMSQ = 8, EPI_KEEP = 9, EPI_SPLIT6_STORE = 10, EPI_CHAIN_SUMSQ = 11,
+       EPI_CHAIN_STORE = 12 };
 __host__ __device__ constexpr bool epi_chained(int epi) { return epi >= EPI_STORE_SCALED && epi != EPI_KEEP; }
 // bf16 parts of an operand
 __host__ __device__ constexpr int epi_planes(int epi) {
-  return epi == EPI_SPLIT6_SCALED || epi == EPI_SPLIT6_SUMSQ || epi == EPI_SPLIT6_STORE ? 3 : epi_chained(epi) && epi != EPI_STORE_SCALED && epi != EPI_CHAIN_SUMSQ ? 2 : 1;
+  return epi == EPI_SPLIT6_SCALED || epi == EPI_SPLIT6_SUMSQ || epi == EPI_SPLIT6_STORE ? 3 : epi == EPI_SPLIT_SCALED || epi == EPI_SPLIT_STORE || epi == EPI_SPLIT_SUMSQ ? 2 : 1;
 }
 __host__ __device__ constexpr bool epi_scaled(int epi) { return epi == EPI_STORE_SCALED || epi == EPI_SPLIT_SCALED || epi == EPI_SPLIT6_SCALED; }
 __host__ __device__ constexpr bool epi_sumsq(int epi) { return epi == EPI_SPLIT_SUMSQ || epi == EPI_SPLIT6_SUMSQ || epi == EPI_CHAIN_SUMSQ; }
-__host__ __device__ constexpr bool epi_stores(int epi) { return epi == EPI_STORE || epi_scaled(epi) || epi == EPI_SPLIT_STORE || epi == EPI_SPLIT6_STORE; }
+// plain products: bias, tiles cut along N
+__host__ __device__ constexpr bool epi_plain(int epi) { return epi == EPI_STORE || epi == EPI_SPLIT_STORE || epi == EPI_SPLIT6_STORE || epi == EPI_CHAIN_STORE; }
+__host__ __device__ constexpr bool epi_stores(int epi) { return epi_plain(epi) || epi_scaled(epi); }
 // eight epilogue warps (two per TMEM lane quarter, 128 columns each) for the store epilogues, four for the norms
 __host__ __device__ constexpr int epi_warps_for(int epi) { return (epi == EPI_STORE || epi == EPI_KEEP || epi_chained(epi)) ? 8 : 4; }
 constexpr int threads_for(int epi) { return 64 + 32 * epi_warps_for(epi); }
@@ -442,7 +446,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   constexpr int STG = A_BYTES + PLANES * B_BYTES;
   constexpr int BN_CTA = BN / CTAS;                      // B columns (rows if K-major) loaded by this CTA
   constexpr int EPI_WARPS = epi_warps_for(EPI);
-  constexpr bool CUTS = EPI == EPI_STORE || EPI == EPI_SPLIT_STORE || EPI == EPI_SPLIT6_STORE;   // may have units of half a tile's columns
+  constexpr bool CUTS = epi_plain(EPI);                  // may have units of half a tile's columns
   static_assert(NST * STG <= STAGES * STAGE_BYTES, "ring size");
   static_assert(CTAS == 1 || EPI_WARPS == 8, "pairs: eight epilogue warps");
   const uint32_t cta_rank = (CTAS == 2) ? cluster_ctarank() : 0u;
@@ -901,7 +905,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             for (int c4 = 0; c4 < 4; ++c4) {
               if (narrow && c4 >= 2) break;
               const int n = n0 + chalf * warp_cols + c4 * 32;
-              if ((EPI == EPI_SPLIT_STORE || EPI == EPI_SPLIT6_STORE) && args.bias != nullptr && n < args.N) add_bias32(args, n, accr + c4 * 32);
+              if (epi_plain(EPI) && args.bias != nullptr && n < args.N) add_bias32(args, n, accr + c4 * 32);
               if (EPI == EPI_SPLIT_STORE || !args.direct_out) store_out32(args, box, &tmOut, accr + c4 * 32, c4, n0 + chalf * warp_cols, m0 + quarter * 32, lane);
             }
             if (EPI != EPI_SPLIT_STORE && args.direct_out)       // (three products: rows and pointers of 16 bytes only)
@@ -2080,13 +2084,22 @@ bool tc_dgrad_ok(int rows, int n_in, int n_out, int dt) {
 size_t tc_gemm_park_bytes(int rows, int K, int N, int products) { return gemm_park_bytes(rows, K, N, products); }
 
 // 16-bit products of any width from 64 on.  Operands whose rows are no multiple of 16 bytes are copied first
-// (tc_pad_bytes each).
+// (tc_pad_bytes each).  With an fp32 output they took the place of FMA kernels and are to be no further from float64: chained, one
+// K stage an accumulator.  Error against float64 and time of FMA kernels / one accumulator for all of K / chained: 8192 rows
+// 3648 -> 64 bf16 5.7e-7 312 us / 3.9e-6 15.0 / 1.5e-7 25.0; 5376 rows 5919 -> 320 fp16 1.4e-6 1195 / 7.0e-6 65 / 2.1e-7 81; 1000 rows
+// 100 -> 65 6.3e-8 14.7 / 9.8e-8 10.8 / 6.5e-8 10.0.
 bool tc_pad_gemm_ok(int rows, int N, int K, int dt) { return (dt == FDP_BF16 || dt == FDP_F16) && rows >= 128 && N >= 64 && K >= 64; }
 size_t tc_pad_bytes(size_t rows, int n) { return n % 8 == 0 ? 0 : align256(rows * pitch8(n) * 2); }
 int tc_pitch(int n) { return pitch8(n); }
 
+template <bool A_MN, bool B_MN, int EPI>
+static int plain_launch(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& a2, const CUtensorMap& b2, const CUtensorMap& o, int ctas,
+                        const TcArgs& args, cudaStream_t s) {
+  return ctas == 2 ? launch<A_MN, B_MN, EPI, 2>(a, b, a2, b2, o, args, s) : launch<A_MN, B_MN, EPI, 1>(a, b, a2, b2, o, args, s);
+}
+
 int tc_dgrad(const void* G, const void* W, void* dX, int* dev_status, int rows, int n_in, int n_out,
-             int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park, int pitch_g, int pitch_w) {
+             int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park, int pitch_g, int pitch_w, bool chained) {
   CUtensorMap mg, mw, mo;
   const int ctas = ctas_per_tile();
   TcArgs args{};
@@ -2103,13 +2116,13 @@ int tc_dgrad(const void* G, const void* W, void* dX, int* dev_status, int rows, 
   // band of G and the whole of W stay in L2 (walking along M first would re-read G per n-tile)
   args.n_fastest = 1;
   args.out = dX; args.out_dt = out_dt; args.scale = 1.0f; args.nk = NoiseKey{};
+  args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = 1;      // (of a chained product)
   if (w_layout == FDP_OUT_IN) {  // W [n_out, n_in]: rows are K, N contiguous
     if (!make_map(&mw, W, n_out, n_in, 64, BK, dt, pitch_w)) return FDP_ERR_LAUNCH;
     args.idesc = make_idesc(dt, false, true, ctas);
     CUtensorMap mp = mg;
     if (!plan_last_round(args, ctas, make_idesc(dt, false, true, ctas, BN / 2), n_out, 1, park, &mp)) return FDP_ERR_LAUNCH;
-    return gemm_fixup(ctas == 2 ? launch<false, true, EPI_STORE, 2>(mg, mw, mp, mw, mo, args, s)
-                                : launch<false, true, EPI_STORE, 1>(mg, mw, mp, mw, mo, args, s), args, ctas, s);
+    return gemm_fixup(chained ? plain_launch<false, true, EPI_CHAIN_STORE>(mg, mw, mp, mw, mo, ctas, args, s) : plain_launch<false, true, EPI_STORE>(mg, mw, mp, mw, mo, ctas, args, s), args, ctas, s);
   }
   // W [n_in, n_out]: K contiguous; a CTA of a pair loads half of the 256 B rows
   CUtensorMap mh;
@@ -2117,14 +2130,13 @@ int tc_dgrad(const void* G, const void* W, void* dX, int* dev_status, int rows, 
   args.idesc = make_idesc(dt, false, false, ctas);
   CUtensorMap mp = mg;
   if (!plan_last_round(args, ctas, make_idesc(dt, false, false, ctas, BN / 2), n_out, 1, park, &mp)) return FDP_ERR_LAUNCH;
-  return gemm_fixup(ctas == 2 ? launch<false, false, EPI_STORE, 2>(mg, mw, mp, mh, mo, args, s)
-                              : launch<false, false, EPI_STORE, 1>(mg, mw, mp, mh, mo, args, s), args, ctas, s);
+  return gemm_fixup(chained ? plain_launch<false, false, EPI_CHAIN_STORE>(mg, mw, mp, mh, mo, ctas, args, s) : plain_launch<false, false, EPI_STORE>(mg, mw, mp, mh, mo, ctas, args, s), args, ctas, s);
 }
 
 // forward: A = X [rows, n_in] K-major; B = W, K-major for [n_out, n_in] (Linear), MN-major for
 // [n_in, n_out] (Conv1D); bias added in the epilogue
 int tc_fwd(const void* X, const void* W, const void* bias, void* Y, int* dev_status, int rows, int n_in,
-           int n_out, int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park, int pitch_x, int pitch_w) {
+           int n_out, int dt, int out_dt, int w_layout, cudaStream_t s, const GemmPark& park, int pitch_x, int pitch_w, bool chained) {
   CUtensorMap mx, mw, mo;
   const int ctas = ctas_per_tile();
   TcArgs args{};
@@ -2140,21 +2152,20 @@ int tc_fwd(const void* X, const void* W, const void* bias, void* Y, int* dev_sta
   args.n_fastest = 1;  // X is streamed once, W stays in L2
   args.out = Y; args.out_dt = out_dt; args.scale = 1.0f; args.nk = NoiseKey{};
   args.bias = bias; args.bias_dt = dt; args.bias_vec = aligned16(bias);
+  args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = 1;
   if (w_layout == FDP_OUT_IN) {  // W [n_out, n_in]: K contiguous
     CUtensorMap mh;
     if (!make_map(&mw, W, n_out, n_in, BK, BN / ctas, dt, pitch_w) || !make_map(&mh, W, n_out, n_in, BK, BN / 2 / ctas, dt, pitch_w)) return FDP_ERR_LAUNCH;
     args.idesc = make_idesc(dt, false, false, ctas);
     CUtensorMap mp = mx;
     if (!plan_last_round(args, ctas, make_idesc(dt, false, false, ctas, BN / 2), n_in, 1, park, &mp)) return FDP_ERR_LAUNCH;
-    return gemm_fixup(ctas == 2 ? launch<false, false, EPI_STORE, 2>(mx, mw, mp, mh, mo, args, s)
-                                : launch<false, false, EPI_STORE, 1>(mx, mw, mp, mh, mo, args, s), args, ctas, s);
+    return gemm_fixup(chained ? plain_launch<false, false, EPI_CHAIN_STORE>(mx, mw, mp, mh, mo, ctas, args, s) : plain_launch<false, false, EPI_STORE>(mx, mw, mp, mh, mo, ctas, args, s), args, ctas, s);
   }
   if (!make_map(&mw, W, n_in, n_out, 64, BK, dt, pitch_w)) return FDP_ERR_LAUNCH;  // W [n_in, n_out]: N contiguous
   args.idesc = make_idesc(dt, false, true, ctas);
   CUtensorMap mp = mx;
   if (!plan_last_round(args, ctas, make_idesc(dt, false, true, ctas, BN / 2), n_in, 1, park, &mp)) return FDP_ERR_LAUNCH;
-  return gemm_fixup(ctas == 2 ? launch<false, true, EPI_STORE, 2>(mx, mw, mp, mw, mo, args, s)
-                              : launch<false, true, EPI_STORE, 1>(mx, mw, mp, mw, mo, args, s), args, ctas, s);
+  return gemm_fixup(chained ? plain_launch<false, true, EPI_CHAIN_STORE>(mx, mw, mp, mw, mo, ctas, args, s) : plain_launch<false, true, EPI_STORE>(mx, mw, mp, mw, mo, ctas, args, s), args, ctas, s);
 }
 
 // ---- fp32 products on the tensor cores: Y[rows, N] = A[rows, K] * W (+ bias) --------------------------

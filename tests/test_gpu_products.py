@@ -203,6 +203,27 @@ def test_16bit_products_of_any_width(ops, rows, K, N, dtype, layout):  # noqa: F
                       G.double().abs() @ w.double().abs().t(), N / 16 + 8, UNIT[out_dtype])
 
 
+@pytest.mark.parametrize("rows,K,N", [(130, 64, 65), (300, 999, 130), (256, 4001, 72), (128, 3648, 100)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("layout", ["out_in", "in_out"])
+def test_fp32_outputs_of_16bit_products_of_any_width(ops, rows, K, N, dtype, layout):  # noqa: F811
+    """In fp32 these are no further from float64 than the FMA kernels that computed them before: an accumulator takes four
+    truncated steps (4 units of 2^-23 at most, of what it holds), its K / 64 contents are added with rounding to nearest, whose
+    errors of at most 2^-24 of the sum are independent.  With terms of one sign no cancellation hides a drift."""
+    X, W = _randn(rows, K, seed=1, dtype=dtype).abs(), _randn(*((N, K) if layout == "out_in" else (K, N)), seed=2, dtype=dtype).abs()
+    G, b = _randn(rows, N, seed=3, dtype=dtype).abs(), _randn(N, seed=4, dtype=dtype).abs()
+    w = (W if layout == "in_out" else W.t()).double()
+
+    def check(got, want, k):
+        assert float((got.double() - want).norm() / want.norm()) < 4 * 2.0 ** -23 + (k / 64 + 1) ** 0.5 * 2.0 ** -24
+    f32 = torch.float32
+    check(ops.linear_forward(X, W, b, layout, out_dtype=f32), X.double() @ w + b.double(), K)
+    check(ops.linear_forward(X, W, None, layout, out_dtype=f32), X.double() @ w, K)
+    check(ops.linear_input_grad(G, W, layout, out_dtype=f32), G.double() @ w.t(), N)
+    wide = _randn(rows, K, seed=5, dtype=dtype).abs()        # the long contraction of an input gradient
+    check(ops.linear_input_grad(wide, W, "in_out" if layout == "out_in" else "out_in", out_dtype=f32), wide.double() @ w, K)
+
+
 # few short samples of wide layers in the product form, every type; and noise drawn by the fix-up kernel
 @pytest.mark.parametrize("B,T,n_in,n_out,dtype", [(3, 44, 1024, 512, torch.bfloat16), (2, 2, 2000, 136, torch.float16), (8, 63, 256, 768, torch.bfloat16),
                                                   (3, 44, 512, 260, torch.float32), (2, 3, 1200, 123, torch.float32), (40, 20, 300, 300, torch.float32)])
