@@ -303,7 +303,8 @@ static int wgrad_run(const void* G, const void* X, void* dW, float* norms_out, f
   }
   if (w.tc.keep) {
     prof_mark(3, s);
-    if ((st = tc_weighted_sum(static_cast<const float*>(w.tc_extra), fs, dW, B, n_in, n_out, out_dtype, layout, inv_div, nk, s)) != FDP_OK)
+    if ((st = tc_weighted_sum(static_cast<const float*>(w.tc_extra), fs, dW, B, n_in, n_out, out_dtype, layout, inv_div, nk, s,
+                              w.tc.planes == 3)) != FDP_OK)
       return st;
   } else if (w.tc.ok) {
     float* split_ws = static_cast<float*>(w.tc_extra);

@@ -170,7 +170,7 @@ bool tc_fused_factors_ok(int B);
 int tc_keep_partials(int n_in, int n_out, int layout);    // norm partials per sample
 bool tc_keep_fused_factors_ok(int B, int nparts);
 int tc_weighted_sum(const float* keep, const TcFactorSource& fs, void* dW, int B, int n_in, int n_out, int out_dt, int layout,
-                    float inv_div, NoiseKey nk, cudaStream_t s);
+                    float inv_div, NoiseKey nk, cudaStream_t s, bool wide);
 // dW = inv_div * sum_b c_b G_b^T X_b + noise over K = B*T.  fs == nullptr: Gs is the pre-scaled copy;
 // otherwise Gs is G itself and c_b is applied per sample in the epilogue.  planes > 1: G and X are split.
 int tc_clipped_wgrad(const void* Gs, const void* X, const TcFactorSource* fs, float* split_ws,

@@ -51,15 +51,14 @@ constexpr int MAX_SMS = 148;           // workers the split-K parking area is si
 // EPI_SPLIT_*: fp32 inputs as bf16 halves, three products per K stage (see TcArgs::plane_a): the clipped sum,
 // a plain product (+ bias), and one sample's product tile squared and summed.
 // EPI_SPLIT6_*: the same with bf16 thirds and six products.
-// EPI_KEEP: one sample's product tile squared and summed, and kept in HBM for weighted_sum_kernel (the SPLIT_SUMSQ
-// ones keep it too when TcArgs::keep is set).
-// EPI_CHAIN_SUMSQ: the same for 16-bit operands whose norms came from FMA kernels before: an accumulator runs for one K
-// stage only, as with split operands (one for all of a sample's stages drifts: 768 rows 6.8e-7, 4000 3.8e-6).
+// The SUMSQ ones of CTA pairs also keep the tile in HBM for weighted_sum_kernel when TcArgs::keep is set.
+// EPI_CHAIN_SUMSQ: one sample's product tile squared and summed for 16-bit operands, in short chains: norms that came from FMA
+// kernels before (an accumulator runs for one K stage only; one for all of a sample's stages drifts: 768 rows 6.8e-7, 4000 3.8e-6)
+// and products that are kept (kept_chain).
 // EPI_CHAIN_STORE: a plain 16-bit product with an fp32 output that FMA kernels computed before, in the same chains.
 enum { EPI_STORE = 0, EPI_SUMSQ = 1, EPI_GRAM = 2, EPI_STORE_SCALED = 3, EPI_SPLIT_SCALED = 4, EPI_SPLIT_STORE = 5,
-       EPI_SPLIT_SUMSQ = 6, EPI_SPLIT6_SCALED = 7, EPI_SPLIT6_SUMSQ = 8, EPI_KEEP = 9, EPI_SPLIT6_STORE = 10, EPI_CHAIN_SUMSQ = 11,
-       EPI_CHAIN_STORE = 12 };
-__host__ __device__ constexpr bool epi_chained(int epi) { return epi >= EPI_STORE_SCALED && epi != EPI_KEEP; }
+       EPI_SPLIT_SUMSQ = 6, EPI_SPLIT6_SCALED = 7, EPI_SPLIT6_SUMSQ = 8, EPI_SPLIT6_STORE = 9, EPI_CHAIN_SUMSQ = 10, EPI_CHAIN_STORE = 11 };
+__host__ __device__ constexpr bool epi_chained(int epi) { return epi >= EPI_STORE_SCALED; }
 // bf16 parts of an operand
 __host__ __device__ constexpr int epi_planes(int epi) {
   return epi == EPI_SPLIT6_SCALED || epi == EPI_SPLIT6_SUMSQ || epi == EPI_SPLIT6_STORE ? 3 : epi == EPI_SPLIT_SCALED || epi == EPI_SPLIT_STORE || epi == EPI_SPLIT_SUMSQ ? 2 : 1;
@@ -70,7 +69,7 @@ __host__ __device__ constexpr bool epi_sumsq(int epi) { return epi == EPI_SPLIT_
 __host__ __device__ constexpr bool epi_plain(int epi) { return epi == EPI_STORE || epi == EPI_SPLIT_STORE || epi == EPI_SPLIT6_STORE || epi == EPI_CHAIN_STORE; }
 __host__ __device__ constexpr bool epi_stores(int epi) { return epi_plain(epi) || epi_scaled(epi); }
 // eight epilogue warps (two per TMEM lane quarter, 128 columns each) for the store epilogues, four for the norms
-__host__ __device__ constexpr int epi_warps_for(int epi) { return (epi == EPI_STORE || epi == EPI_KEEP || epi_chained(epi)) ? 8 : 4; }
+__host__ __device__ constexpr int epi_warps_for(int epi) { return (epi == EPI_STORE || epi_chained(epi)) ? 8 : 4; }
 constexpr int threads_for(int epi) { return 64 + 32 * epi_warps_for(epi); }
 constexpr int smem_for(int epi) {
   return epi_scaled(epi) ? SMEM_BYTES_SCALED : epi_stores(epi) ? SMEM_BYTES_STORE : SMEM_BYTES;
@@ -135,7 +134,8 @@ struct TcArgs {
   int m_group;
   // the output cannot be written by the copy engine (row pitch or base not a multiple of 16 bytes)
   int direct_out;
-  float* keep;          // EPI_KEEP, EPI_*_SUMSQ (may be null there): the product tiles, [tile][CTA of the pair][box]
+  int flush_stages;     // with `keep`: a sample's sum goes to the kept tile every so many K stages (0: at its end), keep_add32
+  float* keep;          // chained EPI_*_SUMSQ (may be null): the product tiles, [tile][CTA of the pair][box]
 };
 
 // ---- PTX wrappers (mbarrier helpers live in fdp_async.cuh) --------------------------------------------
@@ -332,6 +332,22 @@ __device__ __forceinline__ void keep_f32x32(float* dst, const float v[32], int l
 #pragma unroll
   for (int j = 0; j < 8; ++j)
     reinterpret_cast<float4*>(dst)[j * 32 + lane] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+}
+// A long sample's sum in two levels: what has been summed since the last time goes to the kept tile, or is added to what this
+// lane left there, and the registers start again.
+__device__ __forceinline__ void keep_add32(float* dst, float v[32], int lane, bool first, bool last) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    float4* q = reinterpret_cast<float4*>(dst) + j * 32 + lane;
+    if (!first) {
+      const float4 x = *q;
+      v[4 * j] += x.x; v[4 * j + 1] += x.y; v[4 * j + 2] += x.z; v[4 * j + 3] += x.w;
+    }
+    if (!last) {
+      *q = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+      v[4 * j] = 0.f; v[4 * j + 1] = 0.f; v[4 * j + 2] = 0.f; v[4 * j + 3] = 0.f;
+    }
+  }
 }
 // chunk c4 (32 columns) of a warp's 128 columns, in the output type; 16-bit types fill a box with two chunks
 __device__ __forceinline__ void store_out32(const TcArgs& args, uint32_t box, const CUtensorMap* map, const float v[32], int c4,
@@ -837,6 +853,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         int ng = 0, noise_due = 0;
         int sample = ks0 / args.seg_stages, sample_left = (sample + 1) * args.seg_stages - ks0;
         int sub_off = (args.seg_stages - sample_left) % args.sub_stages;
+        const int nb = n0 + chalf * 128;
+        int flush_left = args.flush_stages;      // (0 never comes down to 0)
+        bool flushed = false;
         for (int ks = ks0, sub = 0; ks < ks1 && ok; ++it) {
           const int acc = it % NUM_ACC;
           const uint32_t acc_phase = (it / NUM_ACC) & 1u;
@@ -871,6 +890,17 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
             for (int j = 0; j < 32; ++j) accr[c4 * 32 + j] = fmaf(cbs, __uint_as_float(r[j]), accr[c4 * 32 + j]);
           }
+          if constexpr (epi_planes(EPI) == 3 && epi_sumsq(EPI)) {
+            if (sub == 0 && --flush_left == 0 && ks < ks1) {
+              flush_left = args.flush_stages;
+              if (m0 + quarter * 32 < args.M) {
+#pragma unroll
+                for (int c4 = 0; c4 < 4; ++c4)
+                  if (nb + c4 * 32 < args.N) keep_add32(kept_box(tile, c4), accr + c4 * 32, lane, !flushed, false);
+              }
+              flushed = true;
+            }
+          }
           if (epi_scaled(EPI) && pre_noise) {
             for (noise_due += 32; noise_due >= nseg; noise_due -= nseg, ++ng) {
               float z[4];
@@ -884,7 +914,13 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           // the unit is one sample's product tile: its squares, without the rows and columns past the
           // matrix (with split operands a tile that overhangs reads the other half's columns, not zeros)
           float part = 0.f;
-          const int nb = n0 + chalf * 128;
+          if constexpr (epi_planes(EPI) == 3) {
+            if (flushed && m0 + quarter * 32 < args.M) {
+#pragma unroll
+              for (int c4 = 0; c4 < 4; ++c4)
+                if (nb + c4 * 32 < args.N) keep_add32(kept_box(tile, c4), accr + c4 * 32, lane, false, true);
+            }
+          }
           if (m < args.M) {
 #pragma unroll
             for (int i = 0; i < 128; ++i) {
@@ -925,7 +961,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       tc_fence_after();
       const uint32_t tbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + (EPI == EPI_GRAM ? 0 : acc * BN);
       float part = 0.f;
-      if constexpr (EPI == EPI_STORE || EPI == EPI_KEEP) {
+      if constexpr (EPI == EPI_STORE) {
         // this warp's 128 columns into registers, then the accumulator goes back to the MMA warp at once
         const int col0 = (ew >> 2) * warp_cols;
         float v[128];
@@ -942,22 +978,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           else mbar_arrive_cluster(mapa_u32(tempty_bar(acc), 0));
         }
         ++it;
-        if constexpr (EPI == EPI_KEEP) {
-          // (rows and columns outside the matrix were zero-filled by the loads)
-          float sq[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-          for (int i = 0; i < 128; ++i) sq[i & 3] = fmaf(v[i], v[i], sq[i & 3]);
-          part = warp_sum((sq[0] + sq[1]) + (sq[2] + sq[3]));
-          if (lane == 0) args.partials[(static_cast<size_t>(tile) * CTAS + cta_rank) * EPI_WARPS + ew] = part;
-          if (m0 + quarter * 32 < args.M) {
-#pragma unroll
-            for (int c4 = 0; c4 < 4; ++c4) {
-              const int n = n0 + col0 + c4 * 32;
-              if (n < args.N) keep_f32x32(kept_box(tile, c4), v + c4 * 32, lane);
-            }
-          }
-          continue;
-        }
         if (slot >= 0) {   // K-split unit: park the raw accumulator for the fix-up kernel
 #pragma unroll
           for (int c4 = 0; c4 < 4; ++c4)
@@ -1097,7 +1117,10 @@ __global__ void __launch_bounds__(256) splitk_fixup_kernel(const float* __restri
 // HBM-bound: B fp32 tiles read once, one written.  A block takes one 32 x 32 box of every sample as an epilogue warp
 // left it (keep_f32x32): four adjacent elements a thread, eight samples' loads under way, and the sum goes through
 // shared memory so that rows are written in whole.  Eight samples are summed
-// among themselves and then added to the rest, so the chain of the sum is an eighth of B.
+// among themselves and then added to the rest, so the chain of the sum is an eighth of B.  WIDE, for six products: the sum
+// runs in 64 bits, a chain in fp32 adds as much to the error of such a gradient as its products have, with the next eight samples' loads
+// under way (16 samples, 768 x 3072: 24.8 us in fp32, 27.9 so; 100 samples, 128 x 200: 33 / 26).
+template <bool WIDE>
 __global__ void __launch_bounds__(256) weighted_sum_kernel(const float* __restrict__ P, const TcFactorSource fs, int B, int ctas,
                                                            int tiles_m, size_t sample_stride, int M, int N,
                                                            void* __restrict__ out, int out_dt, int vec_out, float scale, NoiseKey nk) {
@@ -1131,20 +1154,52 @@ __global__ void __launch_bounds__(256) weighted_sum_kernel(const float* __restri
   const float4* p = reinterpret_cast<const float4*>(P) + static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x;
   const size_t stride = sample_stride / 4;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto add = [&](float4& a, float c, const float4& v) {
-    a.x = fmaf(c, v.x, a.x); a.y = fmaf(c, v.y, a.y); a.z = fmaf(c, v.z, a.z); a.w = fmaf(c, v.w, a.w);
-  };
   constexpr int U = 8;
   int b = 0;
-  for (; b + U <= B; b += U, p += U * stride) {
-    float4 v[U], t = make_float4(0.f, 0.f, 0.f, 0.f);
+  if constexpr (WIDE) {
+    double sum[4] = {0.0, 0.0, 0.0, 0.0};
+    auto add = [&](float f, const float4& v) {
+      const double c = static_cast<double>(f) * scale;
+      sum[0] = fma(c, static_cast<double>(v.x), sum[0]); sum[1] = fma(c, static_cast<double>(v.y), sum[1]);
+      sum[2] = fma(c, static_cast<double>(v.z), sum[2]); sum[3] = fma(c, static_cast<double>(v.w), sum[3]);
+    };
+    float4 v[U], w[U];
+    auto fetch = [&](float4 (&to)[U]) {
 #pragma unroll
-    for (int k = 0; k < U; ++k) v[k] = __ldcs(p + k * stride);
+      for (int k = 0; k < U; ++k) to[k] = __ldcs(p + k * stride);
+      p += U * stride;
+    };
+    auto take = [&](const float4 (&from)[U]) {
 #pragma unroll
-    for (int k = 0; k < U; ++k) add(t, factors[b + k] * scale, v[k]);
-    acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
+      for (int k = 0; k < U; ++k) add(factors[b + k], from[k]);
+      b += U;
+    };
+    // (the next samples' loads are under way while these are summed)
+    const int groups = B / U;
+    if (groups > 0) fetch(v);
+    for (int g = 0; g < groups; g += 2) {
+      if (g + 1 < groups) fetch(w);
+      take(v);
+      if (g + 1 >= groups) break;
+      if (g + 2 < groups) fetch(v);
+      take(w);
+    }
+    for (; b < B; ++b, p += stride) add(factors[b], __ldcs(p));
+    acc = make_float4(static_cast<float>(sum[0]), static_cast<float>(sum[1]), static_cast<float>(sum[2]), static_cast<float>(sum[3]));
+  } else {
+    auto add = [&](float4& a, float c, const float4& v) {
+      a.x = fmaf(c, v.x, a.x); a.y = fmaf(c, v.y, a.y); a.z = fmaf(c, v.z, a.z); a.w = fmaf(c, v.w, a.w);
+    };
+    for (; b + U <= B; b += U, p += U * stride) {
+      float4 v[U], t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < U; ++k) v[k] = __ldcs(p + k * stride);
+#pragma unroll
+      for (int k = 0; k < U; ++k) add(t, factors[b + k] * scale, v[k]);
+      acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
+    }
+    for (; b < B; ++b, p += stride) add(acc, factors[b] * scale, __ldcs(p));
   }
-  for (; b < B; ++b, p += stride) add(acc, factors[b] * scale, __ldcs(p));
   box[threadIdx.x >> 5][threadIdx.x & 31] = acc;
   __syncthreads();
   acc = box[threadIdx.x & 7][threadIdx.x >> 3];
@@ -1622,6 +1677,15 @@ static int chain_stages(int seg_stages, int planes) {
   return cap < seg_stages ? cap : seg_stages;
 }
 
+// ... and for 16-bit products that are kept: 8 stages, 32 truncated steps.  16 x 1024 rows, 1024 -> 3072, weight gradient with one
+// accumulator a sample 122 us, in chains of 8 / 4 / 2 stages 125 / 131 / 138; 1 x 4096, 1024 -> 1024, clipping off, error of dW
+// 4.4e-6 with one, 4.8e-7 with 8 stages, and 1.0e-6 when it was contracted twice and cut along K.
+static int kept_chain(int seg_stages, bool pad) {
+  static const int cap = [] { const char* e = getenv("FDP_TC_KEPT_STAGES"); const int v = e ? atoi(e) : 8; return v < 1 ? 1 : v; }();
+  const int n = pad ? 1 : cap;
+  return n < seg_stages ? n : seg_stages;
+}
+
 // fp32 shapes of FDP_FP32_TENSOR's three products: whole 64-column and 64-row K stages, at least 128 of everything
 static bool three_products_ok(int T, int n_in, int n_out) {
   return n_in % BK == 0 && n_out % BK == 0 && n_in >= 128 && n_out >= 128 && T % BK == 0 && T >= 2 * BK;
@@ -1649,6 +1713,16 @@ static int most_product_tiles(int n_in, int n_out) {
 static int product_partials(int n_in, int n_out) {
   const int ctas = ctas_per_tile();
   return ceil_div(n_out, BM * ctas) * ceil_div(n_in, BN) * ctas * epi_warps_for(EPI_STORE_SCALED);
+}
+// K stages of a sample over which six products that are kept are summed at once (two additions a stage): half of what a part
+// of the contraction would sum that they take the place of (one a stage).  Error of dW against float64, contracted twice / summed
+// at once / so: 9 x 2432 rows, 360 -> 835 1.5e-7 / 1.7e-7 / 1.3e-7; 8 x 3264, 128 -> 136 1.4e-7 / 1.9e-7 / 1.3e-7; 2 x 936,
+// 448 -> 1368 9.2e-8 / 1.25e-7 / 9.9e-8.  A visit to the kept tile takes 2 to 3 us: never for less than four stages (8 x 3264 102 us, now
+// 109; 5 x 704, 1344 -> 64 35 / 41; contracted twice 173 and 53).
+static int part_stages(int B, int stages, int n_in, int n_out, int products);
+static int kept_flush(int B, int stages, int n_in, int n_out) {
+  const int n = part_stages(B, stages, n_in, n_out, 6) / 2;
+  return n < 4 ? 4 : n;
 }
 static size_t keep_bytes(int B, int n_in, int n_out) {
   return static_cast<size_t>(B) * most_product_tiles(n_in, n_out) * ctas_per_tile() * BM * BN * sizeof(float);
@@ -1704,6 +1778,10 @@ double fma_sum_us(long long rows, int n_in, int n_out) {
 }
 }  // namespace
 
+// K stages in a part of the clipped sum's contraction
+static int part_stages(int B, int stages, int n_in, int n_out, int products) {
+  return B * stages / plan_tail_split(most_product_tiles(n_in, n_out), B * stages, PLAN_PAIRS, products);
+}
 // Whether keeping the per-sample products beats the plan `p` that contracts twice.  They part where B n_in n_out fp32
 // elements written and read cost what a norm pass costs: 8 x 1024 rows 1024 -> 3072 bf16 70 us kept, 82 contracted twice;
 // 12 x 500, 1024 -> 4096 94 / 80; 16 x 512, 4096 -> 4096 539 / 331; fp32 (three products) 8 x 1024, 1024 -> 3072 182 / 270.
@@ -1712,10 +1790,13 @@ static bool keep_wins(int B, int T, int n_in, int n_out, const TcPlan& p) {
   // 16-bit samples of few rows leave faster than they can be written (64 x 128 rows, 1024 -> 1024: 101 us kept, 47; 48 x 64,
   // 768 -> 3072: 160 / 53); only calls of a few launches gain there (5 x 92, 512 -> 512: 12.6 / 18.6), which the host bounds.
   if (p.planes == 1 && !p.pad && T < 256) return false;
-  // Six products are to be no further from float64 than before: a K split cuts the chain of a long sample's sum, which
-  // keeping does not (one sample of 2816 rows 1.8e-7 against 0.9e-7 in four parts).
+  // No precision is given up for it.  Contracted twice, a tile that is cut along K holds its sums in as many accumulators;
+  // kept, a sample's sum is one: its chain of truncating additions (kept_chain) may not be longer than what a part sums.  (Six
+  // products: kept_flush.)  And the Gram form of the norms has chains of n_in and n_out (bf16 norms from float64, Gram / one
+  // accumulator a sample: 2 x 1024 rows, 256 -> 256 3.9e-7 / 8.5e-7; 1 x 2560, 3624 -> 1288 6.2e-6 / 2.3e-6).
   const int stages = ceil_div(T, BK);
-  if (p.planes == 3 && stages > 16 && B < plan_tail_split(most_product_tiles(n_in, n_out), B * stages, PLAN_PAIRS, 6)) return false;
+  if (p.planes == 1 && p.scaled_epilogue && kept_chain(stages, p.pad) > part_stages(B, stages, n_in, n_out, 1)) return false;
+  if (p.algo == FDP_NORM_GRAM && BK * kept_chain(stages, p.pad) > n_in + n_out) return false;
   // (fp32 calls hold the parts of both operands already: a tenth has to be gained for more)
   return keep_us(B, T, n_in, n_out, p.planes) < (p.planes > 1 ? 0.9 : 0.97) * (norm_us(B, T, n_in, n_out, p.planes, p.algo) +
                                                                              sum_us(B, T, n_in, n_out, p.planes, p.scaled_epilogue));
@@ -1725,7 +1806,7 @@ static bool keep_wins(int B, int T, int n_in, int n_out, const TcPlan& p) {
 // is short of memory gives way where it did before.
 static void plan_keep(TcPlan& p, int B, int n_in, int n_out) {
   p.ok = true; p.keep = true; p.short_seq = false; p.scaled_epilogue = false; p.algo = FDP_NORM_DIRECT;
-  p.nparts = most_product_tiles(n_in, n_out) * ctas_per_tile() * epi_warps_for(EPI_KEEP);
+  p.nparts = most_product_tiles(n_in, n_out) * ctas_per_tile() * epi_warps_for(EPI_CHAIN_SUMSQ);
   p.split_bytes = keep_bytes(B, n_in, n_out);
   if (p.planes > 1 && p.split_bytes < split_ws_bytes()) p.split_bytes = split_ws_bytes();
   p.ws_bytes = p.split_bytes + p.split_g_bytes + p.split_x_bytes + p.pad_g_bytes + p.pad_x_bytes;
@@ -1902,8 +1983,8 @@ int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int
   TcArgs args{};
   args.batch = B; args.batch_rows = T; args.partials = partials; args.status = dev_status; args.T = T;
   args.zero_status = 1;      // the norm pass is the first launch of a weight-gradient call
-  if (pl.planes > 1 || pl.pad) {
-    // fp32 inputs (and 16-bit ones that come as padded copies): the per-sample products G_b^T X_b themselves, on the tiles and CTA pairs of the
+  if (pl.planes > 1 || pl.pad || keep != nullptr) {
+    // fp32 inputs, 16-bit ones that come as padded copies, and products that are kept: the per-sample products G_b^T X_b themselves, on the tiles and CTA pairs of the
     // clipped-sum GEMM, handed to the epilogue every few K stages and summed there in registers; a
     // unit is (sample, tile) and ends with the sum of its squares instead of a store
     const int po = pl.pad ? n_out : pitch8(n_out), pi = pl.pad ? n_in : pitch8(n_in);
@@ -1918,11 +1999,12 @@ int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int
     args.k_stages = ceil_div(T, BK);
     args.plane_a = oi ? po : pi; args.plane_b = oi ? pi : po;
     args.idesc = make_idesc(dt, true, true, ctas);
-    args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = pl.pad ? 1 : chain_stages(args.seg_stages, pl.planes);
+    args.segs = 1; args.seg_stages = args.k_stages; args.sub_stages = pl.planes > 1 ? chain_stages(args.seg_stages, pl.planes) : kept_chain(args.seg_stages, pl.pad);
     args.scale = 1.0f; args.nk = NoiseKey{};
-    if (!pl.pad) { args.zero_status = 0; args.dependent = 1; }     // follows the split kernel, which has cleared the status word
+    if (pl.planes > 1) { args.zero_status = 0; args.dependent = 1; }     // follows the split kernel, which has cleared the status word
     args.keep = keep;
-    if (pl.pad)
+    if (pl.planes == 3 && keep != nullptr) args.flush_stages = kept_flush(B, args.k_stages, n_in, n_out);
+    if (pl.planes == 1)
       return ctas == 2 ? launch<true, true, EPI_CHAIN_SUMSQ, 2>(a, b, a, b, a, args, s)
                        : launch<true, true, EPI_CHAIN_SUMSQ, 1>(a, b, a, b, a, args, s);
     if (pl.planes == 3)
@@ -1930,20 +2012,6 @@ int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int
                        : launch<true, true, EPI_SPLIT6_SUMSQ, 1>(a, b, a, b, a, args, s);
     return ctas == 2 ? launch<true, true, EPI_SPLIT_SUMSQ, 2>(a, b, a, b, a, args, s)
                      : launch<true, true, EPI_SPLIT_SUMSQ, 1>(a, b, a, b, a, args, s);
-  }
-  if (keep != nullptr) {
-    const bool oi = layout == FDP_OUT_IN;
-    const int ctas = ctas_per_tile();
-    args.M = oi ? n_out : n_in; args.N = oi ? n_in : n_out;
-    if (!make_rows_map(oi ? &a : &b, G, B, T, n_out, dt, pitch_g) || !make_rows_map(oi ? &b : &a, X, B, T, n_in, dt, pitch_x))
-      return FDP_ERR_LAUNCH;
-    args.keep = keep;
-    args.tiles_m = ceil_div(args.M, BM * ctas); args.tiles_n = ceil_div(args.N, BN);
-    args.tiles_per_batch = args.tiles_m * args.tiles_n;
-    args.k_stages = ceil_div(T, BK); args.seg_stages = args.k_stages;
-    args.idesc = make_idesc(dt, true, true, ctas);
-    return ctas == 2 ? launch<true, true, EPI_KEEP, 2>(a, b, a, b, a, args, s)
-                     : launch<true, true, EPI_KEEP, 1>(a, b, a, b, a, args, s);
   }
   if (pl.algo == FDP_NORM_DIRECT) {
     if (!make_rows_map(&a, G, B, T, n_out, dt, pitch_g) || !make_rows_map(&b, X, B, T, n_in, dt, pitch_x)) return FDP_ERR_LAUNCH;
@@ -1982,15 +2050,15 @@ int tc_prescale(const void* G, const float* factors, void* Gs, int B, int T, int
 
 static int product_tiles(int M, int N) { return ceil_div(M, BM * ctas_per_tile()) * ceil_div(N, BN); }
 int tc_keep_partials(int n_in, int n_out, int layout) {
-  return product_tiles(layout == FDP_OUT_IN ? n_out : n_in, layout == FDP_OUT_IN ? n_in : n_out) * ctas_per_tile() * epi_warps_for(EPI_KEEP);
+  return product_tiles(layout == FDP_OUT_IN ? n_out : n_in, layout == FDP_OUT_IN ? n_in : n_out) * ctas_per_tile() * epi_warps_for(EPI_CHAIN_SUMSQ);
 }
 bool tc_keep_fused_factors_ok(int B, int nparts) { return B <= KEEP_SMEM_FACTORS && B * nparts <= 2048; }
 int tc_weighted_sum(const float* keep, const TcFactorSource& fs, void* dW, int B, int n_in, int n_out, int out_dt, int layout,
-                    float inv_div, NoiseKey nk, cudaStream_t s) {
+                    float inv_div, NoiseKey nk, cudaStream_t s, bool wide) {
   const int M = layout == FDP_OUT_IN ? n_out : n_in, N = layout == FDP_OUT_IN ? n_in : n_out;
   const int ctas = ctas_per_tile(), tiles = product_tiles(M, N);
   const int vec_out = N % 4 == 0 && reinterpret_cast<uintptr_t>(dW) % (4 * dtype_size(out_dt)) == 0;
-  launch_dependent(weighted_sum_kernel, dim3(tiles * ctas * 32), dim3(256), 0, s, keep, fs, B, ctas, ceil_div(M, BM * ctas),
+  launch_dependent(wide ? weighted_sum_kernel<true> : weighted_sum_kernel<false>, dim3(tiles * ctas * 32), dim3(256), 0, s, keep, fs, B, ctas, ceil_div(M, BM * ctas),
                    static_cast<size_t>(tiles) * ctas * BM * BN, M, N, dW, out_dt, vec_out, inv_div, nk);
   note_launch();
   return FDP_OK;

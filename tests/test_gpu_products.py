@@ -47,6 +47,35 @@ def test_kept_products(ops, B, T, n_in, n_out, dtype, layout):  # noqa: F811
         assert float(((factors.double() - f) / f).abs().max()) < (T / 16 + 12) * 2.0 ** -23 + dropped
 
 
+@pytest.mark.parametrize("B,T,n_in,n_out", [(1, 4096, 1024, 1024), (2, 8192, 256, 256), (4, 4096, 264, 512), (1, 4000, 130, 520)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_long_samples_do_not_drift(ops, B, T, n_in, n_out, dtype):  # noqa: F811
+    """An accumulator takes 32 truncated steps at most, each of which loses a unit of 2^-23 of what it holds at most, whatever the
+    plan; what it holds is added with rounding.  Terms of one sign, clipping off: nothing hides a drift."""
+    X, G = _randn(B, T, n_in, seed=1, dtype=dtype).abs(), _randn(B, T, n_out, seed=2, dtype=dtype, scale=1e-2).abs()
+    per = torch.einsum("bto,bti->boi", G.double(), X.double())
+    want, n = per.sum(0) / B, per.flatten(1).norm(dim=1)
+    dW, norms, _ = ops.dp_linear_weight_grad(X, G, 1e9, 1.0, out_dtype=torch.float32, return_norms=True)
+    bound = 32 * 2.0 ** -23 + (B * T / 512 + 8) ** 0.5 * 2.0 ** -24
+    assert float((dW.double() - want).norm() / want.norm()) < bound
+    if _kept(lambda: ops.dp_linear_weight_grad(X, G, 1.0, 1.0)):
+        assert float(((norms.double() - n) / n).abs().max()) < bound
+
+
+@pytest.mark.parametrize("B,T,n_in,n_out", [(4, 2387, 72, 1024), (8, 3264, 128, 136), (5, 1984, 70, 1648)])
+def test_long_samples_in_six_products_are_summed_in_two_levels(ops, B, T, n_in, n_out):  # noqa: F811
+    """Registers sum two hand-offs a stage over at most max(4, half a part) stages and the kept tile sums what they leave: the
+    rounding errors (2^-24 / sqrt(3) of the running sum each, independent) of a chain of n are sqrt(n / 2) of one, and the
+    truncation of the hand-offs is a unit of 2^-24."""
+    X, G = _randn(B, T, n_in, seed=1, dtype=torch.float32), _randn(B, T, n_out, seed=2, dtype=torch.float32, scale=1e-2)
+    assert _kept(lambda: ops.dp_linear_weight_grad(X, G, 1e9, 1.0))
+    want = torch.einsum("bto,bti->oi", G.double(), X.double()) / B
+    stages, parts = (T + 63) // 64, min(16, 2 * 74 // (-(-n_in // 256) * -(-n_out // 256)))
+    F = max(4, B * stages // parts // 2 + 1)
+    dW = ops.dp_linear_weight_grad(X, G, 1e9, 1.0)
+    assert float((dW.double() - want).norm() / want.norm()) < (((2 * F + stages / F + 1) / 2 / 3) ** 0.5 + 1) * 2.0 ** -24
+
+
 def test_kept_products_noise_and_infinities(ops):  # noqa: F811
     """A zero gradient returns the noise stream of the direct form bit for bit, with rows of any pitch; a sample that is
     not finite has norm inf and factor 0 and leaves the others' elements alone."""
