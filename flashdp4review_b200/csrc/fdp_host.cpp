@@ -349,16 +349,18 @@ void check_status(int st, const char* what) {
   py::gil_scoped_acquire gil;
   python([&] { py_calls->check(st, what); });
 }
-int dtype_code(const Tensor& t) {
-  switch (t.scalar_type()) {
+bool has_code(at::ScalarType t) { return t == at::kFloat || t == at::kBFloat16 || t == at::kHalf; }
+int dtype_code(at::ScalarType t) {
+  switch (t) {
     case at::kFloat: return FDP_F32;
     case at::kBFloat16: return FDP_BF16;
     case at::kHalf: return FDP_F16;
     default: break;
   }
   py::gil_scoped_acquire gil;
-  return python([&] { return py_calls->dtype(t).cast<int>(); });     // raises
+  return python([&] { return py_calls->dtype(at::empty({0}, at::TensorOptions().dtype(t))).cast<int>(); });     // raises
 }
+int dtype_code(const Tensor& t) { return dtype_code(t.scalar_type()); }
 Tensor aligned(const Tensor& t) {
   return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone(at::MemoryFormat::Contiguous);
 }
@@ -386,8 +388,7 @@ at::ScalarType autocast_type(const Tensor& input, const Tensor& weight) {
   return at::autocast::get_autocast_dtype(at::kCUDA);
 }
 bool product_ok(const Tensor& a, int64_t rows, int64_t K, int64_t N) {
-  const auto t = a.scalar_type();
-  if (t != at::kFloat && t != at::kBFloat16 && t != at::kHalf) return false;
+  if (!has_code(a.scalar_type())) return false;
   return python([&] { return py_calls->product(dtype_code(a), rows, K, N).cast<bool>(); });
 }
 
@@ -432,7 +433,8 @@ struct DpLinear : torch::autograd::Function<DpLinear> {
       x3 = x.reshape({x.size(0), -1, x.size(-1)}); g3 = g3.reshape({x.size(0), -1, g3.size(-1)});
     }
     const int64_t B = x3.size(0), K = w.size(in_out ? 1 : 0), N = w.size(in_out ? 0 : 1);
-    const int t = dtype_code(g3);
+    // (a type the kernels do not know is refused only where they are asked: an input gradient alone is torch's then)
+    const int t = has_code(g3.scalar_type()) ? dtype_code(g3) : -1;
     bool native_dx = false;
     OptTensor target;
     fdp_dp_params p{}, pb{};
@@ -440,8 +442,9 @@ struct DpLinear : torch::autograd::Function<DpLinear> {
     {
       py::gil_scoped_acquire gil;
       python([&] {
-        const py::tuple c = py_calls->linear(held(ctx->saved_data["layer"]), weight, B, t, K > 0 ? g3.numel() / K : 0, K, N, need_dx, need_dw);
+        const py::tuple c = py_calls->linear(held(ctx->saved_data["layer"]), weight, B, t, K > 0 ? g3.numel() / K : 0, K, N, need_dx, need_dw, need_db);
         native_dx = c[0].cast<bool>();
+        if (c.size() == 1) return;
         p = params(c[1]); pb = params(c[2]);
         algo = c[3].cast<int>();
         if (!c[4].is_none()) target = c[4].cast<Tensor>();
@@ -455,6 +458,7 @@ struct DpLinear : torch::autograd::Function<DpLinear> {
     Tensor dW, db;
     if (native_dx || need_dw || need_db) {
       if (x3.dim() != 3 || g3.dim() != 3 || x3.size(0) != g3.size(0) || x3.size(1) != g3.size(1)) refuse("expected (B,T,in) and (B,T,out)", g3);
+      dtype_code(g3);
       Tensor G = g3.contiguous();
       if (native_dx || need_dw) G = aligned(G);
       OptTensor X, W;
@@ -463,8 +467,8 @@ struct DpLinear : torch::autograd::Function<DpLinear> {
       if (target.has_value() && (target->sizes() != weight.sizes() || !target->is_contiguous() || target->device() != G.device()))
         refuse("out must be a contiguous tensor of the weight's shape on its device", *target);
       const auto input_type = static_cast<at::ScalarType>(ctx->saved_data["dtype"].toInt());
-      const int dx_dt = input_type == at::kFloat ? FDP_F32 : input_type == at::kBFloat16 ? FDP_BF16 : FDP_F16;
-      const Bwd r = linear_bwd_call(G, X, W, target, static_cast<int>(x3.size(-1)), t, dx_dt, need_dw ? dtype_code(target.has_value() ? *target : weight) : t,
+      const int dx_dt = dtype_code(input_type);
+      const Bwd r = linear_bwd_call(G, X, W, target, static_cast<int>(x3.size(-1)), t, dx_dt, dtype_code(target.has_value() ? *target : weight),
                                     need_db ? dtype_code(bias) : t, in_out ? FDP_IN_OUT : FDP_OUT_IN, algo, p, pb, native_dx, need_dw, need_db);
       check_status(r.st, "fdp_linear_bwd");
       if (native_dx) dX = *r.dX;

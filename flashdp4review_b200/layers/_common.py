@@ -100,11 +100,14 @@ def _product(code, rows, K, N):
     return ops.library_product_ok(_CODES[code], rows, K, N)
 
 
-def _linear_call(layer, weight, B, code, rows, K, N, need_dx, need_dw):
-    """One backward of a Linear / Conv1D layer: whether the input gradient is the library's, the parameters of the
-    weight's and of the bias's gradient, the flags of the call, and the bucket slice the weight gradient goes to."""
+def _linear_call(layer, weight, B, code, rows, K, N, need_dx, need_dw, need_db):
+    """One backward of a Linear / Conv1D layer: whether the input gradient is the library's and, if the call is for
+    anything of the library's, the parameters of the weight's and of the bias's gradient, the flags of the call, and the
+    bucket slice the weight gradient goes to.  `code` is -1 for a dtype that the kernels do not know."""
     step = layer._next_step()
-    native_dx = need_dx and ops.library_product_ok(_CODES[code], rows, K, N)
+    native_dx = need_dx and code >= 0 and ops.library_product_ok(_CODES[code], rows, K, N)
+    if not (native_dx or need_dw or need_db):
+        return (False,)                  # (an empty batch of a frozen layer, for one, has no noise to form)
     w_id, b_id = layer._dp_param_ids
     div, noise = dp_scalars(B, layer.noise_multiplier, w_id, step)
     p = ops._params(layer.C, layer.clamp_value, div, noise)

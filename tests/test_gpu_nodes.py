@@ -124,3 +124,32 @@ def test_nodes_write_into_gradient_buckets(functions):
     assert m.weight.grad is None and len(done) == 1 and done[0] is m.weight
     m(x).sum().backward()
     assert torch.equal(slot, m.weight.grad)
+
+
+@pytest.mark.parametrize("kind", ["linear", "conv1d"])
+def test_nodes_take_and_refuse_what_the_functions_do(functions, kind):
+    """A frozen layer in a dtype of torch's alone returns its input gradient; a float64 input under autocast is refused in
+    backward, not answered in fp16; a frozen layer takes an empty batch, for which no noise could be formed.  The same
+    through the Function classes."""
+    for on in (False, True):
+        functions(on)
+        m = _layer(kind, 128, 192, torch.float64)
+        for p in m.parameters():
+            p.requires_grad_(False)
+        x = torch.randn(4, 64, 128, device=dev(), dtype=torch.float64, requires_grad=True)
+        m(x).sum().backward()
+        w = m.weight if kind == "linear" else m.weight.t()
+        assert torch.allclose(x.grad, w.sum(0).expand_as(x))
+        for width in (192, 33):              # a product of the library's, one of torch's
+            m = _layer(kind, 128, width, torch.float32)
+            y = None
+            with torch.autocast("cuda", dtype=torch.bfloat16):
+                y = m(x)
+            with pytest.raises(KeyError):
+                y.float().sum().backward()
+        m = _layer(kind, 128, 192, torch.float32)
+        for p in m.parameters():
+            p.requires_grad_(False)
+        e = torch.zeros(0, 64, 128, device=dev(), requires_grad=True)
+        m(e).sum().backward()
+        assert e.grad.shape == e.shape and m._dp_step == 1
