@@ -389,6 +389,7 @@ at::ScalarType autocast_type(const Tensor& input, const Tensor& weight) {
 }
 bool product_ok(const Tensor& a, int64_t rows, int64_t K, int64_t N) {
   if (!has_code(a.scalar_type())) return false;
+  py::gil_scoped_acquire gil;
   return python([&] { return py_calls->product(dtype_code(a), rows, K, N).cast<bool>(); });
 }
 
@@ -513,11 +514,21 @@ struct DpLayerNorm : torch::autograd::Function<DpLayerNorm> {
   }
 };
 
+// (the forward runs without the interpreter's lock, as the operator calls do: allocations and launches of one thread do not
+// hold up the others)
 Tensor dp_linear(const Tensor& input, const Tensor& weight, const OptTensor& bias, const py::object& layer, bool in_out, int64_t code) {
-  return boundary([&] { return DpLinear::apply(input, weight, bias, hold(layer), in_out, code); });
+  const c10::IValue held_layer = hold(layer);
+  return boundary([&] {
+    py::gil_scoped_release nogil;
+    return DpLinear::apply(input, weight, bias, held_layer, in_out, code);
+  });
 }
 Tensor dp_layernorm(const Tensor& input, const Tensor& weight, const Tensor& bias, const py::object& layer, double eps) {
-  return boundary([&] { return DpLayerNorm::apply(input, weight, bias, hold(layer), eps); });
+  const c10::IValue held_layer = hold(layer);
+  return boundary([&] {
+    py::gil_scoped_release nogil;
+    return DpLayerNorm::apply(input, weight, bias, held_layer, eps);
+  });
 }
 
 }  // namespace

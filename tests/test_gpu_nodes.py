@@ -153,3 +153,45 @@ def test_nodes_take_and_refuse_what_the_functions_do(functions, kind):
         e = torch.zeros(0, 64, 128, device=dev(), requires_grad=True)
         m(e).sum().backward()
         assert e.grad.shape == e.shape and m._dp_step == 1
+
+
+def test_a_forward_leaves_the_interpreter_to_other_threads(tmp_path):
+    """While one thread is in the library (here an entry point that only sleeps and reports an error) another goes on."""
+    import ctypes
+    import shutil
+    import subprocess
+    import threading
+    import time
+    from flashdp4review_b200 import _lib
+    if shutil.which("gcc") is None:
+        pytest.skip("no C compiler")
+    src = tmp_path / "slow.c"
+    src.write_text("#include <unistd.h>\nint slow(void) { usleep(400000); return -1; }\n")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(tmp_path / "slow.so"), str(src)], check=True)
+    slow = ctypes.cast(ctypes.CDLL(str(tmp_path / "slow.so")).slow, ctypes.c_void_p).value
+    lib, host = _lib.load(), _lib.host()
+    real = {n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in _lib.SIGNATURES}
+    x = torch.randn(4, 64, 128, device=dev())
+    for kind, entry in (("linear", "fdp_linear_fwd"), ("layernorm", "fdp_layernorm_fwd")):
+        m = _layer(kind, 128, 192 if kind == "linear" else 128, torch.float32)
+        m(x)
+        gaps, stop = [0.0], threading.Event()
+
+        def tick():
+            last = time.perf_counter()
+            while not stop.is_set():
+                time.sleep(0.002)
+                now = time.perf_counter()
+                gaps.append(now - last)
+                last = now
+        t = threading.Thread(target=tick)
+        host.bind({**real, entry: slow})
+        try:
+            t.start()
+            with pytest.raises(ValueError):
+                m(x)
+        finally:
+            stop.set()
+            t.join()
+            host.bind(real)
+        assert max(gaps) < 0.3, (kind, max(gaps))
