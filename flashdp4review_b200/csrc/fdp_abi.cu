@@ -475,10 +475,15 @@ static int gemm_split_call(int parts, const void* A, const void* W, const void* 
   // W is [K, N] (w_kn) or [N, K]: either way its rows are split along their own columns
   const SplitJob jobs[2] = {{A, a3, static_cast<size_t>(rows), K, nullptr, 1},
                             {W, w3, static_cast<size_t>(w_kn ? K : N), w_kn ? N : K, nullptr, 1}};
-  const int st = tc_split(jobs, 2, parts, status, s);
-  if (st != FDP_OK) return st;
-  return parts == 2 ? tc_gemm3(a3, w3, bias, Y, status, rows, K, N, out_dtype, w_kn, s, park)
-                    : tc_gemm6(a3, w3, bias, Y, status, rows, K, N, out_dtype, w_kn, s, park);
+  if (parts == 2) {
+    const int st = tc_split(jobs, 2, parts, status, s);
+    return st != FDP_OK ? st : tc_gemm3(a3, w3, bias, Y, status, rows, K, N, out_dtype, w_kn, s, park);
+  }
+  Maxima m[2];
+  int st = tc_split(jobs, 2, parts, status, s, reinterpret_cast<unsigned*>(w3 - SPLIT_MAXIMA_BYTES), m);
+  if (st == FDP_OK) st = tc_gemm6(a3, w3, bias, Y, status, rows, K, N, out_dtype, w_kn, s, park);
+  if (st == FDP_OK) simt_redo(A, W, bias, Y, rows, K, N, out_dtype, w_kn, m[0], m[1], s);
+  return st;
 }
 
 int fdp_linear_dgrad(const void* G, const void* W, void* dX, int rows, int n_in, int n_out,
@@ -569,6 +574,7 @@ struct LinearBwdWs {
   WgradWs w;
   bool shared;
   int dx_parts;       // parts that the input gradient's product takes
+  unsigned* maxima;   // of G and of X and W, for an input gradient in six products
   char* w_parts;      // split copy of W
   GstatsPlan pl;
   float* factors; float* sq_part; float* colsum_part;
@@ -598,6 +604,7 @@ LinearBwdWs linear_bwd_ws(void* base, int B, int T, int n_in, int n_out, int dty
   Carver c(base);
   c.off = q.w.bytes;
   q.w_parts = c.take<char>(!dx ? 0 : q.dx_parts == 3 ? tc_gemm6_w_bytes(n_out, n_in) : tc_gemm3_w_bytes(n_out, n_in, q.w.tc.planes));
+  if (dx && q.dx_parts == 3) q.maxima = c.take<unsigned>(2 * SPLIT_MAXIMA_BYTES / sizeof(unsigned));
   q.pl = gstats_plan(B, T, n_out, dtype);
   q.factors = c.take<float>(B);
   q.sq_part = c.take<float>(static_cast<size_t>(B) * q.pl.row_chunks * q.pl.col_chunks);
@@ -645,14 +652,23 @@ int fdp_linear_bwd(const void* G, const void* X, const void* W, void* dX, void* 
     const bool w_kn = layout == FDP_OUT_IN;      // W's rows are the contraction of dX = G W
     const SplitJob jw{W, q.w_parts, static_cast<size_t>(w_kn ? n_out : n_in), w_kn ? n_in : n_out, nullptr, 1};
     const bool stats = db != nullptr && tc_split_stats_ok(G, n_out);
-    if (stats) {
-      if ((st = tc_split_stats(G, sg, q.colsum_part, q.sq_part, B, T, n_out, planes, q.pl, s)) != FDP_OK) return st;
-    } else {
-      if (db != nullptr) gstats(G, q.colsum_part, q.sq_part, B, T, n_out, in_dtype, q.pl, s);
-      if ((st = tc_split(&jg, 1, planes, nullptr, s)) != FDP_OK) return st;
-    }
     const SplitJob jobs[2] = {jx, jw};
-    if ((st = tc_split(jobs, dX != nullptr ? 2 : 1, planes, q.w.status, s)) != FDP_OK) return st;
+    unsigned* const most_x = q.maxima;           // X's and W's, then G's
+    unsigned* const most_g = q.maxima != nullptr ? q.maxima + SPLIT_MAXIMA_BYTES / sizeof(unsigned) : nullptr;
+    Maxima mg{}, mxw[2] = {};
+    auto split_g = [&] {
+      if (stats) {
+        // (the word beside the status word, which the split of X and W has cleared)
+        unsigned* const word = most_g != nullptr ? reinterpret_cast<unsigned*>(q.w.status) + 1 : nullptr;
+        mg = Maxima{word, 1};
+        return tc_split_stats(G, sg, q.colsum_part, q.sq_part, B, T, n_out, planes, q.pl, s, word);
+      }
+      if (db != nullptr) gstats(G, q.colsum_part, q.sq_part, B, T, n_out, in_dtype, q.pl, s);
+      return tc_split(&jg, 1, planes, nullptr, s, most_g, &mg);
+    };
+    if (q.maxima == nullptr && (st = split_g()) != FDP_OK) return st;
+    if ((st = tc_split(jobs, dX != nullptr ? 2 : 1, planes, q.w.status, s, most_x, mxw)) != FDP_OK) return st;
+    if (q.maxima != nullptr && (st = split_g()) != FDP_OK) return st;
     if ((st = wgrad_run(G, X, dW, nullptr, nullptr, B, T, n_in, n_out, in_dtype, dw_dtype, layout, norm_algo, p, q.w, true, s)) != FDP_OK)
       return st;
     if (dX != nullptr) {
@@ -661,6 +677,7 @@ int fdp_linear_bwd(const void* G, const void* X, const void* W, void* dX, void* 
       st = q.dx_parts == 3 ? tc_gemm6(sg, q.w_parts, nullptr, dX, q.w.status, rows, n_out, n_in, dx_dtype, w_kn, s, park)
                            : tc_gemm3(sg, q.w_parts, nullptr, dX, q.w.status, rows, n_out, n_in, dx_dtype, w_kn, s, park, planes);
       if (st != FDP_OK) return st;
+      if (q.dx_parts == 3) simt_redo(G, W, nullptr, dX, rows, n_out, n_in, dx_dtype, w_kn, mg, mxw[1], s);
     }
     if (db != nullptr) {
       const int div = p_bias->batch_divisor > 0 ? p_bias->batch_divisor : B;

@@ -74,6 +74,13 @@ void simt_dgrad(const void* G, const void* W, void* dX, int rows, int n_in, int 
 // Y[rows,n_out] = X[rows,n_in] * W^T (+ bias); W [n_out,n_in] if w_layout==FDP_OUT_IN else [n_in,n_out]
 void simt_fwd(const void* X, const void* W, const void* bias, void* Y, int rows, int n_in, int n_out, int dt,
               int out_dt, int w_layout, cudaStream_t s);
+// Largest magnitudes of an operand's parts, as bits.
+struct Maxima { const unsigned* words; int n; };
+// A product of split fp32 operands, Y[rows, N] = A[rows, K] * W (+ bias) with W [K, N] if w_kn, else [N, K], once more where an
+// operand's parts cannot stand for it: an infinity (its parts are inf and NaN), a magnitude that bf16 rounds to one, nothing
+// above 2^-100 (the parts run into bf16's smallest numbers).  Otherwise it returns at once.  Follows the product in the stream.
+void simt_redo(const void* A, const void* W, const void* bias, void* Y, int rows, int K, int N, int out_dt, bool w_kn,
+               const Maxima& a, const Maxima& w, cudaStream_t s);
 
 // ---- bias gradient (HBM-bound; G read once) ----------------------------------------------------
 struct GstatsPlan { int vec, cols_per_block, col_chunks, rows_per_chunk, row_chunks; };
@@ -94,7 +101,7 @@ void bias_clip_finalize(const float* colsum_part, const float* sq_part, int npar
 // tc_split of G [B * T, n_out] and gstats in one pass (fp32, plan of gstats_plan)
 bool tc_split_stats_ok(const void* G, int n_out);
 int tc_split_stats(const void* G, void* dst, float* colsum_part, float* sq_part, int B, int T, int n_out, int planes,
-                   const GstatsPlan& pl, cudaStream_t s);
+                   const GstatsPlan& pl, cudaStream_t s, unsigned* maximum = nullptr);
 
 // ---- LayerNorm -----------------------------------------------------------------------------------
 struct LnPlan { int tpr, cpt, cw, rows_per_block, chunks; bool vec; };
@@ -146,7 +153,10 @@ TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo);
 // fp32 [rows, n] -> bf16 [rows, planes, n rounded up to 8]: high parts, then what is left of them, ...; row r is
 // multiplied by factors[r / T] first (factors may be null).  One or two operands; clears *zero_status if not null
 struct SplitJob { const void* src; void* dst; size_t rows; int n; const float* factors; int T; };
-int tc_split(const SplitJob* jobs, int njobs, int planes, int* zero_status, cudaStream_t s);
+// (`zero_status`: two words are cleared).  With planes 3 and `maxima` (SPLIT_MAXIMA_BYTES) the blocks leave their operands'
+// largest magnitudes there, and of_job[k] says which are job k's.
+constexpr size_t SPLIT_MAXIMA_BYTES = 38 * 256;
+int tc_split(const SplitJob* jobs, int njobs, int planes, int* zero_status, cudaStream_t s, unsigned* maxima = nullptr, Maxima* of_job = nullptr);
 // With pl.planes > 1, G and X are the split matrices and dt is FDP_BF16.
 int tc_norms(const void* G, const void* X, float* partials, int* dev_status, int B, int T, int n_in,
              int n_out, int dt, const TcPlan& pl, cudaStream_t s, float* keep = nullptr, int layout = FDP_OUT_IN,

@@ -38,6 +38,7 @@ constexpr int MAX_SMEM_FACTORS = 384;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + BAR_BYTES;
 constexpr int SMEM_BYTES_STORE = SMEM_BYTES + 8 * BOX_BYTES;
 constexpr int SMEM_BYTES_SCALED = SMEM_BYTES_STORE + MAX_SMEM_FACTORS * 4;
+static_assert(SPLIT_MAXIMA_BYTES % 256 == 0 && SPLIT_MAXIMA_BYTES >= (148 * 16 + 2) * sizeof(unsigned), "a word for every block of tc_split");
 static_assert(SMEM_BYTES_SCALED <= 227 * 1024, "shared memory of one CTA");
 constexpr int TMEM_COLS = 512;
 // Per-sample products kept in a call's workspace.  Beyond that there is nothing to gain: 4 x 2048 rows, 4096 -> 11008 bf16,
@@ -1259,10 +1260,21 @@ struct SplitRun {
   unsigned nvec, vec_per_row;
   int n, T, vec;       // vec: n a multiple of 4, src 16-byte aligned
 };
-template <int PLANES>
-__global__ void __launch_bounds__(256) split_kernel(const SplitRun j0, const SplitRun j1, unsigned first, int* zero_status) {
+// MAXIMA: every block also leaves the largest magnitude that it has seen (as bits) in maxima[blockIdx.x], for simt_redo.
+__device__ __forceinline__ unsigned magnitude(float f) { return __float_as_uint(f) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned block_max(unsigned v, unsigned* smem8) {      // 256 threads; valid in thread 0
+  v = __reduce_max_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0) smem8[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int i = 1; i < 8; ++i) v = max(v, smem8[i]);
+  return v;
+}
+template <int PLANES, bool MAXIMA>
+__global__ void __launch_bounds__(256) split_kernel(const SplitRun j0, const SplitRun j1, unsigned first, int* zero_status, unsigned* maxima) {
   pdl_trigger();       // the product that follows sets itself up meanwhile
-  if (zero_status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *zero_status = 0;
+  if (zero_status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) { zero_status[0] = 0; zero_status[1] = 0; }   // (and split_stats_kernel's maximum)
+  unsigned most = 0;
   const bool second = blockIdx.x >= first;
   const SplitRun& j = second ? j1 : j0;
   const unsigned block = second ? blockIdx.x - first : blockIdx.x, blocks = second ? gridDim.x - first : first;
@@ -1277,6 +1289,10 @@ __global__ void __launch_bounds__(256) split_kernel(const SplitRun j0, const Spl
     } else {
 #pragma unroll
       for (int e = 0; e < 8; ++e) f[e] = c0 + e < j.n ? __ldg(p + e) : 0.f;
+    }
+    if (MAXIMA) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) most = max(most, magnitude(f[e]));
     }
     if (j.factors != nullptr) {
       const float c = __ldg(j.factors + row / j.T);
@@ -1293,6 +1309,11 @@ __global__ void __launch_bounds__(256) split_kernel(const SplitRun j0, const Spl
 #pragma unroll
       for (int e = 0; e < 8; ++e) f[e] -= hf[e];
     }
+  }
+  if (MAXIMA) {
+    __shared__ unsigned red[8];
+    most = block_max(most, red);
+    if (threadIdx.x == 0) maxima[blockIdx.x] = most;
   }
 }
 
@@ -1328,11 +1349,14 @@ __global__ void __launch_bounds__(256) pad_kernel(const SplitRun j0, const Split
 // ---- the split of G, with the bias gradient's statistics taken from the pass (grid and partials of gstats_kernel) ---
 // In a whole backward G is split once for both products, and the column sums and sums of squares cost no read of
 // their own: 8192 x 3072 fp32, G 33 + 33 + 23 us (two splits and the statistics) as separate passes, one pass here.
-template <int PLANES>
+// MAXIMA: the largest magnitude goes to *maximum, which an earlier launch has cleared.
+template <int PLANES, bool MAXIMA>
 __global__ void __launch_bounds__(256, 4) split_stats_kernel(const float* __restrict__ G, uint2* __restrict__ dst,
                                                              float* __restrict__ colsum_part, float* __restrict__ sq_part,
                                                              int T, int n_out, int pitch, int rows_per_chunk,
-                                                             int col_chunks, int row_chunks) {
+                                                             int col_chunks, int row_chunks, unsigned* maximum) {
+  pdl_trigger();
+  unsigned most = 0;
   __shared__ float cs[8][32 * 4];
   __shared__ float red[32];
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
@@ -1346,7 +1370,10 @@ __global__ void __launch_bounds__(256, 4) split_stats_kernel(const float* __rest
     auto take = [&](int r, const float4& v) {
       float f[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) { acc[e] += f[e]; sq = fmaf(f[e], f[e], sq); }
+      for (int e = 0; e < 4; ++e) {
+        acc[e] += f[e]; sq = fmaf(f[e], f[e], sq);
+        if (MAXIMA) most = max(most, magnitude(f[e]));
+      }
       uint2* o = dst + ((static_cast<size_t>(b) * T + r) * PLANES * pitch + c0) / 4;
 #pragma unroll
       for (int pl = 0; pl < PLANES; ++pl) {
@@ -1379,6 +1406,11 @@ __global__ void __launch_bounds__(256, 4) split_stats_kernel(const float* __rest
       for (int yy = 0; yy < 8; ++yy) t += cs[yy][c];
       colsum_part[(static_cast<size_t>(b) * row_chunks + rc) * n_out + col] = t;
     }
+  }
+  if (MAXIMA) {
+    __shared__ unsigned mred[8];
+    most = block_max(most, mred);
+    if (threadIdx.x == 0 && most > *static_cast<volatile unsigned*>(maximum)) atomicMax(maximum, most);
   }
 }
 
@@ -1927,7 +1959,7 @@ TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
   return p;
 }
 
-int tc_split(const SplitJob* jobs, int njobs, int planes, int* zero_status, cudaStream_t s) {
+int tc_split(const SplitJob* jobs, int njobs, int planes, int* zero_status, cudaStream_t s, unsigned* maxima, Maxima* of_job) {
   SplitRun r[2] = {};
   unsigned blocks[2] = {0, 0};
   // 32-bit index arithmetic within a launch: an operand past that is cut along its rows
@@ -1951,15 +1983,18 @@ int tc_split(const SplitJob* jobs, int njobs, int planes, int* zero_status, cuda
     }
     if (blocks[0] + blocks[1] == 0) break;
     // 16 blocks an SM in all, shared in proportion to the work
-    const unsigned cap = static_cast<unsigned>(sm_count()) * 16;
+    const unsigned cap = static_cast<unsigned>(sm_count() < MAX_SMS ? sm_count() : MAX_SMS) * 16;
     const unsigned long long all = static_cast<unsigned long long>(blocks[0]) + blocks[1];
     if (all > cap) {
       for (int k = 0; k < 2; ++k)
         if (blocks[k] > 0) blocks[k] = static_cast<unsigned>(blocks[k] * static_cast<unsigned long long>(cap) / all) + 1;
     }
     if (planes == 0) pad_kernel<<<blocks[0] + blocks[1], 256, 0, s>>>(r[0], r[1], blocks[0], zero_status);
-    else if (planes == 2) split_kernel<2><<<blocks[0] + blocks[1], 256, 0, s>>>(r[0], r[1], blocks[0], zero_status);
-    else split_kernel<3><<<blocks[0] + blocks[1], 256, 0, s>>>(r[0], r[1], blocks[0], zero_status);
+    else if (planes == 2) split_kernel<2, false><<<blocks[0] + blocks[1], 256, 0, s>>>(r[0], r[1], blocks[0], zero_status, nullptr);
+    else if (maxima == nullptr) split_kernel<3, false><<<blocks[0] + blocks[1], 256, 0, s>>>(r[0], r[1], blocks[0], zero_status, nullptr);
+    else split_kernel<3, true><<<blocks[0] + blocks[1], 256, 0, s>>>(r[0], r[1], blocks[0], zero_status, maxima);
+    if (maxima != nullptr)       // (operands of one launch: tc_gemm6_ok)
+      for (int k = 0; k < njobs; ++k) of_job[k] = Maxima{maxima + (k == 1 ? blocks[0] : 0), static_cast<int>(blocks[k])};
     note_launch();
   }
   return cudaPeekAtLastError() == cudaSuccess ? FDP_OK : (cudaGetLastError(), FDP_ERR_LAUNCH);
@@ -1967,11 +2002,11 @@ int tc_split(const SplitJob* jobs, int njobs, int planes, int* zero_status, cuda
 
 bool tc_split_stats_ok(const void* G, int n_out) { return n_out % 4 == 0 && aligned16(G); }
 int tc_split_stats(const void* G, void* dst, float* colsum_part, float* sq_part, int B, int T, int n_out, int planes,
-                   const GstatsPlan& pl, cudaStream_t s) {
+                   const GstatsPlan& pl, cudaStream_t s, unsigned* maximum) {
   const unsigned grid = static_cast<unsigned>(static_cast<size_t>(B) * pl.row_chunks * pl.col_chunks);
-  auto kernel = planes == 2 ? split_stats_kernel<2> : split_stats_kernel<3>;
+  auto kernel = planes == 2 ? split_stats_kernel<2, false> : maximum == nullptr ? split_stats_kernel<3, false> : split_stats_kernel<3, true>;
   kernel<<<grid, 256, 0, s>>>(static_cast<const float*>(G), static_cast<uint2*>(dst), colsum_part, sq_part, T, n_out, pitch8(n_out),
-                              pl.rows_per_chunk, pl.col_chunks, pl.row_chunks);
+                              pl.rows_per_chunk, pl.col_chunks, pl.row_chunks, maximum);
   note_launch();
   return cudaPeekAtLastError() == cudaSuccess ? FDP_OK : (cudaGetLastError(), FDP_ERR_LAUNCH);
 }
@@ -2288,13 +2323,18 @@ int tc_gemm3(const void* A3, const void* W3, const void* bias, void* Y, int* dev
 // kernels and are to be no further from float64.  Against cuBLAS (bias added): 1024 rows 1000 -> 1024 21.9 / 43.1 us, error
 // 1.0e-7 / 5.7e-7; 2376 rows 1168 -> 312 27.6 / 54; 5000 rows 900 -> 900 56 / 195; 128 rows 8190 -> 8191 243 / 333; 128 rows
 // 1001 -> 4097 26 / 32; 130 rows 72 -> 100 9.6 / 6.1, which is why the Python layer asks for it from 2^26 multiply-adds on.
-bool tc_gemm6_ok(int rows, int K, int N) { return rows >= 128 && K >= 64 && N >= 64; }
+// Operands that hold an infinity, or what bf16 rounds to one, or nothing but the smallest numbers are done again (simt_redo).
+bool tc_gemm6_ok(int rows, int K, int N) {
+  constexpr size_t ONE_LAUNCH = static_cast<size_t>(1) << 34;       // elements that tc_split takes at once
+  return rows >= 128 && K >= 64 && N >= 64 && static_cast<size_t>(rows) * pitch8(K) < ONE_LAUNCH &&
+         static_cast<size_t>(K) * pitch8(N) < ONE_LAUNCH && static_cast<size_t>(N) * pitch8(K) < ONE_LAUNCH;
+}
 size_t tc_gemm6_w_bytes(int K, int N) {      // in either orientation
   const size_t a = static_cast<size_t>(K) * pitch8(N), b = static_cast<size_t>(N) * pitch8(K);
   return align256((a > b ? a : b) * 6);
 }
 size_t tc_gemm6_ws_bytes(int rows, int K, int N) {
-  return align256(static_cast<size_t>(rows) * pitch8(K) * 6) + tc_gemm6_w_bytes(K, N);
+  return align256(static_cast<size_t>(rows) * pitch8(K) * 6) + SPLIT_MAXIMA_BYTES + tc_gemm6_w_bytes(K, N);
 }
 int tc_gemm6(const void* A3, const void* W3, const void* bias, void* Y, int* dev_status, int rows, int K, int N,
              int out_dt, bool w_kn, cudaStream_t s, const GemmPark& park) {

@@ -92,7 +92,9 @@ enum fdp_norm_algo {
   /* flag, OR-ed into the dtype of fdp_linear_dgrad / fdp_linear_fwd and into fdp_linear_bwd's norm_algo (and those of
    * their workspace queries): fp32 forward and input-gradient products that FDP_FP32_TENSOR's three products do not
    * take, with at least 128 rows and 64 columns on either side, run as six bf16 products, as close to float64 as an
-   * fp32 FMA kernel.  Operands and output need no alignment.  The workspace holds 1.5 times both operands. */
+   * fp32 FMA kernel.  Where an operand holds an infinity, a NaN or a number that bf16 rounds to infinity, or nothing above
+   * 2^-100, FMA kernels do the product once more and the result is theirs.  Operands and output need no alignment.  The
+   * workspace holds 1.5 times both operands and 10 KB. */
   FDP_FP32_WIDE_GEMM = 128,
   /* flag, OR-ed into the same arguments, of any dtype: products of few output tiles and a long contraction are cut along
    * it.  The workspace then has room for the fp32 parts, at most 38.8 MB; in a smaller one the product runs uncut. */

@@ -319,3 +319,41 @@ def test_single_cta_tiles_of_any_width():
     assert r.returncode == 0, r.stderr[-2000:]
     worst = float(r.stdout.strip().split("WORST")[-1])
     assert worst < 20 * 2.0 ** -23, worst
+
+
+# fp32 operands that three bf16 parts cannot stand for: what cuBLAS's and the FMA kernels return.  Cut along K and not
+# (300 x 2000 -> 100), both layouts, every place the operand can be in
+@pytest.mark.parametrize("rows,K,N", [(130, 200, 65), (300, 2000, 100), (1000, 333, 515)])
+@pytest.mark.parametrize("layout", ["out_in", "in_out"])
+def test_fp32_products_of_numbers_that_bf16_lacks(ops, rows, K, N, layout):  # noqa: F811
+    f32, inf = torch.float32, float("inf")
+    X, b = _randn(rows, K, seed=1, dtype=f32), _randn(N, seed=3, dtype=f32)
+    W = _randn(*((N, K) if layout == "out_in" else (K, N)), seed=2, dtype=f32, scale=0.1)
+    G = _randn(rows, N, seed=4, dtype=f32)
+
+    def same(got, want64):
+        want = want64.to(f32)
+        finite = torch.isfinite(want)
+        assert torch.equal(torch.isfinite(got), finite)
+        assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(got[~finite & ~torch.isnan(want)], want[~finite & ~torch.isnan(want)])
+        assert float((got[finite].double() - want64[finite]).norm()) <= 2e-6 * float(want64[finite].norm())
+
+    def check(x, w, g):
+        wkn = (w if layout == "in_out" else w.t()).double()
+        same(ops.linear_forward(x, w, b, layout), x.double() @ wkn + b.double())
+        same(ops.linear_input_grad(g, w, layout), g.double() @ wkn.t())
+        # the whole backward (N and K a multiple of four or not: G's parts come with its statistics or alone)
+        dX, _, _ = ops.dp_linear_backward(x[: rows // 2 * 2].view(2, rows // 2, K), g[: rows // 2 * 2].view(2, rows // 2, N), w, 1.0, 1.0, layout=layout)
+        same(dX.view(-1, K), g[: rows // 2 * 2].double() @ wkn.t())
+
+    def put(t, value, *where):
+        t = t.clone()
+        t[where] = value
+        return t
+    for value in (inf, -inf, float("nan"), 3.4e38, -3.39999e38):
+        check(put(X, value, 3, 5), W, put(G, value, rows - 1, N - 1))
+        check(X, put(W, value, 1, 2), G)
+    check(put(put(X, inf, 7, 0), -inf, 7, 1), W, put(put(G, inf, 0, 0), inf, 0, 1))
+    check(X * 1e-33, W, G * 1e-33)           # everything below 2^-100
+    check(X, W * 1e-33, G)
+    check(torch.zeros_like(X), W, torch.zeros_like(G))
