@@ -1,4 +1,6 @@
 """Shared pieces of the DP layer backward passes."""
+import weakref
+
 import torch
 
 from .. import _lib, runtime
@@ -96,15 +98,54 @@ def native_nodes(input):
     return _native
 
 
+class _NodeState:
+    """What a native node holds of its layer.  Not the layer itself: Python's collector does not see through such a node,
+    and a layer that keeps an output of its own (a hook that captures activations) would be kept alive by it, with its
+    parameters and the graph.  The layer is asked as long as it lives; once it is gone, what it was at its last
+    forward holds, and all of its nodes count their steps on from there."""
+    __slots__ = ("layer", "C", "clamp_value", "noise_multiplier", "norm_algo", "_dp_param_ids", "_dp_step")
+    _next_step = DPLayerMixin._next_step
+
+    def __init__(self, layer):
+        self.layer = weakref.ref(layer)
+
+    def follow(self, layer):
+        self.C, self.clamp_value, self.noise_multiplier = layer.C, layer.clamp_value, layer.noise_multiplier
+        self._dp_param_ids, self._dp_step = layer._dp_param_ids, layer._dp_step
+        self.norm_algo = getattr(layer, "norm_algo", "auto")
+
+
+_states = weakref.WeakKeyDictionary()      # one state a living layer
+
+
+def node_state(layer):
+    """The state that the nodes of this forward hold."""
+    state = _states.get(layer)
+    if state is None:
+        state = _states.setdefault(layer, _NodeState(layer))
+    state.follow(layer)
+    return state
+
+
+def _step_of(state):
+    """The layer, or its state if it is gone, and the step of this backward."""
+    layer = state.layer()
+    if layer is None:
+        return state, state._next_step()
+    step = layer._next_step()
+    state._dp_step = layer._dp_step
+    return layer, step
+
+
 def _product(code, rows, K, N):
     return ops.library_product_ok(_CODES[code], rows, K, N)
 
 
-def _linear_call(layer, weight, B, code, rows, K, N, need_dx, need_dw, need_db):
+def _linear_call(state, weight, B, code, rows, K, N, need_dx, need_dw, need_db):
     """One backward of a Linear / Conv1D layer: whether the input gradient is the library's and, if the call is for
     anything of the library's, the parameters of the weight's and of the bias's gradient, the flags of the call, and the
     bucket slice the weight gradient goes to.  `code` is -1 for a dtype that the kernels do not know."""
-    step = layer._next_step()
+    layer, step = _step_of(state)
     native_dx = need_dx and code >= 0 and ops.library_product_ok(_CODES[code], rows, K, N)
     if not (native_dx or need_dw or need_db):
         return (False,)                  # (an empty batch of a frozen layer, for one, has no noise to form)
@@ -115,7 +156,8 @@ def _linear_call(layer, weight, B, code, rows, K, N, need_dx, need_dw, need_db):
     return native_dx, p, bias, ops.backward_algo(code, layer.norm_algo), direct_grad_target(weight) if need_dw else None
 
 
-def _layernorm_call(layer, B):
+def _layernorm_call(state, B):
+    layer, step = _step_of(state)
     g_id, b_id = layer._dp_param_ids
-    div, noise = dp_scalars(B, layer.noise_multiplier, g_id, layer._next_step(), param_id2=b_id)
+    div, noise = dp_scalars(B, layer.noise_multiplier, g_id, step, param_id2=b_id)
     return ops._params(layer.C, layer.clamp_value, div, noise)

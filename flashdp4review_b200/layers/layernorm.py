@@ -22,7 +22,7 @@ from torch.autograd.function import Function
 
 from ..core import ops
 from .utils import DPParameter as Parameter
-from ._common import DPLayerMixin, dp_scalars, native_nodes
+from ._common import DPLayerMixin, dp_scalars, native_nodes, node_state
 
 
 class _DPLayerNormFunc(Function):
@@ -89,5 +89,5 @@ class DPLayerNorm(nn.LayerNorm, DPLayerMixin):
         bias = self.bias if self.bias is not None else torch.zeros_like(self.weight)
         native = None if self.compat_fused_saturation else native_nodes(input)
         if native is not None:
-            return native.dp_layernorm(input, self.weight, bias, self, float(self.eps))
+            return native.dp_layernorm(input, self.weight, bias, node_state(self), float(self.eps))
         return _DPLayerNormFunc.apply(input, self.weight, bias, self)

@@ -15,7 +15,7 @@ from ..core import ops
 from ..core.ops import RuntimeAutoTuner
 from .utils import DPParameter as Parameter
 from ._common import (DPLayerMixin, reshape_to_3d, dp_scalars, autocast_dtype, direct_grad_target,
-                      direct_grad_done, native_nodes)
+                      direct_grad_done, native_nodes, node_state)
 
 
 class _DPLinearFunc(Function):
@@ -93,5 +93,5 @@ class DPLinear(nn.Linear, DPLayerMixin):
     def forward(self, input):
         native = native_nodes(input)
         if native is not None:
-            return native.dp_linear(input, self.weight, self.bias, self, False, ops.fp32_product_flags())
+            return native.dp_linear(input, self.weight, self.bias, node_state(self), False, ops.fp32_product_flags())
         return _DPLinearFunc.apply(input, self.weight, self.bias, self)

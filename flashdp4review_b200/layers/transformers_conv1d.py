@@ -32,7 +32,7 @@ from ..core import ops
 from ..core.ops import RuntimeAutoTuner
 from .utils import DPParameter as Parameter
 from ._common import (DPLayerMixin, reshape_to_3d, dp_scalars, autocast_dtype, direct_grad_target,
-                      direct_grad_done, native_nodes)
+                      direct_grad_done, native_nodes, node_state)
 
 
 class _DPConv1DFunc(Function):
@@ -115,5 +115,5 @@ class DPConv1D(Conv1D, DPLayerMixin):
         size_out = x.size()[:-1] + (self.nf,)
         native = None if self.compat_inplace_bias_scale else native_nodes(x)
         if native is not None:
-            return native.dp_linear(x, self.weight, self.bias, self, True, ops.fp32_product_flags()).view(size_out)
+            return native.dp_linear(x, self.weight, self.bias, node_state(self), True, ops.fp32_product_flags()).view(size_out)
         return _DPConv1DFunc.apply(self.bias, x, self.weight, self).view(size_out)

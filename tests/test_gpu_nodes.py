@@ -195,3 +195,43 @@ def test_a_forward_leaves_the_interpreter_to_other_threads(tmp_path):
             t.join()
             host.bind(real)
         assert max(gaps) < 0.3, (kind, max(gaps))
+
+
+@pytest.mark.parametrize("kind", ["linear", "conv1d", "layernorm"])
+def test_a_node_does_not_keep_its_layer_alive(kind):
+    """A layer that keeps its own output goes when the program lets go of it; a graph outlives its layer, with the
+    values and the noise that the layer would have given it."""
+    import gc
+    import weakref
+    x = torch.randn(4, 64, 128, device=dev())
+    m = _layer(kind, 128, 192 if kind != "layernorm" else 128, torch.float32)
+    m.register_forward_hook(lambda mod, i, o: setattr(mod, "act", o))
+    m(x)
+    gone = weakref.ref(m)
+    del m
+    gc.collect()
+    assert gone() is None
+
+    grads = []
+    for keep in (True, False):
+        m = _layer(kind, 128, 192 if kind != "layernorm" else 128, torch.float32)
+        m._dp_step = 4
+        params = list(m.parameters())
+        ys = [m(x), m(2.0 * x)]
+        if not keep:
+            del m
+            gc.collect()
+        for y in ys:
+            y.sum().backward()
+        grads.append([p.grad for p in params])
+        if keep:
+            assert m._dp_step == 6
+            m.C = 0.01                # read when a backward runs, as the Function classes do
+            a = torch.autograd.grad(m(x).sum(), params)
+            m._dp_step -= 1
+            m.C = 0.1
+            y = m(x)
+            m.C = 0.01
+            b = torch.autograd.grad(y.sum(), params)
+            assert all(torch.equal(s, t) for s, t in zip(a, b))
+    assert all(torch.equal(s, t) for s, t in zip(*grads))
