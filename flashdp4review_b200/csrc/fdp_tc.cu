@@ -1119,10 +1119,10 @@ __global__ void __launch_bounds__(256) splitk_fixup_kernel(const float* __restri
 // left it (keep_f32x32): four adjacent elements a thread, eight samples' loads under way, and the sum goes through
 // shared memory so that rows are written in whole.  Eight samples are summed
 // among themselves and then added to the rest, so the chain of the sum is an eighth of B.  WIDE, for six products: the sum
-// runs in 64 bits, a chain in fp32 adds as much to the error of such a gradient as its products have, with the next eight samples' loads
+// runs in 64 bits, a chain in fp32 adds as much to the error of such a gradient as its products have, with the next four samples' loads
 // under way (16 samples, 768 x 3072: 24.8 us in fp32, 27.9 so; 100 samples, 128 x 200: 33 / 26).
 template <bool WIDE>
-__global__ void __launch_bounds__(256) weighted_sum_kernel(const float* __restrict__ P, const TcFactorSource fs, int B, int ctas,
+__global__ void __launch_bounds__(256, WIDE ? 4 : 6) weighted_sum_kernel(const float* __restrict__ P, const TcFactorSource fs, int B, int ctas,
                                                            int tiles_m, size_t sample_stride, int M, int N,
                                                            void* __restrict__ out, int out_dt, int vec_out, float scale, NoiseKey nk) {
   // box -> tile, CTA of the pair, epilogue warp (lane quarter, column half), 32 columns
@@ -1155,7 +1155,7 @@ __global__ void __launch_bounds__(256) weighted_sum_kernel(const float* __restri
   const float4* p = reinterpret_cast<const float4*>(P) + static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x;
   const size_t stride = sample_stride / 4;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  constexpr int U = 8;
+  constexpr int U = WIDE ? 4 : 8;
   int b = 0;
   if constexpr (WIDE) {
     double sum[4] = {0.0, 0.0, 0.0, 0.0};
