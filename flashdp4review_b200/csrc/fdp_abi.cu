@@ -349,7 +349,14 @@ int fdp_linear_wgrad(const void* G, const void* X, void* dW, float* norms_out, f
   if (workspace_bytes < w.bytes || !aligned16(workspace)) return FDP_ERR_WORKSPACE;
   // the tensor-core path moves 16-byte vectors (TMA, vector stores); the generic kernels, and the split
   // copies of fp32 operands with six products, take any naturally aligned pointer
-  if (w.tc.ok && !w.tc.any_align && (!aligned16(G) || !aligned16(X) || !aligned16(dW))) return FDP_ERR_ALIGN;
+  if (w.tc.ok && !w.tc.any_align && (!aligned16(G) || !aligned16(X) || !aligned16(dW))) {
+    // (short 16-bit samples that only FDP_KEEP_PRODUCTS brings here: the generic kernels take them, as without the flag)
+    const int less = norm_algo & ~FDP_KEEP_PRODUCTS;
+    const WgradWs u = wgrad_ws(workspace, B, T, n_in, n_out, in_dtype, less);
+    if ((u.tc.ok && !u.tc.any_align) || workspace_bytes < u.bytes) return FDP_ERR_ALIGN;
+    w = u;
+    norm_algo = less;
+  }
 
   return wgrad_run(G, X, dW, norms_out, factors_out, B, T, n_in, n_out, in_dtype, out_dtype, layout, norm_algo, p, w, false,
                    static_cast<cudaStream_t>(stream));

@@ -85,9 +85,10 @@ enum fdp_norm_algo {
    * the 38.8 MB in which the parts of a K split are parked. */
   FDP_FP32_WIDE = 32,
   /* flag, OR-ed into the same arguments: with FDP_NORM_AUTO the tensor-core path may keep every sample's product
-   * G_b^T X_b in the workspace (fp32, B * n_in * n_out elements, at most 512 MiB) where that is expected to be faster
-   * than contracting twice: the norms come from the tiles as they leave, the clipped sum is their weighted sum.
-   * fp32 accumulation throughout, as without the flag. */
+   * G_b^T X_b in the workspace where that is expected to be faster than contracting twice: the norms come from the tiles
+   * as they leave, the clipped sum is their weighted sum.  fp32, in whole tiles of 256 x 256 elements (a product of
+   * 64 x 64 takes one), at most 512 MiB in all, and for fp32 inputs at least the 38.8 MB that their workspace holds without
+   * the flag.  No accumulator runs for longer than without it.  Alignment is asked for where it is without the flag. */
   FDP_KEEP_PRODUCTS = 64,
   /* flag, OR-ed into the dtype of fdp_linear_dgrad / fdp_linear_fwd and into fdp_linear_bwd's norm_algo (and those of
    * their workspace queries): fp32 forward and input-gradient products that FDP_FP32_TENSOR's three products do not
@@ -101,7 +102,9 @@ enum fdp_norm_algo {
   FDP_GEMM_SPLIT_K = 256,
   /* flag, OR-ed into the same arguments and into fdp_linear_wgrad's norm_algo: 16-bit inputs of widths from 64 on, of any
    * number, run on the tensor cores (without it: multiples of 8 from 128 on).  Operands whose rows are no multiple of 16
-   * bytes are copied into the workspace with padded rows; operands and outputs need no alignment. */
+   * bytes are copied into the workspace with padded rows.  Operands and outputs of the widths that the flag adds need no
+   * alignment; fdp_linear_wgrad asks for 16 bytes at the others, as it does without the flag.  fp32 outputs of
+   * fdp_linear_dgrad / fdp_linear_fwd at these widths are as close to float64 as the FMA kernels' were. */
   FDP_PAD_16BIT = 512
 };
 

@@ -357,3 +357,34 @@ def test_fp32_products_of_numbers_that_bf16_lacks(ops, rows, K, N, layout):  # n
     check(X * 1e-33, W, G * 1e-33)           # everything below 2^-100
     check(X, W * 1e-33, G)
     check(torch.zeros_like(X), W, torch.zeros_like(G))
+
+
+@pytest.mark.parametrize("B,T,n_in,n_out", [(3, 44, 256, 512), (5, 20, 1024, 128)])
+@pytest.mark.parametrize("what", ["out", "X", "G"])
+def test_short_samples_take_pointers_of_any_alignment(ops, B, T, n_in, n_out, what):  # noqa: F811
+    """Fewer than 256 rows of short samples ran on the FMA kernels, which take any pointer; where their products are kept
+    now, a pointer off 16 bytes goes where it went (a gradient slice through the operator, operands through the C interface)."""
+    import ctypes
+    from flashdp4review_b200 import _lib
+    bf = torch.bfloat16
+
+    def off(t):
+        flat = torch.empty(t.numel() + 1, device=dev(), dtype=t.dtype)
+        flat[1:] = t.flatten()
+        return flat[1:].view(t.shape)
+    X, G = _randn(B, T, n_in, seed=1, dtype=bf), _randn(B, T, n_out, seed=2, dtype=bf, scale=1e-1)
+    want, norms, _ = ops.dp_linear_weight_grad(X, G, 1.0, 1.0, out_dtype=torch.float32, return_norms=True)
+    assert _kept(lambda: ops.dp_linear_weight_grad(X, G, 1.0, 1.0))
+    if what == "out":
+        out = off(torch.zeros(n_out, n_in, device=dev()))
+        ops.dp_linear_weight_grad(X, G, 1.0, 1.0, out=out)
+    else:
+        lib, algo = _lib.load(), _lib.FDP_KEEP_PRODUCTS | _lib.FDP_PAD_16BIT
+        X, G = (off(X), G) if what == "X" else (X, off(G))
+        out = torch.zeros(n_out, n_in, device=dev())
+        ws = torch.empty(lib.fdp_linear_wgrad_workspace_bytes(B, T, n_in, n_out, _lib.FDP_BF16, algo), dtype=torch.uint8, device=dev())
+        p = _lib.DPParams(1.0, 1.0, 0.0, 0, 0, 0, 0, 0, 0, 1)
+        st = lib.fdp_linear_wgrad(G.data_ptr(), X.data_ptr(), out.data_ptr(), None, None, B, T, n_in, n_out, _lib.FDP_BF16, _lib.FDP_F32, 0,
+                                  algo, ctypes.byref(p), ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+        assert st == 0
+    assert float((out - want).norm()) < 2.0 ** -19 * float(want.norm())       # both in fp32, sums of at most 132 terms
