@@ -1769,8 +1769,10 @@ double rounds(long long units, int on) { return static_cast<double>((units + on 
 double keep_us(int B, int T, int n_in, int n_out, int planes) {
   constexpr double STAGE[3] = {0.38, 1.22, 2.9}, FIXED[3] = {1.8, 2.2, 2.2}, LEAST[3] = {3.5, 5.0, 5.0};
   const double r = ceil_div(T, BK) * STAGE[planes - 1] + FIXED[planes - 1], least = LEAST[planes - 1];
+  // (a product of few boxes keeps few SMs at the sum, sample after sample: 590 x 1 rows, 195 -> 192 bf16 105 us, blocks 86, twice 59)
+  const double hbm = 4.0 * n_in * n_out * (B + 1.0) / 6.4e6, serial = 0.11 * B - 7.0;
   return 9.5 + rounds(static_cast<long long>(B) * most_product_tiles(n_in, n_out), PLAN_PAIRS) * (r > least ? r : least) +
-         4.0 * n_in * n_out * (B + 1.0) / 6.4e6;
+         (hbm > serial ? hbm : serial);
 }
 // a norm pass over product tiles or Gram blocks
 double norm_us(int B, int T, int n_in, int n_out, int planes, int algo) {
