@@ -5,10 +5,13 @@
 //                                     its own TMEM accumulator, added times c_b into registers
 //           MN, MN, STORE, 2          same from a pre-scaled copy of G (T < 256, or mostly padded K stages)
 //   direct  MN, MN, SUMSQ, 1          per-sample ||G_b^T X_b||_F^2: tile squared in the epilogue, never stored
+//   kept    MN, MN, CHAIN_SUMSQ, 2    the same in short chains, the tile kept in the workspace for weighted_sum_kernel; 16-bit
+//                                     widths off the multiples of 8 or below 128 have their norms from it in any case
 //   gram    K,  K,  GRAM, 1           sum_{t,s} (G_b G_b^T)_{ts} (X_b X_b^T)_{ts}, two accumulators in TMEM
 //   dgrad   K,  MN or K, STORE, 2     dX = G W
 //   forward K,  K or MN, STORE, 2     Y = X W^T + bias
-//   fp32    the same products over bf16 parts of the operands: SPLIT_* three products, SPLIT6_* six
+//           CHAIN_STORE for both       16-bit operands of any width, fp32 output: in short chains
+//   fp32    the same products over bf16 parts of the operands: SPLIT_* three products, SPLIT6_* six (SUMSQ, SCALED, STORE)
 // Roles in a CTA: warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner, warps 2-5 (2-9 for the
 // store epilogues) = epilogue, each on the TMEM lane quarter warp % 4.  With two CTAs per tile the
 // even CTA of a 2-CTA cluster issues tcgen05.mma.cta_group::2 for both.  Every mbarrier wait is
@@ -41,8 +44,8 @@ constexpr int SMEM_BYTES_SCALED = SMEM_BYTES_STORE + MAX_SMEM_FACTORS * 4;
 static_assert(SPLIT_MAXIMA_BYTES % 256 == 0 && SPLIT_MAXIMA_BYTES >= (148 * 16 + 2) * sizeof(unsigned), "a word for every block of tc_split");
 static_assert(SMEM_BYTES_SCALED <= 227 * 1024, "shared memory of one CTA");
 constexpr int TMEM_COLS = 512;
-// Per-sample products kept in a call's workspace.  Beyond that there is nothing to gain: 4 x 2048 rows, 4096 -> 11008 bf16,
-// 721 MB of products, a layer's forward and backward 2148 us against 2157.
+// Per-sample products kept in a call's workspace.  Beyond that there was nothing to gain: 4 x 2048 rows, 4096 -> 11008 bf16,
+// 721 MB of products, a layer's forward and backward 2148 us against 2157 (with the GEMMs before the uniform issue).
 constexpr size_t KEEP_LIMIT = static_cast<size_t>(512) << 20;
 constexpr int KEEP_SMEM_FACTORS = 128;
 constexpr int MAX_SMS = 148;           // workers the split-K parking area is sized for
@@ -168,7 +171,8 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // Hands an accumulator back to the leader's MMA warp.  Relaxed: no memory is handed over with it, the accumulator's loads
-// have completed (tcgen05.wait::ld) and tcgen05.fence orders the rest.  A release at cluster scope waits for the warp's
+// have completed (tcgen05.wait::ld), and tcgen05.fence::before_thread_sync here and ::after_thread_sync behind the MMA warp's
+// wait order them before its MMAs, for which the PTX manual's patterns between threads use a relaxed arrive and wait too.  A release at cluster scope waits for the warp's
 // own earlier stores and took 1300 to 2500 cycles, in which the pair's tensor cores ran dry (weight gradients in six products,
 // 16 x 197 rows 768 -> 3072: 151 us, now 134; 5 x 704, 64 -> 7928: 153 / 121; one pair alone in three products, 8192 deep: 89 / 64).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
@@ -1598,7 +1602,7 @@ int ctas_per_tile() { return forced_ctas() == 1 ? 1 : 2; }
 // tiles than workers) are cut into s parts of equal K-stage count, so that the last round keeps more
 // SMs busy; cost in tile-times = ceil(rem*s/workers)/s plus the cost of parking and re-reading the
 // accumulators.  At most 2 * workers parked parts (workers <= MAX_SMS / CTAS).
-// That cost, in K stages of bf16 (0.40 us each): 6 for the fix-up launch, 0.11 per part that it reads back
+// That cost, in K stages of bf16 (0.40 us each when it was taken): 6 for the fix-up launch, 0.11 per part that it reads back
 // (256 KB), 4 for each further round.  Measured, GEMM + fix-up: 48 pair tiles of 256 stages for 74 pairs 110 us
 // unsplit, 117 in two parts, 91 in three; 16 tiles of 128 stages 54 / 37 / 30 / 26 us in one to four parts; 64 tiles
 // of 128 stages 62 us unsplit, 72 in two parts.
@@ -1712,9 +1716,9 @@ static int chain_stages(int seg_stages, int planes) {
 // ... and for 16-bit products that are kept: 8 stages, 32 truncated steps.  16 x 1024 rows, 1024 -> 3072, weight gradient with one
 // accumulator a sample 122 us, in chains of 8 / 4 / 2 stages 125 / 131 / 138; 1 x 4096, 1024 -> 1024, clipping off, error of dW
 // 4.4e-6 with one, 4.8e-7 with 8 stages, and 1.0e-6 when it was contracted twice and cut along K.
+constexpr int KEPT_CHAIN = 8;
 static int kept_chain(int seg_stages, bool pad) {
-  static const int cap = [] { const char* e = getenv("FDP_TC_KEPT_STAGES"); const int v = e ? atoi(e) : 8; return v < 1 ? 1 : v; }();
-  const int n = pad ? 1 : cap;
+  const int n = pad ? 1 : KEPT_CHAIN;
   return n < seg_stages ? n : seg_stages;
 }
 
@@ -1733,8 +1737,6 @@ static bool wide_ok(int B, int T, int n_in, int n_out, int norm_algo) {
   return T >= SHORT_SEQ || (norm_algo != FDP_NORM_DIRECT && static_cast<long long>(B) * T >= 128);
 }
 
-// The tensor-core path needs 16-bit inputs, row pitches that are multiples of 16 bytes, and
-// matrices large enough that the 128x256 tile is not mostly padding.
 // tiles of a sample's product, in the orientation that has more (the workspace query does not know the layout)
 static int most_product_tiles(int n_in, int n_out) {
   const int ctas = ctas_per_tile();
@@ -1760,7 +1762,11 @@ static size_t keep_bytes(int B, int n_in, int n_out) {
   return static_cast<size_t>(B) * most_product_tiles(n_in, n_out) * ctas_per_tile() * BM * BN * sizeof(float);
 }
 // ---- estimates in us by which weight-gradient plans are chosen -----------------------------------------------------
-// Fitted to 36 shapes, B 1 to 64, T 64 to 4096, widths 64 to 11008, every side timed (within 10 % but for the smallest).
+// Fitted to 36 shapes, B 1 to 64, T 64 to 4096, widths 64 to 11008, every side timed, when a CTA pair took 0.30 us a K stage and
+// an accumulator's return held it up (0.19 now): as times they are too high by up to a half, on all sides.  What they are for
+// was timed again with the present kernels: of 315 shapes from T = 64 on the choice between kept and contracted twice is more
+// than 5 % off at 7 (at worst 3 x 681 rows 1712 -> 5304 fp16, 77 us kept, 68 twice), of 419 shorter ones that between three plans
+// more than 8 % off at 9 (at worst 1 x 3, 128 -> 192 fp32, blocks 18 us, kept 12).
 // The SM count is a constant: the workspace query and the launch must pick the same plan.
 namespace {
 constexpr int PLAN_PAIRS = MAX_SMS / 2;
@@ -1817,8 +1823,9 @@ static int part_stages(int B, int stages, int n_in, int n_out, int products) {
   return B * stages / plan_tail_split(most_product_tiles(n_in, n_out), B * stages, PLAN_PAIRS, products);
 }
 // Whether keeping the per-sample products beats the plan `p` that contracts twice.  They part where B n_in n_out fp32
-// elements written and read cost what a norm pass costs: 8 x 1024 rows 1024 -> 3072 bf16 70 us kept, 82 contracted twice;
-// 12 x 500, 1024 -> 4096 94 / 80; 16 x 512, 4096 -> 4096 539 / 331; fp32 (three products) 8 x 1024, 1024 -> 3072 182 / 270.
+// elements written and read cost what a norm pass costs: 8 x 1024 rows 1024 -> 3072 bf16 66 us kept, 76 contracted twice,
+// 1024 -> 1024 27 / 38; fp32 (three products) 8 x 1024, 1024 -> 3072 170 / 252; 12 x 500, 1024 -> 4096 fp16 (67 us) and 16 x 512,
+// 4096 -> 4096 bf16 (238) are contracted twice.
 static bool keep_wins(int B, int T, int n_in, int n_out, const TcPlan& p) {
   if (keep_bytes(B, n_in, n_out) > KEEP_LIMIT) return false;
   // 16-bit samples of few rows leave faster than they can be written (64 x 128 rows, 1024 -> 1024: 101 us kept, 47; 48 x 64,
@@ -1865,6 +1872,8 @@ static void plan_short(TcPlan& p, int B, int T, int n_in, int n_out) {
   p.ws_bytes = p.split_bytes + p.split_g_bytes + p.split_x_bytes + p.pad_g_bytes + p.pad_x_bytes;
 }
 
+// (16-bit inputs without FDP_PAD_16BIT: row pitches that are multiples of 16 bytes, and matrices large enough that the
+// 128 x 256 tile is not mostly padding)
 TcPlan tc_plan(int B, int T, int n_in, int n_out, int dt, int norm_algo) {
   TcPlan p; p.ok = false; p.algo = FDP_NORM_DIRECT; p.ws_bytes = 0; p.nparts = 0; p.scaled_epilogue = false;
   p.short_seq = false; p.any_align = false; p.keep = false; p.split_bytes = 0;
