@@ -21,8 +21,10 @@ class DPLayerMixin:
         self._dp_step = 0
 
     def _next_step(self):
-        self._dp_step += 1
-        return runtime.noise_step(self._dp_step)
+        # (past nn.Module's __setattr__, which takes as long as the rest of a backward's bookkeeping)
+        d = self.__dict__
+        step = d["_dp_step"] = d["_dp_step"] + 1
+        return runtime.noise_step(step)
 
 
 def reshape_to_3d(input, grad_output):
@@ -104,10 +106,13 @@ class _NodeState:
     parameters and the graph.  The layer is asked as long as it lives; once it is gone, what it was at its last
     forward holds, and all of its nodes count their steps on from there."""
     __slots__ = ("layer", "C", "clamp_value", "noise_multiplier", "norm_algo", "_dp_param_ids", "_dp_step")
-    _next_step = DPLayerMixin._next_step
 
     def __init__(self, layer):
         self.layer = weakref.ref(layer)
+
+    def _next_step(self):
+        self._dp_step += 1
+        return runtime.noise_step(self._dp_step)
 
     def follow(self, layer):
         self.C, self.clamp_value, self.noise_multiplier = layer.C, layer.clamp_value, layer.noise_multiplier
